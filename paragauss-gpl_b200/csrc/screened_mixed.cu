@@ -5,8 +5,9 @@
 // N = 240..48, exact INT32 accumulation in TMEM, FP64 combination):
 //
 //   k_sm_quant_pts   phi_t -> INT8 digits, one scale per point          (A of X)
-//   k_sm_rowexp_P,   P -> packed digits P8[nu][mu] (5 bytes of a 64-bit
+//   k_sm_rowexp_P,   P -> packed digits P8[mu][nu] (5 bytes of a 64-bit
 //   k_sm_quant_P     word), one scale per row nu                       (B of X)
+//   k_sm_gather_B    per tile, the digits of P[S_t, S_t] in the MMA layout
 //   k_sm_density     X = phi_t P[S_t, S_t], 128 points x 48 slots per MMA;
 //                    A by bulk copy, B gathered from P8 by four producer
 //                    warps, two TMEM accumulator sets (MMA of slot block j+1
@@ -55,7 +56,7 @@ struct ScreenMixed {
   int64_t chunk_slots = 0, chunk_tiles = 0;
   int max_n = 0;
   int nspin = 1;
-  unsigned long long* P8[2] = {};    // [nbas][nbas] per spin
+  unsigned long long* P8[2] = {};    // [mu][nu], nbas x nbas per spin
   int* e_P[2] = {};                  // [nbas] per spin
   int8_t* tA = nullptr;              // density A digits, [slot block of 32][slice][128 x 32] per tile
   int8_t* tB = nullptr;              // density B digits, [stage][slice][48 x 32] per tile
@@ -101,18 +102,28 @@ __global__ void k_sm_rowexp_P(const double* __restrict__ P, int64_t ldc, int64_t
   if (threadIdx.x == 0) e[blockIdx.x] = scale_exp(red[0]);
 }
 
-// P8[nu][mu]: byte s = digit s of P[nu][mu] at the row scale 2^e_P[nu]
-__global__ void k_sm_quant_P(const double* __restrict__ P, int64_t ldc, int64_t nbas, const int* __restrict__ e_P,
-                             unsigned long long* __restrict__ P8) {
-  const int64_t total = nbas * nbas;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t nu = i / nbas, mu = i - nu * nbas;
+// P8[mu][nu]: byte s = digit s of P[nu][mu] at the row scale 2^e_P[nu].  Stored
+// transposed, so that the gather's lanes (consecutive rows nu of one column mu)
+// read consecutive words.  32 x 32 blocks through shared memory.
+__global__ void __launch_bounds__(256) k_sm_quant_P(const double* __restrict__ P, int64_t ldc, int64_t nbas,
+                                                    const int* __restrict__ e_P, unsigned long long* __restrict__ P8) {
+  __shared__ unsigned long long blk[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t mu0 = (int64_t)blockIdx.x * 32, nu0 = (int64_t)blockIdx.y * 32;
+  for (int r = ty; r < 32; r += 8) {
+    const int64_t nu = nu0 + r, mu = mu0 + tx;
+    if (nu >= nbas || mu >= nbas) continue;
     int8_t d[kSlices];
     digits(P[nu * ldc + mu], e_P[nu], d);
     unsigned long long w = 0;
 #pragma unroll
     for (int s = 0; s < kSlices; ++s) w |= (unsigned long long)(uint8_t)d[s] << (8 * s);
-    P8[i] = w;
+    blk[r][tx] = w;
+  }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8) {
+    const int64_t mu = mu0 + r, nu = nu0 + tx;
+    if (mu < nbas && nu < nbas) P8[mu * nbas + nu] = blk[tx][r];
   }
 }
 
@@ -150,32 +161,46 @@ __global__ void __launch_bounds__(128) k_sm_quant_pts(const int64_t* __restrict_
   }
 }
 
-// byte `sl` of each of 8 packed digit words -> one 64-bit row of 8 digits
-__device__ __forceinline__ unsigned long long gather_slice(const unsigned long long (&w)[8], int sl) {
-  uint32_t lo = 0, hi = 0;
+// The digit bytes of 16 packed words, one 16-byte run per slice: 4 x 4 byte
+// transposes of the low words, byte 0 of the high words for slice 4.
+__device__ __forceinline__ void gather_slices(const uint2 (&w)[16], uint4 (&o)[kSlices]) {
+  uint32_t r[4][kSlices];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    lo |= ((uint32_t)(w[u] >> (8 * sl)) & 0xffu) << (8 * u);
-    hi |= ((uint32_t)(w[u + 4] >> (8 * sl)) & 0xffu) << (8 * u);
+  for (int q = 0; q < 4; ++q) {
+    const uint2 *v = w + 4 * q;
+    const uint32_t b0 = __byte_perm(v[0].x, v[1].x, 0x5140), b1 = __byte_perm(v[2].x, v[3].x, 0x5140);
+    const uint32_t c0 = __byte_perm(v[0].x, v[1].x, 0x7362), c1 = __byte_perm(v[2].x, v[3].x, 0x7362);
+    r[q][0] = __byte_perm(b0, b1, 0x5410);
+    r[q][1] = __byte_perm(b0, b1, 0x7632);
+    r[q][2] = __byte_perm(c0, c1, 0x5410);
+    r[q][3] = __byte_perm(c0, c1, 0x7632);
+    r[q][4] = __byte_perm(__byte_perm(v[0].y, v[1].y, 0x0040), __byte_perm(v[2].y, v[3].y, 0x0040), 0x5410);
   }
-  return (unsigned long long)lo | ((unsigned long long)hi << 32);
+#pragma unroll
+  for (int s = 0; s < kSlices; ++s) o[s] = make_uint4(r[0][s], r[1][s], r[2][s], r[3][s]);
 }
 
 // ---------------------------------------------------------------------------
 // B operand of the density contraction, per tile: for slot block j (48 rows
 // nu) and K step k (32 slots mu) the 5 digit slices of P[fn(nu)][fn(mu)] in
 // the K-major MMA layout, stored at stage b_off[t] + j nK + k; rows past the
-// tile's slots are zero.  One block per tile, thread = (row, 8 K values).
+// tile's slots are zero.  One block per tile; a warp takes 32 consecutive rows
+// and 16 K values at a time: lane = row, so each of the 16 loads runs along one
+// column of P (a shell's functions are consecutive: a few 128-byte lines per
+// instruction), and each lane's 16 words become one whole 16-byte run of each
+// slice in its own registers.  With thread = (row, 8 K values) of the row-major
+// P the 32 lanes of a load touched 32 lines and L1 ran at 97% (200 atoms, 329
+// slots per tile: build 50.5 -> 47.2 ms, this kernel 9.6 -> 6.3; 60 atoms 7.95 -> 7.75 ms).
 // ---------------------------------------------------------------------------
-constexpr int kGatherSplit = 4;  // blocks per tile: block y takes the slot blocks j = y, y + 4, ...
-__global__ void __launch_bounds__(kBlock4(192)) k_sm_gather_B(const int64_t* __restrict__ tso,
-                                                    const int* __restrict__ slot_fn,
-                                                    const int64_t* __restrict__ b_off, int64_t t0, int64_t s0,
-                                                    const unsigned long long* __restrict__ P8,
-                                                    const int* __restrict__ e_P, int64_t nbas,
-                                                    int8_t* __restrict__ tB, double* __restrict__ ps,
-                                                    const int* __restrict__ tile_mol,
-                                                    const SetMolDev* __restrict__ mols) {
+constexpr int kGatherThreads = 256;
+__global__ void __launch_bounds__(kGatherThreads) k_sm_gather_B(const int64_t* __restrict__ tso,
+                                                               const int* __restrict__ slot_fn,
+                                                               const int64_t* __restrict__ b_off, int64_t t0,
+                                                               int64_t s0, const unsigned long long* __restrict__ P8,
+                                                               const int* __restrict__ e_P, int64_t nbas,
+                                                               int8_t* __restrict__ tB, double* __restrict__ ps,
+                                                               const int* __restrict__ tile_mol,
+                                                               const SetMolDev* __restrict__ mols) {
   extern __shared__ int sfn[];
   const int64_t t = t0 + blockIdx.x;
   if (tile_mol) {  // a set: this tile's context
@@ -189,36 +214,32 @@ __global__ void __launch_bounds__(kBlock4(192)) k_sm_gather_B(const int64_t* __r
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const int f = slot_fn[sg + i];
     sfn[i] = f;
-    if (blockIdx.y == 0) ps[sg - s0 + i] = f >= 0 ? pow2(e_P[f]) : 0.0;  // P's row scale for the density epilogue
+    ps[sg - s0 + i] = f >= 0 ? pow2(e_P[f]) : 0.0;  // P's row scale for the density epilogue
   }
   __syncthreads();
-  if (threadIdx.x >= 192) return;  // thread = (row of 48, group of 8 K values)
-  const int nK = n / 32, nN = (n + kN - 1) / kN;
-  const int r = threadIdx.x >> 2, grp = threadIdx.x & 3;
+  const int nK = n / 32, rows = (n + kN - 1) / kN * kN;
+  const int lane = threadIdx.x & 31;
+  const int nh = 2 * nK, units = (rows + 31) / 32 * nh;  // unit = (32 rows, 16 K values)
   int8_t* out = tB + (b_off[t] - b_off[t0]) * kOpB;
-  for (int j = blockIdx.y; j < nN; j += kGatherSplit) {
-    const int nu = j * kN + r;
-    const int fnv = nu < n ? sfn[nu] : -1;
-    const unsigned long long* prow = P8 + (int64_t)max(fnv, 0) * nbas;
-    for (int k = 0; k < nK; k += 2) {  // two K steps per pass: 16 loads in flight (nK is even or ends the loop)
-      unsigned long long w[2][8];
+  for (int u = threadIdx.x >> 5; u < units; u += kGatherThreads / 32) {
+    const int rg = u / nh, h = u - rg * nh;
+    const int nu = rg * 32 + lane;
+    const int fnu = nu < n ? sfn[nu] : -1;
+    const unsigned long long* col = P8 + max(fnu, 0);
+    uint2 w[16];
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int kk = min(k + h, nK - 1);
-          const int fmu = sfn[kk * 32 + grp * 8 + u];
-          w[h][u] = (fnv >= 0 && fmu >= 0) ? __ldg(prow + fmu) : 0ull;
-        }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (k + h >= nK) break;
-        int8_t* o = out + (int64_t)(j * nK + k + h) * kOpB;
-#pragma unroll
-        for (int sl = 0; sl < kSlices; ++sl)
-          *reinterpret_cast<unsigned long long*>(o + sl * kBlkB + blk_off(r, grp * 8)) = gather_slice(w[h], sl);
-      }
+    for (int i = 0; i < 16; ++i) {
+      const int fmu = sfn[h * 16 + i];
+      w[i] = (fnu >= 0 && fmu >= 0) ? __ldg(reinterpret_cast<const uint2*>(col + (int64_t)fmu * nbas))
+                                    : make_uint2(0u, 0u);
     }
+    if (nu >= rows) continue;  // the last group of 32 rows may end inside (48 rows per block)
+    uint4 o[kSlices];
+    gather_slices(w, o);
+    const int j = nu / kN, r = nu - j * kN;
+    int8_t* dst = out + (int64_t)(j * nK + (h >> 1)) * kOpB + blk_off(r, (h & 1) * 16);
+#pragma unroll
+    for (int s = 0; s < kSlices; ++s) *reinterpret_cast<uint4*>(dst + s * kBlkB) = o[s];
   }
 }
 
@@ -939,8 +960,8 @@ void screen_mixed_destroy(ScreenMixed* m) {
 
 int screen_mixed_prepare(ScreenMixed* m, const double* P, int64_t ldc, int spin, cudaStream_t st) {
   k_sm_rowexp_P<<<(unsigned)m->nbas, 256, 0, st>>>(P, ldc, m->nbas, m->e_P[spin]);
-  const unsigned nb = (unsigned)std::max<int64_t>(1, std::min<int64_t>((m->nbas * m->nbas + 255) / 256, 148 * 16));
-  k_sm_quant_P<<<nb, 256, 0, st>>>(P, ldc, m->nbas, m->e_P[spin], m->P8[spin]);
+  const unsigned nb = (unsigned)((m->nbas + 31) / 32);
+  k_sm_quant_P<<<dim3(nb, nb), 256, 0, st>>>(P, ldc, m->nbas, m->e_P[spin], m->P8[spin]);
   return 2;
 }
 
@@ -956,7 +977,7 @@ void screen_mixed_set_gga(ScreenMixed* m, bool gga) { m->gga = gga; }
 
 int screen_mixed_gather(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_t t0, int64_t nt, int64_t s0,
                         int spin, cudaStream_t st, const int* tile_mol, const SetMolDev* mols) {
-  k_sm_gather_B<<<dim3((unsigned)nt, kGatherSplit), kBlock4(192), 4 * m->max_n, st>>>(
+  k_sm_gather_B<<<(unsigned)nt, kGatherThreads, 4 * m->max_n, st>>>(
       tso, slot_fn, m->b_off, t0, s0, m->P8[spin], m->e_P[spin], m->nbas, m->tB, m->ps, tile_mol, mols);
   return 1;
 }
