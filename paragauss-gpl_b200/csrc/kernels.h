@@ -53,6 +53,7 @@ struct BuildArgs {
   double* Cocc = nullptr;
   const double* occ = nullptr;
   double* P = nullptr;        // [ldc][ldc]
+  bool p_symmetric = true;    // P formed here from C; false: the caller's P, which nothing checks
   // potential tiles
   int nt = 0;                 // ldc / 64
   int ntiles = 0;             // nt (nt + 1) / 2

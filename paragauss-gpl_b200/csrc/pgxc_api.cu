@@ -691,7 +691,9 @@ static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given = fal
     CUDA_TRY(c, cudaEventRecord(c->ev[2], s));
     ScreenTimes T;
     std::string e;
-    const int st = screen_run(c->screen, a, c->P2, s, c->d_ham, &T, e);
+    BuildArgs as = a;
+    as.p_symmetric = !p_given;
+    const int st = screen_run(c->screen, as, c->P2, s, c->d_ham, &T, e);
     if (st) return set_err(c, st, e);
     float ms = 0;
     CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev[1], c->ev[2]));

@@ -11,9 +11,9 @@
 //   k_sdensity        X = phi_t P[S_t, S_t] on DMMA, P gathered by cp.async,
 //                     fused rho, grad rho                          [K3]
 //   k_functional      (kernels_fp64.cu)                            [K2]
-//   k_szbuild         Z = A phi (+ B . grad phi)
-//   k_svpot           H[S_t, S_t] += Z_t^T phi_t on DMMA, scatter-added into
-//                     the full matrix with FP64 atomics            [K4]
+//   k_svpot           H[S_t, S_t] += Z_t^T phi_t on DMMA with Z = A phi
+//                     (+ B . grad phi) formed in shared memory, scatter-added
+//                     into the full matrix with FP64 atomics       [K4]
 // then k_spack packs V (LDA: H; GGA: H + H^T, the symmetrisation of
 // modules/xc_hamiltonian.f90:1559-1566) into the tristore order.
 #include <algorithm>
@@ -117,220 +117,327 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pre
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
 }
 
-// B slab of the density GEMM: element (k, n) = P[fn(k0+k)][fn(n0+n)], zero
-// where a slot is padding or n0+n >= n_valid.
-__device__ __forceinline__ void load_gslab(double* s, const double* __restrict__ P, int64_t ldc,
-                                           const int* __restrict__ sfn, int nvalid, int n0, int k0) {
-  const int t = threadIdx.x;
+// ---------------------------------------------------------------------------
+// The two FP64 contractions of a tile run on 64 x 64 CTA tiles of 8 warps, 2
+// (rows) x 4 (columns), 32 x 16 each, on DMMA (mma.sync m8n8k4, 16 K values per
+// shared-memory stage, three stages).  Both are bound by the FP64 tensor pipe
+// (35 TFLOP/s); what the layout is for is keeping it fed: two CTAs (16 warps)
+// per SM at up to 128 registers, a pipeline that runs on across the blocks of
+// a tile, and no work for slots past the listed functions (whole 8-function
+// fragments of a warp are left out).
+// ---------------------------------------------------------------------------
+constexpr int kSThreads = 256;
+constexpr int kSBlk = 64;
+constexpr int kXLd = 66;   // row length of the X block: 2 kXLd = 4 mod 16 (conflict-free fragment stores)
+constexpr int kZLd = 132;  // row length of the Z block: 128 points, 4 mod 16
+
+struct SAcc {
+  double v[4][2][2];
+  __device__ __forceinline__ void zero() {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int c = t + i * kGemmThreads;
-    const int k = c >> 6, nn = c & 63;
-    const int fk = sfn[k0 + k];
-    const int col = n0 + nn;
-    const int fn = col < nvalid ? sfn[col] : -1;
-    const bool ok = fk >= 0 && fn >= 0;
-    cp_async8(s + OpTile<false, 64>::idx(nn, k), ok ? P + (int64_t)fk * ldc + fn : P, ok);
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) v[i][j][0] = v[i][j][1] = 0.0;
+  }
+};
+
+// the row fragments mi (0..4) and column fragments nj (0..2) of a warp that
+// hold functions (warp-uniform)
+__device__ __forceinline__ int live_frags(int first, int listed, int most) {
+  return min(most, max(0, (listed - first + 7) >> 3));
+}
+
+// acc += A B over one 16-deep stage.  a(i, k), b(j, k): shared-memory elements.
+template <typename FA, typename FB>
+__device__ __forceinline__ void s_mma(SAcc& acc, FA a, FB b, int mi, int nj) {
+  if (mi == 4 && nj == 2) {
+#pragma unroll
+    for (int kk = 0; kk < kBK; kk += 4) {
+      double af[4], bf[2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) af[i] = a(i, kk);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) bf[j] = b(j, kk);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) dmma(acc.v[i][j], af[i], bf[j]);
+    }
+  } else if (mi > 0 && nj > 0) {
+#pragma unroll
+    for (int kk = 0; kk < kBK; kk += 4) {
+      double bf[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) bf[j] = b(j, kk);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= mi) continue;
+        const double af = a(i, kk);
+        dmma(acc.v[i][0], af, bf[0]);
+        if (nj > 1) dmma(acc.v[i][1], af, bf[1]);
+      }
+    }
   }
 }
 
-// K3 (screened): CTA = (tile, half of its 128 points); loops over 64-wide
-// blocks of the tile's slots.  The tile's slot -> function list is kept in
-// shared memory after the GEMM stages.
+// K3 (screened): CTA = (tile, half of its 128 points).  X = phi_t P[S_t, S_t]
+// in 64-wide column blocks, P gathered element-wise by 8-byte cp.async (thread
+// = one column, four rows of a stage); each finished block of X passes through
+// shared memory so that a thread then owns one point: the phi and grad phi it
+// meets are read in whole rows and the sums take 4 registers.
+// tri (GGA = false: only rho, a quadratic form): P is symmetric, so column
+// block J takes the rows of the blocks before it doubled and its own block, half
+// the products.  Grid z selects the operand plane and its sum (the three tau
+// sums of a meta-GGA in one launch).
+// 60 atoms, 304 of 690 functions per tile: X block 64 x 64 per 128 threads at 254 registers (two CTAs, 8 warps per SM)
+// kept the DMMA pipe 62% busy
+struct SPlanes {
+  const double *phi0, *phi1, *phi2;
+  double *rho0, *rho1, *rho2;
+  __device__ __forceinline__ const double* phi(int z) const { return z == 0 ? phi0 : (z == 1 ? phi1 : phi2); }
+  __device__ __forceinline__ double* rho(int z) const { return z == 0 ? rho0 : (z == 1 ? rho1 : rho2); }
+};
+// the tile's slot -> function list in shared memory, -1 past its slots up to whole 64-slot blocks
+__host__ __device__ constexpr int sfn_len(int n) { return (n + kSBlk - 1) / kSBlk * kSBlk + kSBlk; }
+__device__ __forceinline__ void load_sfn(int* sfn, const int* __restrict__ slot_fn, int n) {
+  const int len = sfn_len(n);
+  for (int i = threadIdx.x; i < len; i += kSThreads) sfn[i] = i < n ? slot_fn[i] : -1;
+}
 template <bool GGA>
-__global__ void __launch_bounds__(kGemmThreads) k_sdensity(const double* __restrict__ phi,
-                                                          const double* __restrict__ gx,
-                                                          const double* __restrict__ gy,
-                                                          const double* __restrict__ gz,
-                                                          const int64_t* __restrict__ tso, int64_t t0, int64_t s0,
-                                                          const int* __restrict__ slot_fn,
-                                                          const double* __restrict__ P, int64_t ldc,
-                                                          double* __restrict__ rho, double* __restrict__ grx,
-                                                          double* __restrict__ gry, double* __restrict__ grz) {
+__global__ void __launch_bounds__(kSThreads, 2)
+    k_sdensity(SPlanes pl, const double* __restrict__ gx, const double* __restrict__ gy,
+               const double* __restrict__ gz, const int64_t* __restrict__ tso, const int* __restrict__ listed,
+               int64_t t0, int64_t s0, const int* __restrict__ slot_fn, const double* __restrict__ P, int64_t ldc,
+               bool tri, double* __restrict__ grx, double* __restrict__ gry, double* __restrict__ grz) {
   extern __shared__ double smem[];
-  constexpr int EA = OpTile<false, 64>::kElems, EB = OpTile<false, 64>::kElems;
+  constexpr int E = OpTile<false, kSBlk>::kElems;
   double* sA = smem;
-  double* sB = smem + kStages * EA;
-  int* sfn = reinterpret_cast<int*>(smem + kStages * (EA + EB));
+  double* sB = smem + kStages * E;
+  double* sX = smem + 2 * kStages * E;
+  int* sfn = reinterpret_cast<int*>(sX + kSBlk * kXLd);
+  const double* __restrict__ phi = pl.phi(blockIdx.z);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t t = t0 + blockIdx.x;
   const int64_t sb = tso[t] - s0;
-  const int n = (int)(tso[t + 1] - tso[t]);
-  const int m0 = blockIdx.y * 64;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) sfn[i] = slot_fn[tso[t] + i];
+  const int n = (int)(tso[t + 1] - tso[t]), nl = listed[t];
+  const int m0 = blockIdx.y * kSBlk;
+  load_sfn(sfn, slot_fn + sb + s0, n);
   __syncthreads();
-  const double* A = phi + sb * 128;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm0 = (warp >> 1) * 32, wn0 = (warp & 1) * 32;
-  const int fr = lane >> 2, fk = lane & 3;
-  const int nslab = n / kBK;
-  double rp[4][2] = {}, gp[3][4][2] = {};
-  for (int n0 = 0; n0 < n; n0 += 64) {
-    Acc acc;
-    acc.zero();
+  const double* A = phi + sb * 128 + m0;
+  const int wm0 = (warp >> 2) * 32, wn0 = (warp & 3) * 16, fr = lane >> 2, fk = lane & 3;
+  const int nslab = (nl + kBK - 1) / kBK, nblk = (nl + kSBlk - 1) / kSBlk;
+  const int col = tid & 63, kq = tid >> 6;  // this thread's column of every gathered stage, rows kq + 4 i
+  // slabs of column block J: all, or (tri) those up to the end of its own block
+  auto slabs = [&](int J) { return tri ? min(nslab, (J + 1) * (kSBlk / kBK)) : nslab; };
+  int lj = 0, lk = 0;     // next stage to load: column block, slab
+  int fcol = sfn[col];
+  auto load = [&](int st) {
+    if (lj >= nblk) return;
+    double* a = sA + st * E;
+    double* b = sB + st * E;
+    const int k0 = lk * kBK;
 #pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) {
-      if (s < nslab) {
-        load_slab<false>(sA + s * EA, A, 128, m0, (int64_t)s * kBK);
-        load_gslab(sB + s * EB, P, ldc, sfn, n, n0, s * kBK);
-      }
-      cp_async_commit();
+    for (int i = 0; i < 2; ++i) {
+      const int c = tid + i * kSThreads, k = c >> 5, mn = (c & 31) * 2;
+      cp_async16(a + OpTile<false, kSBlk>::idx(mn, k), A + (int64_t)(k0 + k) * 128 + mn);
     }
-    for (int it = 0; it < nslab; ++it) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = kq + 4 * i, f = sfn[k0 + k];
+      const bool ok = f >= 0 && fcol >= 0;
+      cp_async8(b + OpTile<false, kSBlk>::idx(col, k), ok ? P + (int64_t)f * ldc + fcol : P, ok);
+    }
+    if (++lk == slabs(lj)) {
+      lk = 0;
+      ++lj;
+      fcol = sfn[lj * kSBlk + col];
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    load(s);
+    cp_async_commit();
+  }
+  double r = 0.0, g[3] = {0.0, 0.0, 0.0};  // of point m0 + (tid & 63), columns tid >> 6 mod 4
+  int st = 0;
+  for (int J = 0; J < nblk; ++J) {
+    const int n0 = J * kSBlk, ns = slabs(J);
+    const int nj = live_frags(n0 + wn0, nl, 2);
+    SAcc acc;
+    acc.zero();
+    for (int it = 0; it < ns; ++it) {
       cp_async_wait<kStages - 2>();
       __syncthreads();
-      {
-        const int nx = it + kStages - 1;
-        if (nx < nslab) {
-          const int st = nx % kStages;
-          load_slab<false>(sA + st * EA, A, 128, m0, (int64_t)nx * kBK);
-          load_gslab(sB + st * EB, P, ldc, sfn, n, n0, nx * kBK);
-        }
-        cp_async_commit();
-      }
-      const double* a_s = sA + (it % kStages) * EA;
-      const double* b_s = sB + (it % kStages) * EB;
-#pragma unroll
-      for (int kk = 0; kk < kBK; kk += 4) {
-        double af[4], bf[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) af[i] = a_s[OpTile<false, 64>::idx(wm0 + i * 8 + fr, kk + fk)];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bf[j] = b_s[OpTile<false, 64>::idx(wn0 + j * 8 + fr, kk + fk)];
+      load(st >= 1 ? st - 1 : kStages - 1);  // the stage consumed before this one
+      cp_async_commit();
+      if (tri && it * kBK == n0)  // the blocks before J count twice
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) dmma(acc.v[i][j], af[i], bf[j]);
+          for (int j = 0; j < 2; ++j) {
+            acc.v[i][j][0] *= 2.0;
+            acc.v[i][j][1] *= 2.0;
+          }
+      const double* a_s = sA + st * E + wm0 + fr + fk * (kSBlk + kPadMN);
+      const double* b_s = sB + st * E + wn0 + fr + fk * (kSBlk + kPadMN);
+      s_mma(acc, [&](int i, int kk) { return a_s[i * 8 + kk * (kSBlk + kPadMN)]; },
+            [&](int j, int kk) { return b_s[j * 8 + kk * (kSBlk + kPadMN)]; }, 4, nj);
+      st = st == kStages - 1 ? 0 : st + 1;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          sX[(wn0 + j * 8 + 2 * fk + e) * kXLd + wm0 + i * 8 + fr] = acc.v[i][j][e];
+    __syncthreads();
+    const int p = tid & 63, cn = min(kSBlk, nl - n0);
+    const int64_t o0 = (sb + n0) * 128 + m0 + p;
+#pragma unroll 4
+    for (int c = tid >> 6; c < cn; c += 4) {
+      const double x = sX[c * kXLd + p];
+      const int64_t o = o0 + c * 128;
+      r += x * phi[o];
+      if (GGA) {
+        g[0] += x * gx[o];
+        g[1] += x * gy[o];
+        g[2] += x * gz[o];
       }
     }
-    cp_async_wait<0>();
-    __syncthreads();
+    // sX is next written after a further barrier of the stage loop
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  double* red = smem;  // [4 quantities][4 column groups][64 points]
+  red[tid] = r;
+  if (GGA)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) red[(q + 1) * kSThreads + tid] = g[q];
+  __syncthreads();
+  const int q = tid >> 6, p = tid & 63;
+  if (q > 0 && !GGA) return;
+  const double* rq = red + q * kSThreads + p;
+  const double v = (rq[0] + rq[64]) + (rq[128] + rq[192]);
+  double* out = q == 0 ? pl.rho(blockIdx.z) : (q == 1 ? grx : (q == 2 ? gry : grz));
+  out[(int64_t)blockIdx.x * 128 + m0 + p] = q == 0 ? v : 2.0 * v;
+}
+constexpr int sdensity_smem(int max_n) {
+  return (2 * kStages * OpTile<false, kSBlk>::kElems + kSBlk * kXLd) * 8 + 4 * sfn_len(max_n);
+}
+
+// K4 (screened): H[fn_i][fn_j] += sum_p Z[i][p] phi[j][p] for the slots i, j of
+// one tile, Z = A phi (+ B . grad phi).  CTA = (tile, 64 slots i): it forms its
+// block of Z in shared memory once (the whole K = 128 points) and streams the
+// tile's phi against it.  A separate pass that wrote Z for the contraction to
+// read took 2.4 ms of the 60-atom build's 25.
+// kFull: the whole square (GGA: V = H + H^T in k_spack).  kUpper: fn_i <= fn_j
+// only (LDA: H is symmetric).  kTwice: the upper triangle with the off-diagonal
+// elements doubled: the symmetric tau term of a meta-GGA, which k_spack's H + H^T
+// then counts as the whole square does; grid z selects its plane.
+// 60 atoms, 304 of 690 functions per tile: three 128-thread CTAs kept the DMMA pipe 85% busy but a third of it on padding
+enum { kFull, kUpper, kTwice };
+template <int MODE, bool GRAD>
+__global__ void __launch_bounds__(kSThreads, 2)
+    k_svpot(SPlanes pl, const double* __restrict__ gx, const double* __restrict__ gy, const double* __restrict__ gz,
+            const double* __restrict__ A, const double* __restrict__ Bx, const double* __restrict__ By,
+            const double* __restrict__ Bz, const int64_t* __restrict__ tso, const int* __restrict__ listed, int64_t t0,
+            int64_t s0, const int* __restrict__ slot_fn, double* __restrict__ V, int64_t ldv) {
+  extern __shared__ double smem[];
+  constexpr int E = OpTile<true, kSBlk>::kElems;
+  const int64_t t = t0 + blockIdx.x;
+  const int nl = listed[t], I0 = blockIdx.y * kSBlk;
+  if (I0 >= nl) return;
+  double* sZ = smem;
+  double* sF = smem + kSBlk * kZLd;
+  int* sfn = reinterpret_cast<int*>(sF + kStages * E);
+  const double* __restrict__ phi = pl.phi(blockIdx.z);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t sb = tso[t] - s0;
+  const double* F = phi + sb * 128;
+  const int J0 = MODE == kFull ? 0 : blockIdx.y, nJ = (nl + kSBlk - 1) / kSBlk;
+  int lj = J0, lk = 0;  // next stage to load: 64-slot block, slab of 16 points
+  auto load = [&](int st) {
+    if (lj >= nJ) return;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int c = tid + i * kSThreads, row = c >> 3, k = (c & 7) * 2;
+      cp_async16(sF + st * E + OpTile<true, kSBlk>::idx(row, k), F + (int64_t)(lj * kSBlk + row) * 128 + lk * kBK + k);
+    }
+    if (++lk == 128 / kBK) {
+      lk = 0;
+      ++lj;
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    load(s);
+    cp_async_commit();
+  }
+  load_sfn(sfn, slot_fn + sb + s0, (int)(tso[t + 1] - tso[t]));
+  {
+    // Z rows tid >> 7, + 2, ...; this thread's point is tid & 127 throughout
+    const int p = tid & 127;
+    const int64_t pt = (int64_t)blockIdx.x * 128 + p;
+    const double a = A[pt];
+    double b[3] = {0.0, 0.0, 0.0};
+    if (GRAD) {
+      b[0] = Bx[pt];
+      b[1] = By[pt];
+      b[2] = Bz[pt];
+    }
+    const int nz = min(kSBlk, nl - I0);
+#pragma unroll 8
+    for (int i = tid >> 7; i < kSBlk; i += 2) {
+      double z = 0.0;
+      if (i < nz) {
+        const int64_t o = (sb + I0 + i) * 128 + p;
+        z = a * phi[o];
+        if (GRAD) z += b[0] * gx[o] + b[1] * gy[o] + b[2] * gz[o];
+      }
+      sZ[i * kZLd + p] = z;
+    }
+  }
+  const int wm0 = (warp >> 2) * 32, wn0 = (warp & 3) * 16, fr = lane >> 2, fk = lane & 3;
+  const int nj = live_frags(I0 + wn0, nl, 2);
+  int st = 0;
+  for (int J = J0; J < nJ; ++J) {
+    const int j0 = J * kSBlk + wm0;
+    // rows j of the fragment, columns i: a warp's atomics run along rows of V
+    const int mi = MODE != kFull && j0 + 31 < I0 + wn0 ? 0 : live_frags(j0, nl, 4);
+    SAcc acc;
+    acc.zero();
+    for (int it = 0; it < 128 / kBK; ++it) {
+      cp_async_wait<kStages - 2>();
+      __syncthreads();
+      load(st >= 1 ? st - 1 : kStages - 1);
+      cp_async_commit();
+      const double* f_s = sF + st * E + (wm0 + fr) * (kBK + kPadK) + fk;
+      const double* z_s = sZ + (wn0 + fr) * kZLd + it * kBK + fk;
+      s_mma(acc, [&](int i, int kk) { return f_s[i * 8 * (kBK + kPadK) + kk]; },
+            [&](int j, int kk) { return z_s[j * 8 * kZLd + kk]; }, mi, nj);
+      st = st == kStages - 1 ? 0 : st + 1;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int r = m0 + wm0 + i * 8 + (lane >> 2);
+      const int j = j0 + i * 8 + fr;
+      const int fj = sfn[j];  // -1 past the listed functions
+      if (i >= mi || fj < 0) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int c = n0 + wn0 + j * 8 + 2 * (lane & 3) + e;
-          if (c < n) {
-            const double x = acc.v[i][j][e];
-            const int64_t o = (sb + c) * 128 + r;
-            rp[i][e] += x * phi[o];
-            if (GGA) {
-              gp[0][i][e] += x * gx[o];
-              gp[1][i][e] += x * gy[o];
-              gp[2][i][e] += x * gz[o];
-            }
-          }
+          const int fi = sfn[I0 + wn0 + c * 8 + 2 * fk + e];
+          if (fi < 0) continue;
+          double v = acc.v[i][c][e];
+          if (MODE == kTwice && fj != fi) v *= 2.0;
+          if (MODE == kFull || fj >= fi) atomicAdd(V + (int64_t)fi * ldv + fj, v);
         }
     }
   }
-  // reduce the 4 lanes of a row, then the two column-warps through smem
-  double* red = smem;  // [2 warps-n][4 quantities][64 rows]
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    double v[4];
-    v[0] = rp[i][0] + rp[i][1];
-    if (GGA) {
-      v[1] = gp[0][i][0] + gp[0][i][1];
-      v[2] = gp[1][i][0] + gp[1][i][1];
-      v[3] = gp[2][i][0] + gp[2][i][1];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (q > 0 && !GGA) break;
-      v[q] += __shfl_xor_sync(0xffffffffu, v[q], 1);
-      v[q] += __shfl_xor_sync(0xffffffffu, v[q], 2);
-      if ((lane & 3) == 0) red[((warp & 1) * 4 + q) * 64 + wm0 + i * 8 + (lane >> 2)] = v[q];
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 64) {
-    const int r = threadIdx.x;
-    const int64_t o = (int64_t)blockIdx.x * 128 + m0 + r;
-    rho[o] = red[0 * 64 + r] + red[4 * 64 + r];
-    if (GGA) {
-      grx[o] = 2.0 * (red[1 * 64 + r] + red[5 * 64 + r]);
-      gry[o] = 2.0 * (red[2 * 64 + r] + red[6 * 64 + r]);
-      grz[o] = 2.0 * (red[3 * 64 + r] + red[7 * 64 + r]);
-    }
-  }
 }
-
-// Z[s][p] = A[p] phi[s][p] (+ B[p] . grad phi[s][p]) over the chunk's slots
-template <bool GGA>
-__global__ void k_szbuild(int64_t nslots, const int* __restrict__ slot_tile, int64_t t0,
-                          const double* __restrict__ phi, const double* __restrict__ gx,
-                          const double* __restrict__ gy, const double* __restrict__ gz,
-                          const double* __restrict__ A, const double* __restrict__ Bx,
-                          const double* __restrict__ By, const double* __restrict__ Bz, double* __restrict__ Z) {
-  const int64_t total = nslots * 128;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = ((int64_t)slot_tile[e >> 7] - t0) * 128 + (e & 127);
-    double z = A[p] * phi[e];
-    if (GGA) z += Bx[p] * gx[e] + By[p] * gy[e] + Bz[p] * gz[e];
-    Z[e] = z;
-  }
-}
-
-// (I, J) of pair q of the tile's nb 64-slot blocks: all nb^2 (GGA) or I <= J (LDA)
-__device__ __forceinline__ void pair_of(int q, int nb, bool all, int& I, int& J) {
-  if (all) {
-    I = q / nb;
-    J = q % nb;
-    return;
-  }
-  I = 0;
-  while (q >= nb - I) {
-    q -= nb - I;
-    ++I;
-  }
-  J = I + q;
-}
-
-// K4 (screened): H[fn_i][fn_j] += sum_p Z[i][p] phi[j][p] for the slots i, j
-// of one tile; LDA keeps fn_i <= fn_j only (H is symmetric), GGA the whole
-// square (V = H + H^T in k_spack).
-template <bool GGA>
-__global__ void __launch_bounds__(kGemmThreads) k_svpot(const double* __restrict__ phi, const double* __restrict__ Z,
-                                                       const int64_t* __restrict__ tso, int64_t t0, int64_t s0,
-                                                       const int* __restrict__ slot_fn, double* __restrict__ V,
-                                                       int64_t ldv) {
-  extern __shared__ double smem[];
-  constexpr int kGemmDoubles = kStages * (OpTile<true, 64>::kElems + OpTile<true, 64>::kElems);
-  int* sfn = reinterpret_cast<int*>(smem + kGemmDoubles);
-  const int64_t t = t0 + blockIdx.x;
-  const int64_t sb = tso[t] - s0;
-  const int n = (int)(tso[t + 1] - tso[t]);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) sfn[i] = slot_fn[tso[t] + i];
-  __syncthreads();
-  const int nb = (n + 63) / 64;
-  const int npairs = GGA ? nb * nb : nb * (nb + 1) / 2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm0 = (warp >> 1) * 32, wn0 = (warp & 1) * 32;
-  for (int q = blockIdx.y; q < npairs; q += gridDim.y) {
-    int I, J;
-    pair_of(q, nb, GGA, I, J);
-    Acc acc;
-    acc.zero();
-    // acc[j][i] = sum_p phi_j Z_i: rows of the fragment run along j, so the
-    // atomics of a warp instruction hit 4 rows of V in runs of 8 functions
-    gemm_tile<true, true>(acc, phi + sb * 128, 128, (int64_t)J * 64, Z + sb * 128, 128, (int64_t)I * 64, 0, 128,
-                          smem);
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const int j = J * 64 + wm0 + jj * 8 + (lane >> 2);
-      const int fj = j < n ? sfn[j] : -1;
-#pragma unroll
-      for (int ii = 0; ii < 4; ++ii)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = I * 64 + wn0 + ii * 8 + 2 * (lane & 3) + e;
-          const int fi = i < n ? sfn[i] : -1;
-          if (fi >= 0 && fj >= 0 && (GGA || fj >= fi)) atomicAdd(V + (int64_t)fi * ldv + fj, acc.v[jj][ii][e]);
-        }
-    }
-  }
+constexpr int svpot_smem(int max_n) {
+  return (kSBlk * kZLd + kStages * OpTile<true, kSBlk>::kElems) * 8 + 4 * sfn_len(max_n);
 }
 
 }  // namespace
@@ -519,7 +626,7 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
   }
   // --- per-tile lists --------------------------------------------------------
   std::vector<int64_t> tso((size_t)ntiles + 1, 0);
-  std::vector<int> slot_fn, slot_tile, listed_t((size_t)ntiles, 0);
+  std::vector<int> slot_fn, listed_t((size_t)ntiles, 0);
   std::vector<BasisItem> items[kMaxL + 1];
   std::vector<int64_t> tile_items[kMaxL + 1];  // items before tile t, per L
   for (int l = 0; l <= kMaxL; ++l) tile_items[l].assign((size_t)ntiles + 1, 0);
@@ -561,7 +668,6 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     const int64_t nt = (int64_t)slot_fn.size() - base;
     sp->sum_n2 += (double)listed * (double)listed;
     sp->max_n = std::max(sp->max_n, (int)nt);
-    slot_tile.resize(slot_fn.size(), (int)t);
     tso[(size_t)t + 1] = (int64_t)slot_fn.size();
   }
   for (int l = 0; l <= kMaxL; ++l) {
@@ -586,7 +692,7 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     }
     freeb -= (size_t)need;
   }
-  const int64_t per_slot = 128 * (16 + (in.gga ? 3 * (sp->gf32 ? 4 : 8) : 0)) + (mixed ? screen_mixed_bytes_per_slot() : 0);
+  const int64_t per_slot = 128 * (8 + (in.gga ? 3 * (sp->gf32 ? 4 : 8) : 0)) + (mixed ? screen_mixed_bytes_per_slot() : 0);
   const int64_t per_tile = 128 * 8 * 8 * in.ispin + (mixed ? screen_mixed_bytes_per_tile() : 0);
   int64_t budget_slots = (int64_t)(0.45 * (double)freeb) / per_slot;
   budget_slots = std::max<int64_t>(budget_slots, sp->max_n);
@@ -632,11 +738,8 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
   SP_TRY(sp_alloc(sp, &sp->listed, listed_t.size()), "cudaMalloc");
   SP_TRY(cudaMemcpy(sp->listed, listed_t.data(), sizeof(int) * listed_t.size(), cudaMemcpyHostToDevice), "copy");
   SP_TRY(sp_alloc(sp, &sp->slot_fn, slot_fn.size()), "cudaMalloc");
-  SP_TRY(sp_alloc(sp, &sp->slot_tile, slot_tile.size()), "cudaMalloc");
   if (!slot_fn.empty()) {
     SP_TRY(cudaMemcpy(sp->slot_fn, slot_fn.data(), sizeof(int) * slot_fn.size(), cudaMemcpyHostToDevice), "copy");
-    SP_TRY(cudaMemcpy(sp->slot_tile, slot_tile.data(), sizeof(int) * slot_tile.size(), cudaMemcpyHostToDevice),
-           "copy");
   }
   for (int l = 0; l <= kMaxL; ++l) {
     SP_TRY(sp_alloc(sp, &sp->items[l], items[l].size()), "cudaMalloc");
@@ -648,9 +751,7 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
   // basis arrays: one chunk's rows, or every slot of the grid when they stay resident
   const size_t brows = sp->keep ? (size_t)(sp->nslots + kSlack) * 128 : rows;
   SP_TRY(sp_alloc(sp, &sp->phi, brows), "cudaMalloc (phi)");
-  SP_TRY(sp_alloc(sp, &sp->Z, rows), "cudaMalloc (Z)");
   SP_TRY(cudaMemset(sp->phi, 0, sizeof(double) * brows), "memset");
-  SP_TRY(cudaMemset(sp->Z, 0, sizeof(double) * rows), "memset");
   if (in.gga && sp->gf32) {
     SP_TRY(sp_alloc(sp, &sp->fx, brows), "cudaMalloc (grad phi)");
     SP_TRY(sp_alloc(sp, &sp->fy, brows), "cudaMalloc (grad phi)");
@@ -815,33 +916,32 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
           T.launches += screen_mixed_density(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, phi, gxc, gyc, gzc,
                                              b[s].rho, b[s].grx, b[s].gry, b[s].grz, so, to, st);
       } else {
-        const int smem = gemm_smem_bytes<false, false>() + (int)sizeof(int) * sp->max_n;
-        dim3 grid((unsigned)nt, 2);
+        const int smem = sdensity_smem(sp->max_n);
+        const SPlanes pl{phi, phi, phi, b[s].rho, b[s].rho, b[s].rho};
         if (gga) {
           raise_smem_limit(k_sdensity<true>, smem);
-          k_sdensity<true><<<grid, kGemmThreads, smem, st>>>(phi, gxc, gyc, gzc, sp->tso, t0, s0,
-                                                             sp->slot_fn, P[s], a.ldc, b[s].rho, b[s].grx, b[s].gry,
-                                                             b[s].grz);
+          k_sdensity<true><<<dim3((unsigned)nt, 2), kSThreads, smem, st>>>(
+              pl, gxc, gyc, gzc, sp->tso, sp->listed, t0, s0, sp->slot_fn, P[s], a.ldc, false, b[s].grx, b[s].gry,
+              b[s].grz);
         } else {
           raise_smem_limit(k_sdensity<false>, smem);
-          k_sdensity<false><<<grid, kGemmThreads, smem, st>>>(phi, nullptr, nullptr, nullptr, sp->tso, t0, s0,
-                                                              sp->slot_fn, P[s], a.ldc, b[s].rho, nullptr, nullptr,
-                                                              nullptr);
+          k_sdensity<false><<<dim3((unsigned)nt, 2), kSThreads, smem, st>>>(
+              pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, P[s], a.ldc, a.p_symmetric,
+              nullptr, nullptr, nullptr);
         }
         ++T.launches;
       }
       if (sp->mgga || (extra && extra->tau)) {
         // 2 tau_j = sum_nu (d_j phi P)_nu d_j phi_nu: the density contraction with d_j phi in the
         // place of phi (FP64 DMMA in every precision mode)
-        const int smem = gemm_smem_bytes<false, false>() + (int)sizeof(int) * sp->max_n;
+        const int smem = sdensity_smem(sp->max_n);
         raise_smem_limit(k_sdensity<false>, smem);
-        const double* gj[3] = {gxc, gyc, gzc};
-        for (int j = 0; j < 3; ++j) {
-          k_sdensity<false><<<dim3((unsigned)nt, 2), kGemmThreads, smem, st>>>(
-              gj[j], nullptr, nullptr, nullptr, sp->tso, t0, s0, sp->slot_fn, P[s], a.ldc,
-              sp->tq + (4 * s + j) * cp, nullptr, nullptr, nullptr);
-          ++T.launches;
-        }
+        double* tau = sp->tq + 4 * s * cp;
+        const SPlanes pl{gxc, gyc, gzc, tau, tau + cp, tau + 2 * cp};
+        k_sdensity<false><<<dim3((unsigned)nt, 2, 3), kSThreads, smem, st>>>(
+            pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, P[s], a.ldc, a.p_symmetric,
+            nullptr, nullptr, nullptr);
+        ++T.launches;
       }
     }
     if (timed) SR_TRY(cudaEventRecord(ev[5], st));
@@ -864,51 +964,41 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
       cudaEvent_t k0 = timed ? ev[7 + 3 * s] : nullptr, k1 = timed ? ev[8 + 3 * s] : nullptr;
       if (sp->mixed) {
         if (gf)
-          T.launches += screen_mixed_potential(sp->mixed, sp->tso, sp->slot_fn, sp->slot_tile, t0, nt, s0, ns, phi,
+          T.launches += screen_mixed_potential(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, phi,
                                                fxc, fyc, fzc, b[s].A, b[s].Bx, b[s].By, b[s].Bz, Vs, sp->nbas,
                                                st, k0, k1);
         else
-          T.launches += screen_mixed_potential(sp->mixed, sp->tso, sp->slot_fn, sp->slot_tile, t0, nt, s0, ns, phi,
+          T.launches += screen_mixed_potential(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, phi,
                                                gxc, gyc, gzc, b[s].A, b[s].Bx, b[s].By, b[s].Bz, Vs, sp->nbas,
                                                st, k0, k1);
       } else {
-        const unsigned nbk = (unsigned)std::max<int64_t>(1, std::min<int64_t>((ns * 128 + 255) / 256, 148 * 32));
-        if (gga)
-          k_szbuild<true><<<nbk, 256, 0, st>>>(ns, sp->slot_tile + s0, t0, phi, gxc, gyc, gzc, b[s].A,
-                                               b[s].Bx, b[s].By, b[s].Bz, sp->Z);
-        else
-          k_szbuild<false><<<nbk, 256, 0, st>>>(ns, sp->slot_tile + s0, t0, phi, nullptr, nullptr, nullptr,
-                                                b[s].A, nullptr, nullptr, nullptr, sp->Z);
+        const int smem = svpot_smem(sp->max_n);
+        const dim3 grid((unsigned)nt, (unsigned)((sp->max_n + kSBlk - 1) / kSBlk));
+        const SPlanes pl{phi, phi, phi, nullptr, nullptr, nullptr};
         if (timed) SR_TRY(cudaEventRecord(k0, st));
-        const int smem = gemm_smem_bytes<true, true>() + (int)sizeof(int) * sp->max_n;
-        dim3 grid((unsigned)nt, 4);
         if (gga) {
-          raise_smem_limit(k_svpot<true>, smem);
-          k_svpot<true><<<grid, kGemmThreads, smem, st>>>(phi, sp->Z, sp->tso, t0, s0, sp->slot_fn, Vs,
-                                                          sp->nbas);
+          raise_smem_limit(k_svpot<kFull, true>, smem);
+          k_svpot<kFull, true><<<grid, kSThreads, smem, st>>>(pl, gxc, gyc, gzc, b[s].A, b[s].Bx, b[s].By, b[s].Bz,
+                                                              sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas);
         } else {
-          raise_smem_limit(k_svpot<false>, smem);
-          k_svpot<false><<<grid, kGemmThreads, smem, st>>>(phi, sp->Z, sp->tso, t0, s0, sp->slot_fn, Vs,
-                                                           sp->nbas);
+          raise_smem_limit(k_svpot<kUpper, false>, smem);
+          k_svpot<kUpper, false><<<grid, kSThreads, smem, st>>>(pl, nullptr, nullptr, nullptr, b[s].A, nullptr, nullptr,
+                                                                nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs,
+                                                                sp->nbas);
         }
         if (timed) SR_TRY(cudaEventRecord(k1, st));
-        T.launches += 2;
+        ++T.launches;
       }
       if (sp->mgga) {
-        // tau term: per direction Z = C d_j phi and H += Z^T d_j phi over the whole square of
+        // tau term: per direction Z = C d_j phi and H += Z^T d_j phi over the upper triangle of
         // each tile (k_spack then forms H + H^T), FP64 DMMA in every precision mode
-        const unsigned nbk = (unsigned)std::max<int64_t>(1, std::min<int64_t>((ns * 128 + 255) / 256, 148 * 32));
-        const int smem = gemm_smem_bytes<true, true>() + (int)sizeof(int) * sp->max_n;
-        raise_smem_limit(k_svpot<true>, smem);
-        const double* gj[3] = {gxc, gyc, gzc};
-        const double* Cs = sp->tq + (4 * s + 3) * cp;
-        for (int j = 0; j < 3; ++j) {
-          k_szbuild<false><<<nbk, 256, 0, st>>>(ns, sp->slot_tile + s0, t0, gj[j], nullptr, nullptr, nullptr, Cs,
-                                                nullptr, nullptr, nullptr, sp->Z);
-          k_svpot<true><<<dim3((unsigned)nt, 4), kGemmThreads, smem, st>>>(gj[j], sp->Z, sp->tso, t0, s0,
-                                                                            sp->slot_fn, Vs, sp->nbas);
-          T.launches += 2;
-        }
+        const int smem = svpot_smem(sp->max_n);
+        raise_smem_limit(k_svpot<kTwice, false>, smem);
+        const SPlanes pl{gxc, gyc, gzc, nullptr, nullptr, nullptr};
+        k_svpot<kTwice, false><<<dim3((unsigned)nt, (unsigned)((sp->max_n + kSBlk - 1) / kSBlk), 3), kSThreads, smem,
+                                 st>>>(pl, nullptr, nullptr, nullptr, sp->tq + (4 * s + 3) * cp, nullptr, nullptr,
+                                       nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas);
+        ++T.launches;
       }
     }
     // further functionals on the same density (after K4, whose A and B they overwrite)
@@ -1425,7 +1515,7 @@ int screen_set_run(ScreenSet* S, cudaStream_t st, std::string& err) {
     launch_functional_tiles(b, t0 * 128, nt, gga, st);
     k_set_sum<<<(unsigned)c.nseg, 128, 0, st>>>(S->partial, S->segs + c.seg0, S->outs);
     launches += 2;
-    launches += screen_mixed_potential(S->mixed, S->tso, S->slot_fn, nullptr, t0, nt, s0, 0, S->phi, gxc, gyc, gzc, b.A,
+    launches += screen_mixed_potential(S->mixed, S->tso, S->slot_fn, t0, nt, s0, S->phi, gxc, gyc, gzc, b.A,
                                        b.Bx, b.By, b.Bz, nullptr, 0, st, nullptr, nullptr, S->tile_mol, S->mols);
   }
   k_set_pack<<<(unsigned)S->mem.size(), 256, 0, st>>>(S->outs);

@@ -1051,23 +1051,19 @@ int screen_mixed_density(ScreenMixed* m, const int64_t* tso, const int* slot_fn,
   return mixed_density<float>(m, tso, slot_fn, t0, nt, s0, phi, gx, gy, gz, rho, grx, gry, grz, so, to, st);
 }
 
-int screen_mixed_potential(ScreenMixed* m, const int64_t* tso, const int* slot_fn, const int* slot_tile, int64_t t0,
-                           int64_t nt, int64_t s0, int64_t ns, const double* phi, const double* gx, const double* gy,
+int screen_mixed_potential(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_t t0,
+                           int64_t nt, int64_t s0, const double* phi, const double* gx, const double* gy,
                            const double* gz, const double* A, const double* Bx, const double* By, const double* Bz,
                            double* V, int64_t ldv, cudaStream_t st, cudaEvent_t k0, cudaEvent_t k1,
                            const int* tile_mol, const SetMolDev* mols) {
-  (void)slot_tile;
-  (void)ns;
   return mixed_potential<double>(m, tso, slot_fn, t0, nt, s0, phi, gx, gy, gz, A, Bx, By, Bz, V, ldv, st, k0, k1,
                                  tile_mol, mols);
 }
-int screen_mixed_potential(ScreenMixed* m, const int64_t* tso, const int* slot_fn, const int* slot_tile, int64_t t0,
-                           int64_t nt, int64_t s0, int64_t ns, const double* phi, const float* gx, const float* gy,
+int screen_mixed_potential(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_t t0,
+                           int64_t nt, int64_t s0, const double* phi, const float* gx, const float* gy,
                            const float* gz, const double* A, const double* Bx, const double* By, const double* Bz,
                            double* V, int64_t ldv, cudaStream_t st, cudaEvent_t k0, cudaEvent_t k1,
                            const int* tile_mol, const SetMolDev* mols) {
-  (void)slot_tile;
-  (void)ns;
   return mixed_potential<float>(m, tso, slot_fn, t0, nt, s0, phi, gx, gy, gz, A, Bx, By, Bz, V, ldv, st, k0, k1,
                                 tile_mol, mols);
 }

@@ -30,7 +30,6 @@ struct ScreenPlan {
   double *qx = nullptr, *qy = nullptr, *qz = nullptr, *qw = nullptr;  // Morton-ordered points [ntiles*128]
   int64_t* tso = nullptr;   // [ntiles+1] first slot of each tile
   int* slot_fn = nullptr;   // [nslots] function of each slot, -1 for padding
-  int* slot_tile = nullptr; // [nslots]
   int* listed = nullptr;    // [ntiles] listed (not padding) slots of each tile
   int64_t* b_off = nullptr;  // [ntiles+1] first density B stage of each tile (INT8 path)
   BasisItem* items[kMaxL + 1] = {};
@@ -41,7 +40,7 @@ struct ScreenPlan {
   std::vector<int64_t> tile_item[kMaxL + 1];       // items before tile t, per L ([ntiles + 1])
   int64_t chunk_slots = 0, chunk_tiles = 0;        // buffer capacities
   // device, per chunk
-  double *phi = nullptr, *gx = nullptr, *gy = nullptr, *gz = nullptr, *Z = nullptr;
+  double *phi = nullptr, *gx = nullptr, *gy = nullptr, *gz = nullptr;
   // INT8 build (not a meta-GGA): grad phi in 32-bit planes instead of gx/gy/gz
   bool gf32 = false;
   float *fx = nullptr, *fy = nullptr, *fz = nullptr;
