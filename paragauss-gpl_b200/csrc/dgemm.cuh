@@ -59,7 +59,7 @@ __device__ __forceinline__ void load_slab(double* s, const double* __restrict__ 
 }
 
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
 }

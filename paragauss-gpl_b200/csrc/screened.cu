@@ -118,185 +118,193 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pre
 }
 
 // ---------------------------------------------------------------------------
-// The two FP64 contractions of a tile run on 64 x 64 CTA tiles of 8 warps, 2
-// (rows) x 4 (columns), 32 x 16 each, on DMMA (mma.sync m8n8k4, 16 K values per
-// shared-memory stage, three stages).  Both are bound by the FP64 tensor pipe
-// (35 TFLOP/s); what the layout is for is keeping it fed: two CTAs (16 warps)
-// per SM at up to 128 registers, a pipeline that runs on across the blocks of
-// a tile, and no work for slots past the listed functions (whole 8-function
-// fragments of a warp are left out).
+// The two FP64 contractions of a tile run on DMMA (mma.sync m8n8k4) in CTAs of
+// four warps, 16 K values per shared-memory stage.  Both are bound
+// by the FP64 tensor pipe (35 TFLOP/s); what the layout is for is keeping it
+// fed.  Each SM sub-partition has its own DMMA unit and a CTA holds one warp of
+// each, so that three independent CTAs per SM fill one another's barriers and
+// epilogues (with eight warps and two CTAs the pipe ran at 63%).  Whole 8-function
+// fragments past the listed functions are left out, and the warps' places rotate
+// with the tile so that the warps a ragged block leaves idle do not all fall on
+// one sub-partition.
 // ---------------------------------------------------------------------------
-constexpr int kSThreads = 256;
-constexpr int kSBlk = 64;
-constexpr int kXLd = 66;   // row length of the X block: 2 kXLd = 4 mod 16 (conflict-free fragment stores)
-constexpr int kZLd = 132;  // row length of the Z block: 128 points, 4 mod 16
+constexpr int kSThreads = 128;
+constexpr int kSBlk = 64;   // functions (and points) of a block
+constexpr int kRows = 32;   // functions i of a potential CTA, and functions j of a warp's block
+constexpr int kSStages = 2;
+constexpr int kDK = 16, kDStages = 3, kDLd = kSBlk + kPadMN;  // density stages
+constexpr int kXLd = 66;    // row length of the X block: 2 kXLd = 4 mod 16 (conflict-free fragment stores)
+constexpr int kZLd = 132;   // row length of the Z block: 128 points, 4 mod 16
 
+template <int NI, int NJ>
 struct SAcc {
-  double v[4][2][2];
+  double v[NI][NJ][2];
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < NI; ++i)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) v[i][j][0] = v[i][j][1] = 0.0;
+      for (int j = 0; j < NJ; ++j) v[i][j][0] = v[i][j][1] = 0.0;
   }
 };
 
-// the row fragments mi (0..4) and column fragments nj (0..2) of a warp that
-// hold functions (warp-uniform)
+// the fragments (0..most) of eight functions from `first` on that hold listed ones (warp-uniform)
 __device__ __forceinline__ int live_frags(int first, int listed, int most) {
   return min(most, max(0, (listed - first + 7) >> 3));
 }
 
-// acc += A B over one 16-deep stage.  a(i, k), b(j, k): shared-memory elements.
-template <typename FA, typename FB>
-__device__ __forceinline__ void s_mma(SAcc& acc, FA a, FB b, int mi, int nj) {
-  if (mi == 4 && nj == 2) {
+// acc += A B over one K-deep stage, row fragments < mi and column fragments
+// < nj.  a(i, k), b(j, k): shared-memory elements.  The fragments of the next
+// four K values are read before the products of the current ones are issued.
+template <int K, int NI, int NJ, typename FA, typename FB>
+__device__ __forceinline__ void s_mma(SAcc<NI, NJ>& acc, FA a, FB b, int mi, int nj) {
+  if (mi == 0 || nj == 0) return;
+  double af[2][NI], bf[2][NJ];
+  auto frags = [&](int u, int kk) {
 #pragma unroll
-    for (int kk = 0; kk < kBK; kk += 4) {
-      double af[4], bf[2];
+    for (int i = 0; i < NI; ++i) af[u][i] = a(i, kk);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) af[i] = a(i, kk);
+    for (int j = 0; j < NJ; ++j) bf[u][j] = b(j, kk);
+  };
+  frags(0, 0);
+  if (mi == NI && nj == NJ) {
 #pragma unroll
-      for (int j = 0; j < 2; ++j) bf[j] = b(j, kk);
+    for (int q = 0; q < K / 4; ++q) {
+      if (q + 1 < K / 4) frags((q + 1) & 1, 4 * q + 4);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) dmma(acc.v[i][j], af[i], bf[j]);
+        for (int j = 0; j < NJ; ++j) dmma(acc.v[i][j], af[q & 1][i], bf[q & 1][j]);
     }
-  } else if (mi > 0 && nj > 0) {
+  } else {
 #pragma unroll
-    for (int kk = 0; kk < kBK; kk += 4) {
-      double bf[2];
+    for (int q = 0; q < K / 4; ++q) {
+      if (q + 1 < K / 4) frags((q + 1) & 1, 4 * q + 4);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) bf[j] = b(j, kk);
+      for (int i = 0; i < NI; ++i) {
+        if (i >= mi) break;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i >= mi) continue;
-        const double af = a(i, kk);
-        dmma(acc.v[i][0], af, bf[0]);
-        if (nj > 1) dmma(acc.v[i][1], af, bf[1]);
+        for (int j = 0; j < NJ; ++j)
+          if (j < nj) dmma(acc.v[i][j], af[q & 1][i], bf[q & 1][j]);
       }
     }
   }
 }
 
-// K3 (screened): CTA = (tile, half of its 128 points).  X = phi_t P[S_t, S_t]
-// in 64-wide column blocks, P gathered element-wise by 8-byte cp.async (thread
-// = one column, four rows of a stage); each finished block of X passes through
-// shared memory so that a thread then owns one point: the phi and grad phi it
-// meets are read in whole rows and the sums take 4 registers.
-// tri (GGA = false: only rho, a quadratic form): P is symmetric, so column
-// block J takes the rows of the blocks before it doubled and its own block, half
-// the products.  Grid z selects the operand plane and its sum (the three tau
-// sums of a meta-GGA in one launch).
-// 60 atoms, 304 of 690 functions per tile: X block 64 x 64 per 128 threads at 254 registers (two CTAs, 8 warps per SM)
-// kept the DMMA pipe 62% busy
+// up to three operand planes and their sums, chosen by grid z
 struct SPlanes {
   const double *phi0, *phi1, *phi2;
   double *rho0, *rho1, *rho2;
   __device__ __forceinline__ const double* phi(int z) const { return z == 0 ? phi0 : (z == 1 ? phi1 : phi2); }
   __device__ __forceinline__ double* rho(int z) const { return z == 0 ? rho0 : (z == 1 ? rho1 : rho2); }
 };
-// the tile's slot -> function list in shared memory, -1 past its slots up to whole 64-slot blocks
+// The tile's slot -> function list in shared memory, -1 from its slots to a
+// whole block past them: every index the kernels form is inside it, guarded or
+// not (a guarded shared-memory load may be executed all the same).
 __host__ __device__ constexpr int sfn_len(int n) { return (n + kSBlk - 1) / kSBlk * kSBlk + kSBlk; }
 __device__ __forceinline__ void load_sfn(int* sfn, const int* __restrict__ slot_fn, int n) {
   const int len = sfn_len(n);
   for (int i = threadIdx.x; i < len; i += kSThreads) sfn[i] = i < n ? slot_fn[i] : -1;
 }
+
+// K3 (screened): CTA = (tile, half of its 128 points).  X = phi_t P[S_t, S_t]
+// in 64-wide column blocks, P gathered element-wise by 8-byte cp.async (thread
+// = one column, every second row of a stage); each finished block of X passes
+// through shared memory so that a thread then owns one point: the phi and grad phi it meets are read in whole rows and the sums take
+// 4 registers.
+// tri (GGA = false: only rho, a quadratic form): P is symmetric, so column
+// block J takes the rows of the blocks before it doubled and its own block, half
+// the products.  Grid z selects the operand plane and its sum (the three tau
+// sums of a meta-GGA in one launch).
+// Three CTAs per SM: 60 atoms, 304 of 690 functions per tile (226 GF, 6.4 ms at
+// the pipe's rate) 10.8 -> 8.9 ms against one 128-thread CTA form that kept two
+// CTAs at 254 registers; four CTAs at 128 registers 9.2, 32-deep stages 9.4.
 template <bool GGA>
-__global__ void __launch_bounds__(kSThreads, 2)
+__global__ void __launch_bounds__(kSThreads, 3)
     k_sdensity(SPlanes pl, const double* __restrict__ gx, const double* __restrict__ gy,
                const double* __restrict__ gz, const int64_t* __restrict__ tso, const int* __restrict__ listed,
                int64_t t0, int64_t s0, const int* __restrict__ slot_fn, const double* __restrict__ P, int64_t ldc,
                bool tri, double* __restrict__ grx, double* __restrict__ gry, double* __restrict__ grz) {
   extern __shared__ double smem[];
-  constexpr int E = OpTile<false, kSBlk>::kElems;
+  constexpr int E = kDK * kDLd;  // one operand of a stage
+  static_assert(kSBlk * kXLd <= 2 * kDStages * E, "the X block lies in the stages");
   double* sA = smem;
-  double* sB = smem + kStages * E;
-  double* sX = smem + 2 * kStages * E;
-  int* sfn = reinterpret_cast<int*>(sX + kSBlk * kXLd);
+  double* sB = smem + kDStages * E;
+  double* sX = smem;
+  int* sfn = reinterpret_cast<int*>(smem + 2 * kDStages * E);
   const double* __restrict__ phi = pl.phi(blockIdx.z);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = ((tid >> 5) + blockIdx.x) & 3;
   const int64_t t = t0 + blockIdx.x;
   const int64_t sb = tso[t] - s0;
-  const int n = (int)(tso[t + 1] - tso[t]), nl = listed[t];
+  const int nl = listed[t];
   const int m0 = blockIdx.y * kSBlk;
-  load_sfn(sfn, slot_fn + sb + s0, n);
-  __syncthreads();
+  load_sfn(sfn, slot_fn + sb + s0, (int)(tso[t + 1] - tso[t]));
   const double* A = phi + sb * 128 + m0;
-  const int wm0 = (warp >> 2) * 32, wn0 = (warp & 3) * 16, fr = lane >> 2, fk = lane & 3;
-  const int nslab = (nl + kBK - 1) / kBK, nblk = (nl + kSBlk - 1) / kSBlk;
-  const int col = tid & 63, kq = tid >> 6;  // this thread's column of every gathered stage, rows kq + 4 i
-  // slabs of column block J: all, or (tri) those up to the end of its own block
-  auto slabs = [&](int J) { return tri ? min(nslab, (J + 1) * (kSBlk / kBK)) : nslab; };
-  int lj = 0, lk = 0;     // next stage to load: column block, slab
-  int fcol = sfn[col];
-  auto load = [&](int st) {
-    if (lj >= nblk) return;
-    double* a = sA + st * E;
-    double* b = sB + st * E;
-    const int k0 = lk * kBK;
+  const int wm0 = (warp >> 1) * 32, wn0 = (warp & 1) * 32, fr = lane >> 2, fk = lane & 3;
+  const int nslab = (nl + kDK - 1) / kDK;
+  const int col = tid & 63, kq = tid >> 6;  // this thread's column of every gathered stage, rows kq + 2 i
+  double r = 0.0, g[3] = {0.0, 0.0, 0.0};   // of point m0 + (tid & 63), columns tid >> 6 mod 2
+  for (int n0 = 0; n0 < nl; n0 += kSBlk) {
+    const int ns = tri ? min(nslab, n0 / kDK + kSBlk / kDK) : nslab;
+    __syncthreads();  // sfn written; the X block before this one read
+    const int fcol = sfn[n0 + col];
+    auto load = [&](int it) {
+      double* a = sA + it % kDStages * E;
+      double* b = sB + it % kDStages * E;
+      const int k0 = it * kDK;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int c = tid + i * kSThreads, k = c >> 5, mn = (c & 31) * 2;
-      cp_async16(a + OpTile<false, kSBlk>::idx(mn, k), A + (int64_t)(k0 + k) * 128 + mn);
-    }
+      for (int i = 0; i < kDK / 4; ++i) {
+        const int c = tid + i * kSThreads, k = c >> 5, mn = (c & 31) * 2;
+        cp_async16(a + k * kDLd + mn, A + (int64_t)(k0 + k) * 128 + mn);
+      }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = kq + 4 * i, f = sfn[k0 + k];
-      const bool ok = f >= 0 && fcol >= 0;
-      cp_async8(b + OpTile<false, kSBlk>::idx(col, k), ok ? P + (int64_t)f * ldc + fcol : P, ok);
-    }
-    if (++lk == slabs(lj)) {
-      lk = 0;
-      ++lj;
-      fcol = sfn[lj * kSBlk + col];
-    }
-  };
+      for (int i = 0; i < kDK / 2; ++i) {
+        const int k = kq + 2 * i, f = sfn[k0 + k];
+        const bool ok = f >= 0 && fcol >= 0;
+        cp_async8(b + k * kDLd + col, ok ? P + (int64_t)f * ldc + fcol : P, ok);
+      }
+    };
 #pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) {
-    load(s);
-    cp_async_commit();
-  }
-  double r = 0.0, g[3] = {0.0, 0.0, 0.0};  // of point m0 + (tid & 63), columns tid >> 6 mod 4
-  int st = 0;
-  for (int J = 0; J < nblk; ++J) {
-    const int n0 = J * kSBlk, ns = slabs(J);
-    const int nj = live_frags(n0 + wn0, nl, 2);
-    SAcc acc;
+    for (int s = 0; s < kDStages - 1; ++s) {
+      if (s < ns) load(s);
+      cp_async_commit();
+    }
+    const int nj = live_frags(n0 + wn0, nl, 4);
+    SAcc<4, 4> acc;
     acc.zero();
     for (int it = 0; it < ns; ++it) {
-      cp_async_wait<kStages - 2>();
+      cp_async_wait<kDStages - 2>();
       __syncthreads();
-      load(st >= 1 ? st - 1 : kStages - 1);  // the stage consumed before this one
+      if (it + kDStages - 1 < ns) load(it + kDStages - 1);
       cp_async_commit();
-      if (tri && it * kBK == n0)  // the blocks before J count twice
+      if (tri && it * kDK == n0) {  // the blocks before this one count twice
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
+          for (int j = 0; j < 4; ++j) {
             acc.v[i][j][0] *= 2.0;
             acc.v[i][j][1] *= 2.0;
           }
-      const double* a_s = sA + st * E + wm0 + fr + fk * (kSBlk + kPadMN);
-      const double* b_s = sB + st * E + wn0 + fr + fk * (kSBlk + kPadMN);
-      s_mma(acc, [&](int i, int kk) { return a_s[i * 8 + kk * (kSBlk + kPadMN)]; },
-            [&](int j, int kk) { return b_s[j * 8 + kk * (kSBlk + kPadMN)]; }, 4, nj);
-      st = st == kStages - 1 ? 0 : st + 1;
+      }
+      const double* a_s = sA + it % kDStages * E + wm0 + fr + fk * kDLd;
+      const double* b_s = sB + it % kDStages * E + wn0 + fr + fk * kDLd;
+      s_mma<kDK>(acc, [&](int i, int kk) { return a_s[i * 8 + kk * kDLd]; },
+                 [&](int j, int kk) { return b_s[j * 8 + kk * kDLd]; }, 4, nj);
     }
+    cp_async_wait<0>();
+    __syncthreads();  // the stages are read: X takes their place
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int e = 0; e < 2; ++e)
           sX[(wn0 + j * 8 + 2 * fk + e) * kXLd + wm0 + i * 8 + fr] = acc.v[i][j][e];
     __syncthreads();
-    const int p = tid & 63, cn = min(kSBlk, nl - n0);
-    const int64_t o0 = (sb + n0) * 128 + m0 + p;
+    const int cn = min(kSBlk, nl - n0);
+    const int64_t o0 = (sb + n0) * 128 + m0 + col;
 #pragma unroll 4
-    for (int c = tid >> 6; c < cn; c += 4) {
-      const double x = sX[c * kXLd + p];
+    for (int c = kq; c < cn; c += 2) {
+      const double x = sX[c * kXLd + col];
       const int64_t o = o0 + c * 128;
       r += x * phi[o];
       if (GGA) {
@@ -305,80 +313,78 @@ __global__ void __launch_bounds__(kSThreads, 2)
         g[2] += x * gz[o];
       }
     }
-    // sX is next written after a further barrier of the stage loop
   }
-  cp_async_wait<0>();
   __syncthreads();
-  double* red = smem;  // [4 quantities][4 column groups][64 points]
+  double* red = smem;  // [4 quantities][2 column groups][64 points]
   red[tid] = r;
-  if (GGA)
+  if (GGA) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) red[(q + 1) * kSThreads + tid] = g[q];
+  }
   __syncthreads();
-  const int q = tid >> 6, p = tid & 63;
-  if (q > 0 && !GGA) return;
-  const double* rq = red + q * kSThreads + p;
-  const double v = (rq[0] + rq[64]) + (rq[128] + rq[192]);
-  double* out = q == 0 ? pl.rho(blockIdx.z) : (q == 1 ? grx : (q == 2 ? gry : grz));
-  out[(int64_t)blockIdx.x * 128 + m0 + p] = q == 0 ? v : 2.0 * v;
+  for (int q = kq; q < (GGA ? 4 : 1); q += 2) {
+    const double v = red[q * kSThreads + col] + red[q * kSThreads + 64 + col];
+    double* out = q == 0 ? pl.rho(blockIdx.z) : (q == 1 ? grx : (q == 2 ? gry : grz));
+    out[(int64_t)blockIdx.x * 128 + m0 + col] = q == 0 ? v : 2.0 * v;
+  }
 }
 constexpr int sdensity_smem(int max_n) {
-  return (2 * kStages * OpTile<false, kSBlk>::kElems + kSBlk * kXLd) * 8 + 4 * sfn_len(max_n);
+  return 2 * kDStages * kDK * kDLd * 8 + 4 * sfn_len(max_n);
 }
 
 // K4 (screened): H[fn_i][fn_j] += sum_p Z[i][p] phi[j][p] for the slots i, j of
-// one tile, Z = A phi (+ B . grad phi).  CTA = (tile, 64 slots i): it forms its
-// block of Z in shared memory once (the whole K = 128 points) and streams the
-// tile's phi against it.  A separate pass that wrote Z for the contraction to
-// read took 2.4 ms of the 60-atom build's 25.
+// one tile, Z = A phi (+ B . grad phi).  CTA = (tile, 32 slots i): it forms its
+// rows of Z in shared memory once (the whole K = 128 points) and streams the
+// tile's phi against them, each warp its own blocks of 32 slots j through stages
+// of its own: no barrier after Z.  A tile's CTAs follow one another in the grid,
+// so that its phi comes from L2.  A separate pass that wrote Z
+// for the contraction to read took 2.4 ms of the 60-atom build's 25.
 // kFull: the whole square (GGA: V = H + H^T in k_spack).  kUpper: fn_i <= fn_j
 // only (LDA: H is symmetric).  kTwice: the upper triangle with the off-diagonal
 // elements doubled: the symmetric tau term of a meta-GGA, which k_spack's H + H^T
 // then counts as the whole square does; grid z selects its plane.
-// 60 atoms, 304 of 690 functions per tile: three 128-thread CTAs kept the DMMA pipe 85% busy but a third of it on padding
+// 60 atoms, 304 of 690 functions per tile: 11.1 -> 8.4 ms with the Z pass (8.7
+// the contraction alone, a third of it on padding).
 enum { kFull, kUpper, kTwice };
 template <int MODE, bool GRAD>
-__global__ void __launch_bounds__(kSThreads, 2)
+__global__ void __launch_bounds__(kSThreads, 3)
     k_svpot(SPlanes pl, const double* __restrict__ gx, const double* __restrict__ gy, const double* __restrict__ gz,
             const double* __restrict__ A, const double* __restrict__ Bx, const double* __restrict__ By,
             const double* __restrict__ Bz, const int64_t* __restrict__ tso, const int* __restrict__ listed, int64_t t0,
-            int64_t s0, const int* __restrict__ slot_fn, double* __restrict__ V, int64_t ldv) {
+            int64_t s0, const int* __restrict__ slot_fn, double* __restrict__ V, int64_t ldv, unsigned nI) {
   extern __shared__ double smem[];
-  constexpr int E = OpTile<true, kSBlk>::kElems;
-  const int64_t t = t0 + blockIdx.x;
-  const int nl = listed[t], I0 = blockIdx.y * kSBlk;
+  constexpr int E = OpTile<true, kRows>::kElems;
+  const unsigned tile = blockIdx.x / nI;
+  const int64_t t = t0 + tile;
+  const int nl = listed[t], I0 = (int)(blockIdx.x - tile * nI) * kRows;
   if (I0 >= nl) return;
   double* sZ = smem;
-  double* sF = smem + kSBlk * kZLd;
-  int* sfn = reinterpret_cast<int*>(sF + kStages * E);
+  int* sfn = reinterpret_cast<int*>(smem + kRows * kZLd + 4 * kSStages * E);
   const double* __restrict__ phi = pl.phi(blockIdx.z);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = ((tid >> 5) + tile) & 3;
   const int64_t sb = tso[t] - s0;
   const double* F = phi + sb * 128;
-  const int J0 = MODE == kFull ? 0 : blockIdx.y, nJ = (nl + kSBlk - 1) / kSBlk;
-  int lj = J0, lk = 0;  // next stage to load: 64-slot block, slab of 16 points
-  auto load = [&](int st) {
-    if (lj >= nJ) return;
+  // The warp's run: blocks of 32 slots j (every fourth of the tile's), 8 stages
+  // of 16 points each, streamed through stages of its own.
+  double* sF = smem + kRows * kZLd + warp * (kSStages * E);
+  int lj = (MODE == kFull ? 0 : I0) + warp * kRows, lk = 0;  // the next stage to load
+  auto load = [&]() {
+    if (lj < nl) {
+      const double* src = F + (int64_t)(lj + (lane >> 3)) * 128 + lk * kBK + (lane & 7) * 2;
+      double* dst = sF + (lk & 1) * E + OpTile<true, kRows>::idx(lane >> 3, (lane & 7) * 2);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int c = tid + i * kSThreads, row = c >> 3, k = (c & 7) * 2;
-      cp_async16(sF + st * E + OpTile<true, kSBlk>::idx(row, k), F + (int64_t)(lj * kSBlk + row) * 128 + lk * kBK + k);
+      for (int i = 0; i < 8; ++i) cp_async16(dst + 4 * i * (kBK + kPadK), src + 4 * i * 128);
     }
+    cp_async_commit();
     if (++lk == 128 / kBK) {
       lk = 0;
-      ++lj;
+      lj += 4 * kRows;
     }
   };
-#pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) {
-    load(s);
-    cp_async_commit();
-  }
+  load();
   load_sfn(sfn, slot_fn + sb + s0, (int)(tso[t + 1] - tso[t]));
   {
-    // Z rows tid >> 7, + 2, ...; this thread's point is tid & 127 throughout
-    const int p = tid & 127;
-    const int64_t pt = (int64_t)blockIdx.x * 128 + p;
+    const int64_t pt = (int64_t)tile * 128 + tid;  // thread = point
     const double a = A[pt];
     double b[3] = {0.0, 0.0, 0.0};
     if (GRAD) {
@@ -386,58 +392,54 @@ __global__ void __launch_bounds__(kSThreads, 2)
       b[1] = By[pt];
       b[2] = Bz[pt];
     }
-    const int nz = min(kSBlk, nl - I0);
 #pragma unroll 8
-    for (int i = tid >> 7; i < kSBlk; i += 2) {
-      double z = 0.0;
-      if (i < nz) {
-        const int64_t o = (sb + I0 + i) * 128 + p;
-        z = a * phi[o];
-        if (GRAD) z += b[0] * gx[o] + b[1] * gy[o] + b[2] * gz[o];
-      }
-      sZ[i * kZLd + p] = z;
+    for (int i = 0; i < kRows; ++i) {  // rows past the listed functions are the tile's zero padding
+      const int64_t o = (sb + I0 + i) * 128 + tid;
+      double z = a * phi[o];
+      if (GRAD) z += b[0] * gx[o] + b[1] * gy[o] + b[2] * gz[o];
+      sZ[i * kZLd + tid] = z;
     }
   }
-  const int wm0 = (warp >> 2) * 32, wn0 = (warp & 3) * 16, fr = lane >> 2, fk = lane & 3;
-  const int nj = live_frags(I0 + wn0, nl, 2);
-  int st = 0;
-  for (int J = J0; J < nJ; ++J) {
-    const int j0 = J * kSBlk + wm0;
-    // rows j of the fragment, columns i: a warp's atomics run along rows of V
-    const int mi = MODE != kFull && j0 + 31 < I0 + wn0 ? 0 : live_frags(j0, nl, 4);
-    SAcc acc;
+  __syncthreads();  // Z and sfn; the warps run on their own from here
+  const int fr = lane >> 2, fk = lane & 3;
+  const int nj = live_frags(I0, nl, 4);
+  // rows of the fragments are slots j, so that a warp's atomics run along rows of V
+  for (int j0 = (MODE == kFull ? 0 : I0) + warp * kRows; j0 < nl; j0 += 4 * kRows) {
+    const int mi = live_frags(j0, nl, 4);
+    SAcc<4, 4> acc;
     acc.zero();
+#pragma unroll 2
     for (int it = 0; it < 128 / kBK; ++it) {
-      cp_async_wait<kStages - 2>();
-      __syncthreads();
-      load(st >= 1 ? st - 1 : kStages - 1);
-      cp_async_commit();
-      const double* f_s = sF + st * E + (wm0 + fr) * (kBK + kPadK) + fk;
-      const double* z_s = sZ + (wn0 + fr) * kZLd + it * kBK + fk;
-      s_mma(acc, [&](int i, int kk) { return f_s[i * 8 * (kBK + kPadK) + kk]; },
+      cp_async_wait<0>();
+      __syncwarp();
+      load();  // into the stage read before this one
+      const double* f_s = sF + (it & 1) * E + fr * (kBK + kPadK) + fk;
+      const double* z_s = sZ + fr * kZLd + it * kBK + fk;
+      s_mma<kBK>(acc, [&](int i, int kk) { return f_s[i * 8 * (kBK + kPadK) + kk]; },
             [&](int j, int kk) { return z_s[j * 8 * kZLd + kk]; }, mi, nj);
-      st = st == kStages - 1 ? 0 : st + 1;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int j = j0 + i * 8 + fr;
-      const int fj = sfn[j];  // -1 past the listed functions
-      if (i >= mi || fj < 0) continue;
+      if (i >= mi) break;
+      const int fj = sfn[j0 + i * 8 + fr];  // -1 past the listed functions
+      if (fj < 0) continue;
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+      for (int c = 0; c < 4; ++c) {
+        if (c >= nj) break;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int fi = sfn[I0 + wn0 + c * 8 + 2 * fk + e];
+          const int fi = sfn[I0 + c * 8 + 2 * fk + e];
           if (fi < 0) continue;
           double v = acc.v[i][c][e];
           if (MODE == kTwice && fj != fi) v *= 2.0;
           if (MODE == kFull || fj >= fi) atomicAdd(V + (int64_t)fi * ldv + fj, v);
         }
+      }
     }
   }
 }
 constexpr int svpot_smem(int max_n) {
-  return (kSBlk * kZLd + kStages * OpTile<true, kSBlk>::kElems) * 8 + 4 * sfn_len(max_n);
+  return (kRows * kZLd + 4 * kSStages * OpTile<true, kRows>::kElems) * 8 + 4 * sfn_len(max_n);
 }
 
 }  // namespace
@@ -973,18 +975,19 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
                                                st, k0, k1);
       } else {
         const int smem = svpot_smem(sp->max_n);
-        const dim3 grid((unsigned)nt, (unsigned)((sp->max_n + kSBlk - 1) / kSBlk));
+        const unsigned nI = (unsigned)((sp->max_n + kRows - 1) / kRows);
+        const dim3 grid((unsigned)nt * nI);
         const SPlanes pl{phi, phi, phi, nullptr, nullptr, nullptr};
         if (timed) SR_TRY(cudaEventRecord(k0, st));
         if (gga) {
           raise_smem_limit(k_svpot<kFull, true>, smem);
           k_svpot<kFull, true><<<grid, kSThreads, smem, st>>>(pl, gxc, gyc, gzc, b[s].A, b[s].Bx, b[s].By, b[s].Bz,
-                                                              sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas);
+                                                              sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas, nI);
         } else {
           raise_smem_limit(k_svpot<kUpper, false>, smem);
           k_svpot<kUpper, false><<<grid, kSThreads, smem, st>>>(pl, nullptr, nullptr, nullptr, b[s].A, nullptr, nullptr,
                                                                 nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs,
-                                                                sp->nbas);
+                                                                sp->nbas, nI);
         }
         if (timed) SR_TRY(cudaEventRecord(k1, st));
         ++T.launches;
@@ -995,9 +998,10 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         const int smem = svpot_smem(sp->max_n);
         raise_smem_limit(k_svpot<kTwice, false>, smem);
         const SPlanes pl{gxc, gyc, gzc, nullptr, nullptr, nullptr};
-        k_svpot<kTwice, false><<<dim3((unsigned)nt, (unsigned)((sp->max_n + kSBlk - 1) / kSBlk), 3), kSThreads, smem,
+        const unsigned nI = (unsigned)((sp->max_n + kRows - 1) / kRows);
+        k_svpot<kTwice, false><<<dim3((unsigned)nt * nI, 1, 3), kSThreads, smem,
                                  st>>>(pl, nullptr, nullptr, nullptr, sp->tq + (4 * s + 3) * cp, nullptr, nullptr,
-                                       nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas);
+                                       nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas, nI);
         ++T.launches;
       }
     }
