@@ -119,9 +119,10 @@ int check_device(pgxc_ctx* c, int want) {
     if (cudaGetDevice(&dev) != cudaSuccess) return set_err(c, PGXC_ENODEV, "cudaGetDevice failed");
   }
   if (dev >= n) return set_err(c, PGXC_EINVAL, "device ordinal out of range");
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return set_err(c, PGXC_ENODEV, "device query failed");
-  if (prop.major != 10) return set_err(c, PGXC_ENODEV, "libpgxc is built for sm_100a (B200) only");
+  int major = 0;
+  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess)
+    return set_err(c, PGXC_ENODEV, "device query failed");
+  if (major != 10) return set_err(c, PGXC_ENODEV, "libpgxc is built for sm_100a (B200) only");
   if (c) c->device = dev;
   return PGXC_OK;
 }

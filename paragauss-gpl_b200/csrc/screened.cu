@@ -89,6 +89,102 @@ __global__ void __launch_bounds__(128) k_tile_atom_d2(const double* __restrict__
   }
 }
 
+// The listing of a tile: shell s has the radial functions whose squared listing
+// radius r2[s][rr] exceeds the tile's smallest squared distance to its atom.
+__device__ __forceinline__ unsigned long long plan_mask(const DevShell& S, double dd, const double* __restrict__ r2) {
+  unsigned long long m = 0;
+  for (int rr = 0; rr < S.nrad; ++rr)
+    if (dd < r2[rr]) m |= 1ull << rr;
+  return m;
+}
+
+// cnt[t] = {listed functions, basis items of l = 0..3} of tile t (block per tile)
+__global__ void __launch_bounds__(128) k_plan_count(const float* __restrict__ d2, int natm,
+                                                    const DevShell* __restrict__ shells, int nsh,
+                                                    const double* __restrict__ r2, const int* __restrict__ r2off,
+                                                    int* __restrict__ cnt) {
+  __shared__ int sum[1 + kMaxL + 1];
+  const int64_t t = blockIdx.x;
+  if (threadIdx.x < 2 + kMaxL) sum[threadIdx.x] = 0;
+  __syncthreads();
+  for (int s = threadIdx.x; s < nsh; s += 128) {
+    const DevShell S = shells[s];
+    const int n = __popcll(plan_mask(S, d2[t * natm + S.atom], r2 + r2off[s]));
+    if (!n) continue;
+    atomicAdd(&sum[0], n * (2 * S.l + 1));
+    atomicAdd(&sum[1 + S.l], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 + kMaxL) cnt[t * (2 + kMaxL) + threadIdx.x] = sum[threadIdx.x];
+}
+
+struct PlanItems {
+  BasisItem* items[kMaxL + 1];
+};
+// The slot list (shell by shell: independent function -> radial function, then
+// padding) and the basis items of every tile, in shell order: 128 shells at a
+// time, their places by a block scan.  start[t] = {first item of l = 0..3}.
+__global__ void __launch_bounds__(128) k_plan_fill(const float* __restrict__ d2, int natm,
+                                                   const double* __restrict__ atoms,
+                                                   const DevShell* __restrict__ shells, int nsh,
+                                                   const double* __restrict__ r2, const int* __restrict__ r2off,
+                                                   const int64_t* __restrict__ tso, const int64_t* __restrict__ start,
+                                                   int* __restrict__ slot_fn, PlanItems out) {
+  __shared__ int scan_n[128];
+  __shared__ unsigned scan_l[128];  // four 8-bit counts (at most 128 shells each)
+  const int64_t t = blockIdx.x;
+  const int tid = threadIdx.x;
+  int64_t slot0 = tso[t], item0[kMaxL + 1];
+  for (int l = 0; l <= kMaxL; ++l) item0[l] = start[t * (kMaxL + 1) + l];
+  for (int s0 = 0; s0 < nsh; s0 += 128) {
+    const int s = s0 + tid;
+    DevShell S{};
+    unsigned long long mask = 0;
+    if (s < nsh) {
+      S = shells[s];
+      mask = plan_mask(S, d2[t * natm + S.atom], r2 + r2off[s]);
+    }
+    const int nsig = __popcll(mask), n = nsig * (2 * S.l + 1);
+    const unsigned one = nsig ? 1u << (8 * S.l) : 0u;
+    scan_n[tid] = n;
+    scan_l[tid] = one;
+    __syncthreads();
+    for (int o = 1; o < 128; o <<= 1) {
+      const int vn = tid >= o ? scan_n[tid - o] : 0;
+      const unsigned vl = tid >= o ? scan_l[tid - o] : 0u;
+      __syncthreads();
+      scan_n[tid] += vn;
+      scan_l[tid] += vl;
+      __syncthreads();
+    }
+    if (nsig) {
+      const int64_t slot = slot0 + scan_n[tid] - n;
+      BasisItem it{};
+      it.ax = atoms[3 * S.atom];
+      it.ay = atoms[3 * S.atom + 1];
+      it.az = atoms[3 * S.atom + 2];
+      it.tile = (int)t;
+      it.slot = slot;
+      it.nsig = nsig;
+      it.mask = mask;
+      it.exp_off = S.exp_off;
+      it.con_off = S.con_off;
+      it.rad_off = S.rad_off;
+      it.nexp = S.nexp;
+      it.nunc = S.nunc;
+      it.seg = S.seg;
+      out.items[S.l][item0[S.l] + ((scan_l[tid] - one) >> (8 * S.l) & 255u)] = it;
+      int64_t o = slot;
+      for (int i = 0; i < 2 * S.l + 1; ++i)
+        for (unsigned long long m = mask; m; m &= m - 1) slot_fn[o++] = S.f0 + i * S.nrad + __ffsll((long long)m) - 1;
+    }
+    slot0 += scan_n[127];
+    for (int l = 0; l <= kMaxL; ++l) item0[l] += scan_l[127] >> (8 * l) & 255u;
+    __syncthreads();
+  }
+  for (int64_t o = slot0 + tid; o < tso[t + 1]; o += 128) slot_fn[o] = -1;
+}
+
 // ---------------------------------------------------------------------------
 // FP64 kernels
 // ---------------------------------------------------------------------------
@@ -498,7 +594,20 @@ double listing_r2(const DevShell& S, int rr, const double* exps, const double* n
   const double rcut = std::sqrt(r2cut);
   const int nstep = 4000;
   const double dr = rcut / nstep;
-  for (int i = nstep; i >= 0; --i) {
+  // every term exp(-a r^2) r^k, k <= l + 1, falls for r >= sqrt((l + 1) / (2 a)): from the smallest
+  // exponent's radius on the bound falls, and its last step at or above the threshold is found by halving
+  int hi = std::min(nstep, (int)std::ceil(std::sqrt((l + 1) / (2.0 * amin)) / dr));
+  if (bound(hi * dr) >= threshold) {
+    int lo = hi;
+    hi = nstep + 1;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) / 2;
+      (bound(mid * dr) >= threshold ? lo : hi) = mid;
+    }
+    const double R = std::min(rcut, lo * dr + dr);
+    return R * R;
+  }
+  for (int i = hi - 1; i >= 0; --i) {
     const double r = i * dr;
     if (bound(r) >= threshold) {
       const double R = std::min(rcut, r + dr);
@@ -593,17 +702,6 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     cudaFree(dperm);
     SP_TRY(e, "grid reordering");
   }
-  // --- tile-atom distances ------------------------------------------------
-  std::vector<float> d2((size_t)ntiles * in.natm);
-  {
-    float* dd2;
-    SP_TRY(cudaMalloc(&dd2, sizeof(float) * d2.size()), "cudaMalloc");
-    k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, in.natm, dd2);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = cudaMemcpy(d2.data(), dd2, sizeof(float) * d2.size(), cudaMemcpyDeviceToHost);
-    cudaFree(dd2);
-    SP_TRY(e, "tile distances");
-  }
   // --- listing radii -------------------------------------------------------
   double sa_fac[kMaxL + 1];
   for (int l = 0; l <= kMaxL; ++l) {
@@ -616,67 +714,84 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
       }
   }
   const int nsh = (int)shells.size();
-  std::vector<std::vector<double>> R2((size_t)nsh);
-  std::vector<double> shR2((size_t)nsh, 0.0);
+  std::vector<double> R2;
+  std::vector<int> r2off((size_t)nsh);
   for (int s = 0; s < nsh; ++s) {
     const DevShell& S = shells[(size_t)s];
-    R2[(size_t)s].resize((size_t)S.nrad);
-    for (int rr = 0; rr < S.nrad; ++rr) {
-      R2[(size_t)s][(size_t)rr] = listing_r2(S, rr, in.exps, in.norms, in.contr, in.threshold, sa_fac[S.l]);
-      shR2[(size_t)s] = std::max(shR2[(size_t)s], R2[(size_t)s][(size_t)rr]);
-    }
+    r2off[(size_t)s] = (int)R2.size();
+    for (int rr = 0; rr < S.nrad; ++rr)
+      R2.push_back(listing_r2(S, rr, in.exps, in.norms, in.contr, in.threshold, sa_fac[S.l]));
   }
-  // --- per-tile lists --------------------------------------------------------
+  // --- per-tile lists, on the device: distances, counts, then (their places known) the lists.  On the
+  // host the lists of a 41-atom grid (2,710 tiles, 170,000 items of 80 bytes, copied from pageable
+  // memory) were most of the 30 ms of a context's creation.
   std::vector<int64_t> tso((size_t)ntiles + 1, 0);
-  std::vector<int> slot_fn, listed_t((size_t)ntiles, 0);
-  std::vector<BasisItem> items[kMaxL + 1];
-  std::vector<int64_t> tile_items[kMaxL + 1];  // items before tile t, per L
-  for (int l = 0; l <= kMaxL; ++l) tile_items[l].assign((size_t)ntiles + 1, 0);
-  slot_fn.reserve((size_t)ntiles * 64);
-  for (int64_t t = 0; t < ntiles; ++t) {
-    const int64_t base = (int64_t)slot_fn.size();
-    for (int l = 0; l <= kMaxL; ++l) tile_items[l][(size_t)t] = (int64_t)items[l].size();
-    for (int s = 0; s < nsh; ++s) {
-      const DevShell& S = shells[(size_t)s];
-      const double dd = d2[(size_t)t * in.natm + S.atom];
-      if (!(dd < shR2[(size_t)s])) continue;
-      uint64_t mask = 0;
-      for (int rr = 0; rr < S.nrad; ++rr)
-        if (dd < R2[(size_t)s][(size_t)rr]) mask |= 1ull << rr;
-      const int nsig = __builtin_popcountll(mask);
-      BasisItem it{};
-      it.ax = in.atoms[3 * S.atom];
-      it.ay = in.atoms[3 * S.atom + 1];
-      it.az = in.atoms[3 * S.atom + 2];
-      it.tile = (int)t;
-      it.slot = (int64_t)slot_fn.size();
-      it.nsig = nsig;
-      it.mask = mask;
-      it.exp_off = S.exp_off;
-      it.con_off = S.con_off;
-      it.rad_off = S.rad_off;
-      it.nexp = S.nexp;
-      it.nunc = S.nunc;
-      it.seg = S.seg;
-      items[S.l].push_back(it);
-      for (int i = 0; i < 2 * S.l + 1; ++i)
-        for (int rr = 0; rr < S.nrad; ++rr)
-          if (mask >> rr & 1) slot_fn.push_back(S.f0 + i * S.nrad + rr);
-    }
-    const int64_t listed = (int64_t)slot_fn.size() - base;
-    listed_t[(size_t)t] = (int)listed;
-    sp->nlisted += listed;
-    while (((int64_t)slot_fn.size() - base) % kSlotAlign) slot_fn.push_back(-1);
-    const int64_t nt = (int64_t)slot_fn.size() - base;
-    sp->sum_n2 += (double)listed * (double)listed;
-    sp->max_n = std::max(sp->max_n, (int)nt);
-    tso[(size_t)t + 1] = (int64_t)slot_fn.size();
+  std::vector<int> listed_t((size_t)ntiles, 0);
+  {
+    constexpr int kCnt = 2 + kMaxL;
+    float* dd2 = nullptr;
+    double* dR2 = nullptr;
+    int *dr2off = nullptr, *dcnt = nullptr;
+    int64_t* dstart = nullptr;
+    std::vector<int> cnt((size_t)ntiles * kCnt);
+    std::vector<int64_t> start((size_t)ntiles * (kMaxL + 1));
+    auto plan = [&]() -> cudaError_t {
+#define PL_TRY(call)                      \
+  do {                                    \
+    cudaError_t e_ = (call);              \
+    if (e_ != cudaSuccess) return e_;     \
+  } while (0)
+      // one scratch allocation for the five tables
+      const size_t n8 = (size_t)ntiles * (kMaxL + 1) + std::max<size_t>(R2.size(), 1);
+      const size_t n4 = (size_t)ntiles * in.natm + (size_t)ntiles * kCnt + (size_t)nsh;
+      PL_TRY(cudaMalloc(&dstart, 8 * n8 + 4 * n4));
+      dR2 = (double*)(dstart + (size_t)ntiles * (kMaxL + 1));
+      dd2 = (float*)(dstart + n8);
+      dcnt = (int*)(dd2 + (size_t)ntiles * in.natm);
+      dr2off = dcnt + (size_t)ntiles * kCnt;
+      PL_TRY(cudaMemcpyAsync(dR2, R2.data(), sizeof(double) * R2.size(), cudaMemcpyHostToDevice, st));
+      PL_TRY(cudaMemcpyAsync(dr2off, r2off.data(), sizeof(int) * r2off.size(), cudaMemcpyHostToDevice, st));
+      k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, in.natm, dd2);
+      k_plan_count<<<(unsigned)ntiles, 128, 0, st>>>(dd2, in.natm, a.shells, nsh, dR2, dr2off, dcnt);
+      PL_TRY(cudaGetLastError());
+      PL_TRY(cudaMemcpyAsync(cnt.data(), dcnt, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, st));
+      PL_TRY(cudaStreamSynchronize(st));
+      int64_t items[kMaxL + 1] = {};
+      for (int l = 0; l <= kMaxL; ++l) sp->tile_item[l].assign((size_t)ntiles + 1, 0);
+      for (int64_t t = 0; t < ntiles; ++t) {
+        const int* c = &cnt[(size_t)t * kCnt];
+        listed_t[(size_t)t] = c[0];
+        const int nt = (c[0] + kSlotAlign - 1) / kSlotAlign * kSlotAlign;
+        sp->nlisted += c[0];
+        sp->sum_n2 += (double)c[0] * (double)c[0];
+        sp->max_n = std::max(sp->max_n, nt);
+        tso[(size_t)t + 1] = tso[(size_t)t] + nt;
+        for (int l = 0; l <= kMaxL; ++l) {
+          start[(size_t)t * (kMaxL + 1) + l] = items[l];
+          items[l] += c[1 + l];
+          sp->tile_item[l][(size_t)t + 1] = items[l];
+        }
+      }
+      sp->nslots = tso[(size_t)ntiles];
+      PL_TRY(sp_alloc(sp, &sp->tso, tso.size()));
+      PL_TRY(sp_alloc(sp, &sp->listed, listed_t.size()));
+      PL_TRY(sp_alloc(sp, &sp->slot_fn, (size_t)sp->nslots));
+      for (int l = 0; l <= kMaxL; ++l) PL_TRY(sp_alloc(sp, &sp->items[l], (size_t)items[l]));
+      PL_TRY(cudaMemcpyAsync(sp->tso, tso.data(), sizeof(int64_t) * tso.size(), cudaMemcpyHostToDevice, st));
+      PL_TRY(cudaMemcpyAsync(sp->listed, listed_t.data(), sizeof(int) * listed_t.size(), cudaMemcpyHostToDevice, st));
+      PL_TRY(cudaMemcpyAsync(dstart, start.data(), sizeof(int64_t) * start.size(), cudaMemcpyHostToDevice, st));
+      PlanItems out{};
+      for (int l = 0; l <= kMaxL; ++l) out.items[l] = sp->items[l];
+      k_plan_fill<<<(unsigned)ntiles, 128, 0, st>>>(dd2, in.natm, a.atoms, a.shells, nsh, dR2, dr2off, sp->tso, dstart,
+                                                    sp->slot_fn, out);
+      PL_TRY(cudaGetLastError());
+      return cudaStreamSynchronize(st);
+#undef PL_TRY
+    };
+    const cudaError_t e = plan();
+    cudaFree(dstart);
+    SP_TRY(e, "tile lists");
   }
-  for (int l = 0; l <= kMaxL; ++l) {
-    tile_items[l][(size_t)ntiles] = (int64_t)items[l].size();
-    sp->tile_item[l] = tile_items[l];
-  }
-  sp->nslots = (int64_t)slot_fn.size();
   sp->h_tso = tso;
   // --- chunks -------------------------------------------------------------------
   const bool mixed = in.precision != PGXC_PREC_FP64;
@@ -733,48 +848,33 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     chunk_bstages = std::max(chunk_bstages, boff[(size_t)t1] - boff[(size_t)t0]);
   }
   for (int l = 0; l <= kMaxL; ++l)
-    for (size_t c = 0; c <= nch; ++c) sp->item_off[l].push_back(tile_items[l][(size_t)sp->chunk_t0[c]]);
-  // --- device copies and buffers ------------------------------------------------
-  SP_TRY(sp_alloc(sp, &sp->tso, tso.size()), "cudaMalloc");
-  SP_TRY(cudaMemcpy(sp->tso, tso.data(), sizeof(int64_t) * tso.size(), cudaMemcpyHostToDevice), "copy");
-  SP_TRY(sp_alloc(sp, &sp->listed, listed_t.size()), "cudaMalloc");
-  SP_TRY(cudaMemcpy(sp->listed, listed_t.data(), sizeof(int) * listed_t.size(), cudaMemcpyHostToDevice), "copy");
-  SP_TRY(sp_alloc(sp, &sp->slot_fn, slot_fn.size()), "cudaMalloc");
-  if (!slot_fn.empty()) {
-    SP_TRY(cudaMemcpy(sp->slot_fn, slot_fn.data(), sizeof(int) * slot_fn.size(), cudaMemcpyHostToDevice), "copy");
-  }
-  for (int l = 0; l <= kMaxL; ++l) {
-    SP_TRY(sp_alloc(sp, &sp->items[l], items[l].size()), "cudaMalloc");
-    if (!items[l].empty())
-      SP_TRY(cudaMemcpy(sp->items[l], items[l].data(), sizeof(BasisItem) * items[l].size(), cudaMemcpyHostToDevice),
-             "copy");
-  }
+    for (size_t c = 0; c <= nch; ++c) sp->item_off[l].push_back(sp->tile_item[l][(size_t)sp->chunk_t0[c]]);
+  // --- buffers ------------------------------------------------------------------
   const size_t rows = (size_t)(sp->chunk_slots + kSlack) * 128;
   // basis arrays: one chunk's rows, or every slot of the grid when they stay resident
   const size_t brows = sp->keep ? (size_t)(sp->nslots + kSlack) * 128 : rows;
-  SP_TRY(sp_alloc(sp, &sp->phi, brows), "cudaMalloc (phi)");
-  SP_TRY(cudaMemset(sp->phi, 0, sizeof(double) * brows), "memset");
+  // (padding slots are zeroed by every evaluation; the rows after the last slot are read by whole-block copies)
+  auto plane = [&](auto** p) -> cudaError_t {
+    cudaError_t e = sp_alloc(sp, p, brows);
+    if (e == cudaSuccess) e = cudaMemsetAsync(*p + (brows - kSlack * 128), 0, sizeof(**p) * kSlack * 128, st);
+    return e;
+  };
+  SP_TRY(plane(&sp->phi), "cudaMalloc (phi)");
   if (in.gga && sp->gf32) {
-    SP_TRY(sp_alloc(sp, &sp->fx, brows), "cudaMalloc (grad phi)");
-    SP_TRY(sp_alloc(sp, &sp->fy, brows), "cudaMalloc (grad phi)");
-    SP_TRY(sp_alloc(sp, &sp->fz, brows), "cudaMalloc (grad phi)");
-    SP_TRY(cudaMemset(sp->fx, 0, sizeof(float) * brows), "memset");
-    SP_TRY(cudaMemset(sp->fy, 0, sizeof(float) * brows), "memset");
-    SP_TRY(cudaMemset(sp->fz, 0, sizeof(float) * brows), "memset");
+    SP_TRY(plane(&sp->fx), "cudaMalloc (grad phi)");
+    SP_TRY(plane(&sp->fy), "cudaMalloc (grad phi)");
+    SP_TRY(plane(&sp->fz), "cudaMalloc (grad phi)");
   } else if (in.gga) {
-    SP_TRY(sp_alloc(sp, &sp->gx, brows), "cudaMalloc (grad phi)");
-    SP_TRY(sp_alloc(sp, &sp->gy, brows), "cudaMalloc (grad phi)");
-    SP_TRY(sp_alloc(sp, &sp->gz, brows), "cudaMalloc (grad phi)");
-    SP_TRY(cudaMemset(sp->gx, 0, sizeof(double) * brows), "memset");
-    SP_TRY(cudaMemset(sp->gy, 0, sizeof(double) * brows), "memset");
-    SP_TRY(cudaMemset(sp->gz, 0, sizeof(double) * brows), "memset");
+    SP_TRY(plane(&sp->gx), "cudaMalloc (grad phi)");
+    SP_TRY(plane(&sp->gy), "cudaMalloc (grad phi)");
+    SP_TRY(plane(&sp->gz), "cudaMalloc (grad phi)");
   }
   const int64_t cp = sp->chunk_tiles * 128;
   SP_TRY(sp_alloc(sp, &sp->pt, 8 * (size_t)in.ispin * cp), "cudaMalloc");
-  SP_TRY(cudaMemset(sp->pt, 0, sizeof(double) * 8 * in.ispin * cp), "memset");
+  SP_TRY(cudaMemsetAsync(sp->pt, 0, sizeof(double) * 8 * in.ispin * cp, st), "memset");
   if (in.mgga) {
     SP_TRY(sp_alloc(sp, &sp->tq, 4 * (size_t)in.ispin * cp), "cudaMalloc");
-    SP_TRY(cudaMemset(sp->tq, 0, sizeof(double) * 4 * in.ispin * cp), "memset");
+    SP_TRY(cudaMemsetAsync(sp->tq, 0, sizeof(double) * 4 * in.ispin * cp, st), "memset");
   }
   SP_TRY(sp_alloc(sp, &sp->partial, 2 * (size_t)((cp + 255) / 256) + 2), "cudaMalloc");
   SP_TRY(sp_alloc(sp, &sp->V, (size_t)in.ispin * in.nbas * in.nbas), "cudaMalloc (V)");

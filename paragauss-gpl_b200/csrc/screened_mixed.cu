@@ -909,10 +909,12 @@ int screen_mixed_create(ScreenMixed** out, const ScreenMixedInput& in, std::stri
   if (e == cudaSuccess) e = sm_alloc(m, &m->ps, (size_t)in.chunk_slots);
   if (e == cudaSuccess) e = sm_alloc(m, &m->err, 1);
   // the slack rows after a chunk's last slot are read (never used) by whole-block copies
-  if (e == cudaSuccess) e = cudaMemset(m->tA, 0, dig_a);
-  if (e == cudaSuccess) e = cudaMemset(m->tZ, 0, dig);
-  if (e == cudaSuccess) e = cudaMemset(m->tF, 0, dig);
+  const size_t slack = (size_t)std::min<int64_t>(in.chunk_slots, 128) * kDigBytesPerSlot;
+  if (e == cudaSuccess) e = cudaMemset(m->tA + dig_a - slack, 0, slack);
+  if (e == cudaSuccess) e = cudaMemset(m->tZ + dig - slack, 0, slack);
+  if (e == cudaSuccess) e = cudaMemset(m->tF + dig - slack, 0, slack);
   if (e == cudaSuccess) e = cudaMemset(m->err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) {
     err = std::string("screened mixed-precision buffers: ") + cudaGetErrorString(e);
     screen_mixed_destroy(m);

@@ -210,7 +210,8 @@ def i32p(a):
 class Marshalled:
     """Keeps the numpy buffers alive while the C structs point into them."""
 
-    def __init__(self, case, weighted=True):
+    def __init__(self, case, weighted=True, grid=True):
+        """grid: marshal the host grid too (not needed where the library builds it)."""
         self._keep = []
         c = case
         coords = np.ascontiguousarray(c.coords, dtype=np.float64).reshape(-1)
@@ -224,11 +225,12 @@ class Marshalled:
         self._keep += arrs + flt + [sa]
         self.basis = Basis(len(c.shell_l), *[i32p(a) for a in arrs], *[f64p(a) for a in flt],
                            f64p(sa), int(c.sa_lmax))
-        w = c.grid_w if (weighted and c.grid_w is not None) else c.grid_wraw
+        self.weights_are_raw = raw = 0 if (weighted and c.grid_w is not None) else 1
+        if not grid:
+            return
+        w = c.grid_wraw if raw else c.grid_w
         grd = np.concatenate([c.grid_xyz[:, 0], c.grid_xyz[:, 1], c.grid_xyz[:, 2], w])
         grd = np.ascontiguousarray(grd, dtype=np.float64)
         pa = np.ascontiguousarray(c.point_atom, dtype=np.int32)
         self._keep += [grd, pa]
-        raw = 0 if (weighted and c.grid_w is not None) else 1
         self.grid = Grid(len(w), f64p(grd), raw, i32p(pa))
-        self.weights_are_raw = raw

@@ -92,7 +92,7 @@ class Context:
         device (pgxc_create_on_grid) instead of passing the host grid."""
         L = lib()
         self.case = case
-        self._m = abi.Marshalled(case, weighted=weighted)
+        self._m = abi.Marshalled(case, weighted=weighted, grid=not on_grid)
         o = abi.Options()
         L.pgxc_default_options(ct.byref(o))
         o.functional = abi.XC_IDS[case.functional]
