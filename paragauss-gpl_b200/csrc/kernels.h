@@ -45,7 +45,7 @@ struct BuildArgs {
   double* Bx = nullptr;
   double* By = nullptr;
   double* Bz = nullptr;
-  double* partial = nullptr;  // 2 per functional block
+  double* partial = nullptr;  // 2 per functional block, then a counter (0 between launches)
   double* acc = nullptr;      // {E, cE, N, cN}
   // density matrix
   int64_t ldc = 0;            // nbas padded to 64
@@ -53,6 +53,8 @@ struct BuildArgs {
   double* Cocc = nullptr;
   const double* occ = nullptr;
   double* P = nullptr;        // [ldc][ldc]
+  bool cleared = false;       // acc and the plan's potential matrix are already 0
+  double* exc_nel = nullptr;  // device {E_xc, N_el} written by the packing, when not null
   bool p_symmetric = true;    // P formed here from C; false: the caller's P, which nothing checks
   // potential tiles
   int nt = 0;                 // ldc / 64
@@ -71,6 +73,11 @@ void launch_basis(const BuildArgs& a, const double* px, const double* py, const 
 void launch_basis_points_f64(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t n,
                              int64_t ld, double* phi, double* gx, double* gy, double* gz, cudaStream_t st);
 void launch_pmat_f64(const BuildArgs& a, int64_t kpad, cudaStream_t st);
+// P from Cocc and C already padded and scaled
+void launch_pmat_scaled(const BuildArgs& a, int64_t kpad, cudaStream_t st);
+// P from unpadded device orbitals C (nbas x nocc) and occ; z0[n0] and z1[n1] are cleared in the same launch
+void launch_pmat_raw(const BuildArgs& a, const double* C, const double* occ, int64_t nbas, int nocc, int64_t kpad,
+                     double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st);
 void launch_density_f64(const BuildArgs& a, bool gga, cudaStream_t st);
 void launch_functional_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool gga, cudaStream_t st);
 // the functional on ntiles whole 128-point tiles, one partial pair per tile (no reduction)

@@ -15,6 +15,7 @@
 // The density is formed from P rather than from the occupied orbitals as the
 // reference does (density_calc_nl, modules/density_calc_module.f90:1447-1576);
 // the two are equal, P = C diag(occ) C^T, up to rounding.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -64,6 +65,25 @@ void launch_basis_points_f64(const BuildArgs& a, const double* px, const double*
 // ---------------------------------------------------------------------------
 // Density matrix: Cocc[j][mu] = occ_j C[j][mu];  P = sum_j C[j][mu] Cocc[j][nu]
 // ---------------------------------------------------------------------------
+// The caller's orbitals (nbas x nocc, column-major) and occupations into the
+// padded rows C[j][mu] and Cocc[j][mu] = occ_j C[j][mu] (zero past nocc and
+// nbas), and two accumulators cleared: one launch for what were two clears, a
+// strided copy, a copy and the scaling.
+__global__ void k_load_orbitals(const double* __restrict__ C, const double* __restrict__ occ, int64_t nbas, int nocc,
+                                int64_t ldc, int64_t kpad, double* __restrict__ Cp, double* __restrict__ Cocc,
+                                double* __restrict__ z0, int64_t n0, double* __restrict__ z1, int64_t n1) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = first; i < ldc * kpad; i += step) {
+    const int64_t j = i / ldc, mu = i - j * ldc;
+    const bool in = j < nocc && mu < nbas;
+    const double c = in ? C[j * nbas + mu] : 0.0;
+    Cp[i] = c;
+    Cocc[i] = in ? c * occ[j] : 0.0;
+  }
+  for (int64_t i = first; i < n0; i += step) z0[i] = 0.0;
+  for (int64_t i = first; i < n1; i += step) z1[i] = 0.0;
+}
+
 __global__ void k_scale_occ(const double* __restrict__ C, const double* __restrict__ occ, int64_t ldc, int nocc,
                             double* __restrict__ Cocc) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -96,8 +116,20 @@ __global__ void __launch_bounds__(kGemmThreads) k_pmat(const double* __restrict_
 void launch_pmat_f64(const BuildArgs& a, int64_t kpad, cudaStream_t st) {
   const int64_t n = a.ldc * kpad;
   k_scale_occ<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a.C, a.occ, a.ldc, (int)kpad, a.Cocc);
+  launch_pmat_scaled(a, kpad, st);
+}
+
+void launch_pmat_raw(const BuildArgs& a, const double* C, const double* occ, int64_t nbas, int nocc, int64_t kpad,
+                     double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st) {
+  const int64_t n = std::max(a.ldc * kpad, n0);
+  const unsigned nb = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8);
+  k_load_orbitals<<<nb, 256, 0, st>>>(C, occ, nbas, nocc, a.ldc, kpad, a.C, a.Cocc, z0, n0, z1, n1);
+  launch_pmat_scaled(a, kpad, st);
+}
+
+void launch_pmat_scaled(const BuildArgs& a, int64_t kpad, cudaStream_t st) {
   constexpr int smem = gemm_smem_bytes<false, false>();
-  cudaFuncSetAttribute(k_pmat, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  raise_smem_limit(k_pmat, smem);
   dim3 grid((unsigned)(a.ldc / 64), (unsigned)(a.ldc / 64));
   k_pmat<<<grid, kGemmThreads, smem, st>>>(a.C, a.Cocc, a.ldc, kpad, a.P);
 }
@@ -191,13 +223,69 @@ void launch_density_f64(const BuildArgs& a, bool gga, cudaStream_t st) {
 // w*f and w*rho (exc_int, charge_int).  rho is clamped at 0: in P form it can
 // round to tiny negative values where the reference's sum of squares is +0.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void kahan_add(double* acc, double e, double q) {
+  const double vals[2] = {e, q};
+  for (int k = 0; k < 2; ++k) {
+    const double y = vals[k] - acc[2 * k + 1];
+    const double t = acc[2 * k] + y;
+    acc[2 * k + 1] = (t - acc[2 * k]) - y;
+    acc[2 * k] = t;
+  }
+}
+
+// fixed-order block sum of (e, q) into se[0], sq[0] (deterministic; blockDim a power of two <= 256)
+__device__ __forceinline__ void block_sum2(double* se, double* sq, double e, double q) {
+  se[threadIdx.x] = e;
+  sq[threadIdx.x] = q;
+  __syncthreads();
+  for (int s = blockDim.x >> 1; s > 0; s >>= 1) {
+    if (threadIdx.x < s) {
+      se[threadIdx.x] += se[threadIdx.x + s];
+      sq[threadIdx.x] += sq[threadIdx.x + s];
+    }
+    __syncthreads();
+  }
+}
+
+// The block's sums of w f and w rho into its partials; with acc, the last
+// block to finish (a counter behind the partials, left at 0) sums all partials
+// in their fixed order and Kahan-adds them into acc[4] = {E, cE, N, cN}: the
+// sums of k_sum_partials without a launch of their own.
+__device__ __forceinline__ void sum_points(double e, double q, double* partial, double* acc) {
+  __shared__ double se[256], sq[256];
+  __shared__ bool last;
+  block_sum2(se, sq, e, q);
+  if (threadIdx.x == 0) {
+    partial[2 * blockIdx.x] = se[0];
+    partial[2 * blockIdx.x + 1] = sq[0];
+    if (acc) {
+      __threadfence();
+      unsigned* done = reinterpret_cast<unsigned*>(partial + 2 * gridDim.x);
+      last = atomicAdd(done, 1u) == gridDim.x - 1;
+      if (last) *done = 0;
+    }
+  }
+  if (!acc) return;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  e = q = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+    e += __ldcg(partial + 2 * i);
+    q += __ldcg(partial + 2 * i + 1);
+  }
+  __syncthreads();
+  block_sum2(se, sq, e, q);
+  if (threadIdx.x == 0) kahan_add(acc, se[0], sq[0]);
+}
+
 template <bool GGA>
 __global__ void __launch_bounds__(256) k_functional(XcConst K, int64_t p0, int64_t nvalid, int64_t n, const double* __restrict__ w,
                                                     const double* __restrict__ rho, const double* __restrict__ grx,
                                                     const double* __restrict__ gry, const double* __restrict__ grz,
                                                     double* __restrict__ A, double* __restrict__ Bx,
                                                     double* __restrict__ By, double* __restrict__ Bz,
-                                                    double* __restrict__ partial) {
+                                                    double* partial, double* acc) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double e = 0.0, q = 0.0;
   if (p < n) {
@@ -222,22 +310,7 @@ __global__ void __launch_bounds__(256) k_functional(XcConst K, int64_t p0, int64
     }
     q = r * wt;
   }
-  // fixed-order block reduction (deterministic; blockDim a power of two <= 256)
-  __shared__ double se[256], sq[256];
-  se[threadIdx.x] = e;
-  sq[threadIdx.x] = q;
-  __syncthreads();
-  for (int s = blockDim.x >> 1; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      se[threadIdx.x] += se[threadIdx.x + s];
-      sq[threadIdx.x] += sq[threadIdx.x + s];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    partial[2 * blockIdx.x] = se[0];
-    partial[2 * blockIdx.x + 1] = sq[0];
-  }
+  sum_points(e, q, partial, acc);
 }
 
 // Sum the block partials in a fixed order and Kahan-add them into acc[4]
@@ -249,25 +322,8 @@ __global__ void k_sum_partials(const double* __restrict__ partial, int nblocks, 
     e += partial[2 * i];
     q += partial[2 * i + 1];
   }
-  se[threadIdx.x] = e;
-  sq[threadIdx.x] = q;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      se[threadIdx.x] += se[threadIdx.x + s];
-      sq[threadIdx.x] += sq[threadIdx.x + s];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double vals[2] = {se[0], sq[0]};
-    for (int k = 0; k < 2; ++k) {
-      const double y = vals[k] - acc[2 * k + 1];
-      const double t = acc[2 * k] + y;
-      acc[2 * k + 1] = (t - acc[2 * k]) - y;
-      acc[2 * k] = t;
-    }
-  }
+  block_sum2(se, sq, e, q);
+  if (threadIdx.x == 0) kahan_add(acc, se[0], sq[0]);
 }
 
 // Open shell (ispin = 2).  pa / pb hold the point arrays of spin a / b, each
@@ -279,7 +335,7 @@ template <bool GGA>
 __global__ void __launch_bounds__(256) k_functional2(XcConst K, int64_t p0, int64_t nvalid, int64_t n,
                                                      const double* __restrict__ w, double* __restrict__ pa,
                                                      double* __restrict__ pb, int64_t ld,
-                                                     double* __restrict__ partial) {
+                                                     double* partial, double* acc) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double e = 0.0, q = 0.0;
   if (p < n) {
@@ -311,21 +367,7 @@ __global__ void __launch_bounds__(256) k_functional2(XcConst K, int64_t p0, int6
     e = f * wt;
     q = (rho[0] + rho[1]) * wt;
   }
-  __shared__ double se[256], sq[256];
-  se[threadIdx.x] = e;
-  sq[threadIdx.x] = q;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      se[threadIdx.x] += se[threadIdx.x + s];
-      sq[threadIdx.x] += sq[threadIdx.x + s];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    partial[2 * blockIdx.x] = se[0];
-    partial[2 * blockIdx.x + 1] = sq[0];
-  }
+  sum_points(e, q, partial, acc);
 }
 
 void launch_sum_partials(const double* partial, int nblocks, double* acc, cudaStream_t st) {
@@ -335,20 +377,18 @@ void launch_sum_partials(const double* partial, int nblocks, double* acc, cudaSt
 void launch_functional2_f64(const XcConst& K, const double* w, double* pa, double* pb, int64_t ld, int64_t p0,
                             int64_t nvalid, bool gga, double* partial, double* acc, cudaStream_t st) {
   const unsigned nb = (unsigned)((ld + 255) / 256);
-  if (gga) k_functional2<true><<<nb, 256, 0, st>>>(K, p0, nvalid, ld, w, pa, pb, ld, partial);
-  else k_functional2<false><<<nb, 256, 0, st>>>(K, p0, nvalid, ld, w, pa, pb, ld, partial);
-  k_sum_partials<<<1, 256, 0, st>>>(partial, (int)nb, acc);
+  if (gga) k_functional2<true><<<nb, 256, 0, st>>>(K, p0, nvalid, ld, w, pa, pb, ld, partial, acc);
+  else k_functional2<false><<<nb, 256, 0, st>>>(K, p0, nvalid, ld, w, pa, pb, ld, partial, acc);
 }
 
 void launch_functional_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool gga, cudaStream_t st) {
   const unsigned nb = (unsigned)((a.ldp + 255) / 256);
   if (gga)
     k_functional<true><<<nb, 256, 0, st>>>(a.xc, p0, nvalid, a.ldp, a.w, a.rho, a.grx, a.gry, a.grz, a.A, a.Bx, a.By,
-                                           a.Bz, a.partial);
+                                           a.Bz, a.partial, a.acc);
   else
     k_functional<false><<<nb, 256, 0, st>>>(a.xc, p0, nvalid, a.ldp, a.w, a.rho, nullptr, nullptr, nullptr, a.A, nullptr,
-                                            nullptr, nullptr, a.partial);
-  k_sum_partials<<<1, 256, 0, st>>>(a.partial, (int)nb, a.acc);
+                                            nullptr, nullptr, a.partial, a.acc);
 }
 
 // One block per 128-point tile of a set's chunk: partial[2 t], partial[2 t + 1]
@@ -357,10 +397,10 @@ void launch_functional_tiles(const BuildArgs& a, int64_t p0, int64_t ntiles, boo
   const int64_t n = ntiles * 128;
   if (gga)
     k_functional<true><<<(unsigned)ntiles, 128, 0, st>>>(a.xc, p0, n, n, a.w, a.rho, a.grx, a.gry, a.grz, a.A, a.Bx,
-                                                         a.By, a.Bz, a.partial);
+                                                         a.By, a.Bz, a.partial, nullptr);
   else
     k_functional<false><<<(unsigned)ntiles, 128, 0, st>>>(a.xc, p0, n, n, a.w, a.rho, nullptr, nullptr, nullptr, a.A,
-                                                          nullptr, nullptr, nullptr, a.partial);
+                                                          nullptr, nullptr, nullptr, a.partial, nullptr);
 }
 
 // ---------------------------------------------------------------------------

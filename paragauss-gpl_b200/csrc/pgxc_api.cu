@@ -47,7 +47,7 @@ struct SymPlan {
 struct pgxc_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
-  cudaEvent_t ev[8] = {};
+  cudaEvent_t ev[9] = {};
   cudaEvent_t kev[4] = {};
   std::string err;
   pgxc_options opt;
@@ -72,6 +72,8 @@ struct pgxc_ctx {
   MixedState* mixed = nullptr;  // tensor-core mixed-precision path (dense)
   ScreenPlan* screen = nullptr; // screened (tile-sparse) build, when screen_threshold >= 0
   SymPlan* sym = nullptr;       // symmetry adaptation, when set
+  double* d_raw = nullptr;      // host builds' orbitals and occupations as the caller passed them
+  int64_t raw_cap = 0;
   double* d_eacc = nullptr;     // {E, cE, N, cN} per functional of pgxc_xc_energies
   void* grad_scr = nullptr;     // scratch of pgxc_xc_gradient, kept across calls (grows only)
   size_t grad_scr_bytes = 0;
@@ -127,10 +129,16 @@ int check_device(pgxc_ctx* c, int want) {
   return PGXC_OK;
 }
 
+// no NaN or infinity (exponent bits not all ones), without an early exit: the loop vectorises
 bool all_finite(const double* p, int64_t n) {
-  for (int64_t i = 0; i < n; ++i)
-    if (!std::isfinite(p[i])) return false;
-  return true;
+  constexpr uint64_t kExp = 0x7ff0000000000000ull;
+  uint64_t bad = 0;
+  for (int64_t i = 0; i < n; ++i) {
+    uint64_t u;
+    std::memcpy(&u, p + i, 8);
+    bad |= (uint64_t)((u & kExp) == kExp);
+  }
+  return bad == 0;
 }
 
 // A device copy of a host vector (a context allocation).
@@ -492,8 +500,8 @@ int create_impl(const pgxc_geometry* geo, const pgxc_basis* bas, const pgxc_grid
     // accumulators and the packed matrix are shared with the dense layout
     if ((st = dalloc(c, &a.acc, 4)) || (st = dalloc(c, &a.P, (size_t)a.ldc * a.ldc))) return fail(st);
     if (o.ispin == 2 && (st = dalloc(c, &c->P2, (size_t)a.ldc * a.ldc))) return fail(st);
-    if ((st = dalloc(c, &c->d_ham, (size_t)o.ispin * c->nbas * (c->nbas + 1) / 2))) return fail(st);
-    CUDA_TRY(c, cudaMallocHost(&c->h_ham, sizeof(double) * o.ispin * c->nbas * (c->nbas + 1) / 2));
+    if ((st = dalloc(c, &c->d_ham, (size_t)o.ispin * c->nbas * (c->nbas + 1) / 2 + 2))) return fail(st);
+    CUDA_TRY(c, cudaMallocHost(&c->h_ham, sizeof(double) * (o.ispin * c->nbas * (c->nbas + 1) / 2 + 2)));
     CUDA_TRY(c, cudaMallocHost(&c->h_acc, sizeof(double) * 4));
     ScreenInput in;
     in.shells = &c->shells;
@@ -558,8 +566,9 @@ int create_impl(const pgxc_geometry* geo, const pgxc_basis* bas, const pgxc_grid
   if ((st = dalloc(c, &pp, 8 * (size_t)chunk))) return fail(st);
   a.rho = pp; a.grx = pp + chunk; a.gry = pp + 2 * chunk; a.grz = pp + 3 * chunk;
   a.A = pp + 4 * chunk; a.Bx = pp + 5 * chunk; a.By = pp + 6 * chunk; a.Bz = pp + 7 * chunk;
-  if ((st = dalloc(c, &a.partial, 2 * (size_t)((chunk + 255) / 256) + 2)) || (st = dalloc(c, &a.acc, 4)))
-    return fail(st);
+  const size_t npart = 2 * (size_t)((chunk + 255) / 256);
+  if ((st = dalloc(c, &a.partial, npart + 2)) || (st = dalloc(c, &a.acc, 4))) return fail(st);
+  CUDA_TRY(c, cudaMemsetAsync(a.partial + npart, 0, 2 * sizeof(double), c->stream));
   if ((st = dalloc(c, &a.P, (size_t)a.ldc * a.ldc))) return fail(st);
   // potential tiles: upper triangle of 64x64 tiles, split over points
   {
@@ -581,8 +590,8 @@ int create_impl(const pgxc_geometry* geo, const pgxc_basis* bas, const pgxc_grid
   a.nsplit = ns64;
   a.kspan = chunk / ns64;
   if ((st = dalloc(c, &a.vpart, (size_t)a.nsplit * a.ntiles * kTile * kTile))) return fail(st);
-  if ((st = dalloc(c, &c->d_ham, (size_t)o.ispin * c->nbas * (c->nbas + 1) / 2))) return fail(st);
-  CUDA_TRY(c, cudaMallocHost(&c->h_ham, sizeof(double) * o.ispin * c->nbas * (c->nbas + 1) / 2));
+  if ((st = dalloc(c, &c->d_ham, (size_t)o.ispin * c->nbas * (c->nbas + 1) / 2 + 2))) return fail(st);
+  CUDA_TRY(c, cudaMallocHost(&c->h_ham, sizeof(double) * (o.ispin * c->nbas * (c->nbas + 1) / 2 + 2)));
   CUDA_TRY(c, cudaMallocHost(&c->h_acc, sizeof(double) * 4));
   if (o.precision != PGXC_PREC_FP64) {
     st = mixed_create(&c->mixed, a, c->nbas, gga, o.precision, c->err);
@@ -672,41 +681,44 @@ static int upload_orbitals(pgxc_ctx* c, const double* C, const double* occ, int3
 
 // The device part of a build; C / occ already in a.C / a.occ (padded).
 // p_given: the density matrices are already in a.P (and P2), written by the caller's P.
-static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given = false) {
+// rawC, rawocc (screened contexts): device orbitals as the caller passes them
+// (nbas x nocc per spin, nocc per spin), read in place of a.C / a.occ.  ham,
+// exc_nel: device outputs (the packed matrix, and {E_xc, N_el} unless null).
+// A screened build is only enqueued (finish_build completes it).
+static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given, const double* rawC, const double* rawocc,
+                     double* ham, double* exc_nel) {
   BuildArgs& a = c->a;
   cudaStream_t s = c->stream;
   const bool gga = PGXC_XC_IS_GGA(c->opt.functional);
   const int64_t kpad = round_up(std::max(nocc, 1), 16);
   if (c->screen) {
-    CUDA_TRY(c, cudaMemsetAsync(a.acc, 0, 4 * sizeof(double), s));
     CUDA_TRY(c, cudaEventRecord(c->ev[1], s));
-    if (!p_given) launch_pmat_f64(a, kpad, s);
-    if (c->opt.ispin == 2 && !p_given) {
-      BuildArgs b = a;  // second spin: its orbitals and occupations into P2 (Cocc is scratch)
-      b.C = c->C2;
-      b.occ = c->occ2;
-      b.P = c->P2;
-      launch_pmat_f64(b, kpad, s);
-    }
-    CUDA_TRY(c, cudaGetLastError());
-    CUDA_TRY(c, cudaEventRecord(c->ev[2], s));
-    ScreenTimes T;
-    std::string e;
     BuildArgs as = a;
     as.p_symmetric = !p_given;
-    const int st = screen_run(c->screen, as, c->P2, s, c->d_ham, &T, e);
-    if (st) return set_err(c, st, e);
-    float ms = 0;
-    CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev[1], c->ev[2]));
-    if (tm) {
-      tm->basis_ms = T.basis;
-      tm->density_ms = T.density + ms;
-      tm->functional_ms = T.functional;
-      tm->potential_ms = T.potential;
-      tm->xgemm_ms = T.x;
-      tm->vgemm_ms = T.v;
-      tm->kernel_launches = T.launches + (p_given ? 0 : 2 * c->opt.ispin);
+    as.cleared = rawC != nullptr;
+    as.exc_nel = exc_nel;
+    int64_t nv = 0;
+    double* V = screen_potential(c->screen, &nv);
+    if (!as.cleared) CUDA_TRY(c, cudaMemsetAsync(a.acc, 0, 4 * sizeof(double), s));
+    for (int sp = 0; sp < c->opt.ispin && !p_given; ++sp) {
+      BuildArgs b = a;
+      if (sp) {  // second spin: its orbitals and occupations into P2 (Cocc is scratch)
+        b.C = c->C2;
+        b.occ = c->occ2;
+        b.P = c->P2;
+      }
+      if (rawC)
+        launch_pmat_raw(b, rawC + (size_t)sp * c->nbas * nocc, rawocc + (size_t)sp * nocc, c->nbas, nocc, kpad, V,
+                        sp ? 0 : nv, a.acc, sp ? 0 : 4, s);
+      else
+        launch_pmat_f64(b, kpad, s);
     }
+    CUDA_TRY(c, cudaGetLastError());
+    ScreenTimes T;
+    std::string e;
+    const int st = screen_run(c->screen, as, c->P2, s, ham, &T, e);
+    if (st) return set_err(c, st, e);
+    tm->kernel_launches = T.launches + (p_given ? 0 : 2 * c->opt.ispin);
     return PGXC_OK;
   }
   float t_basis = 0, t_dens = 0, t_func = 0, t_pot = 0, t_x = 0, t_v = 0;
@@ -784,6 +796,41 @@ static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given = fal
   return PGXC_OK;
 }
 
+// Complete a run_build: for a screened context wait for it, read its phase
+// times and error flag (a dense build is already complete).
+static int finish_build(pgxc_ctx* c, pgxc_timings* tm) {
+  if (!c->screen) return PGXC_OK;
+  ScreenTimes T;
+  std::string e;
+  const int st = screen_finish(c->screen, c->stream, c->ev[1], &T, e);
+  if (st) return set_err(c, st, e);
+  tm->basis_ms = T.basis;
+  tm->density_ms = T.density;
+  tm->functional_ms = T.functional;
+  tm->potential_ms = T.potential;
+  tm->xgemm_ms = T.x;
+  tm->vgemm_ms = T.v;
+  return PGXC_OK;
+}
+
+// Device copy of host orbitals and occupations as the caller holds them (one
+// buffer: C of both spins, then occ of both), grown when nocc grows.
+static int stage_orbitals(pgxc_ctx* c, const double* C, const double* occ, int32_t nbas, int32_t nocc, double** dC,
+                          double** docc) {
+  const int64_t nC = (int64_t)c->opt.ispin * nbas * nocc, no = (int64_t)c->opt.ispin * nocc;
+  if (nC + no > c->raw_cap || !c->d_raw) {
+    if (int st = dalloc(c, &c->d_raw, (size_t)(nC + no))) return st;
+    c->raw_cap = nC + no;
+  }
+  *dC = c->d_raw;
+  *docc = c->d_raw + nC;
+  if (nocc > 0) {
+    CUDA_TRY(c, cudaMemcpyAsync(*dC, C, sizeof(double) * nC, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(*docc, occ, sizeof(double) * no, cudaMemcpyHostToDevice, c->stream));
+  }
+  return PGXC_OK;
+}
+
 static int check_build_args(pgxc_ctx* c, int32_t nbas, int32_t nocc, int32_t ispin, int64_t xc_length) {
   if (nbas != c->nbas) return set_err(c, PGXC_EINVAL, "nbas does not match the context's basis");
   if (ispin != c->opt.ispin) return set_err(c, PGXC_EINVAL, "ispin does not match the context");
@@ -793,8 +840,8 @@ static int check_build_args(pgxc_ctx* c, int32_t nbas, int32_t nocc, int32_t isp
   return PGXC_OK;
 }
 
-static int host_build_tail(pgxc_ctx* c, int nocc, bool p_given, double* ham, int64_t xc_length, double* exc,
-                           double* nel, pgxc_timings* tm);
+static int host_build_tail(pgxc_ctx* c, int nocc, bool p_given, const double* rawC, const double* rawocc, double* ham,
+                           int64_t xc_length, double* exc, double* nel, pgxc_timings* tm);
 
 int pgxc_build(pgxc_ctx* c, const double* C, const double* occ, int32_t nbas, int32_t nocc, int32_t ispin,
                double* ham, int64_t xc_length, double* exc, double* nel, pgxc_timings* tm) {
@@ -808,39 +855,45 @@ int pgxc_build(pgxc_ctx* c, const double* C, const double* occ, int32_t nbas, in
   if ((st = ensure_occ(c, nocc))) return st;
   const int64_t kpad = round_up(std::max(nocc, 1), 16);
   CUDA_TRY(c, cudaEventRecord(c->ev[0], c->stream));
-  if ((st = upload_orbitals(c, C, occ, nbas, nocc, kpad, cudaMemcpyHostToDevice))) return st;
-  return host_build_tail(c, nocc, false, ham, xc_length, exc, nel, tm);
+  double *rawC = nullptr, *rawocc = nullptr;
+  if (c->screen) st = stage_orbitals(c, C, occ, nbas, nocc, &rawC, &rawocc);
+  else st = upload_orbitals(c, C, occ, nbas, nocc, kpad, cudaMemcpyHostToDevice);
+  if (st) return st;
+  return host_build_tail(c, nocc, false, rawC, rawocc, ham, xc_length, exc, nel, tm);
 }
 
 // The rest of a host-buffer build whose inputs were enqueued after c->ev[0]:
 // the device build, the D2H of the packed matrix and of the two sums, added
 // into the caller's arrays.
-static int host_build_tail(pgxc_ctx* c, int nocc, bool p_given, double* ham, int64_t xc_length, double* exc,
-                           double* nel, pgxc_timings* tm) {
-  BuildArgs& a = c->a;
+static int host_build_tail(pgxc_ctx* c, int nocc, bool p_given, const double* rawC, const double* rawocc, double* ham,
+                           int64_t xc_length, double* exc, double* nel, pgxc_timings* tm) {
   cudaStream_t s = c->stream;
   int st;
-  CUDA_TRY(c, cudaEventRecord(c->ev[1], s));
-  CUDA_TRY(c, cudaEventSynchronize(c->ev[1]));
-  float h2d = 0;
-  CUDA_TRY(c, cudaEventElapsedTime(&h2d, c->ev[0], c->ev[1]));
+  cudaEvent_t up = c->ev[8], e0 = c->ev[5], e1 = c->ev[6];
+  if (!c->screen) CUDA_TRY(c, cudaEventRecord(up, s));  // (a screened build records ev[1] at the same place)
+  else up = c->ev[1];
   pgxc_timings local{};
-  if ((st = run_build(c, nocc, &local, p_given))) return st;
-  // D2H of the packed matrix and the two sums
-  cudaEvent_t e0 = c->ev[5], e1 = c->ev[6];
+  if ((st = run_build(c, nocc, &local, p_given, rawC, rawocc, c->d_ham, c->d_ham + xc_length))) return st;
+  if (!c->screen) {
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_ham + xc_length, c->a.acc, sizeof(double), cudaMemcpyDeviceToDevice, s));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_ham + xc_length + 1, c->a.acc + 2, sizeof(double), cudaMemcpyDeviceToDevice, s));
+  }
+  // D2H of the packed matrix and the two sums behind it
   CUDA_TRY(c, cudaEventRecord(e0, s));
-  CUDA_TRY(c, cudaMemcpyAsync(c->h_ham, c->d_ham, sizeof(double) * xc_length, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(c, cudaMemcpyAsync(c->h_acc, a.acc, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(c, cudaMemcpyAsync(c->h_ham, c->d_ham, sizeof(double) * (xc_length + 2), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(c, cudaEventRecord(e1, s));
   CUDA_TRY(c, cudaEventSynchronize(e1));
-  float d2h = 0, tot = 0;
+  if ((st = finish_build(c, &local))) return st;
+  const double* sums = c->h_ham + xc_length;
+  float h2d = 0, d2h = 0, tot = 0;
+  CUDA_TRY(c, cudaEventElapsedTime(&h2d, c->ev[0], up));
   CUDA_TRY(c, cudaEventElapsedTime(&d2h, e0, e1));
   CUDA_TRY(c, cudaEventElapsedTime(&tot, c->ev[0], e1));
-  if (!std::isfinite(c->h_acc[0]) || !std::isfinite(c->h_acc[2]))
+  if (!std::isfinite(sums[0]) || !std::isfinite(sums[1]))
     return set_err(c, PGXC_ENONFINITE, "non-finite E_xc or N_el");
   for (int64_t i = 0; i < xc_length; ++i) ham[i] += c->h_ham[i];
-  *exc += c->h_acc[0];
-  *nel += c->h_acc[2];
+  *exc += sums[0];
+  *nel += sums[1];
   if (tm) {
     *tm = local;
     tm->h2d_ms = h2d;
@@ -867,7 +920,7 @@ int pgxc_build_density(pgxc_ctx* c, const double* P, int32_t nbas, int32_t ispin
     CUDA_TRY(c, cudaMemcpy2DAsync(dP, sizeof(double) * a.ldc, P + (size_t)sp * nbas * nbas, sizeof(double) * nbas,
                                   sizeof(double) * nbas, nbas, cudaMemcpyHostToDevice, s));
   }
-  return host_build_tail(c, 0, true, ham, xc_length, exc, nel, tm);
+  return host_build_tail(c, 0, true, nullptr, nullptr, ham, xc_length, exc, nel, tm);
 }
 
 int pgxc_build_device(pgxc_ctx* c, const double* d_C, const double* d_occ, int32_t nbas, int32_t nocc, int32_t ispin,
@@ -882,16 +935,23 @@ int pgxc_build_device(pgxc_ctx* c, const double* d_C, const double* d_occ, int32
   cudaStream_t s = c->stream;
   const int64_t kpad = round_up(std::max(nocc, 1), 16);
   CUDA_TRY(c, cudaEventRecord(c->ev[0], s));
-  if ((st = upload_orbitals(c, d_C, d_occ, nbas, nocc, kpad, cudaMemcpyDeviceToDevice))) return st;
   pgxc_timings local{};
-  if ((st = run_build(c, nocc, &local))) return st;
-  CUDA_TRY(c, cudaMemcpyAsync(d_ham, c->d_ham, sizeof(double) * xc_length, cudaMemcpyDeviceToDevice, s));
-  CUDA_TRY(c, cudaMemcpyAsync(d_exc_nel, a.acc, sizeof(double), cudaMemcpyDeviceToDevice, s));
-  CUDA_TRY(c, cudaMemcpyAsync(d_exc_nel + 1, a.acc + 2, sizeof(double), cudaMemcpyDeviceToDevice, s));
-  CUDA_TRY(c, cudaEventRecord(c->ev[1], s));
-  CUDA_TRY(c, cudaEventSynchronize(c->ev[1]));
+  if (c->screen) {
+    // the operands are read, and the outputs written, in place (nocc = 0: no orbital is read)
+    if ((st = run_build(c, nocc, &local, false, nocc > 0 ? d_C : a.C, nocc > 0 ? d_occ : a.occ, d_ham, d_exc_nel)))
+      return st;
+  } else {
+    if ((st = upload_orbitals(c, d_C, d_occ, nbas, nocc, kpad, cudaMemcpyDeviceToDevice))) return st;
+    if ((st = run_build(c, nocc, &local, false, nullptr, nullptr, nullptr, nullptr))) return st;
+    CUDA_TRY(c, cudaMemcpyAsync(d_ham, c->d_ham, sizeof(double) * xc_length, cudaMemcpyDeviceToDevice, s));
+    CUDA_TRY(c, cudaMemcpyAsync(d_exc_nel, a.acc, sizeof(double), cudaMemcpyDeviceToDevice, s));
+    CUDA_TRY(c, cudaMemcpyAsync(d_exc_nel + 1, a.acc + 2, sizeof(double), cudaMemcpyDeviceToDevice, s));
+  }
+  CUDA_TRY(c, cudaEventRecord(c->ev[6], s));
+  CUDA_TRY(c, cudaEventSynchronize(c->ev[6]));
+  if ((st = finish_build(c, &local))) return st;
   float tot = 0;
-  CUDA_TRY(c, cudaEventElapsedTime(&tot, c->ev[0], c->ev[1]));
+  CUDA_TRY(c, cudaEventElapsedTime(&tot, c->ev[0], c->ev[6]));
   if (tm) {
     *tm = local;
     tm->total_ms = tot;
@@ -1414,12 +1474,12 @@ int pgxc_build_sym(pgxc_ctx* c, const double* const* C, const double* const* occ
   int64_t ntot = 0;
   int st;
   if ((st = sym_expand(c, C, occ, nocc, ispin, &ntot))) return st;
-  CUDA_TRY(c, cudaEventRecord(c->ev[1], s));
-  CUDA_TRY(c, cudaEventSynchronize(c->ev[1]));
+  CUDA_TRY(c, cudaEventRecord(c->ev[7], s));
+  CUDA_TRY(c, cudaEventSynchronize(c->ev[7]));
   float h2d = 0;
-  CUDA_TRY(c, cudaEventElapsedTime(&h2d, c->ev[0], c->ev[1]));
+  CUDA_TRY(c, cudaEventElapsedTime(&h2d, c->ev[0], c->ev[7]));
   pgxc_timings local{};
-  if ((st = run_build(c, (int)ntot, &local))) return st;
+  if ((st = run_build(c, (int)ntot, &local, false, nullptr, nullptr, c->d_ham, nullptr))) return st;
   cudaEvent_t e0 = c->ev[5], e1 = c->ev[6];
   CUDA_TRY(c, cudaEventRecord(e0, s));
   launch_sym_potential(P->dev, P->max_dim, ispin, c->d_ham, P->d_ham, s);
@@ -1431,6 +1491,7 @@ int pgxc_build_sym(pgxc_ctx* c, const double* const* C, const double* const* occ
   CUDA_TRY(c, cudaMemcpyAsync(c->h_acc, a.acc, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(c, cudaEventRecord(e1, s));
   CUDA_TRY(c, cudaEventSynchronize(e1));
+  if ((st = finish_build(c, &local))) return st;
   float d2h = 0, tot = 0;
   CUDA_TRY(c, cudaEventElapsedTime(&d2h, e0, e1));
   CUDA_TRY(c, cudaEventElapsedTime(&tot, c->ev[0], e1));
@@ -1463,24 +1524,24 @@ static int enqueue_screened_build(pgxc_ctx* c, const double* d_C, const double* 
   BuildArgs& a = c->a;
   cudaStream_t s = c->stream;
   const int64_t kpad = round_up(std::max(nocc, 1), 16);
-  int st = upload_orbitals(c, d_C, d_occ, (int32_t)c->nbas, nocc, kpad, cudaMemcpyDeviceToDevice);
-  if (st) return st;
-  CUDA_TRY(c, cudaMemsetAsync(a.acc, 0, 4 * sizeof(double), s));
-  launch_pmat_f64(a, kpad, s);
-  if (c->opt.ispin == 2) {
+  int64_t nv = 0;
+  double* V = screen_potential(c->screen, &nv);
+  for (int sp = 0; sp < c->opt.ispin; ++sp) {
     BuildArgs b = a;
-    b.C = c->C2;
-    b.occ = c->occ2;
-    b.P = c->P2;
-    launch_pmat_f64(b, kpad, s);
+    if (sp) {
+      b.C = c->C2;
+      b.occ = c->occ2;
+      b.P = c->P2;
+    }
+    launch_pmat_raw(b, d_C + (size_t)sp * c->nbas * nocc, d_occ + (size_t)sp * nocc, c->nbas, nocc, kpad, V,
+                    sp ? 0 : nv, a.acc, sp ? 0 : 4, s);
   }
   CUDA_TRY(c, cudaGetLastError());
   std::string e;
-  if ((st = screen_run(c->screen, a, c->P2, s, c->d_ham, nullptr, e))) return set_err(c, st, e);
-  const int64_t len = (int64_t)c->opt.ispin * c->nbas * (c->nbas + 1) / 2;
-  CUDA_TRY(c, cudaMemcpyAsync(d_ham, c->d_ham, sizeof(double) * len, cudaMemcpyDeviceToDevice, s));
-  CUDA_TRY(c, cudaMemcpyAsync(d_exc_nel, a.acc, sizeof(double), cudaMemcpyDeviceToDevice, s));
-  CUDA_TRY(c, cudaMemcpyAsync(d_exc_nel + 1, a.acc + 2, sizeof(double), cudaMemcpyDeviceToDevice, s));
+  BuildArgs as = a;
+  as.cleared = true;
+  as.exc_nel = d_exc_nel;
+  if (int st = screen_run(c->screen, as, c->P2, s, d_ham, nullptr, e)) return set_err(c, st, e);
   return PGXC_OK;
 }
 
@@ -1491,10 +1552,9 @@ static int enqueue_set_member(pgxc_ctx* c, const double* d_C, const double* d_oc
   BuildArgs& a = c->a;
   cudaStream_t s = c->stream;
   const int64_t kpad = round_up(std::max(nocc, 1), 16);
-  int st = upload_orbitals(c, d_C, d_occ, (int32_t)c->nbas, nocc, kpad, cudaMemcpyDeviceToDevice);
-  if (st) return st;
-  CUDA_TRY(c, cudaMemsetAsync(a.acc, 0, 4 * sizeof(double), s));
-  launch_pmat_f64(a, kpad, s);
+  int64_t nv = 0;
+  double* V = screen_potential(c->screen, &nv);
+  launch_pmat_raw(a, d_C, d_occ, c->nbas, nocc, kpad, V, nv, a.acc, 4, s);
   CUDA_TRY(c, cudaGetLastError());
   if (screen_set_prepare_member(c->screen, a.P, a.ldc, s)) return set_err(c, PGXC_ECUDA, "set member preparation");
   return PGXC_OK;

@@ -7,7 +7,8 @@
 //                     basis work items (tile, shell, radial mask) and chunks.
 // Per build (screen_run), per chunk of tiles:
 //   k_basis_items     phi, grad phi of listed functions only     [K1]
-//   k_pad_zero        zero the padding slots at the end of each tile's list
+//   k_tile_init       (first) clears: the padding slots at the end of each tile's
+//                     list, and what the INT8 stages add or max into
 //   k_sdensity        X = phi_t P[S_t, S_t] on DMMA, P gathered by cp.async,
 //                     fused rho, grad rho                          [K3]
 //   k_functional      (kernels_fp64.cu)                            [K2]
@@ -188,13 +189,23 @@ __global__ void __launch_bounds__(128) k_plan_fill(const float* __restrict__ d2,
 // ---------------------------------------------------------------------------
 // FP64 kernels
 // ---------------------------------------------------------------------------
-// Zero the padding slots of each tile (the slots after its listed
-// functions: tso[t] + listed[t] .. tso[t+1]).  grid = chunk tiles.
+// Clears of one chunk before its basis values (grid = chunk tiles): the padding
+// slots of each tile (after its listed functions: tso[t] + listed[t] ..
+// tso[t+1]; phi not null), the points' largest |phi| (pmax not null) and the
+// density columns the INT8 contraction adds into (rho not null: ncol columns of
+// ld per spin, spins 8 ld apart).
 template <bool GGA, typename GT = double>
-__global__ void __launch_bounds__(128) k_pad_zero(const int64_t* __restrict__ tso, const int* __restrict__ listed,
+__global__ void __launch_bounds__(128) k_tile_init(const int64_t* __restrict__ tso, const int* __restrict__ listed,
                                                   int64_t t0, int64_t s0, double* __restrict__ phi,
                                                   GT* __restrict__ gx, GT* __restrict__ gy,
-                                                  GT* __restrict__ gz) {
+                                                  GT* __restrict__ gz, unsigned long long* __restrict__ pmax,
+                                                  double* __restrict__ rho, int64_t ld, int nspin) {
+  const int64_t p = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (pmax) pmax[p] = 0;
+  if (rho)
+    for (int s = 0; s < nspin; ++s)
+      for (int c = 0; c < (GGA ? 4 : 1); ++c) rho[(8 * s + c) * ld + p] = 0.0;
+  if (!phi) return;
   const int64_t t = t0 + blockIdx.x;
   const int64_t r0 = tso[t] - s0 + listed[t], r1 = tso[t + 1] - s0;
   for (int64_t e = r0 * 128 + threadIdx.x; e < r1 * 128; e += 128) {
@@ -541,9 +552,11 @@ constexpr int svpot_smem(int max_n) {
 }  // namespace
 
 // ham[spin + ispin*(j(j+1)/2 + k)] = H(k, j), k <= j; GGA: H(k, j) + H(j, k)
+// (exc_nel not null: and {E_xc, N_el} from acc)
 __global__ void k_spack(const double* __restrict__ V, int64_t nbas, bool sym2, int ispin, int spin,
-                        double* __restrict__ ham) {
+                        double* __restrict__ ham, const double* __restrict__ acc, double* __restrict__ exc_nel) {
   const int64_t len = nbas * (nbas + 1) / 2;
+  if (exc_nel && blockIdx.x == 0 && threadIdx.x < 2) exc_nel[threadIdx.x] = acc[2 * threadIdx.x];
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < len;
        idx += (int64_t)gridDim.x * blockDim.x) {
     int64_t j = (int64_t)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
@@ -623,8 +636,9 @@ void screen_destroy(ScreenPlan* sp) {
   if (!sp) return;
   if (sp->mixed) screen_mixed_destroy(sp->mixed);
   for (void* p : sp->allocs) cudaFree(p);
-  for (auto& e : sp->ev)
-    if (e) cudaEventDestroy(e);
+  for (auto& c : sp->cev)
+    for (auto& e : c)
+      if (e) cudaEventDestroy(e);
   delete sp;
 }
 
@@ -674,7 +688,6 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
       screen_destroy(sp);
       return PGXC_ENOTSUP;
     }
-  for (auto& e : sp->ev) SP_TRY(cudaEventCreate(&e), "cudaEventCreate");
   {
     int dev = 0;
     SP_TRY(cudaGetDevice(&dev), "cudaGetDevice");
@@ -876,7 +889,9 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     SP_TRY(sp_alloc(sp, &sp->tq, 4 * (size_t)in.ispin * cp), "cudaMalloc");
     SP_TRY(cudaMemsetAsync(sp->tq, 0, sizeof(double) * 4 * in.ispin * cp, st), "memset");
   }
-  SP_TRY(sp_alloc(sp, &sp->partial, 2 * (size_t)((cp + 255) / 256) + 2), "cudaMalloc");
+  const size_t npart = 2 * (size_t)((cp + 255) / 256);
+  SP_TRY(sp_alloc(sp, &sp->partial, npart + 2), "cudaMalloc");
+  SP_TRY(cudaMemsetAsync(sp->partial + npart, 0, sizeof(double) * 2, st), "memset");
   SP_TRY(sp_alloc(sp, &sp->V, (size_t)in.ispin * in.nbas * in.nbas), "cudaMalloc (V)");
   if (mixed) {
     ScreenMixedInput mi;
@@ -917,7 +932,6 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
   // resident basis values filled by an earlier build: skip their evaluation (K1)
   const bool eval_basis = !(sp->keep && sp->basis_ready);
   ScreenTimes T;
-  cudaEvent_t* ev = sp->ev;
 #define SR_TRY(call)                                                          \
   do {                                                                        \
     cudaError_t e_ = (call);                                                  \
@@ -926,13 +940,16 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
       return PGXC_ECUDA;                                                      \
     }                                                                         \
   } while (0)
-  SR_TRY(cudaMemsetAsync(sp->V, 0, sizeof(double) * ispin * nb2, st));
+  if (!a.cleared) SR_TRY(cudaMemsetAsync(sp->V, 0, sizeof(double) * ispin * nb2, st));
   if (sp->mixed) {
-    if (timed) SR_TRY(cudaEventRecord(ev[0], st));
     for (int s = 0; s < ispin; ++s) T.launches += screen_mixed_prepare(sp->mixed, P[s], a.ldc, s, st);
     SR_TRY(cudaGetLastError());
-    if (timed) SR_TRY(cudaEventRecord(ev[1], st));
   }
+  if (timed)
+    while (sp->cev.size() < sp->chunk_t0.size() - 1) {
+      sp->cev.emplace_back();
+      for (auto& e : sp->cev.back()) SR_TRY(cudaEventCreate(&e));
+    }
   const int64_t cp = sp->chunk_tiles * 128;
   // per-chunk point arrays of spin s: 8 columns of cp (rho, grad rho, A, B) from pt + 8 s cp
   BuildArgs b[2];
@@ -952,8 +969,8 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
     b[s].partial = sp->partial;
   }
   const size_t nch = sp->chunk_t0.size() - 1;
-  float ms;
   for (size_t c = 0; c < nch; ++c) {
+    cudaEvent_t* ev = timed ? sp->cev[c].data() : nullptr;
     const int64_t t0 = sp->chunk_t0[c], t1 = sp->chunk_t0[c + 1], nt = t1 - t0;
     const int64_t s0 = sp->h_tso[(size_t)t0], ns = sp->h_tso[(size_t)t1] - s0;
     const int64_t npt = nt * 128;
@@ -967,12 +984,26 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
     float* fxc = gga && gf ? sp->fx + so * 128 : nullptr;
     float* fyc = gga && gf ? sp->fy + so * 128 : nullptr;
     float* fzc = gga && gf ? sp->fz + so * 128 : nullptr;
-    if (timed) SR_TRY(cudaEventRecord(ev[2], st));
+    if (timed) SR_TRY(cudaEventRecord(ev[0], st));
     // K1
+    {
+      double* ip = eval_basis ? phi : nullptr;
+      double* ir = sp->mixed ? sp->pt : nullptr;
+      unsigned long long* im = eval_basis ? sp->pmax : nullptr;
+      const unsigned g = (unsigned)nt;
+      if (!ip && !ir) {
+      } else if (gga && gf) {
+        k_tile_init<true, float><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, ip, fxc, fyc, fzc, im, ir, cp, ispin);
+      } else if (gga) {
+        k_tile_init<true><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, ip, gxc, gyc, gzc, im, ir, cp, ispin);
+      } else {
+        k_tile_init<false><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, ip, gxc, gyc, gzc, im, ir, cp, ispin);
+      }
+      ++T.launches;
+    }
     if (!eval_basis) {
       if (sp->mixed) T.launches += screen_mixed_gather(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, 0, st);
     } else {
-      if (sp->pmax) SR_TRY(cudaMemsetAsync(sp->pmax, 0, sizeof(unsigned long long) * nt * 128, st));
       auto launch_l = [&](auto Lc) {
         constexpr int L = decltype(Lc)::value;
         const int64_t i0 = sp->item_off[L][c], i1 = sp->item_off[L][c + 1];
@@ -997,17 +1028,11 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
       launch_l(std::integral_constant<int, 1>());
       launch_l(std::integral_constant<int, 2>());
       launch_l(std::integral_constant<int, 3>());
-      if (gga && gf) k_pad_zero<true, float><<<(unsigned)nt, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, phi, fxc, fyc, fzc);
-      else if (gga) k_pad_zero<true><<<(unsigned)nt, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, phi, gxc, gyc, gzc);
-      else k_pad_zero<false, double><<<(unsigned)nt, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, phi, (double*)nullptr,
-                                                                   (double*)nullptr, (double*)nullptr);
-      ++T.launches;
       if (sp->mixed)
         T.launches += screen_mixed_basis(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, phi, sp->pmax, so, to, st);
     }
-    if (timed) SR_TRY(cudaEventRecord(ev[3], st));
+    if (timed) SR_TRY(cudaEventRecord(ev[1], st));
     // K3, per spin
-    if (timed) SR_TRY(cudaEventRecord(ev[4], st));
     for (int s = 0; s < ispin; ++s) {
       if (sp->mixed) {
         if (s > 0) T.launches += screen_mixed_gather(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, s, st);
@@ -1046,7 +1071,7 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         ++T.launches;
       }
     }
-    if (timed) SR_TRY(cudaEventRecord(ev[5], st));
+    if (timed) SR_TRY(cudaEventRecord(ev[2], st));
     // K2
     if (sp->mgga) {
       launch_functional_mgga(sp->functional, ispin, sp->qw, sp->pt, sp->tq, cp, t0 * 128, npt, sp->partial, a.acc,
@@ -1058,12 +1083,12 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
     } else {
       launch_functional2_f64(a.xc, sp->qw, b[0].rho, b[1].rho, cp, t0 * 128, npt, gga, sp->partial, a.acc, st);
     }
-    T.launches += 2;
-    if (timed) SR_TRY(cudaEventRecord(ev[6], st));
-    // K4, per spin: the contraction of spin s is bracketed by ev[7 + 3s], ev[8 + 3s]
+    T.launches += sp->mgga ? 2 : 1;
+    if (timed) SR_TRY(cudaEventRecord(ev[3], st));
+    // K4, per spin: the contraction of spin s is bracketed by ev[4 + 2s], ev[5 + 2s]
     for (int s = 0; s < ispin && potential; ++s) {
       double* Vs = sp->V + s * nb2;
-      cudaEvent_t k0 = timed ? ev[7 + 3 * s] : nullptr, k1 = timed ? ev[8 + 3 * s] : nullptr;
+      cudaEvent_t k0 = timed ? ev[4 + 2 * s] : nullptr, k1 = timed ? ev[5 + 2 * s] : nullptr;
       if (sp->mixed) {
         if (gf)
           T.launches += screen_mixed_potential(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, phi,
@@ -1123,37 +1148,53 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
       T.launches += 2;
     }
     SR_TRY(cudaGetLastError());
-    if (!timed) continue;
-    SR_TRY(cudaEventRecord(ev[9], st));
-    SR_TRY(cudaEventSynchronize(ev[9]));
-    SR_TRY(cudaEventElapsedTime(&ms, ev[2], ev[3])); T.basis += ms;
-    SR_TRY(cudaEventElapsedTime(&ms, ev[4], ev[5])); T.density += ms; T.x += ms;
-    SR_TRY(cudaEventElapsedTime(&ms, ev[5], ev[6])); T.functional += ms;
-    SR_TRY(cudaEventElapsedTime(&ms, ev[6], ev[9])); T.potential += ms;
-    for (int s = 0; s < ispin; ++s) {
-      SR_TRY(cudaEventElapsedTime(&ms, ev[7 + 3 * s], ev[8 + 3 * s]));
-      T.v += ms;
-    }
+    // the packing counts with the last chunk's potential
+    if (timed && c + 1 < nch) SR_TRY(cudaEventRecord(ev[8], st));
   }
-  if (sp->mixed && timed) {
-    SR_TRY(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-    T.density += ms;
-  }
-  if (timed) SR_TRY(cudaEventRecord(ev[2], st));
   if (potential) {
     const int64_t len = sp->nbas * (sp->nbas + 1) / 2;
     const unsigned nbk = (unsigned)std::min<int64_t>((len + 255) / 256, 148 * 8);
     for (int s = 0; s < ispin; ++s) {
-      k_spack<<<nbk, 256, 0, st>>>(sp->V + s * nb2, sp->nbas, gga, ispin, s, ham);
+      k_spack<<<nbk, 256, 0, st>>>(sp->V + s * nb2, sp->nbas, gga, ispin, s, ham, a.acc, s == 0 ? a.exc_nel : nullptr);
       ++T.launches;
     }
   }
   SR_TRY(cudaGetLastError());
-  if (!timed) return PGXC_OK;
-  SR_TRY(cudaEventRecord(ev[3], st));
-  SR_TRY(cudaEventSynchronize(ev[3]));
-  SR_TRY(cudaEventElapsedTime(&ms, ev[2], ev[3]));
-  T.potential += ms;
+  if (timed) {
+    SR_TRY(cudaEventRecord(sp->cev[nch - 1][8], st));
+    *tm = T;
+  }
+#undef SR_TRY
+  return PGXC_OK;
+}
+
+int screen_finish(ScreenPlan* sp, cudaStream_t st, cudaEvent_t start, ScreenTimes* tm, std::string& err) {
+  float ms;
+  ScreenTimes& T = *tm;
+#define SF_TRY(call)                                                          \
+  do {                                                                        \
+    cudaError_t e_ = (call);                                                  \
+    if (e_ != cudaSuccess) {                                                  \
+      err = std::string("screened build: ") + cudaGetErrorString(e_);         \
+      return PGXC_ECUDA;                                                      \
+    }                                                                         \
+  } while (0)
+  SF_TRY(cudaStreamSynchronize(st));
+  const size_t nch = sp->chunk_t0.size() - 1;
+  SF_TRY(cudaEventElapsedTime(&ms, start, sp->cev[0][0]));
+  T.density += ms;  // the density matrix and its digits
+  for (size_t c = 0; c < nch; ++c) {
+    const auto& ev = sp->cev[c];
+    SF_TRY(cudaEventElapsedTime(&ms, ev[0], ev[1])); T.basis += ms;
+    SF_TRY(cudaEventElapsedTime(&ms, ev[1], ev[2])); T.density += ms; T.x += ms;
+    SF_TRY(cudaEventElapsedTime(&ms, ev[2], ev[3])); T.functional += ms;
+    SF_TRY(cudaEventElapsedTime(&ms, ev[3], ev[8])); T.potential += ms;
+    for (int s = 0; s < sp->ispin; ++s) {
+      SF_TRY(cudaEventElapsedTime(&ms, ev[4 + 2 * s], ev[5 + 2 * s]));
+      T.v += ms;
+    }
+  }
+#undef SF_TRY
   if (sp->mixed) {
     int flag = 0;
     if (screen_mixed_error_flag(sp->mixed, st, &flag) != PGXC_OK) {
@@ -1165,10 +1206,13 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
       return PGXC_ETIMEOUT;
     }
   }
-#undef SR_TRY
   if (sp->keep) sp->basis_ready = true;  // a completed build has filled the resident basis values
-  *tm = T;
   return PGXC_OK;
+}
+
+double* screen_potential(ScreenPlan* sp, int64_t* n) {
+  *n = sp->ispin * sp->nbas * sp->nbas;
+  return sp->V;
 }
 
 int screen_enable_tau(ScreenPlan* sp, std::string& err) {
@@ -1574,7 +1618,13 @@ int screen_set_run(ScreenSet* S, cudaStream_t st, std::string& err) {
     float* gxc = gga ? S->gx : nullptr;
     float* gyc = gga ? S->gy : nullptr;
     float* gzc = gga ? S->gz : nullptr;
-    cudaMemsetAsync(S->pmax, 0, sizeof(unsigned long long) * nt * 128, st);
+    if (gga)
+      k_tile_init<true, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc, S->pmax,
+                                                             S->pt, cp, 1);
+    else
+      k_tile_init<false, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc, S->pmax,
+                                                              S->pt, cp, 1);
+    ++launches;
     auto launch_l = [&](auto Lc) {
       constexpr int L = decltype(Lc)::value;
       const int64_t i0 = c.i0[L], n = c.i1[L] - c.i0[L];
@@ -1594,10 +1644,6 @@ int screen_set_run(ScreenSet* S, cudaStream_t st, std::string& err) {
     launch_l(std::integral_constant<int, 1>());
     launch_l(std::integral_constant<int, 2>());
     launch_l(std::integral_constant<int, 3>());
-    if (gga) k_pad_zero<true, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc);
-    else k_pad_zero<false, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, (float*)nullptr,
-                                                                (float*)nullptr, (float*)nullptr);
-    ++launches;
     screen_mixed_set_gga(S->mixed, gga);
     launches += screen_mixed_basis(S->mixed, S->tso, S->slot_fn, t0, nt, s0, S->phi, S->pmax, 0, 0, st, S->tile_mol,
                                    S->mols);
@@ -1636,7 +1682,6 @@ int screen_set_run(ScreenSet* S, cudaStream_t st, std::string& err) {
 int screen_set_error_flag(ScreenSet* S, cudaStream_t st, int* flag) { return screen_mixed_error_flag(S->mixed, st, flag); }
 
 int screen_set_prepare_member(ScreenPlan* sp, const double* P, int64_t ldc, cudaStream_t st) {
-  if (cudaMemsetAsync(sp->V, 0, sizeof(double) * sp->nbas * sp->nbas, st) != cudaSuccess) return PGXC_ECUDA;
   screen_mixed_prepare(sp->mixed, P, ldc, 0, st);
   return cudaGetLastError() == cudaSuccess ? PGXC_OK : PGXC_ECUDA;
 }

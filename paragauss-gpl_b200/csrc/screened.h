@@ -56,10 +56,12 @@ void screen_destroy(ScreenPlan* sp);
 // One build: the FP64 density matrices must be ready (a.P; for an open shell
 // also Pb, the second spin's, with the same leading dimension a.ldc); E_xc /
 // N_el are Kahan-added into a.acc; the packed matrix (both spins interleaved
-// for an open shell) is written to ham.  With t == nullptr the build is only
-// enqueued: no event records, synchronisation or host reads, so that it can be
-// captured into a CUDA graph; screen_error_flag then reports a bounded wait
-// of the INT8 kernels that ran out.
+// for an open shell) is written to ham.  The build is only enqueued, without
+// synchronisation or host reads.  With t it records timing events, and
+// screen_finish completes it (one wait per build, not one per chunk and phase);
+// with t == nullptr there are none, so that it can be captured into a CUDA
+// graph, and screen_error_flag reports a bounded wait of the INT8 kernels that
+// ran out.
 // Further functionals evaluated on the same density (energies only): E_xc and
 // N_el of functional i are Kahan-added into acc[4 i .. 4 i + 3] ({E, cE, N,
 // cN}, zeroed by the caller); with potential == false the potential
@@ -76,6 +78,12 @@ struct ScreenExtra {
 int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_t st, double* ham, ScreenTimes* t,
                std::string& err, const ScreenExtra* extra = nullptr);
 int screen_error_flag(ScreenPlan* sp, cudaStream_t st, int* flag);
+// After a timed screen_run: waits for the stream, adds the phase times (the
+// time from `start` to the first chunk counts as density) to *t and reads the
+// error flag.
+int screen_finish(ScreenPlan* sp, cudaStream_t st, cudaEvent_t start, ScreenTimes* t, std::string& err);
+// The plan's potential accumulator (both spins), which a caller may clear itself (BuildArgs::cleared).
+double* screen_potential(ScreenPlan* sp, int64_t* n);
 // The kinetic-energy density for meta-GGA energies on the density of a plan
 // that does not form it in its builds: its buffer, allocated once.  Needs FP64
 // gradient planes (a GGA plan of the FP64 build); PGXC_ENOTSUP otherwise.
@@ -108,8 +116,8 @@ void screen_set_destroy(ScreenSet* s);
 // potential accumulator (zeroed) and acc (zeroed) must be ready on st.
 int screen_set_run(ScreenSet* s, cudaStream_t st, std::string& err);
 int screen_set_error_flag(ScreenSet* s, cudaStream_t st, int* flag);
-// A member's per-build preparation on st: its potential accumulator zeroed
-// and its density matrix P (leading dimension ldc) in digit form.
+// A member's per-build preparation on st: its density matrix P (leading
+// dimension ldc) in digit form.
 int screen_set_prepare_member(ScreenPlan* sp, const double* P, int64_t ldc, cudaStream_t st);
 // whether a context's plan can join a set (screened INT8, closed shell, basis not kept)
 bool screen_set_eligible(const ScreenPlan* sp);

@@ -67,7 +67,8 @@ struct ScreenMixed {
   double* zs = nullptr;              // [chunk_slots] 2^e of each slot's Z digits
   double* fs = nullptr;              // [chunk_slots] 2^(e - 40) of each slot's phi digits (the combine shift folded in)
   double* ps = nullptr;              // [chunk_slots] 2^e_P of each slot's function (0 for padding)
-  int* err = nullptr;
+  int* err = nullptr;                // device view of h_err
+  volatile int* h_err = nullptr;     // mapped host word: written by a kernel only when a wait runs out
   int nsm = 148;
   std::vector<void*> allocs;
 };
@@ -907,13 +908,16 @@ int screen_mixed_create(ScreenMixed** out, const ScreenMixedInput& in, std::stri
   if (e == cudaSuccess) e = sm_alloc(m, &m->zs, (size_t)in.chunk_slots);
   if (e == cudaSuccess) e = sm_alloc(m, &m->fs, (size_t)in.chunk_slots);
   if (e == cudaSuccess) e = sm_alloc(m, &m->ps, (size_t)in.chunk_slots);
-  if (e == cudaSuccess) e = sm_alloc(m, &m->err, 1);
+  if (e == cudaSuccess) e = cudaHostAlloc((void**)&m->h_err, sizeof(int), cudaHostAllocMapped);
+  if (e == cudaSuccess) {
+    *m->h_err = 0;
+    e = cudaHostGetDevicePointer((void**)&m->err, (void*)m->h_err, 0);
+  }
   // the slack rows after a chunk's last slot are read (never used) by whole-block copies
   const size_t slack = (size_t)std::min<int64_t>(in.chunk_slots, 128) * kDigBytesPerSlot;
   if (e == cudaSuccess) e = cudaMemset(m->tA + dig_a - slack, 0, slack);
   if (e == cudaSuccess) e = cudaMemset(m->tZ + dig - slack, 0, slack);
   if (e == cudaSuccess) e = cudaMemset(m->tF + dig - slack, 0, slack);
-  if (e == cudaSuccess) e = cudaMemset(m->err, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) {
     err = std::string("screened mixed-precision buffers: ") + cudaGetErrorString(e);
@@ -957,6 +961,7 @@ int screen_mixed_create(ScreenMixed** out, const ScreenMixedInput& in, std::stri
 void screen_mixed_destroy(ScreenMixed* m) {
   if (!m) return;
   for (void* p : m->allocs) cudaFree(p);
+  if (m->h_err) cudaFreeHost((void*)m->h_err);
   delete m;
 }
 
@@ -992,12 +997,6 @@ int mixed_density(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_
                   double* grz, int64_t so, int64_t to, cudaStream_t st) {
   const int8_t* tA = m->tA + so * kDigBytesPerSlot;
   const int* e_pt = m->e_pt + to * 128;
-  cudaMemsetAsync(rho, 0, sizeof(double) * nt * 128, st);
-  if (m->gga) {
-    cudaMemsetAsync(grx, 0, sizeof(double) * nt * 128, st);
-    cudaMemsetAsync(gry, 0, sizeof(double) * nt * 128, st);
-    cudaMemsetAsync(grz, 0, sizeof(double) * nt * 128, st);
-  }
   const unsigned grid = (unsigned)std::min<int64_t>(nt, m->nsm);
   const int smem = tc::kWholeSmSmem;
   if (m->gga)
@@ -1076,11 +1075,9 @@ void screen_mixed_p8(ScreenMixed* m, int spin, const unsigned long long** P8, co
 }
 
 int screen_mixed_error_flag(ScreenMixed* m, cudaStream_t st, int* flag) {
-  int h = 0;
-  if (cudaMemcpyAsync(&h, m->err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return PGXC_ECUDA;
-  if (cudaMemsetAsync(m->err, 0, sizeof(int), st) != cudaSuccess) return PGXC_ECUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return PGXC_ECUDA;
-  *flag = h;
+  *flag = *m->h_err;
+  *m->h_err = 0;
   return PGXC_OK;
 }
 

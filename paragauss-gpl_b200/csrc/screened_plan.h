@@ -9,6 +9,7 @@
 #include "basis.cuh"
 #include "screened.h"
 #include "screened_mixed.h"
+#include <array>
 
 namespace pgxc {
 
@@ -52,7 +53,7 @@ struct ScreenPlan {
   double* V = nullptr;       // [ispin][nbas][nbas]
   unsigned long long* pmax = nullptr;  // [chunk_tiles*128] largest |phi| per point (INT8 path)
   ScreenMixed* mixed = nullptr;
-  cudaEvent_t ev[12] = {};
+  std::vector<std::array<cudaEvent_t, 9>> cev;  // timing events of each chunk (made by the first timed build)
   int nsm = 148;
   std::vector<void*> allocs;
 };
