@@ -13,6 +13,8 @@
 // All arithmetic is FP64 in both precision modes.
 #pragma once
 
+#include <type_traits>
+
 #include "pgxc_common.cuh"
 
 namespace pgxc {
@@ -288,12 +290,11 @@ __global__ void __launch_bounds__(128) k_basis_l(const DevShell* __restrict__ sh
 // of the chunk (tile - t0) is max-reduced into it.
 //
 // An item carries every field its evaluation needs (atom position, primitive
-// and contraction offsets), so that the loads of the next items do not depend
-// on one another.  A block walks a contiguous range of items; each warp keeps
-// the item records lane-distributed (lane k holds 32-bit word k) two items
-// ahead, and the current item's exponents and norms in lanes (lane e holds
-// primitive e), broadcast with shuffles.  Consecutive items of a tile reuse
-// the point coordinates.
+// and contraction offsets), so that the loads of the next item do not depend
+// on one another.  A block walks a contiguous range of items; the next item's
+// record is loaded (whole 16-byte words, the same for every lane) while the
+// current one is evaluated, and consecutive items of a tile reuse the point
+// coordinates.
 // ---------------------------------------------------------------------------
 struct BasisItem {
   double ax, ay, az;        // words 0-5: atom position
@@ -309,17 +310,13 @@ struct BasisItem {
   int seg;                  // 17
   int pad_[2];
 };
-static_assert(sizeof(BasisItem) == 80, "BasisItem is read as 20 words");
-constexpr int kItemWords = 20;
+static_assert(sizeof(BasisItem) == 80, "BasisItem is read as five 16-byte words");
 
-__device__ __forceinline__ int item_i(unsigned w, int k) { return (int)__shfl_sync(0xffffffffu, w, k); }
-__device__ __forceinline__ double item_d(unsigned w, int k) {
-  const unsigned lo = __shfl_sync(0xffffffffu, w, k), hi = __shfl_sync(0xffffffffu, w, k + 1);
-  return __hiloint2double((int)hi, (int)lo);
-}
-__device__ __forceinline__ unsigned long long item_u64(unsigned w, int k) {
-  const unsigned lo = __shfl_sync(0xffffffffu, w, k), hi = __shfl_sync(0xffffffffu, w, k + 1);
-  return ((unsigned long long)hi << 32) | lo;
+__device__ __forceinline__ void load_item(BasisItem& it, const BasisItem* __restrict__ p) {
+  uint4* d = reinterpret_cast<uint4*>(&it);
+  const uint4* src = reinterpret_cast<const uint4*>(p);
+#pragma unroll
+  for (int i = 0; i < 5; ++i) d[i] = __ldg(src + i);
 }
 
 // GT: the element type of the gradient planes (double; float in the INT8
@@ -333,172 +330,223 @@ template <int L, bool GRAD>
 constexpr int basis_blocks() {
   return GRAD ? (L == 0 ? 6 : (L == 1 ? 5 : 4)) : (L <= 2 ? 8 : 7);
 }
-template <int L, bool GRAD, typename GT = double>
-__global__ void __launch_bounds__(128, (basis_blocks<L, GRAD>())) k_basis_items(const BasisItem* __restrict__ items, int64_t nitems,
-                                                     const double* __restrict__ exps, const double* __restrict__ norms,
-                                                     const double* __restrict__ contr,
-                                                     const int2* __restrict__ rng, DevSA sa,
-                                                     const double* __restrict__ qx, const double* __restrict__ qy,
-                                                     const double* __restrict__ qz, int64_t s0, int64_t t0,
-                                                     double* __restrict__ phi, GT* __restrict__ gx,
-                                                     GT* __restrict__ gy, GT* __restrict__ gz,
-                                                     unsigned long long* __restrict__ pmax) {
-  const int lane = threadIdx.x & 31;
-  const int64_t per = (nitems + gridDim.x - 1) / gridDim.x;
-  const int64_t i0 = (int64_t)blockIdx.x * per, i1 = min(nitems, i0 + per);
+// The tables and point arrays of a launch.
+template <typename GT>
+struct BasisIO {
+  const double* exps;
+  const double* norms;
+  const double* contr;
+  const int2* rng;
+  const double2* prim;  // {exponent, norm x coefficient} of the primitives of segmented shells
+  const double *qx, *qy, *qz;
+  int64_t s0, t0;
+  double* phi;
+  GT *gx, *gy, *gz;
+  unsigned long long* pmax;
+};
+
+// Items [i0, i1) by one block.  Bound by instruction issue (2.9 of 4 per
+// cycle with lane-broadcast records and primitives, every primitive of a shell
+// looked at for every function): so of a segmented shell only the primitives
+// that reach some point of the warp are visited, a bit mask made once per item
+// from the warp's smallest r^2; their exponent and coefficient (the norm folded
+// in) come as one 16-byte load; and the largest |phi| takes one step per radial
+// function (max_k fl(|Y_k| |R|) = fl(max_k |Y_k| |R|)).
+template <int L, bool GRAD, typename GT>
+__device__ __forceinline__ void basis_items(const BasisItem* __restrict__ items, int64_t i0, int64_t i1,
+                                            const BasisIO<GT>& io, const DevSA& sa) {
   if (i0 >= i1) return;
-  const unsigned* words = reinterpret_cast<const unsigned*>(items);
-  auto load_item = [&](int64_t i) -> unsigned {
-    return lane < kItemWords ? __ldg(words + min(i, i1 - 1) * kItemWords + lane) : 0u;
-  };
-  unsigned wc = load_item(i0), wn = load_item(i0 + 1);
-  int nexp = item_i(wc, 15), eoff = item_i(wc, 12);
-  double pe = 0.0, pn = 0.0;  // lane e: exponent and norm of primitive e of the current item
-  if (lane < nexp) { pe = __ldg(exps + eoff + lane); pn = __ldg(norms + eoff + lane); }
-  int tile = item_i(wc, 10);
-  double px = __ldg(qx + (int64_t)tile * 128 + threadIdx.x);
-  double py = __ldg(qy + (int64_t)tile * 128 + threadIdx.x);
-  double pz = __ldg(qz + (int64_t)tile * 128 + threadIdx.x);
+  const int lane = threadIdx.x & 31;
+  BasisItem it;
+  load_item(it, items + i0);
+  double px = __ldg(io.qx + (int64_t)it.tile * 128 + threadIdx.x);
+  double py = __ldg(io.qy + (int64_t)it.tile * 128 + threadIdx.x);
+  double pz = __ldg(io.qz + (int64_t)it.tile * 128 + threadIdx.x);
   double tmax = 0.0;
   for (int64_t i = i0; i < i1; ++i) {
-    // loads for the next items, issued ahead of this item's arithmetic
-    const unsigned wnn = load_item(i + 2);
-    const int n_nexp = item_i(wn, 15), n_eoff = item_i(wn, 12), n_tile = item_i(wn, 10);
-    double ne = 0.0, nn = 0.0;
-    if (lane < n_nexp) { ne = __ldg(exps + n_eoff + lane); nn = __ldg(norms + n_eoff + lane); }
-    double nx = px, ny = py, nz = pz;
-    if (n_tile != tile) {
-      const int64_t qn = (int64_t)n_tile * 128 + threadIdx.x;
-      nx = __ldg(qx + qn); ny = __ldg(qy + qn); nz = __ldg(qz + qn);
+    BasisItem nx;
+    load_item(nx, items + min(i + 1, i1 - 1));
+    const double x = px - it.ax, y = py - it.ay, z = pz - it.az;
+    const double r2 = x * x + y * y + z * z;
+    const int nsel = it.nsig, nexp = it.nexp;
+    // the primitives (of the first 32) with alpha r^2 < 50 somewhere in the warp
+    unsigned live = 0;
+    if (it.seg && nexp <= 32) {
+      const float rmin = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(__double2float_rd(r2))));
+      const bool on = lane < nexp && __ldg(io.exps + it.exp_off + min(lane, nexp - 1)) * (double)rmin < 50.0;
+      live = __ballot_sync(0xffffffffu, on);
     }
-    // this item
-    {
-      const double x = px - item_d(wc, 0), y = py - item_d(wc, 2), z = pz - item_d(wc, 4);
-      const int64_t base = (int64_t)item_u64(wc, 6) - s0;
-      const uint64_t mask = item_u64(wc, 8);
-      const int nsel = item_i(wc, 11), coff = item_i(wc, 13), roff = item_i(wc, 14), nunc = item_i(wc, 16);
-      const bool seg = item_i(wc, 17) != 0;
-      double Y[16];
-      double dY[3][16];
-      solid_harmonics<L, double>(x, y, z, Y, dY);
-      const double r2 = x * x + y * y + z * z;
-      double Ys[2 * L + 1], dYs[3][2 * L + 1];
+    double Y[16];
+    double dY[3][16];
+    solid_harmonics<L, double>(x, y, z, Y, dY);
+    double Ys[2 * L + 1], dYs[3][2 * L + 1], ymax = 0.0;
 #pragma unroll
-      for (int k = 0; k < 2 * L + 1; ++k) {
-        if (sa.identity) {
-          Ys[k] = Y[L * L + k];
+    for (int k = 0; k < 2 * L + 1; ++k) {
+      if (sa.identity) {
+        Ys[k] = Y[L * L + k];
 #pragma unroll
-          for (int c = 0; c < 3; ++c) dYs[c][k] = dY[c][L * L + k];
-        } else {
-          double v = 0, g0 = 0, g1 = 0, g2 = 0;
+        for (int c = 0; c < 3; ++c) dYs[c][k] = dY[c][L * L + k];
+      } else {
+        double v = 0, g0 = 0, g1 = 0, g2 = 0;
 #pragma unroll
-          for (int m = 0; m < 2 * L + 1; ++m) {
-            const double cf = sa.c[L][k][m];
-            v += cf * Y[L * L + m];
-            g0 += cf * dY[0][L * L + m];
-            g1 += cf * dY[1][L * L + m];
-            g2 += cf * dY[2][L * L + m];
-          }
-          Ys[k] = v; dYs[0][k] = g0; dYs[1][k] = g1; dYs[2][k] = g2;
+        for (int m = 0; m < 2 * L + 1; ++m) {
+          const double cf = sa.c[L][k][m];
+          v += cf * Y[L * L + m];
+          g0 += cf * dY[0][L * L + m];
+          g1 += cf * dY[1][L * L + m];
+          g2 += cf * dY[2][L * L + m];
+        }
+        Ys[k] = v; dYs[0][k] = g0; dYs[1][k] = g1; dYs[2][k] = g2;
+      }
+      ymax = fmax(ymax, fabs(Ys[k]));
+    }
+    const int64_t row0 = (it.slot - io.s0) * 128 + threadIdx.x;
+    double vmax = 0.0;
+    // radial function k of the item: its 2 L + 1 functions
+    auto store = [&](int k, double Rv, double dRv) {
+      vmax = fmax(vmax, fabs(Rv));
+#pragma unroll
+      for (int m = 0; m < 2 * L + 1; ++m) {
+        const int64_t o = row0 + (m * nsel + k) * 128;
+        io.phi[o] = Ys[m] * Rv;
+        if (GRAD) {
+          const double h = Ys[m] * dRv;
+          io.gx[o] = (GT)(x * h + dYs[0][m] * Rv);
+          io.gy[o] = (GT)(y * h + dYs[1][m] * Rv);
+          io.gz[o] = (GT)(z * h + dYs[2][m] * Rv);
         }
       }
-      // primitive e's exponent and norm: from lane e, or memory past 32 primitives
-      auto prim = [&](int e, double& alpha, double& nrm) {
-        if (e < 32) {
-          alpha = __shfl_sync(0xffffffffu, pe, e);
-          nrm = __shfl_sync(0xffffffffu, pn, e);
+    };
+    uint64_t rem = it.mask;
+    if (it.seg) {
+      // segmented contractions: each selected radial function sums only its own primitives
+      const double2* pr = io.prim + it.exp_off;
+      for (int k = 0; k < nsel; ++k) {
+        const int rr = __ffsll((long long)rem) - 1;
+        rem &= rem - 1;
+        const int2 rg = __ldg(io.rng + it.rad_off + rr);
+        double Rr = 0.0, dR = 0.0;
+        auto add = [&](int e) {
+          const double2 p = __ldg(pr + e);
+          const double ar2 = p.x * r2;
+          const double v = ar2 < 50.0 ? p.y * exp(-ar2) : 0.0;
+          Rr += v;
+          dR += (-2.0 * p.x) * v;
+        };
+        if (nexp <= 32) {
+          unsigned m = rg.y > rg.x ? live & (0xffffffffu >> (32 - (rg.y - rg.x))) << rg.x : 0u;
+          for (; m; m &= m - 1) add(__ffs((int)m) - 1);
         } else {
-          alpha = __ldg(exps + eoff + e);
-          nrm = __ldg(norms + eoff + e);
+          for (int e = rg.x; e < rg.y; ++e) add(e);
         }
-      };
-      double vmax = 0.0;
-      auto store = [&](int64_t f, double Rv, double dRv, int k) {
-        const int64_t o = f * 128 + threadIdx.x;
-        phi[o] = Ys[k] * Rv;
-        vmax = fmax(vmax, fabs(Ys[k] * Rv));
-        if (GRAD) {
-          const double h = Ys[k] * dRv;
-          gx[o] = (GT)(x * h + dYs[0][k] * Rv);
-          gy[o] = (GT)(y * h + dYs[1][k] * Rv);
-          gz[o] = (GT)(z * h + dYs[2][k] * Rv);
-        }
-      };
-      if (seg) {
-        // segmented contractions: each selected radial function sums only its own primitives
-        uint64_t rem = mask;
-        for (int k = 0; k < nsel; ++k) {
-          const int rr = __ffsll((long long)rem) - 1;
-          rem &= rem - 1;
-          const int2 rg = __ldg(rng + roff + rr);
-          double Rr = 0.0, dR = 0.0;
-          for (int e = rg.x; e < rg.y; ++e) {
-            double alpha, nrm;
-            prim(e, alpha, nrm);
-            const double v = prim_value(alpha, nrm, r2);
-            const double cf = __ldg(contr + coff + e + (int64_t)nexp * rr);
-            Rr += cf * v;
-            dR += cf * ((-2.0 * alpha) * v);
-          }
+        store(k, Rr, dR);
+      }
+    } else {
+      for (int k0 = 0; k0 < nsel; k0 += kRadGroup) {
+        int rr[kRadGroup];
 #pragma unroll
-          for (int k2 = 0; k2 < 2 * L + 1; ++k2) store(base + (int64_t)k2 * nsel + k, Rr, dR, k2);
+        for (int r = 0; r < kRadGroup; ++r) {
+          if (k0 + r < nsel) {
+            rr[r] = __ffsll((long long)rem) - 1;
+            rem &= rem - 1;
+          } else {
+            rr[r] = -1;
+          }
         }
-      } else {
-        uint64_t rem = mask;
-        for (int k0 = 0; k0 < nsel; k0 += kRadGroup) {
-          int rr[kRadGroup];
+        double Rr[kRadGroup], dR[kRadGroup];
+#pragma unroll
+        for (int r = 0; r < kRadGroup; ++r) { Rr[r] = 0.0; dR[r] = 0.0; }
+        for (int e = 0; e < nexp; ++e) {
+          const double alpha = __ldg(io.exps + it.exp_off + e);
+          const double v = prim_value(alpha, __ldg(io.norms + it.exp_off + e), r2);
+          const double dv = (-2.0 * alpha) * v;
 #pragma unroll
           for (int r = 0; r < kRadGroup; ++r) {
-            if (k0 + r < nsel) {
-              rr[r] = __ffsll((long long)rem) - 1;
-              rem &= rem - 1;
-            } else {
-              rr[r] = -1;
+            if (rr[r] >= 0) {
+              const double cf = rr[r] < it.nunc ? (e == rr[r] ? 1.0 : 0.0)
+                                                : __ldg(io.contr + it.con_off + e + (int64_t)nexp * (rr[r] - it.nunc));
+              Rr[r] += cf * v;
+              dR[r] += cf * dv;
             }
-          }
-          double Rr[kRadGroup], dR[kRadGroup];
-#pragma unroll
-          for (int r = 0; r < kRadGroup; ++r) { Rr[r] = 0.0; dR[r] = 0.0; }
-          for (int e = 0; e < nexp; ++e) {
-            double alpha, nrm;
-            prim(e, alpha, nrm);
-            const double v = prim_value(alpha, nrm, r2);
-            const double dv = (-2.0 * alpha) * v;
-#pragma unroll
-            for (int r = 0; r < kRadGroup; ++r) {
-              if (rr[r] >= 0) {
-                const double cf = rr[r] < nunc ? (e == rr[r] ? 1.0 : 0.0)
-                                               : __ldg(contr + coff + e + (int64_t)nexp * (rr[r] - nunc));
-                Rr[r] += cf * v;
-                dR[r] += cf * dv;
-              }
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < 2 * L + 1; ++k) {
-#pragma unroll
-            for (int r = 0; r < kRadGroup; ++r)
-              if (rr[r] >= 0) store(base + (int64_t)k * nsel + k0 + r, Rr[r], dR[r], k);
           }
         }
-      }
-      // largest |phi| of each point over the tile's functions, max-reduced once per run of
-      // items of one tile (non-negative doubles order like their bits)
-      tmax = fmax(tmax, vmax);
-      if (pmax && (n_tile != tile || i + 1 == i1)) {
-        atomicMax(pmax + ((int64_t)tile - t0) * 128 + threadIdx.x, (unsigned long long)__double_as_longlong(tmax));
-        tmax = 0.0;
+#pragma unroll
+        for (int r = 0; r < kRadGroup; ++r)
+          if (rr[r] >= 0) store(k0 + r, Rr[r], dR[r]);
       }
     }
-    wc = wn;
-    wn = wnn;
-    nexp = n_nexp;
-    eoff = n_eoff;
-    pe = ne;
-    pn = nn;
-    tile = n_tile;
-    px = nx; py = ny; pz = nz;
+    // largest |phi| of each point over the tile's functions, max-reduced once per run of
+    // items of one tile (non-negative doubles order like their bits)
+    tmax = fmax(tmax, ymax * vmax);
+    if (io.pmax && (nx.tile != it.tile || i + 1 == i1)) {
+      atomicMax(io.pmax + ((int64_t)it.tile - io.t0) * 128 + threadIdx.x,
+                (unsigned long long)__double_as_longlong(tmax));
+      tmax = 0.0;
+    }
+    if (nx.tile != it.tile) {
+      const int64_t qn = (int64_t)nx.tile * 128 + threadIdx.x;
+      px = __ldg(io.qx + qn); py = __ldg(io.qy + qn); pz = __ldg(io.qz + qn);
+    }
+    it = nx;
   }
+}
+
+template <int L, bool GRAD, typename GT>
+__global__ void __launch_bounds__(128, (basis_blocks<L, GRAD>()))
+    k_basis_items(const BasisItem* __restrict__ items, int64_t nitems, BasisIO<GT> io, DevSA sa) {
+  const int64_t per = (nitems + gridDim.x - 1) / gridDim.x;
+  const int64_t i0 = (int64_t)blockIdx.x * per;
+  basis_items<L, GRAD, GT>(items, i0, min(nitems, i0 + per), io, sa);
+}
+
+// The same for every l in one launch, one item per block: grids of few tiles,
+// where each launch is one short wave and the launches one after another are
+// what takes the time.  n.v[l] items of each l.
+struct BasisCounts {
+  const BasisItem* items[kMaxL + 1];
+  unsigned v[kMaxL + 1];
+};
+template <bool GRAD, typename GT>
+__global__ void __launch_bounds__(128, 4) k_basis_small(BasisCounts n, BasisIO<GT> io, DevSA sa) {
+  unsigned b = blockIdx.x;
+  if (b < n.v[0]) return basis_items<0, GRAD, GT>(n.items[0], b, b + 1, io, sa);
+  b -= n.v[0];
+  if (b < n.v[1]) return basis_items<1, GRAD, GT>(n.items[1], b, b + 1, io, sa);
+  b -= n.v[1];
+  if (b < n.v[2]) return basis_items<2, GRAD, GT>(n.items[2], b, b + 1, io, sa);
+  b -= n.v[2];
+  basis_items<3, GRAD, GT>(n.items[3], b, b + 1, io, sa);
+}
+
+// Basis values of a chunk: items[l][0 .. n[l]).  One launch per l, blocks that
+// each walk a range of items, or a single one while all items together are no
+// more than the blocks of one such launch.  Returns launches.
+template <bool GRAD, typename GT>
+int launch_basis_items(const BasisItem* const (&items)[kMaxL + 1], const int64_t (&n)[kMaxL + 1], int nsm,
+                       int blocks_per_sm, const BasisIO<GT>& io, const DevSA& sa, cudaStream_t st) {
+  const int64_t most = (int64_t)nsm * blocks_per_sm, all = n[0] + n[1] + n[2] + n[3];
+  if (all == 0) return 0;
+  if (all <= most) {
+    BasisCounts c;
+    for (int l = 0; l <= kMaxL; ++l) {
+      c.items[l] = items[l];
+      c.v[l] = (unsigned)n[l];
+    }
+    k_basis_small<GRAD, GT><<<(unsigned)all, 128, 0, st>>>(c, io, sa);
+    return 1;
+  }
+  int launches = 0;
+  auto one = [&](auto Lc) {
+    constexpr int L = decltype(Lc)::value;
+    if (n[L] == 0) return;
+    k_basis_items<L, GRAD, GT><<<(unsigned)(n[L] < most ? n[L] : most), 128, 0, st>>>(items[L], n[L], io, sa);
+    ++launches;
+  };
+  one(std::integral_constant<int, 0>());
+  one(std::integral_constant<int, 1>());
+  one(std::integral_constant<int, 2>());
+  one(std::integral_constant<int, 3>());
+  return launches;
 }
 
 }  // namespace pgxc

@@ -22,6 +22,7 @@ struct BuildArgs {
   const double* norms = nullptr;
   const double* contr = nullptr;
   const int2* rng = nullptr;       // [lo, hi) primitive range of each contraction of segmented shells
+  const double2* prim = nullptr;   // {exponent, norm x its contraction's coefficient} of each primitive (segmented shells)
   DevSA sa;
   XcConst xc;
   // grid (SoA, whole grid)

@@ -270,6 +270,7 @@ __device__ __forceinline__ void sum_points(double e, double q, double* partial, 
   if (!last) return;
   __threadfence();
   e = q = 0.0;
+#pragma unroll 8
   for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
     e += __ldcg(partial + 2 * i);
     q += __ldcg(partial + 2 * i + 1);

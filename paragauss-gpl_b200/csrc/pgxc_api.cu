@@ -415,6 +415,7 @@ int create_impl(const pgxc_geometry* geo, const pgxc_basis* bas, const pgxc_grid
     // and every contraction's nonzero coefficients form its own contiguous,
     // disjoint range of primitives (each primitive then feeds one function)
     std::vector<int2> rng;
+    std::vector<double2> prim((size_t)nexp_tot, make_double2(0.0, 0.0));
     for (DevShell& S : c->shells) {
       S.seg = 0;
       S.rad_off = (int)rng.size();
@@ -438,12 +439,19 @@ int create_impl(const pgxc_geometry* geo, const pgxc_basis* bas, const pgxc_grid
       }
       if (!seg) continue;
       S.seg = 1;
+      for (int e = 0; e < S.nexp; ++e) {
+        const double cf = owner[(size_t)e] < 0 ? 0.0 : bas->contractions[S.con_off + e + (int64_t)S.nexp * owner[(size_t)e]];
+        prim[(size_t)(S.exp_off + e)] = make_double2(bas->exponents[S.exp_off + e], bas->norms[S.exp_off + e] * cf);
+      }
       rng.insert(rng.end(), r.begin(), r.end());
     }
     int2* drng = nullptr;
     if ((st = dalloc(c, &drng, std::max<size_t>(rng.size(), 1)))) return fail(st);
     if (!rng.empty()) CUDA_TRY(c, cudaMemcpy(drng, rng.data(), rng.size() * sizeof(int2), cudaMemcpyHostToDevice));
     a.rng = drng;
+    double2* dprim = nullptr;
+    if ((st = upload_vec(c, prim, &dprim))) return fail(st);
+    a.prim = dprim;
     CUDA_TRY(c, cudaMemcpy(dsh, c->shells.data(), c->shells.size() * sizeof(DevShell), cudaMemcpyHostToDevice));
   }
   {

@@ -1004,30 +1004,22 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
     if (!eval_basis) {
       if (sp->mixed) T.launches += screen_mixed_gather(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, 0, st);
     } else {
-      auto launch_l = [&](auto Lc) {
-        constexpr int L = decltype(Lc)::value;
-        const int64_t i0 = sp->item_off[L][c], i1 = sp->item_off[L][c + 1];
-        if (i1 <= i0) return;
-        // persistent-style blocks, each walking a contiguous range of items
-        const unsigned nb = (unsigned)std::min<int64_t>(i1 - i0, (int64_t)sp->nsm * kBasisBlocksPerSM);
-        if (gga && gf)
-          k_basis_items<L, true, float><<<nb, 128, 0, st>>>(sp->items[L] + i0, i1 - i0, a.exps, a.norms, a.contr,
-                                                            a.rng, a.sa, sp->qx, sp->qy, sp->qz, s0, t0, phi, fxc, fyc,
-                                                            fzc, sp->pmax);
-        else if (gga)
-          k_basis_items<L, true><<<nb, 128, 0, st>>>(sp->items[L] + i0, i1 - i0, a.exps, a.norms, a.contr, a.rng,
-                                                     a.sa, sp->qx, sp->qy, sp->qz, s0, t0, phi, gxc, gyc, gzc, sp->pmax);
-        else
-          k_basis_items<L, false, double><<<nb, 128, 0, st>>>(sp->items[L] + i0, i1 - i0, a.exps, a.norms, a.contr,
-                                                              a.rng, a.sa, sp->qx, sp->qy, sp->qz, s0, t0, phi,
-                                                              (double*)nullptr, (double*)nullptr, (double*)nullptr,
-                                                              sp->pmax);
-        ++T.launches;
+      const BasisItem* items[kMaxL + 1];
+      int64_t ni[kMaxL + 1];
+      for (int l = 0; l <= kMaxL; ++l) {
+        items[l] = sp->items[l] + sp->item_off[l][c];
+        ni[l] = sp->item_off[l][c + 1] - sp->item_off[l][c];
+      }
+      auto io = [&](auto* gx, auto* gy, auto* gz) {
+        using GT = std::remove_pointer_t<decltype(gx)>;
+        return BasisIO<GT>{a.exps, a.norms, a.contr, a.rng, a.prim, sp->qx, sp->qy, sp->qz, s0, t0, phi, gx, gy, gz, sp->pmax};
       };
-      launch_l(std::integral_constant<int, 0>());
-      launch_l(std::integral_constant<int, 1>());
-      launch_l(std::integral_constant<int, 2>());
-      launch_l(std::integral_constant<int, 3>());
+      if (gga && gf)
+        T.launches += launch_basis_items<true, float>(items, ni, sp->nsm, kBasisBlocksPerSM, io(fxc, fyc, fzc), a.sa, st);
+      else if (gga)
+        T.launches += launch_basis_items<true, double>(items, ni, sp->nsm, kBasisBlocksPerSM, io(gxc, gyc, gzc), a.sa, st);
+      else
+        T.launches += launch_basis_items<false, double>(items, ni, sp->nsm, kBasisBlocksPerSM, io(gxc, gyc, gzc), a.sa, st);
       if (sp->mixed)
         T.launches += screen_mixed_basis(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, phi, sp->pmax, so, to, st);
     }
@@ -1352,6 +1344,7 @@ struct ScreenSet {
   BasisItem* items[kMaxL + 1] = {};
   double *exps = nullptr, *norms = nullptr, *contr = nullptr;
   int2* rng = nullptr;
+  double2* prim = nullptr;
   SetMolDev* mols = nullptr;
   SetOutDev* outs = nullptr;
   SetSeg* segs = nullptr;
@@ -1459,6 +1452,7 @@ int screen_set_create(ScreenSet** out, const std::vector<SetMember>& members, in
   SS_TRY(alloc(&S->tile_mol, (size_t)T), "cudaMalloc");
   SS_TRY(alloc(&S->exps, (size_t)eoff[nm]), "cudaMalloc");
   SS_TRY(alloc(&S->norms, (size_t)eoff[nm]), "cudaMalloc");
+  SS_TRY(alloc(&S->prim, (size_t)eoff[nm]), "cudaMalloc");
   SS_TRY(alloc(&S->contr, (size_t)coff[nm]), "cudaMalloc");
   SS_TRY(alloc(&S->rng, (size_t)roff[nm]), "cudaMalloc");
   for (int l = 0; l <= kMaxL; ++l) SS_TRY(alloc(&S->items[l], (size_t)ioff[l][nm]), "cudaMalloc");
@@ -1481,6 +1475,8 @@ int screen_set_create(ScreenSet** out, const std::vector<SetMember>& members, in
     SS_TRY(cudaMemcpyAsync(S->exps + eoff[i], a->exps, sizeof(double) * sp->n_exps, cudaMemcpyDeviceToDevice, st),
            "copy");
     SS_TRY(cudaMemcpyAsync(S->norms + eoff[i], a->norms, sizeof(double) * sp->n_exps, cudaMemcpyDeviceToDevice, st),
+           "copy");
+    SS_TRY(cudaMemcpyAsync(S->prim + eoff[i], a->prim, sizeof(double2) * sp->n_exps, cudaMemcpyDeviceToDevice, st),
            "copy");
     if (sp->n_contr)
       SS_TRY(cudaMemcpyAsync(S->contr + coff[i], a->contr, sizeof(double) * sp->n_contr, cudaMemcpyDeviceToDevice,
@@ -1625,25 +1621,16 @@ int screen_set_run(ScreenSet* S, cudaStream_t st, std::string& err) {
       k_tile_init<false, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc, S->pmax,
                                                               S->pt, cp, 1);
     ++launches;
-    auto launch_l = [&](auto Lc) {
-      constexpr int L = decltype(Lc)::value;
-      const int64_t i0 = c.i0[L], n = c.i1[L] - c.i0[L];
-      if (n <= 0) return;
-      const unsigned nb = (unsigned)std::min<int64_t>(n, (int64_t)S->nsm * kBasisBlocksPerSM);
-      if (gga)
-        k_basis_items<L, true, float><<<nb, 128, 0, st>>>(S->items[L] + i0, n, S->exps, S->norms, S->contr, S->rng,
-                                                          S->sa, S->qx, S->qy, S->qz, s0, t0, S->phi, gxc, gyc, gzc,
-                                                          S->pmax);
-      else
-        k_basis_items<L, false, float><<<nb, 128, 0, st>>>(S->items[L] + i0, n, S->exps, S->norms, S->contr, S->rng,
-                                                           S->sa, S->qx, S->qy, S->qz, s0, t0, S->phi, (float*)nullptr,
-                                                           (float*)nullptr, (float*)nullptr, S->pmax);
-      ++launches;
-    };
-    launch_l(std::integral_constant<int, 0>());
-    launch_l(std::integral_constant<int, 1>());
-    launch_l(std::integral_constant<int, 2>());
-    launch_l(std::integral_constant<int, 3>());
+    const BasisItem* items[kMaxL + 1];
+    int64_t ni[kMaxL + 1];
+    for (int l = 0; l <= kMaxL; ++l) {
+      items[l] = S->items[l] + c.i0[l];
+      ni[l] = c.i1[l] - c.i0[l];
+    }
+    const BasisIO<float> io{S->exps, S->norms, S->contr, S->rng, S->prim, S->qx, S->qy, S->qz,
+                            s0,      t0,       S->phi,   gxc,    gyc,     gzc,   S->pmax};
+    launches += gga ? launch_basis_items<true, float>(items, ni, S->nsm, kBasisBlocksPerSM, io, S->sa, st)
+                    : launch_basis_items<false, float>(items, ni, S->nsm, kBasisBlocksPerSM, io, S->sa, st);
     screen_mixed_set_gga(S->mixed, gga);
     launches += screen_mixed_basis(S->mixed, S->tso, S->slot_fn, t0, nt, s0, S->phi, S->pmax, 0, 0, st, S->tile_mol,
                                    S->mols);
