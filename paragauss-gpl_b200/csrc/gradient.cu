@@ -1,8 +1,15 @@
-// gradient.cu -- kernels of the post-SCF XC nuclear gradient (gradient.h).
+// gradient.cu -- the post-SCF XC nuclear gradient (gradient.h).
 //
-// FP64 throughout.  The gradient runs once per geometry, after the SCF: the
-// kernels are plain per-point / per-function loops; the four contractions
-// per spin (X = Phi P, Y_j = d_j Phi P) are library DGEMMs issued by the caller.
+// FP64 throughout, on the Morton-ordered 128-point tiles of a plan whose lists
+// hold every function that is not identically zero on the tile (threshold 0,
+// whatever the context's own screening): per chunk of tiles
+//   k_hess_items   phi, grad phi and Hessians of the listed functions
+//   grad_contract  X = phi P[S_t, S_t] with rho, grad rho (screened.cu, DMMA)
+//   k_grad_coef    the functional and the coefficients of each point
+//   k_grad_w       W = sum_j b_j d_j phi, then V = W P[S_t, S_t]
+//   k_grad_orb     the orbital terms
+// and over all tiles k_grad_weights, the Becke weight term (its points in the
+// same order: a warp's points then share their live atoms).
 #include <cmath>
 
 #include "basis.cuh"
@@ -10,6 +17,7 @@
 #include "gradient.h"
 #include "xc_functional.cuh"
 #include "xc_mgga.cuh"
+#include "screened_plan.h"
 
 namespace pgxc {
 
@@ -108,82 +116,107 @@ __device__ __forceinline__ void solid_harmonics_h(double x, double y, double z, 
   }
 }
 
-// grid = (ld / 128, shells of L): phi, grad and Hessian of every function of the shell
+// phi, grad phi and (hess) the Hessian of the items' functions on their tiles:
+// plane c (phi; x, y, z; xx, xy, xz, yy, yz, zz) at out + c plane, rows of 128
+// points per slot.  Block = the 128 points of a tile, a range of items.
 template <int L>
-__global__ void __launch_bounds__(128) k_basis_hess(const DevShell* __restrict__ shells, const int* __restrict__ ids,
-                                                    const double* __restrict__ atoms, const double* __restrict__ exps,
-                                                    const double* __restrict__ norms, const double* __restrict__ contr,
-                                                    const int2* __restrict__ rng, DevSA sa,
-                                                    const double* __restrict__ px, const double* __restrict__ py,
-                                                    const double* __restrict__ pz, int64_t p0, int64_t nvalid,
-                                                    int64_t ld, int64_t plane, double* __restrict__ out) {
-  const DevShell S = shells[ids[blockIdx.y]];
-  const int64_t p = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (p >= ld) return;
-  const bool valid = p < nvalid;
-  double x = 0, y = 0, z = 0;
-  if (valid) {
-    x = px[p0 + p] - atoms[3 * S.atom];
-    y = py[p0 + p] - atoms[3 * S.atom + 1];
-    z = pz[p0 + p] - atoms[3 * S.atom + 2];
-  }
-  double Y[16], dY[3][16], H[6][16];
-  solid_harmonics_h<L>(x, y, z, Y, dY, H);
-  const double r2 = x * x + y * y + z * z;
-  const double xv[3] = {x, y, z};
+__global__ void __launch_bounds__(128) k_hess_items(const BasisItem* __restrict__ items, int64_t nitems,
+                                                    BasisIO<double> io, DevSA sa, bool hess, int64_t plane,
+                                                    double* __restrict__ out) {
+  const int64_t per = (nitems + gridDim.x - 1) / gridDim.x;
+  const int64_t i0 = (int64_t)blockIdx.x * per, i1 = min(nitems, i0 + per);
   constexpr int ci[6] = {0, 0, 0, 1, 1, 2}, di[6] = {0, 1, 2, 1, 2, 2};
-  // symmetry-adapted harmonics of this l
-  double Ys[2 * L + 1], dYs[3][2 * L + 1], Hs[6][2 * L + 1];
-  for (int i = 0; i < 2 * L + 1; ++i) {
-    double v = 0, g[3] = {0, 0, 0}, h[6] = {0, 0, 0, 0, 0, 0};
+  for (int64_t i = i0; i < i1; ++i) {
+    BasisItem it;
+    load_item(it, items + i);
+    const int64_t q = (int64_t)it.tile * 128 + threadIdx.x;
+    const double x = __ldg(io.qx + q) - it.ax, y = __ldg(io.qy + q) - it.ay, z = __ldg(io.qz + q) - it.az;
+    double Y[16], dY[3][16], H[6][16];
+    solid_harmonics_h<L>(x, y, z, Y, dY, H);
+    const double r2 = x * x + y * y + z * z;
+    const double xv[3] = {x, y, z};
+    // symmetry-adapted harmonics of this l
+    double Ys[2 * L + 1], dYs[3][2 * L + 1], Hs[6][2 * L + 1];
+#pragma unroll
     for (int m = 0; m < 2 * L + 1; ++m) {
-      const double cf = sa.identity ? (m == i ? 1.0 : 0.0) : sa.c[L][i][m];
-      v += cf * Y[L * L + m];
-      for (int c = 0; c < 3; ++c) g[c] += cf * dY[c][L * L + m];
-      for (int k = 0; k < 6; ++k) h[k] += cf * H[k][L * L + m];
+      if (sa.identity) {
+        Ys[m] = Y[L * L + m];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) dYs[c][m] = dY[c][L * L + m];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) Hs[k][m] = H[k][L * L + m];
+      } else {
+        double v = 0, g[3] = {0, 0, 0}, h[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int n = 0; n < 2 * L + 1; ++n) {
+          const double cf = sa.c[L][m][n];
+          v += cf * Y[L * L + n];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) g[c] += cf * dY[c][L * L + n];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) h[k] += cf * H[k][L * L + n];
+        }
+        Ys[m] = v;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) dYs[c][m] = g[c];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) Hs[k][m] = h[k];
+      }
     }
-    Ys[i] = v;
-    for (int c = 0; c < 3; ++c) dYs[c][i] = g[c];
-    for (int k = 0; k < 6; ++k) Hs[k][i] = h[k];
+    uint64_t rem = it.mask;
+    for (int k = 0; k < it.nsig; ++k) {
+      const int rr = __ffsll((long long)rem) - 1;
+      rem &= rem - 1;
+      // R, dR = sum c (-2 alpha) v and d2R = sum c (4 alpha^2) v of radial function rr:
+      // d_c R = x_c dR, d_c d_d R = delta_cd dR + x_c x_d d2R
+      double R = 0.0, dR = 0.0, d2R = 0.0;
+      auto add = [&](double alpha, double c) {
+        const double ar2 = alpha * r2;
+        if (!__any_sync(0xffffffffu, ar2 < 50.0)) return;
+        const double v = ar2 < 50.0 ? c * exp(-ar2) : 0.0;
+        R += v;
+        dR += (-2.0 * alpha) * v;
+        d2R += (4.0 * alpha * alpha) * v;
+      };
+      if (it.seg) {
+        const int2 rg = __ldg(io.rng + it.rad_off + rr);
+        for (int e = rg.x; e < rg.y; ++e) {
+          const double2 p = __ldg(io.prim + it.exp_off + e);
+          add(p.x, p.y);
+        }
+      } else {
+        const int e0 = rr < it.nunc ? rr : 0, e1 = rr < it.nunc ? rr + 1 : it.nexp;
+        for (int e = e0; e < e1; ++e) {
+          const double cf = rr < it.nunc ? 1.0 : __ldg(io.contr + it.con_off + e + (int64_t)it.nexp * (rr - it.nunc));
+          add(__ldg(io.exps + it.exp_off + e), cf * __ldg(io.norms + it.exp_off + e));
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 2 * L + 1; ++m) {
+        double* o = out + (it.slot - io.s0 + (int64_t)m * it.nsig + k) * 128 + threadIdx.x;
+        o[0] = Ys[m] * R;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o[(1 + c) * plane] = dYs[c][m] * R + Ys[m] * xv[c] * dR;
+        if (hess) {
+#pragma unroll
+          for (int h = 0; h < 6; ++h) {
+            const int c = ci[h], d = di[h];
+            o[(4 + h) * plane] = Hs[h][m] * R + (dYs[c][m] * xv[d] + dYs[d][m] * xv[c]) * dR +
+                                 Ys[m] * ((c == d ? dR : 0.0) + xv[c] * xv[d] * d2R);
+          }
+        }
+      }
+    }
   }
-  const double* ex = exps + S.exp_off;
-  const double* nr = norms + S.exp_off;
-  const double* cc = contr + S.con_off;
-  for (int rr = 0; rr < S.nrad; ++rr) {
-    // R, dR = sum c (-2 alpha) v and d2R = sum c (4 alpha^2) v of radial function rr:
-    // d_c R = x_c dR, d_c d_d R = delta_cd dR + x_c x_d d2R
-    double R = 0.0, dR = 0.0, d2R = 0.0;
-    if (valid) {
-      int e0 = 0, e1 = S.nexp;
-      if (S.seg) {
-        const int2 rg = rng[S.rad_off + rr];
-        e0 = rg.x;
-        e1 = rg.y;
-      }
-      for (int e = e0; e < e1; ++e) {
-        double cf;
-        if (S.seg) cf = cc[e + (int64_t)S.nexp * rr];
-        else if (rr < S.nunc) cf = (e == rr) ? 1.0 : 0.0;
-        else cf = cc[e + (int64_t)S.nexp * (rr - S.nunc)];
-        const double alpha = ex[e];
-        const double v = prim_value(alpha, nr[e], r2);
-        R += cf * v;
-        dR += cf * (-2.0 * alpha) * v;
-        d2R += cf * (4.0 * alpha * alpha) * v;
-      }
-    }
-    for (int i = 0; i < 2 * L + 1; ++i) {
-      const int64_t f = S.f0 + (int64_t)i * S.nrad + rr;
-      double* o = out + f * ld + p;
-      o[0] = Ys[i] * R;
-      for (int c = 0; c < 3; ++c) o[(1 + c) * plane] = dYs[c][i] * R + Ys[i] * xv[c] * dR;
-      for (int k = 0; k < 6; ++k) {
-        const int c = ci[k], d = di[k];
-        o[(4 + k) * plane] = Hs[k][i] * R + (dYs[c][i] * xv[d] + dYs[d][i] * xv[c]) * dR +
-                             Ys[i] * ((c == d ? dR : 0.0) + xv[c] * xv[d] * d2R);
-      }
-    }
-  }
+}
+
+// Zero the padding slots of each tile in the first np planes (grid = chunk tiles).
+__global__ void __launch_bounds__(128) k_grad_pads(const int64_t* __restrict__ tso, const int* __restrict__ listed,
+                                                   int64_t t0, int64_t s0, int np, int64_t plane,
+                                                   double* __restrict__ out) {
+  const int64_t t = t0 + blockIdx.x;
+  for (int64_t r = tso[t] - s0 + listed[t]; r < tso[t + 1] - s0; ++r)
+    for (int c = 0; c < np; ++c) out[c * plane + r * 128 + threadIdx.x] = 0.0;
 }
 
 // index of the Hessian component (c, d) in xx, xy, xz, yy, yz, zz
@@ -195,167 +228,171 @@ __device__ __forceinline__ int hidx(int c, int d) {
 // coef planes per spin: a, b_x, b_y, b_z, c (c = w df/dtau, meta-GGAs)
 constexpr int kCoefPlanes = 5;
 
-__global__ void k_grad_points(XcConst K, int functional, bool gga, int ispin, int64_t nbas, int64_t ld, int64_t p0,
-                              int64_t nvalid, const double* __restrict__ w, const double* __restrict__ wraw,
-                              const double* __restrict__ B, int64_t plane, const double* __restrict__ XY,
-                              double* __restrict__ coef, double* __restrict__ ef, double* __restrict__ exc) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= ld) return;
-  if (p >= nvalid) {
-    for (int s = 0; s < ispin; ++s)
-      for (int c = 0; c < kCoefPlanes; ++c) coef[(kCoefPlanes * s + c) * ld + p] = 0.0;
-    ef[p] = 0.0;
-    return;
-  }
+// Per point of the chunk: the functional at rho_s, grad rho_s (den[(7 s + c) ld
+// + p], c = 0..3) and for meta-GGAs tau_s = 1/2 sum_j (2 tau_j) (c = 4..6), and
+// the coefficients a_s, b_s, c_s (0 on padding points); ef = w_raw f, and
+// sum w f is added into *exc.
+__global__ void __launch_bounds__(128) k_grad_coef(XcConst K, int functional, bool gga, int ispin, int64_t ld,
+                                                   const double* __restrict__ w, const double* __restrict__ wraw,
+                                                   const double* __restrict__ den, double* __restrict__ coef,
+                                                   double* __restrict__ ef, double* __restrict__ exc) {
+  const int64_t p = (int64_t)blockIdx.x * 128 + threadIdx.x;
   const bool mgga = PGXC_XC_IS_MGGA(functional);
-  // rho_s, grad rho_s and (meta-GGAs) tau_s = 1/2 sum_j d_j phi P_s d_j phi = 1/2 sum_j,f d_j phi_f Y_j,f
-  double rho[2] = {0, 0}, gr[2][3] = {{0, 0, 0}, {0, 0, 0}}, tau[2] = {0, 0};
-  for (int s = 0; s < ispin; ++s) {
-    const double* X = XY + (4 * s) * plane;
-    for (int64_t f = 0; f < nbas; ++f) {
-      const double xv = X[f * ld + p];
-      rho[s] += B[f * ld + p] * xv;
-      if (gga)
-        for (int c = 0; c < 3; ++c) gr[s][c] += 2.0 * B[(1 + c) * plane + f * ld + p] * xv;
-      if (mgga)
-        for (int c = 0; c < 3; ++c) tau[s] += 0.5 * B[(1 + c) * plane + f * ld + p] * X[(1 + c) * plane + f * ld + p];
-    }
-  }
-  const double wp = w[p0 + p];
-  double f = 0.0, fr[2] = {0, 0}, fg[3] = {0, 0, 0}, ft[2] = {0, 0};
-  if (ispin == 1) {
-    const double g = gr[0][0] * gr[0][0] + gr[0][1] * gr[0][1] + gr[0][2] * gr[0][2];
-    if (mgga) mgga::mgga_closed(functional, rho[0], g, tau[0], f, fr[0], fg[0], ft[0]);
-    else if (gga) xc_gga(K, rho[0], g, f, fr[0], fg[0]);
-    else xc_vwn(K, rho[0], f, fr[0]);
-    coef[p] = wp * fr[0];
-    for (int c = 0; c < 3; ++c) coef[(1 + c) * ld + p] = gga ? wp * 2.0 * fg[0] * gr[0][c] : 0.0;
-    coef[4 * ld + p] = wp * ft[0];
+  const double wp = w[p], wr = wraw[p];
+  double f = 0.0;
+  if (wp == 0.0 && wr == 0.0) {
+    for (int c = 0; c < kCoefPlanes * ispin; ++c) coef[c * ld + p] = 0.0;
   } else {
-    const double r2[2] = {rho[0], rho[1]};
-    const double g3[3] = {gr[0][0] * gr[0][0] + gr[0][1] * gr[0][1] + gr[0][2] * gr[0][2],
-                          gr[1][0] * gr[1][0] + gr[1][1] * gr[1][1] + gr[1][2] * gr[1][2],
-                          gr[0][0] * gr[1][0] + gr[0][1] * gr[1][1] + gr[0][2] * gr[1][2]};
-    double fr2[2], fg3[3];
-    if (mgga) mgga::mgga_open(functional, r2, g3, tau, f, fr2, fg3, ft);
-    else if (gga) xc_open<true>(K, r2, g3, f, fr2, fg3);
-    else xc_open<false>(K, r2, g3, f, fr2, fg3);
-    for (int s = 0; s < 2; ++s) {
-      coef[(kCoefPlanes * s) * ld + p] = wp * fr2[s];
-      for (int c = 0; c < 3; ++c)
-        coef[(kCoefPlanes * s + 1 + c) * ld + p] = gga ? wp * (2.0 * fg3[s] * gr[s][c] + fg3[2] * gr[1 - s][c]) : 0.0;
-      coef[(kCoefPlanes * s + 4) * ld + p] = wp * ft[s];
+    double rho[2] = {0, 0}, gr[2][3] = {{0, 0, 0}, {0, 0, 0}}, tau[2] = {0, 0};
+    for (int s = 0; s < ispin; ++s) {
+      const double* d = den + (int64_t)(7 * s) * ld + p;
+      rho[s] = d[0];
+      if (gga)
+        for (int c = 0; c < 3; ++c) gr[s][c] = d[(1 + c) * ld];
+      if (mgga) tau[s] = 0.5 * (d[4 * ld] + d[5 * ld] + d[6 * ld]);
+    }
+    double fr[2] = {0, 0}, fg[3] = {0, 0, 0}, ft[2] = {0, 0};
+    if (ispin == 1) {
+      const double g = gr[0][0] * gr[0][0] + gr[0][1] * gr[0][1] + gr[0][2] * gr[0][2];
+      if (mgga) mgga::mgga_closed(functional, rho[0], g, tau[0], f, fr[0], fg[0], ft[0]);
+      else if (gga) xc_gga(K, rho[0], g, f, fr[0], fg[0]);
+      else xc_vwn(K, rho[0], f, fr[0]);
+      coef[p] = wp * fr[0];
+      for (int c = 0; c < 3; ++c) coef[(1 + c) * ld + p] = gga ? wp * 2.0 * fg[0] * gr[0][c] : 0.0;
+      coef[4 * ld + p] = wp * ft[0];
+    } else {
+      const double r2[2] = {rho[0], rho[1]};
+      const double g3[3] = {gr[0][0] * gr[0][0] + gr[0][1] * gr[0][1] + gr[0][2] * gr[0][2],
+                            gr[1][0] * gr[1][0] + gr[1][1] * gr[1][1] + gr[1][2] * gr[1][2],
+                            gr[0][0] * gr[1][0] + gr[0][1] * gr[1][1] + gr[0][2] * gr[1][2]};
+      double fr2[2], fg3[3];
+      if (mgga) mgga::mgga_open(functional, r2, g3, tau, f, fr2, fg3, ft);
+      else if (gga) xc_open<true>(K, r2, g3, f, fr2, fg3);
+      else xc_open<false>(K, r2, g3, f, fr2, fg3);
+      for (int s = 0; s < 2; ++s) {
+        coef[(kCoefPlanes * s) * ld + p] = wp * fr2[s];
+        for (int c = 0; c < 3; ++c)
+          coef[(kCoefPlanes * s + 1 + c) * ld + p] =
+              gga ? wp * (2.0 * fg3[s] * gr[s][c] + fg3[2] * gr[1 - s][c]) : 0.0;
+        coef[(kCoefPlanes * s + 4) * ld + p] = wp * ft[s];
+      }
     }
   }
-  ef[p] = wraw[p0 + p] * f;
-  atomicAdd(exc, wp * f);
+  ef[p] = wr * f;
+  double e = wp * f;
+  for (int off = 16; off > 0; off >>= 1) e += __shfl_down_sync(0xffffffffu, e, off);
+  if ((threadIdx.x & 31) == 0 && e != 0.0) atomicAdd(exc, e);
+}
+
+// GGAs (not meta-GGAs): the Y_j enter the orbital terms only as
+// sum_j b_j Y_j = W P with W = sum_j b_j d_j phi, one product instead of
+// three.  Padding rows are zero (grid = chunk tiles).
+__global__ void __launch_bounds__(128) k_grad_w(const int64_t* __restrict__ tso, const int* __restrict__ listed,
+                                                int64_t t0, int64_t s0, const double* __restrict__ B, int64_t plane,
+                                                const double* __restrict__ cb, int64_t ld, double* __restrict__ W) {
+  const int64_t t = t0 + blockIdx.x, p = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  const double b0 = cb[p], b1 = cb[ld + p], b2 = cb[2 * ld + p];
+  const int64_t o0 = (tso[t] - s0) * 128 + threadIdx.x;
+  const int n = (int)(tso[t + 1] - tso[t]), nl = listed[t];
+#pragma unroll 4
+  for (int r = 0; r < nl; ++r) {
+    const int64_t o = o0 + r * 128;
+    W[o] = b0 * B[plane + o] + b1 * B[2 * plane + o] + b2 * B[3 * plane + o];
+  }
+  for (int r = nl; r < n; ++r) W[o0 + r * 128] = 0.0;
 }
 
 // The orbital terms in one pass: q^s_mu,k(p) is formed once per function and
-// point.  Block = 256 points x kGradFB functions: each thread takes one point
-// and loops over the block's functions; -q goes to atom(mu) through a warp
-// reduction and the block's shared sums, +q to the point's host through the
-// thread's running sum, reduced over the warp when all its points share a
-// host (the usual case: the raw grid is atom by atom) and the block's shared
-// per-atom sums.
-// GGAs (not meta-GGAs): the Y_j enter the orbital terms only as
-// sum_j b_j Y_j = W P with W = sum_j b_j d_j phi, one product instead of
-// three.  W[f][p] for f < nbas, and zero rows nbas .. kpad - 1 (read by the
-// product's K loop, which meets P's zero rows there).
-__global__ void k_grad_w(int64_t nbas, int64_t kpad, int64_t ld, const double* __restrict__ B, int64_t plane,
-                         const double* __restrict__ cb, double* __restrict__ W) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kpad * ld) return;
-  const int64_t f = i / ld, p = i - f * ld;
-  double w = 0.0;
-  if (f < nbas)
-    for (int j = 0; j < 3; ++j) w += cb[j * ld + p] * B[(1 + j) * plane + i];
-  W[i] = w;
-}
-
-constexpr int kGradFB = 32;
-
-__global__ void __launch_bounds__(256) k_grad_orb(bool gga, bool mgga, int ispin, int64_t nbas, int64_t ld, int64_t p0,
-                                                  int64_t nvalid, int natm, const int* __restrict__ fatom,
-                                                  const int* __restrict__ owner, const double* __restrict__ B,
-                                                  int64_t plane, const double* __restrict__ XY,
-                                                  const double* __restrict__ coef, double* __restrict__ grad) {
-  extern __shared__ double sh[];  // [kGradFB][3] function sums, then [natm][3] host sums
-  double* gq = sh;
-  double* gh = sh + 3 * kGradFB;
-  for (int i = threadIdx.x; i < 3 * (kGradFB + natm); i += blockDim.x) sh[i] = 0.0;
+// point.  Block = a tile, thread = point; a tile's slots come atom by atom, so
+// -q is summed over an atom's functions in registers and reduced over the warp
+// once per atom (a reduction per function took most of the instructions), +q
+// goes to the point's host through the thread's running sum.
+__global__ void __launch_bounds__(128) k_grad_orb(bool gga, bool mgga, int ispin, int natm,
+                                                  const int64_t* __restrict__ tso, const int* __restrict__ listed,
+                                                  const int* __restrict__ slot_fn, int64_t t0, int64_t s0,
+                                                  const int* __restrict__ fatom, const int* __restrict__ owner,
+                                                  const double* __restrict__ B, int64_t plane,
+                                                  const double* __restrict__ XY, int nxy,
+                                                  const double* __restrict__ coef, int64_t ld,
+                                                  double* __restrict__ grad) {
+  extern __shared__ double gs[];  // [natm][3]
+  for (int i = threadIdx.x; i < 3 * natm; i += 128) gs[i] = 0.0;
   __syncthreads();
-  const int64_t p = (int64_t)blockIdx.y * blockDim.x + threadIdx.x;
-  const bool live = p < nvalid;
-  const int lane = threadIdx.x & 31;
-  const int64_t f0 = (int64_t)blockIdx.x * kGradFB, f1 = min(nbas, f0 + kGradFB);
-  // the point's coefficients, once for all its functions
+  const int64_t t = t0 + blockIdx.x, p = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  const int lane = threadIdx.x & 31, nl = listed[t];
+  const int* fn = slot_fn + tso[t];
   double a[2] = {0, 0}, b[2][3] = {{0, 0, 0}, {0, 0, 0}}, ct[2] = {0, 0};
-  if (live)
-    for (int sp = 0; sp < ispin; ++sp) {
-      a[sp] = coef[(kCoefPlanes * sp) * ld + p];
-      if (gga)
-        for (int j = 0; j < 3; ++j) b[sp][j] = coef[(kCoefPlanes * sp + 1 + j) * ld + p];
-      if (mgga) ct[sp] = coef[(kCoefPlanes * sp + 4) * ld + p];
+  for (int sp = 0; sp < ispin; ++sp) {
+    a[sp] = coef[(kCoefPlanes * sp) * ld + p];
+    if (gga)
+      for (int j = 0; j < 3; ++j) b[sp][j] = coef[(kCoefPlanes * sp + 1 + j) * ld + p];
+    if (mgga) ct[sp] = coef[(kCoefPlanes * sp + 4) * ld + p];
+  }
+  double tot[3] = {0, 0, 0}, qa[3] = {0, 0, 0};
+  int atom = nl > 0 ? fatom[fn[0]] : 0;
+  auto flush = [&]() {
+    for (int k = 0; k < 3; ++k) {
+      tot[k] += qa[k];
+      double v = qa[k];
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+      if (lane == 0) atomicAdd(&gs[3 * atom + k], -v);
+      qa[k] = 0.0;
     }
-  double t[3] = {0, 0, 0};
-  for (int64_t f = f0; f < f1; ++f) {
-    double q[3] = {0, 0, 0};
-    if (live) {
-      const int64_t o = f * ld + p;
-      double d[3], H[6];
-      for (int c = 0; c < 3; ++c) d[c] = B[(1 + c) * plane + o];
-      if (gga)
-        for (int k = 0; k < 6; ++k) H[k] = B[(4 + k) * plane + o];
-      for (int sp = 0; sp < ispin; ++sp) {
-        const double X = XY[(4 * sp) * plane + o];
-        for (int k = 0; k < 3; ++k) q[k] += 2.0 * a[sp] * d[k] * X;
-        if (!gga) continue;
-        if (!mgga) {  // sum_j b_j Y_j = (sum_j b_j d_j phi) P = V, plane 2 of the spin
-          const double V = XY[(4 * sp + 2) * plane + o];
-          for (int k = 0; k < 3; ++k) {
-            double u = d[k] * V;
-            for (int j = 0; j < 3; ++j) u += b[sp][j] * H[hidx(k, j)] * X;
-            q[k] += 2.0 * u;
-          }
-          continue;
-        }
-        double Yj[3];
-        for (int j = 0; j < 3; ++j) Yj[j] = XY[(4 * sp + 1 + j) * plane + o];
+  };
+  const int64_t o0 = (tso[t] - s0) * 128 + threadIdx.x;
+#pragma unroll 2
+  for (int r = 0; r < nl; ++r) {
+    const int at = fatom[fn[r]];
+    if (at != atom) {
+      flush();
+      atom = at;
+    }
+    const int64_t o = o0 + r * 128;
+    double d[3], H[6];
+    for (int c = 0; c < 3; ++c) d[c] = B[(1 + c) * plane + o];
+    if (gga)
+      for (int k = 0; k < 6; ++k) H[k] = B[(4 + k) * plane + o];
+    for (int sp = 0; sp < ispin; ++sp) {
+      const double* xy = XY + (int64_t)(nxy * sp) * plane + o;
+      const double X = xy[0];
+      for (int k = 0; k < 3; ++k) qa[k] += 2.0 * a[sp] * d[k] * X;
+      if (!gga) continue;
+      if (!mgga) {  // sum_j b_j Y_j = (sum_j b_j d_j phi) P = V
+        const double V = xy[plane];
         for (int k = 0; k < 3; ++k) {
-          double u = 0.0;
-          for (int j = 0; j < 3; ++j) u += b[sp][j] * (H[hidx(k, j)] * X + d[k] * Yj[j]);
-          q[k] += 2.0 * u;
-          // meta-GGAs: tau moves with the functions through d_k d_j phi
-          if (mgga)
-            for (int j = 0; j < 3; ++j) q[k] += ct[sp] * H[hidx(k, j)] * Yj[j];
+          double u = d[k] * V;
+          for (int j = 0; j < 3; ++j) u += b[sp][j] * H[hidx(k, j)] * X;
+          qa[k] += 2.0 * u;
         }
+        continue;
+      }
+      double Yj[3];
+      for (int j = 0; j < 3; ++j) Yj[j] = xy[(1 + j) * plane];
+      for (int k = 0; k < 3; ++k) {
+        double u = 0.0;
+        for (int j = 0; j < 3; ++j) u += b[sp][j] * (H[hidx(k, j)] * X + d[k] * Yj[j]);
+        qa[k] += 2.0 * u;
+        // meta-GGAs: tau moves with the functions through d_k d_j phi
+        for (int j = 0; j < 3; ++j) qa[k] += ct[sp] * H[hidx(k, j)] * Yj[j];
       }
     }
-    for (int k = 0; k < 3; ++k) {
-      t[k] += q[k];
-      double v = q[k];
-      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-      if (lane == 0 && v != 0.0) atomicAdd(&gq[3 * (f - f0) + k], v);
-    }
   }
+  flush();
   // host sums: one shared atomic per warp when its points share a host
-  const int h = live ? owner[p0 + p] : -1;
+  const int h = owner[t * 128 + threadIdx.x];
   const int h0 = __shfl_sync(0xffffffffu, h, 0);
-  if (__all_sync(0xffffffffu, h == h0) && h0 >= 0) {
+  if (__all_sync(0xffffffffu, h == h0)) {
     for (int k = 0; k < 3; ++k) {
-      double v = t[k];
+      double v = tot[k];
       for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-      if (lane == 0) atomicAdd(&gh[3 * h0 + k], v);
+      if (lane == 0) atomicAdd(&gs[3 * h0 + k], v);
     }
-  } else if (live) {
-    for (int k = 0; k < 3; ++k) atomicAdd(&gh[3 * h + k], t[k]);
+  } else {
+    for (int k = 0; k < 3; ++k) atomicAdd(&gs[3 * h + k], tot[k]);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 3 * (int)(f1 - f0); i += blockDim.x)
-    if (gq[i] != 0.0) atomicAdd(grad + 3 * fatom[f0 + i / 3] + i % 3, -gq[i]);
-  for (int i = threadIdx.x; i < 3 * natm; i += blockDim.x)
-    if (gh[i] != 0.0) atomicAdd(grad + i, gh[i]);
+  for (int i = threadIdx.x; i < 3 * natm; i += 128)
+    if (gs[i] != 0.0) atomicAdd(grad + i, gs[i]);
 }
 
 // Thread per point.  Pass 1 stores, per atom b, the point's distance d_b,
@@ -601,81 +638,57 @@ __global__ void __launch_bounds__(128) k_grad_weights(const double* __restrict__
     if (G[i] != 0.0) atomicAdd(grad + i, G[i]);
 }
 
-// X (component 0) or Y_j (components 1..3) = (d_j Phi) P on the FP64 tensor
-// pipe (DMMA): C[f][p] = sum_g A[g][p] P[g][f] for f < nbas, with the 64 x 64
-// tile engine of dgemm.cuh (A: basis component rows of ld points, P: ldc x
-// ldc, zero past nbas).  K runs to nbas rounded up to 16: the rows read past
-// nbas belong to the next basis plane and meet P's zero rows.
-__global__ void __launch_bounds__(kGemmThreads) k_grad_xy(const double* __restrict__ A, int64_t ld,
-                                                         const double* __restrict__ P, int64_t ldc, int64_t nbas,
-                                                         int64_t kend, double* __restrict__ C) {
-  extern __shared__ double smem[];
-  const int64_t m0 = (int64_t)blockIdx.x * 64, n0 = (int64_t)blockIdx.y * 64;
-  Acc acc;
-  acc.zero();
-  gemm_tile<false, false>(acc, A, ld, m0, P, ldc, n0, 0, kend, smem);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm0 = (warp >> 1) * 32, wn0 = (warp & 1) * 32;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int64_t p = m0 + wm0 + i * 8 + (lane >> 2);
-        const int64_t f = n0 + wn0 + j * 8 + 2 * (lane & 3) + e;
-        if (f < nbas) C[f * ld + p] = acc.v[i][j][e];
-      }
-}
-
-template <int L>
-void launch_hess_l(const BuildArgs& a, int64_t p0, int64_t nvalid, int64_t ld, int64_t plane, double* out,
-                   cudaStream_t st) {
-  if (a.nshl[L] == 0) return;
-  dim3 grid((unsigned)((ld + 127) / 128), (unsigned)a.nshl[L]);
-  k_basis_hess<L><<<grid, 128, 0, st>>>(a.shells, a.shl[L], a.atoms, a.exps, a.norms, a.contr, a.rng, a.sa, a.px, a.py,
-                                        a.pz, p0, nvalid, ld, plane, out);
-}
-
 }  // namespace
 
-void launch_basis_hess(const BuildArgs& a, int64_t p0, int64_t nvalid, int64_t ld, int64_t plane, double* out,
-                       cudaStream_t st) {
-  launch_hess_l<0>(a, p0, nvalid, ld, plane, out, st);
-  launch_hess_l<1>(a, p0, nvalid, ld, plane, out, st);
-  launch_hess_l<2>(a, p0, nvalid, ld, plane, out, st);
-  launch_hess_l<3>(a, p0, nvalid, ld, plane, out, st);
+int64_t grad_planes(bool gga, bool mgga, int ispin) {
+  return mgga ? 10 + 4 * ispin : gga ? 11 + 2 * ispin : 4 + ispin;
 }
 
-void launch_grad_points(const XcConst& K, int functional, bool gga, int ispin, int64_t nbas, int64_t ld, int64_t p0,
-                        int64_t nvalid, const double* w, const double* wraw, const double* basis, int64_t plane,
-                        const double* XY, double* coef, double* ef, double* exc, cudaStream_t st) {
-  k_grad_points<<<(unsigned)((ld + 127) / 128), 128, 0, st>>>(K, functional, gga, ispin, nbas, ld, p0, nvalid, w,
-                                                               wraw, basis, plane, XY, coef, ef, exc);
-}
-
-void launch_grad_orbital(bool gga, bool mgga, int ispin, int64_t nbas, int64_t ld, int64_t p0, int64_t nvalid,
-                         int natm, const int* fatom, const int* owner, const double* basis, int64_t plane,
-                         const double* XY, const double* coef, double* grad, cudaStream_t st) {
-  const size_t smem = sizeof(double) * 3 * (kGradFB + natm);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_grad_orb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid((unsigned)((nbas + kGradFB - 1) / kGradFB), (unsigned)((ld + 255) / 256));
-  k_grad_orb<<<grid, 256, smem, st>>>(gga, mgga, ispin, nbas, ld, p0, nvalid, natm, fatom, owner, basis, plane, XY,
-                                      coef, grad);
-}
-
-void launch_grad_w(int64_t nbas, int64_t ld, const double* basis, int64_t plane, const double* coef_b, double* W,
-                   cudaStream_t st) {
-  const int64_t n = round_up(nbas, 16) * ld;
-  k_grad_w<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nbas, round_up(nbas, 16), ld, basis, plane, coef_b, W);
-}
-
-void launch_grad_xy(const double* basis_j, int64_t ld, const double* P, int64_t ldc, int64_t nbas, double* out,
-                    cudaStream_t st) {
-  constexpr int smem = gemm_smem_bytes<false, false>();
-  cudaFuncSetAttribute(k_grad_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  const dim3 grid((unsigned)(ld / 64), (unsigned)((nbas + 63) / 64));
-  k_grad_xy<<<grid, kGemmThreads, smem, st>>>(basis_j, ld, P, ldc, nbas, round_up(nbas, 16), out);
+void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan* sp, size_t c, cudaStream_t st) {
+  const int64_t t0 = sp->chunk_t0[c], nt = sp->chunk_t0[c + 1] - t0, s0 = sp->h_tso[(size_t)t0], ld = g.ld;
+  const int64_t plane = g.plane;
+  double* B = g.rows;                                  // phi, grad phi and (GGAs) the Hessian
+  double* XY = B + (g.gga ? 10 : 4) * plane;           // per spin X; X, V (GGA); X, Y_j (meta-GGA)
+  const int nxy = g.mgga ? 4 : g.gga ? 2 : 1;
+  double* W = XY + (int64_t)nxy * g.ispin * plane;
+  const BasisIO<double> io{a.exps, a.norms, a.contr,  a.rng,   a.prim,  sp->qx,  sp->qy, sp->qz,
+                           s0,     t0,      nullptr, nullptr, nullptr, nullptr, nullptr};
+  auto hess = [&](auto Lc) {
+    constexpr int L = decltype(Lc)::value;
+    const BasisItem* it = sp->items[L] + sp->tile_item[L][(size_t)t0];
+    const int64_t n = sp->tile_item[L][(size_t)(t0 + nt)] - sp->tile_item[L][(size_t)t0];
+    if (n > 0)
+      k_hess_items<L><<<(unsigned)std::min<int64_t>(n, (int64_t)sp->nsm * 32), 128, 0, st>>>(it, n, io, a.sa, g.gga,
+                                                                                             plane, B);
+  };
+  hess(std::integral_constant<int, 0>());
+  hess(std::integral_constant<int, 1>());
+  hess(std::integral_constant<int, 2>());
+  hess(std::integral_constant<int, 3>());
+  k_grad_pads<<<(unsigned)nt, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, g.mgga ? 4 : 1, plane, B);
+  const double *gx = B + plane, *gy = B + 2 * plane, *gz = B + 3 * plane;
+  for (int s = 0; s < g.ispin; ++s) {
+    double* d = g.den + (int64_t)(7 * s) * ld;
+    double* X = XY + (int64_t)(nxy * s) * plane;
+    grad_contract(sp, t0, nt, s0, B, g.gga ? gx : nullptr, gy, gz, g.P[s], a.ldc, X, d, d + ld, d + 2 * ld, d + 3 * ld,
+                  st);
+    // the Y_j only for meta-GGAs (tau and its terms), GGAs take V = W P after the coefficients
+    for (int j = 0; j < 3 && g.mgga; ++j)
+      grad_contract(sp, t0, nt, s0, B + (1 + j) * plane, nullptr, nullptr, nullptr, g.P[s], a.ldc, X + (1 + j) * plane,
+                    d + (4 + j) * ld, nullptr, nullptr, nullptr, st);
+  }
+  k_grad_coef<<<(unsigned)nt, 128, 0, st>>>(a.xc, g.functional, g.gga, g.ispin, ld, sp->qw + t0 * 128,
+                                            sp->qwraw + t0 * 128, g.den, g.coef, g.ef + t0 * 128, g.exc);
+  for (int s = 0; s < g.ispin && g.gga && !g.mgga; ++s) {
+    k_grad_w<<<(unsigned)nt, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, B, plane,
+                                           g.coef + (int64_t)(kCoefPlanes * s + 1) * ld, ld, W);
+    grad_contract(sp, t0, nt, s0, W, nullptr, nullptr, nullptr, g.P[s], a.ldc, XY + (int64_t)(nxy * s + 1) * plane,
+                  g.den, nullptr, nullptr, nullptr, st);  // (rho is done with: its sum goes to scratch)
+  }
+  const int smem = (int)sizeof(double) * 3 * g.natm;
+  if (smem > 48 * 1024) raise_smem_limit(k_grad_orb, smem);
+  k_grad_orb<<<(unsigned)nt, 128, smem, st>>>(g.gga, g.mgga, g.ispin, g.natm, sp->tso, sp->listed, sp->slot_fn, t0, s0,
+                                              g.fatom, sp->qowner, B, plane, XY, nxy, g.coef, ld, g.grad);
 }
 
 void launch_grad_weights(const double* atoms, const double* dist, int natm, const double* px, const double* py,

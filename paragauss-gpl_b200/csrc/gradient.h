@@ -7,7 +7,7 @@
 // gradients with moving grid and weight gradients (post_scf_module.f90
 // :2930-3060, density_calc_ph_nl, grid_module.f90 becke1).
 //
-// With X^s = Phi P^s and Y^s_j = d_j Phi P^s (per chunk of points),
+// With X^s = Phi P^s and Y^s_j = d_j Phi P^s (per tile of points, its listed functions),
 //   q^s_mu,k(g) = 2 [a_s d_k phi_mu X^s_mu + sum_j b_sj (d_k d_j phi_mu X^s_mu + d_k phi_mu Y^s_j,mu)],
 // a_s = w df/drho_s and b_s = w (2 df/dgamma_ss grad rho_s + df/dgamma_ab grad rho_s'), the
 // orbital terms are  -sum_g q_mu(g) to atom(mu)  and  +sum_mu q_mu(g) to host(g);
@@ -21,34 +21,29 @@
 
 namespace pgxc {
 
-// Basis values, gradients and Hessians of every function on points
-// [p0, p0 + nvalid) of the context's grid: out[c * plane + f * ld + p],
-// c = 0 phi, 1..3 d/dx, d/dy, d/dz, 4..9 xx, xy, xz, yy, yz, zz.
-void launch_basis_hess(const BuildArgs& a, int64_t p0, int64_t nvalid, int64_t ld, int64_t plane, double* out,
-                       cudaStream_t st);
+struct ScreenPlan;
 
-// Per point of the chunk: rho_s, grad rho_s (and for meta-GGAs tau_s) from X,
-// Y and the basis values, the functional, and the coefficients a_s, b_s, c_s
-// (coef[(5 s + c) ld + p]; c_s = w df/dtau_s, 0 below meta-GGAs) and
-// ef = w_raw f; E_xc = sum w f is added into *exc.
-// out[f][p] = sum_g basis_j[g][p] P[g][f], f < nbas, p < ld (ld a multiple of
-// 64; basis_j followed by at least 15 more rows of ld; P ldc x ldc, zero past nbas)
-void launch_grad_xy(const double* basis_j, int64_t ld, const double* P, int64_t ldc, int64_t nbas, double* out,
-                    cudaStream_t st);
-void launch_grad_points(const XcConst& K, int functional, bool gga, int ispin, int64_t nbas, int64_t ld, int64_t p0,
-                        int64_t nvalid, const double* w, const double* wraw, const double* basis, int64_t plane,
-                        const double* XY, double* coef, double* ef, double* exc, cudaStream_t st);
+// [slot][128] planes of a chunk: phi, grad phi, (GGAs) Hessian, and the products
+int64_t grad_planes(bool gga, bool mgga, int ispin);
 
-// GGAs (not meta-GGAs): W = sum_j b_j d_j phi of the chunk (coef_b: the three
-// b planes of one spin), rows nbas .. round_up(nbas, 16) - 1 zero; the orbital
-// terms then take V = W P (plane 2 of the spin) in place of the three Y_j.
-void launch_grad_w(int64_t nbas, int64_t ld, const double* basis, int64_t plane, const double* coef_b, double* W,
-                   cudaStream_t st);
-
-// The orbital terms: -sum_g q to atom(mu) (fatom[mu]) and +sum_mu q to host(g).
-void launch_grad_orbital(bool gga, bool mgga, int ispin, int64_t nbas, int64_t ld, int64_t p0, int64_t nvalid,
-                         int natm, const int* fatom, const int* owner, const double* basis, int64_t plane,
-                         const double* XY, const double* coef, double* grad, cudaStream_t st);
+// One gradient's buffers and kind.
+struct GradChunk {
+  bool gga, mgga;            // meta-GGAs set both
+  int ispin, functional, natm;
+  const double* P[2];        // density matrices, leading dimension BuildArgs::ldc
+  const int* fatom;          // atom of each function
+  double* rows;              // grad_planes planes of `plane` doubles
+  int64_t plane;
+  int64_t ld;                // points of the largest chunk
+  double* den;               // 7 ispin ld: rho, grad rho, 2 tau_j
+  double* coef;              // 5 ispin ld: a, b, c
+  double* ef;                // w_raw f of every point of the plan
+  double* exc;               // sum w f is added
+  double* grad;              // the orbital terms are added
+};
+// The orbital terms of chunk c of the plan (grad_plan_create): -sum_g q to atom(mu)
+// and +sum_mu q to host(g); also ef and E_xc.
+void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan* sp, size_t c, cudaStream_t st);
 
 // The weight term sum_g ef_g dW_host(r_g)/dR over the chunk's points; dist is
 // the natm x natm atom distance matrix followed by its reciprocals (the

@@ -20,6 +20,7 @@
 #include "mixed.h"
 #include "pgxc_common.cuh"
 #include "screened.h"
+#include "screened_plan.h"
 #include "symmetry.h"
 
 using namespace pgxc;
@@ -75,6 +76,9 @@ struct pgxc_ctx {
   double* d_raw = nullptr;      // host builds' orbitals and occupations as the caller passed them
   int64_t raw_cap = 0;
   double* d_eacc = nullptr;     // {E, cE, N, cN} per functional of pgxc_xc_energies
+  std::vector<double> grad_r2;     // listing radii of the exact (threshold 0) lists of the gradient
+  std::vector<int> grad_r2off;
+  ScreenPlan* gplan = nullptr;  // tiles and lists of pgxc_xc_gradient, made by the first call
   void* grad_scr = nullptr;     // scratch of pgxc_xc_gradient, kept across calls (grows only)
   size_t grad_scr_bytes = 0;
   int eacc_cap = 0;
@@ -192,6 +196,7 @@ void pgxc_destroy(pgxc_ctx* c) {
   if (c->screen) screen_destroy(c->screen);
   delete c->sym;
   for (void* p : c->allocs) cudaFree(p);
+  if (c->gplan) screen_destroy(c->gplan);
   if (c->grad_scr) cudaFree(c->grad_scr);
   if (c->h_ham) cudaFreeHost(c->h_ham);
   if (c->h_acc) cudaFreeHost(c->h_acc);
@@ -497,6 +502,7 @@ int create_impl(const pgxc_geometry* geo, const pgxc_basis* bas, const pgxc_grid
     if ((st = dalloc(c, &c->d_wraw, n))) return fail(st);
     CUDA_TRY(c, cudaMemcpy(c->d_wraw, dgrid + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToDevice));
     c->d_owner = downer;
+    screen_listing_radii(c->shells, bas->exponents, bas->norms, bas->contractions, 0.0, a.sa, c->grad_r2, c->grad_r2off);
     CUDA_TRY(c, launch_becke(datoms, c->d_dist, c->natm, a.px, a.py, a.pz, downer, n, dbecke, c->stream));
     launch_scale_inplace(dgrid + 3 * n, dbecke, n, c->stream);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -989,23 +995,31 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   std::vector<int> fatom((size_t)nbas);
   for (const DevShell& S : c->shells)
     for (int f = 0; f < (2 * S.l + 1) * S.nrad; ++f) fatom[(size_t)S.f0 + f] = S.atom;
-  // chunk of points: 10 basis planes + 4 ispin X/Y planes of nbas x ld, under ~4 GB
-  int64_t ld = 65536;
-  while (ld > 128 && (double)(10 + 4 * ispin) * nbas * ld * 8.0 > 4.0e9) ld /= 2;
-  const int64_t plane = (int64_t)nbas * ld;
-  // The weight term needs only each point's w_raw f (ef, kept for the whole
-  // grid: whole chunks of ld, which k_grad_points fills to the end) and runs after the chunk loop in launches of ldw points, as many as
-  // its per-(atom, point) scratch of 3.5 natm ldw doubles allows under ~2 GB:
-  // far more blocks than one basis chunk would give (its per-point loops over
-  // atom pairs are long, and a few blocks per SM leave it latency-bound).
-  int64_t ldw = round_up(c->npts, 128);
+  const bool mgga = PGXC_XC_IS_MGGA(c->opt.functional);
+  const bool gga = PGXC_XC_IS_GGA(c->opt.functional) || mgga;
+  const int64_t planes = grad_planes(gga, mgga, ispin);
+  if (!c->gplan) {
+    // tiles and lists, once per context (its threshold does not matter: every function that is not
+    // identically zero on a tile is listed), in chunks of under ~4 GB of slot rows
+    std::string e;
+    const int st = grad_plan_create(&c->gplan, a, c->natm, c->npts, c->shells, c->grad_r2, c->grad_r2off, c->d_wraw,
+                                    c->d_owner, (int64_t)(4.0e9 / (1024.0 * planes)), s, e);
+    if (st) return set_err(c, st, "gradient plan: " + e);
+  }
+  const ScreenPlan* gp = c->gplan;
+  const int64_t nq = gp->ntiles * 128, ld = gp->chunk_tiles * 128;
+  const int64_t plane = (gp->chunk_slots + kSlack) * 128;
+  // The weight term needs only each point's w_raw f and runs after the chunk loop in launches of ldw
+  // points, as many as its per-(atom, point) scratch of 3.5 natm ldw doubles allows under ~2 GB (its
+  // per-point loops over atom pairs are long, and a few blocks per SM leave it latency-bound).
+  int64_t ldw = nq;
   while (ldw > 128 && 28.0 * c->natm * ldw > 2.0e9) ldw = round_up(ldw / 2, 128);
   // one scratch buffer, carved in 256-byte aligned pieces and kept in the
   // context for the next call (allocation and release of several GB per call
   // would cost more than the gradient's kernels)
-  const size_t sizes[8] = {sizeof(double) * 10 * plane,         sizeof(double) * 4 * ispin * plane,
-                           sizeof(double) * 5 * ispin * ld,      sizeof(double) * (size_t)round_up(c->npts, ld),
-                           sizeof(double) * 3 * c->natm,         sizeof(double),
+  const size_t sizes[8] = {sizeof(double) * (size_t)(planes * plane), sizeof(double) * 7 * ispin * (size_t)ld,
+                           sizeof(double) * 5 * ispin * (size_t)ld,   sizeof(double) * (size_t)nq,
+                           sizeof(double) * 3 * c->natm,              sizeof(double),
                            sizeof(double) * ((size_t)7 * c->natm * ldw / 2 + 1), sizeof(int) * (size_t)nbas};
   size_t offs[8], total = 0;
   for (int i = 0; i < 8; ++i) {
@@ -1024,16 +1038,25 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     c->grad_scr_bytes = total;
   }
   char* base = (char*)c->grad_scr;
-  double* basis = (double*)(base + offs[0]);
-  double* XY = (double*)(base + offs[1]);
-  double* coef = (double*)(base + offs[2]);
-  double* ef = (double*)(base + offs[3]);
-  double* dgrad = (double*)(base + offs[4]);
-  double* de = (double*)(base + offs[5]);
+  GradChunk g;
+  g.gga = gga;
+  g.mgga = mgga;
+  g.ispin = ispin;
+  g.functional = c->opt.functional;
+  g.natm = c->natm;
+  g.P[0] = a.P;
+  g.P[1] = c->P2;
+  g.rows = (double*)(base + offs[0]);
+  g.plane = plane;
+  g.ld = ld;
+  g.den = (double*)(base + offs[1]);
+  g.coef = (double*)(base + offs[2]);
+  double* ef = g.ef = (double*)(base + offs[3]);
+  double* dgrad = g.grad = (double*)(base + offs[4]);
+  double* de = g.exc = (double*)(base + offs[5]);
   double* wscr = (double*)(base + offs[6]);
   int* dfatom = (int*)(base + offs[7]);
-  const bool mgga = PGXC_XC_IS_MGGA(c->opt.functional);
-  const bool gga = PGXC_XC_IS_GGA(c->opt.functional) || mgga;
+  g.fatom = dfatom;
   int rc = PGXC_OK;
   do {
     if (cudaMemcpyAsync(dfatom, fatom.data(), sizeof(int) * nbas, cudaMemcpyHostToDevice, s) != cudaSuccess ||
@@ -1042,35 +1065,10 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
       rc = set_err(c, PGXC_ECUDA, "gradient set-up copies failed");
       break;
     }
-    for (int64_t p0 = 0; p0 < c->npts && rc == PGXC_OK; p0 += ld) {
-      const int64_t nv = std::min<int64_t>(ld, c->npts - p0);
-      launch_basis_hess(a, p0, nv, ld, plane, basis, s);
-      for (int sp = 0; sp < ispin; ++sp) {
-        const double* P = sp ? c->P2 : a.P;
-        // X (j = 0) or Y_j = (d_j Phi) P: (ld x nbas) = (ld x nbas)(nbas x nbas), P symmetric; the
-        // Y_j only for meta-GGAs (tau and its terms), GGAs take V = W P after the coefficients
-        for (int j = 0; j < (mgga ? 4 : 1); ++j)
-          launch_grad_xy(basis + j * plane, ld, P, a.ldc, nbas, XY + (4 * sp + j) * plane, s);
-      }
-      if (rc) break;
-      launch_grad_points(a.xc, c->opt.functional, gga, ispin, nbas, ld, p0, nv, a.w, c->d_wraw, basis, plane, XY,
-                         coef, ef + p0, de, s);
-      if (gga && !mgga)
-        for (int sp = 0; sp < ispin; ++sp) {
-          double* W = XY + (4 * sp + 1) * plane;
-          launch_grad_w(nbas, ld, basis, plane, coef + (5 * sp + 1) * ld, W, s);
-          launch_grad_xy(W, ld, sp ? c->P2 : a.P, a.ldc, nbas, XY + (4 * sp + 2) * plane, s);
-        }
-      launch_grad_orbital(gga, mgga, ispin, nbas, ld, p0, nv, c->natm, dfatom, c->d_owner, basis, plane, XY, coef,
-                          dgrad, s);
-      if (cudaGetLastError() != cudaSuccess) rc = set_err(c, PGXC_ECUDA, "gradient kernel launch failed");
-    }
-    if (rc) break;
-    for (int64_t p0 = 0; p0 < c->npts; p0 += ldw) {
-      const int64_t nv = std::min<int64_t>(ldw, c->npts - p0);
-      launch_grad_weights(a.atoms, c->d_dist, c->natm, a.px, a.py, a.pz, c->d_owner, p0, nv, ldw, ef + p0, wscr,
-                          dgrad, s);
-    }
+    for (size_t ch = 0; ch + 1 < gp->chunk_t0.size(); ++ch) launch_grad_chunk(g, a, gp, ch, s);
+    for (int64_t p0 = 0; p0 < nq; p0 += ldw)
+      launch_grad_weights(a.atoms, c->d_dist, c->natm, gp->qx, gp->qy, gp->qz, gp->qowner, p0,
+                          std::min<int64_t>(ldw, nq - p0), ldw, ef + p0, wscr, dgrad, s);
     if (cudaGetLastError() != cudaSuccess) rc = set_err(c, PGXC_ECUDA, "gradient kernel launch failed");
     if (rc) break;
     std::vector<double> hg((size_t)3 * c->natm);

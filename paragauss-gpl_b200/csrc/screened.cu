@@ -321,16 +321,18 @@ __device__ __forceinline__ void load_sfn(int* sfn, const int* __restrict__ slot_
 // tri (GGA = false: only rho, a quadratic form): P is symmetric, so column
 // block J takes the rows of the blocks before it doubled and its own block, half
 // the products.  Grid z selects the operand plane and its sum (the three tau
-// sums of a meta-GGA in one launch).
+// sums of a meta-GGA in one launch).  STORE: X itself is written too (the
+// gradient's terms).
 // Three CTAs per SM: 60 atoms, 304 of 690 functions per tile (226 GF, 6.4 ms at
 // the pipe's rate) 10.8 -> 8.9 ms against one 128-thread CTA form that kept two
 // CTAs at 254 registers; four CTAs at 128 registers 9.2, 32-deep stages 9.4.
-template <bool GGA>
+template <bool GGA, bool STORE = false>
 __global__ void __launch_bounds__(kSThreads, 3)
     k_sdensity(SPlanes pl, const double* __restrict__ gx, const double* __restrict__ gy,
                const double* __restrict__ gz, const int64_t* __restrict__ tso, const int* __restrict__ listed,
                int64_t t0, int64_t s0, const int* __restrict__ slot_fn, const double* __restrict__ P, int64_t ldc,
-               bool tri, double* __restrict__ grx, double* __restrict__ gry, double* __restrict__ grz) {
+               bool tri, double* __restrict__ grx, double* __restrict__ gry, double* __restrict__ grz,
+               double* __restrict__ X = nullptr) {
   extern __shared__ double smem[];
   constexpr int E = kDK * kDLd;  // one operand of a stage
   static_assert(kSBlk * kXLd <= 2 * kDStages * E, "the X block lies in the stages");
@@ -413,6 +415,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
     for (int c = kq; c < cn; c += 2) {
       const double x = sX[c * kXLd + col];
       const int64_t o = o0 + c * 128;
+      if (STORE) X[o] = x;
       r += x * phi[o];
       if (GGA) {
         g[0] += x * gx[o];
@@ -632,6 +635,139 @@ double listing_r2(const DevShell& S, int rr, const double* exps, const double* n
 
 }  // namespace
 
+void screen_listing_radii(const std::vector<DevShell>& shells, const double* exps, const double* norms,
+                          const double* contr, double threshold, const DevSA& sa, std::vector<double>& R2,
+                          std::vector<int>& r2off) {
+  double sa_fac[kMaxL + 1];
+  for (int l = 0; l <= kMaxL; ++l) {
+    sa_fac[l] = 1.0;
+    if (!sa.identity)
+      for (int i = 0; i < 2 * l + 1; ++i) {
+        double s = 0.0;
+        for (int m = 0; m < 2 * l + 1; ++m) s += std::fabs(sa.c[l][i][m]);
+        sa_fac[l] = std::max(sa_fac[l], s);
+      }
+  }
+  for (const DevShell& S : shells) {
+    r2off.push_back((int)R2.size());
+    for (int rr = 0; rr < S.nrad; ++rr) R2.push_back(listing_r2(S, rr, exps, norms, contr, threshold, sa_fac[S.l]));
+  }
+}
+
+// The tiles and their lists: Morton-ordered points, per tile the listed
+// functions (those whose listing radius exceeds the tile's distance to their
+// atom) and the basis items.  perm: the Morton order is kept in it (caller
+// frees) when not null.
+static int build_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
+                       const std::vector<double>& R2, const std::vector<int>& r2off, int64_t** perm, cudaStream_t st,
+                       std::string& err) {
+#define BL_TRY(call, what)                                                       \
+  do {                                                                           \
+    cudaError_t e_ = (call);                                                     \
+    if (e_ != cudaSuccess) {                                                     \
+      err = std::string(what) + ": " + cudaGetErrorString(e_);                   \
+      return e_ == cudaErrorMemoryAllocation ? PGXC_ENOMEM : PGXC_ECUDA;         \
+    }                                                                            \
+  } while (0)
+  const int nsh = (int)shells.size();
+  // --- Morton-ordered, 128-point tiles -----------------------------------
+  const int64_t n = npts;
+  const int64_t ntiles = (n + 127) / 128;
+  sp->ntiles = ntiles;
+  {
+    // Morton order of the points, on the device (ties by point index)
+    const int64_t nq = ntiles * 128;
+    int64_t* dperm;
+    BL_TRY(cudaMalloc(&dperm, sizeof(int64_t) * nq), "cudaMalloc");
+    cudaError_t e = morton_perm_device(a.px, a.py, a.pz, n, nq, dperm, st);
+    if (e == cudaSuccess) e = sp_alloc(sp, &sp->qx, 4 * nq);
+    if (e == cudaSuccess) {
+      sp->qy = sp->qx + nq;
+      sp->qz = sp->qx + 2 * nq;
+      sp->qw = sp->qx + 3 * nq;
+      k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(dperm, nq, a.px, a.py, a.pz, a.w, sp->qx,
+                                                                   sp->qy, sp->qz, sp->qw);
+      e = cudaStreamSynchronize(st);
+    }
+    if (perm && e == cudaSuccess) *perm = dperm;
+    else cudaFree(dperm);
+    BL_TRY(e, "grid reordering");
+  }
+  // --- per-tile lists, on the device: distances, counts, then (their places known) the lists.  On the
+  // host the lists of a 41-atom grid (2,710 tiles, 170,000 items of 80 bytes, copied from pageable
+  // memory) were most of the 30 ms of a context's creation.
+  std::vector<int64_t> tso((size_t)ntiles + 1, 0);
+  std::vector<int> listed_t((size_t)ntiles, 0);
+  {
+    constexpr int kCnt = 2 + kMaxL;
+    float* dd2 = nullptr;
+    double* dR2 = nullptr;
+    int *dr2off = nullptr, *dcnt = nullptr;
+    int64_t* dstart = nullptr;
+    std::vector<int> cnt((size_t)ntiles * kCnt);
+    std::vector<int64_t> start((size_t)ntiles * (kMaxL + 1));
+    auto plan = [&]() -> cudaError_t {
+#define PL_TRY(call)                      \
+  do {                                    \
+    cudaError_t e_ = (call);              \
+    if (e_ != cudaSuccess) return e_;     \
+  } while (0)
+      // one scratch allocation for the five tables
+      const size_t n8 = (size_t)ntiles * (kMaxL + 1) + std::max<size_t>(R2.size(), 1);
+      const size_t n4 = (size_t)ntiles * natm + (size_t)ntiles * kCnt + (size_t)nsh;
+      PL_TRY(cudaMalloc(&dstart, 8 * n8 + 4 * n4));
+      dR2 = (double*)(dstart + (size_t)ntiles * (kMaxL + 1));
+      dd2 = (float*)(dstart + n8);
+      dcnt = (int*)(dd2 + (size_t)ntiles * natm);
+      dr2off = dcnt + (size_t)ntiles * kCnt;
+      PL_TRY(cudaMemcpyAsync(dR2, R2.data(), sizeof(double) * R2.size(), cudaMemcpyHostToDevice, st));
+      PL_TRY(cudaMemcpyAsync(dr2off, r2off.data(), sizeof(int) * r2off.size(), cudaMemcpyHostToDevice, st));
+      k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, natm, dd2);
+      k_plan_count<<<(unsigned)ntiles, 128, 0, st>>>(dd2, natm, a.shells, nsh, dR2, dr2off, dcnt);
+      PL_TRY(cudaGetLastError());
+      PL_TRY(cudaMemcpyAsync(cnt.data(), dcnt, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, st));
+      PL_TRY(cudaStreamSynchronize(st));
+      int64_t items[kMaxL + 1] = {};
+      for (int l = 0; l <= kMaxL; ++l) sp->tile_item[l].assign((size_t)ntiles + 1, 0);
+      for (int64_t t = 0; t < ntiles; ++t) {
+        const int* c = &cnt[(size_t)t * kCnt];
+        listed_t[(size_t)t] = c[0];
+        const int nt = (c[0] + kSlotAlign - 1) / kSlotAlign * kSlotAlign;
+        sp->nlisted += c[0];
+        sp->sum_n2 += (double)c[0] * (double)c[0];
+        sp->max_n = std::max(sp->max_n, nt);
+        tso[(size_t)t + 1] = tso[(size_t)t] + nt;
+        for (int l = 0; l <= kMaxL; ++l) {
+          start[(size_t)t * (kMaxL + 1) + l] = items[l];
+          items[l] += c[1 + l];
+          sp->tile_item[l][(size_t)t + 1] = items[l];
+        }
+      }
+      sp->nslots = tso[(size_t)ntiles];
+      PL_TRY(sp_alloc(sp, &sp->tso, tso.size()));
+      PL_TRY(sp_alloc(sp, &sp->listed, listed_t.size()));
+      PL_TRY(sp_alloc(sp, &sp->slot_fn, (size_t)sp->nslots));
+      for (int l = 0; l <= kMaxL; ++l) PL_TRY(sp_alloc(sp, &sp->items[l], (size_t)items[l]));
+      PL_TRY(cudaMemcpyAsync(sp->tso, tso.data(), sizeof(int64_t) * tso.size(), cudaMemcpyHostToDevice, st));
+      PL_TRY(cudaMemcpyAsync(sp->listed, listed_t.data(), sizeof(int) * listed_t.size(), cudaMemcpyHostToDevice, st));
+      PL_TRY(cudaMemcpyAsync(dstart, start.data(), sizeof(int64_t) * start.size(), cudaMemcpyHostToDevice, st));
+      PlanItems out{};
+      for (int l = 0; l <= kMaxL; ++l) out.items[l] = sp->items[l];
+      k_plan_fill<<<(unsigned)ntiles, 128, 0, st>>>(dd2, natm, a.atoms, a.shells, nsh, dR2, dr2off, sp->tso, dstart,
+                                                    sp->slot_fn, out);
+      PL_TRY(cudaGetLastError());
+      return cudaStreamSynchronize(st);
+#undef PL_TRY
+    };
+    const cudaError_t e = plan();
+    cudaFree(dstart);
+    BL_TRY(e, "tile lists");
+  }
+  sp->h_tso = std::move(tso);
+  return PGXC_OK;
+#undef BL_TRY
+}
+
 void screen_destroy(ScreenPlan* sp) {
   if (!sp) return;
   if (sp->mixed) screen_mixed_destroy(sp->mixed);
@@ -693,119 +829,18 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     SP_TRY(cudaGetDevice(&dev), "cudaGetDevice");
     SP_TRY(cudaDeviceGetAttribute(&sp->nsm, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
   }
-  // --- Morton-ordered, 128-point tiles -----------------------------------
-  const int64_t n = in.npts;
-  const int64_t ntiles = (n + 127) / 128;
-  sp->ntiles = ntiles;
+  // --- tiles and lists ----------------------------------------------------
   {
-    // Morton order of the points, on the device (ties by point index)
-    const int64_t nq = ntiles * 128;
-    int64_t* dperm;
-    SP_TRY(cudaMalloc(&dperm, sizeof(int64_t) * nq), "cudaMalloc");
-    cudaError_t e = morton_perm_device(a.px, a.py, a.pz, n, nq, dperm, st);
-    if (e == cudaSuccess) e = sp_alloc(sp, &sp->qx, 4 * nq);
-    if (e == cudaSuccess) {
-      sp->qy = sp->qx + nq;
-      sp->qz = sp->qx + 2 * nq;
-      sp->qw = sp->qx + 3 * nq;
-      k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(dperm, nq, a.px, a.py, a.pz, a.w, sp->qx,
-                                                                   sp->qy, sp->qz, sp->qw);
-      e = cudaStreamSynchronize(st);
+    std::vector<double> R2;
+    std::vector<int> r2off;
+    screen_listing_radii(shells, in.exps, in.norms, in.contr, in.threshold, a.sa, R2, r2off);
+    if (const int st2 = build_lists(sp, a, in.natm, in.npts, shells, R2, r2off, nullptr, st, err)) {
+      screen_destroy(sp);
+      return st2;
     }
-    cudaFree(dperm);
-    SP_TRY(e, "grid reordering");
   }
-  // --- listing radii -------------------------------------------------------
-  double sa_fac[kMaxL + 1];
-  for (int l = 0; l <= kMaxL; ++l) {
-    sa_fac[l] = 1.0;
-    if (!a.sa.identity)
-      for (int i = 0; i < 2 * l + 1; ++i) {
-        double s = 0.0;
-        for (int m = 0; m < 2 * l + 1; ++m) s += std::fabs(a.sa.c[l][i][m]);
-        sa_fac[l] = std::max(sa_fac[l], s);
-      }
-  }
-  const int nsh = (int)shells.size();
-  std::vector<double> R2;
-  std::vector<int> r2off((size_t)nsh);
-  for (int s = 0; s < nsh; ++s) {
-    const DevShell& S = shells[(size_t)s];
-    r2off[(size_t)s] = (int)R2.size();
-    for (int rr = 0; rr < S.nrad; ++rr)
-      R2.push_back(listing_r2(S, rr, in.exps, in.norms, in.contr, in.threshold, sa_fac[S.l]));
-  }
-  // --- per-tile lists, on the device: distances, counts, then (their places known) the lists.  On the
-  // host the lists of a 41-atom grid (2,710 tiles, 170,000 items of 80 bytes, copied from pageable
-  // memory) were most of the 30 ms of a context's creation.
-  std::vector<int64_t> tso((size_t)ntiles + 1, 0);
-  std::vector<int> listed_t((size_t)ntiles, 0);
-  {
-    constexpr int kCnt = 2 + kMaxL;
-    float* dd2 = nullptr;
-    double* dR2 = nullptr;
-    int *dr2off = nullptr, *dcnt = nullptr;
-    int64_t* dstart = nullptr;
-    std::vector<int> cnt((size_t)ntiles * kCnt);
-    std::vector<int64_t> start((size_t)ntiles * (kMaxL + 1));
-    auto plan = [&]() -> cudaError_t {
-#define PL_TRY(call)                      \
-  do {                                    \
-    cudaError_t e_ = (call);              \
-    if (e_ != cudaSuccess) return e_;     \
-  } while (0)
-      // one scratch allocation for the five tables
-      const size_t n8 = (size_t)ntiles * (kMaxL + 1) + std::max<size_t>(R2.size(), 1);
-      const size_t n4 = (size_t)ntiles * in.natm + (size_t)ntiles * kCnt + (size_t)nsh;
-      PL_TRY(cudaMalloc(&dstart, 8 * n8 + 4 * n4));
-      dR2 = (double*)(dstart + (size_t)ntiles * (kMaxL + 1));
-      dd2 = (float*)(dstart + n8);
-      dcnt = (int*)(dd2 + (size_t)ntiles * in.natm);
-      dr2off = dcnt + (size_t)ntiles * kCnt;
-      PL_TRY(cudaMemcpyAsync(dR2, R2.data(), sizeof(double) * R2.size(), cudaMemcpyHostToDevice, st));
-      PL_TRY(cudaMemcpyAsync(dr2off, r2off.data(), sizeof(int) * r2off.size(), cudaMemcpyHostToDevice, st));
-      k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, in.natm, dd2);
-      k_plan_count<<<(unsigned)ntiles, 128, 0, st>>>(dd2, in.natm, a.shells, nsh, dR2, dr2off, dcnt);
-      PL_TRY(cudaGetLastError());
-      PL_TRY(cudaMemcpyAsync(cnt.data(), dcnt, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, st));
-      PL_TRY(cudaStreamSynchronize(st));
-      int64_t items[kMaxL + 1] = {};
-      for (int l = 0; l <= kMaxL; ++l) sp->tile_item[l].assign((size_t)ntiles + 1, 0);
-      for (int64_t t = 0; t < ntiles; ++t) {
-        const int* c = &cnt[(size_t)t * kCnt];
-        listed_t[(size_t)t] = c[0];
-        const int nt = (c[0] + kSlotAlign - 1) / kSlotAlign * kSlotAlign;
-        sp->nlisted += c[0];
-        sp->sum_n2 += (double)c[0] * (double)c[0];
-        sp->max_n = std::max(sp->max_n, nt);
-        tso[(size_t)t + 1] = tso[(size_t)t] + nt;
-        for (int l = 0; l <= kMaxL; ++l) {
-          start[(size_t)t * (kMaxL + 1) + l] = items[l];
-          items[l] += c[1 + l];
-          sp->tile_item[l][(size_t)t + 1] = items[l];
-        }
-      }
-      sp->nslots = tso[(size_t)ntiles];
-      PL_TRY(sp_alloc(sp, &sp->tso, tso.size()));
-      PL_TRY(sp_alloc(sp, &sp->listed, listed_t.size()));
-      PL_TRY(sp_alloc(sp, &sp->slot_fn, (size_t)sp->nslots));
-      for (int l = 0; l <= kMaxL; ++l) PL_TRY(sp_alloc(sp, &sp->items[l], (size_t)items[l]));
-      PL_TRY(cudaMemcpyAsync(sp->tso, tso.data(), sizeof(int64_t) * tso.size(), cudaMemcpyHostToDevice, st));
-      PL_TRY(cudaMemcpyAsync(sp->listed, listed_t.data(), sizeof(int) * listed_t.size(), cudaMemcpyHostToDevice, st));
-      PL_TRY(cudaMemcpyAsync(dstart, start.data(), sizeof(int64_t) * start.size(), cudaMemcpyHostToDevice, st));
-      PlanItems out{};
-      for (int l = 0; l <= kMaxL; ++l) out.items[l] = sp->items[l];
-      k_plan_fill<<<(unsigned)ntiles, 128, 0, st>>>(dd2, in.natm, a.atoms, a.shells, nsh, dR2, dr2off, sp->tso, dstart,
-                                                    sp->slot_fn, out);
-      PL_TRY(cudaGetLastError());
-      return cudaStreamSynchronize(st);
-#undef PL_TRY
-    };
-    const cudaError_t e = plan();
-    cudaFree(dstart);
-    SP_TRY(e, "tile lists");
-  }
-  sp->h_tso = tso;
+  const std::vector<int64_t>& tso = sp->h_tso;
+  const int64_t ntiles = sp->ntiles;
   // --- chunks -------------------------------------------------------------------
   const bool mixed = in.precision != PGXC_PREC_FP64;
   size_t freeb = 0, totb = 0;
@@ -919,6 +954,72 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
   }
   *out = sp;
   return PGXC_OK;
+}
+
+namespace {
+// raw weight (0 for padding) and host atom of the Morton-ordered points
+__global__ void k_gather_hosts(const int64_t* __restrict__ perm, int64_t nq, const double* __restrict__ wraw,
+                               const int* __restrict__ owner, double* __restrict__ qwraw, int* __restrict__ qowner) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nq) return;
+  const int64_t i = perm[q];
+  qwraw[q] = i >= 0 ? wraw[i] : 0.0;
+  qowner[q] = owner[i >= 0 ? i : perm[q & ~(int64_t)127]];
+}
+}  // namespace
+
+int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
+                     const std::vector<double>& R2, const std::vector<int>& r2off, const double* wraw,
+                     const int* owner, int64_t max_rows, cudaStream_t st, std::string& err) {
+  *out = nullptr;
+  ScreenPlan* sp = new ScreenPlan();
+  SP_TRY(cudaGetDevice(&sp->nsm), "cudaGetDevice");
+  SP_TRY(cudaDeviceGetAttribute(&sp->nsm, cudaDevAttrMultiProcessorCount, sp->nsm), "cudaDeviceGetAttribute");
+  int64_t* perm = nullptr;
+  if (const int st2 = build_lists(sp, a, natm, npts, shells, R2, r2off, &perm, st, err)) {
+    cudaFree(perm);
+    screen_destroy(sp);
+    return st2;
+  }
+  const int64_t nq = sp->ntiles * 128;
+  cudaError_t e = sp_alloc(sp, &sp->qwraw, nq);
+  if (e == cudaSuccess) e = sp_alloc(sp, &sp->qowner, nq);
+  if (e == cudaSuccess) {
+    k_gather_hosts<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(perm, nq, wraw, owner, sp->qwraw, sp->qowner);
+    e = cudaStreamSynchronize(st);
+  }
+  cudaFree(perm);
+  SP_TRY(e, "gradient plan");
+  max_rows = std::max<int64_t>(max_rows, sp->max_n);
+  sp->chunk_t0.push_back(0);
+  for (int64_t t = 1; t <= sp->ntiles; ++t) {
+    const int64_t t0 = sp->chunk_t0.back();
+    if (t == sp->ntiles || sp->h_tso[(size_t)t + 1] - sp->h_tso[(size_t)t0] > max_rows) sp->chunk_t0.push_back(t);
+  }
+  for (size_t c = 0; c + 1 < sp->chunk_t0.size(); ++c) {
+    const int64_t t0 = sp->chunk_t0[c], t1 = sp->chunk_t0[c + 1];
+    sp->chunk_tiles = std::max(sp->chunk_tiles, t1 - t0);
+    sp->chunk_slots = std::max(sp->chunk_slots, sp->h_tso[(size_t)t1] - sp->h_tso[(size_t)t0]);
+  }
+  *out = sp;
+  return PGXC_OK;
+}
+
+void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
+                   const double* gy, const double* gz, const double* P, int64_t ldc, double* X, double* rho,
+                   double* grx, double* gry, double* grz, cudaStream_t st) {
+  const int smem = sdensity_smem(sp->max_n);
+  const SPlanes pl{F, F, F, rho, rho, rho};
+  const dim3 grid((unsigned)nt, 2);
+  if (gx) {
+    raise_smem_limit(k_sdensity<true, true>, smem);
+    k_sdensity<true, true><<<grid, kSThreads, smem, st>>>(pl, gx, gy, gz, sp->tso, sp->listed, t0, s0, sp->slot_fn, P,
+                                                          ldc, false, grx, gry, grz, X);
+  } else {
+    raise_smem_limit(k_sdensity<false, true>, smem);
+    k_sdensity<false, true><<<grid, kSThreads, smem, st>>>(pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0,
+                                                           sp->slot_fn, P, ldc, false, nullptr, nullptr, nullptr, X);
+  }
 }
 
 int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_t st, double* ham, ScreenTimes* tm,

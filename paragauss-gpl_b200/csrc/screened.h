@@ -53,6 +53,10 @@ struct ScreenInput {
 
 int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, cudaStream_t st, std::string& err);
 void screen_destroy(ScreenPlan* sp);
+// Squared listing radius of every radial function (shell s: R2[r2off[s] ...]).
+void screen_listing_radii(const std::vector<DevShell>& shells, const double* exps, const double* norms,
+                          const double* contr, double threshold, const DevSA& sa, std::vector<double>& R2,
+                          std::vector<int>& r2off);
 // One build: the FP64 density matrices must be ready (a.P; for an open shell
 // also Pb, the second spin's, with the same leading dimension a.ldc); E_xc /
 // N_el are Kahan-added into a.acc; the packed matrix (both spins interleaved

@@ -56,7 +56,22 @@ struct ScreenPlan {
   std::vector<std::array<cudaEvent_t, 9>> cev;  // timing events of each chunk (made by the first timed build)
   int nsm = 148;
   std::vector<void*> allocs;
+  // gradient plans: raw weight and host atom of the Morton-ordered points
+  double* qwraw = nullptr;
+  int* qowner = nullptr;
 };
+
+// A plan of tiles and lists alone (no build buffers), in chunks of at most
+// max_rows slot rows, for the nuclear gradient; R2 with threshold 0, so that
+// unlisted functions and their derivatives are exactly zero on the tile.
+int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
+                     const std::vector<double>& R2, const std::vector<int>& r2off, const double* wraw,
+                     const int* owner, int64_t max_rows, cudaStream_t st, std::string& err);
+// X = F_t P[S_t, S_t] of the chunk's tiles ([slot][128] rows, padding rows of F
+// zero), with rho[p] = sum X F and (gx not null) gr[p] = 2 sum X grad phi.
+void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
+                   const double* gy, const double* gz, const double* P, int64_t ldc, double* X, double* rho,
+                   double* grx, double* gry, double* grz, cudaStream_t st);
 
 
 }  // namespace pgxc

@@ -54,3 +54,43 @@ def test_unsymmetric_density_matrix():
     # rounding of sums of products up to max|A| rho-sized terms
     assert abs(got[1] - ref[1]) < 1e-9 and abs(got[2] - ref[2]) < 1e-9
     assert float(np.max(np.abs(got[0] - ref[0]))) < 1e-8
+
+
+# the gradient on compact tiles: a shell with bare primitives only (not segmented), the most radial
+# functions a shell may have, and the block sizes
+def _wide(c, nrad):
+    """The case's first shell replaced by nrad bare primitives."""
+    ne, nc = int(c.shell_nexp[0]), int(c.shell_ncontr[0])
+    e = np.exp(np.linspace(np.log(0.2), np.log(60.0), nrad))
+    c.exponents = np.concatenate([e, c.exponents[ne:]])
+    c.norms = np.concatenate([cases.primitive_norm(int(c.shell_l[0]), e), c.norms[ne:]])
+    c.contractions = c.contractions[ne * nc:]
+    for a, v in ((c.shell_nexp, nrad), (c.shell_nunc, nrad), (c.shell_ncontr, 0)):
+        a[0] = v
+    c.nbas += nrad - nc
+    rng = np.random.default_rng(5)
+    c.C = rng.normal(size=(c.nbas, c.nocc, c.ispin)) / c.nbas
+    return c
+
+
+@pytest.mark.parametrize("nrad,threshold", [(5, 0.0), (64, -1.0)])
+@pytest.mark.parametrize("functional", ["VWN", "PBE"])
+def test_gradient_of_unsegmented_shells(functional, nrad, threshold):
+    c = _wide(cases.small_case(functional, seed=66, natoms=4, nrad=12, nang=50, nocc=5), nrad)
+    ref, re = O.xc_gradient(c)
+    with lib.Context(c, weighted=False, screen_threshold=threshold) as ctx:
+        g, e = ctx.xc_gradient()
+    scale = max(1.0, float(np.max(np.abs(ref))))
+    assert abs(e - re) < 1e-10 * max(1.0, abs(re))
+    np.testing.assert_allclose(g, ref, rtol=0, atol=1e-10 * scale)
+
+
+@pytest.mark.parametrize("natoms,lmax", [(3, 0), (5, 3), (9, 3), (12, 2)])
+def test_gradient_block_remainders(natoms, lmax):
+    c = cases.small_case("PBE", seed=40 + natoms, natoms=natoms, nrad=9, nang=26, nocc=max(2, natoms), lmax=lmax)
+    ref, re = O.xc_gradient(c)
+    with lib.Context(c, weighted=False, screen_threshold=1e-10) as ctx:
+        g, e = ctx.xc_gradient()
+    scale = max(1.0, float(np.max(np.abs(ref))))
+    assert abs(e - re) < 1e-10 * max(1.0, abs(re))
+    np.testing.assert_allclose(g, ref, rtol=0, atol=1e-10 * scale)
