@@ -291,10 +291,9 @@ __global__ void __launch_bounds__(128) k_basis_l(const DevShell* __restrict__ sh
 //
 // An item carries every field its evaluation needs (atom position, primitive
 // and contraction offsets), so that the loads of the next item do not depend
-// on one another.  A block walks a contiguous range of items; the next item's
-// record is loaded (whole 16-byte words, the same for every lane) while the
-// current one is evaluated, and consecutive items of a tile reuse the point
-// coordinates.
+// on one another.  A block walks contiguous ranges of items (records as whole
+// 16-byte words, the same for every lane); consecutive items of a tile reuse the
+// point coordinates.
 // ---------------------------------------------------------------------------
 struct BasisItem {
   double ax, ay, az;        // words 0-5: atom position
@@ -321,14 +320,10 @@ __device__ __forceinline__ void load_item(BasisItem& it, const BasisItem* __rest
 
 // GT: the element type of the gradient planes (double; float in the INT8
 // build, whose potential and density gradient tolerate 24-bit gradients).
-// Blocks per SM: with gradients 6, 5, 4, 4 for l = 0..3 (at most 80, 96, 128
-// and 128 registers), without them 8, 8, 8, 7.  Without a bound the f-shell
-// kernel took 164 registers and ran three blocks per SM, the slower form for
-// the 500-atom grid; a bound of one block lets the compiler take 144-188
-// registers for l <= 2, which cost the 60-atom build 0.6 ms.
+// Blocks per SM that the registers are bounded for.
 template <int L, bool GRAD>
 constexpr int basis_blocks() {
-  return GRAD ? (L == 0 ? 6 : (L == 1 ? 5 : 4)) : (L <= 2 ? 8 : 7);
+  return GRAD ? (L == 0 ? 5 : L == 1 ? 4 : 4) : (L <= 1 ? 5 : 7);
 }
 // The tables and point arrays of a launch.
 template <typename GT>
@@ -345,75 +340,126 @@ struct BasisIO {
   unsigned long long* pmax;
 };
 
-// Items [i0, i1) by one block.  Bound by instruction issue (2.9 of 4 per
-// cycle with lane-broadcast records and primitives, every primitive of a shell
-// looked at for every function): so of a segmented shell only the primitives
-// that reach some point of the warp are visited, a bit mask made once per item
-// from the warp's smallest r^2; their exponent and coefficient (the norm folded
-// in) come as one 16-byte load; and the largest |phi| takes one step per radial
-// function (max_k fl(|Y_k| |R|) = fl(max_k |Y_k| |R|)).
+// Points per thread: two consecutive ones for s and p functions (16-byte stores,
+// and what an item and a primitive cost besides arithmetic is paid once for two
+// points, whose chains run side by side), one for d and f functions, whose values
+// would take 230 registers and more (60 atoms: basis phase 2.31 ms, 2.35 with two
+// points for d too).
+template <int L>
+constexpr int kBasisPts = L <= 1 ? 2 : 1;
+
+template <int N, typename T>
+__device__ __forceinline__ void put_points(T* p, const double (&v)[N]) {
+  if constexpr (N == 1) *p = (T)v[0];
+  else if constexpr (sizeof(T) == 8) *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+  else *reinterpret_cast<float2*>(p) = make_float2((float)v[0], (float)v[1]);
+}
+template <int N>
+__device__ __forceinline__ void get_points(const double* p, double (&v)[N]) {
+  if constexpr (N == 1) {
+    v[0] = __ldg(p);
+  } else {
+    const double2 d = __ldg(reinterpret_cast<const double2*>(p));
+    v[0] = d.x;
+    v[1] = d.y;
+  }
+}
+
+// Items [i0, i1) by 128 / kBasisPts threads (whole warps; p0: the thread's
+// first point).  Bound by instruction issue (2.9 of 4 per cycle with one point
+// per thread, lane-broadcast records and every primitive of a shell looked at
+// for every function): so of a segmented shell only the primitives that reach
+// some point of the warp are visited, a bit mask made once per item from the
+// warp's smallest r^2; their exponent and coefficient (the norm folded in) come
+// as one 16-byte load; and the largest |phi| takes one step per radial function
+// (max_k fl(|Y_k| |R|) = fl(max_k |Y_k| |R|)).
+// 60 atoms, threshold 0 (2.77 million listed functions x 128 points, 11.4 GB
+// written): 3.20 -> 2.93 ms with these, 2.31 with two points per thread.
 template <int L, bool GRAD, typename GT>
-__device__ __forceinline__ void basis_items(const BasisItem* __restrict__ items, int64_t i0, int64_t i1,
+__device__ __forceinline__ void basis_items(const BasisItem* __restrict__ items, int64_t i0, int64_t i1, int p0,
                                             const BasisIO<GT>& io, const DevSA& sa) {
   if (i0 >= i1) return;
+  constexpr int N = kBasisPts<L>, M = 2 * L + 1;
   const int lane = threadIdx.x & 31;
-  BasisItem it;
-  load_item(it, items + i0);
-  double px = __ldg(io.qx + (int64_t)it.tile * 128 + threadIdx.x);
-  double py = __ldg(io.qy + (int64_t)it.tile * 128 + threadIdx.x);
-  double pz = __ldg(io.qz + (int64_t)it.tile * 128 + threadIdx.x);
-  double tmax = 0.0;
+  double px[N], py[N], pz[N], tmax[N] = {};
+  auto points = [&](int tile) {
+    const int64_t q = (int64_t)tile * 128 + p0;
+    get_points(io.qx + q, px);
+    get_points(io.qy + q, py);
+    get_points(io.qz + q, pz);
+  };
+  points(__ldg(&items[i0].tile));
   for (int64_t i = i0; i < i1; ++i) {
-    BasisItem nx;
-    load_item(nx, items + min(i + 1, i1 - 1));
-    const double x = px - it.ax, y = py - it.ay, z = pz - it.az;
-    const double r2 = x * x + y * y + z * z;
+    BasisItem it;
+    load_item(it, items + i);
+    // the next item's tile: also what brings its record into L1 a whole item ahead
+    const int ntile = __ldg(&items[min(i + 1, i1 - 1)].tile);
     const int nsel = it.nsig, nexp = it.nexp;
+    double x[N], y[N], z[N], r2[N], Ys[N][M], dYs[N][3][M], ymax[N], vmax[N] = {};
+    float rmin = __int_as_float(0x7f800000);
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      x[u] = px[u] - it.ax;
+      y[u] = py[u] - it.ay;
+      z[u] = pz[u] - it.az;
+      r2[u] = x[u] * x[u] + y[u] * y[u] + z[u] * z[u];
+      rmin = fminf(rmin, __double2float_rd(r2[u]));
+      double Y[16];
+      double dY[3][16];
+      solid_harmonics<L, double>(x[u], y[u], z[u], Y, dY);
+      ymax[u] = 0.0;
+#pragma unroll
+      for (int k = 0; k < M; ++k) {
+        if (sa.identity) {
+          Ys[u][k] = Y[L * L + k];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) dYs[u][c][k] = dY[c][L * L + k];
+        } else {
+          double v = 0, g0 = 0, g1 = 0, g2 = 0;
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            const double cf = sa.c[L][k][m];
+            v += cf * Y[L * L + m];
+            g0 += cf * dY[0][L * L + m];
+            g1 += cf * dY[1][L * L + m];
+            g2 += cf * dY[2][L * L + m];
+          }
+          Ys[u][k] = v; dYs[u][0][k] = g0; dYs[u][1][k] = g1; dYs[u][2][k] = g2;
+        }
+        ymax[u] = fmax(ymax[u], fabs(Ys[u][k]));
+      }
+    }
     // the primitives (of the first 32) with alpha r^2 < 50 somewhere in the warp
     unsigned live = 0;
     if (it.seg && nexp <= 32) {
-      const float rmin = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(__double2float_rd(r2))));
+      rmin = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(rmin)));
       const bool on = lane < nexp && __ldg(io.exps + it.exp_off + min(lane, nexp - 1)) * (double)rmin < 50.0;
       live = __ballot_sync(0xffffffffu, on);
     }
-    double Y[16];
-    double dY[3][16];
-    solid_harmonics<L, double>(x, y, z, Y, dY);
-    double Ys[2 * L + 1], dYs[3][2 * L + 1], ymax = 0.0;
-#pragma unroll
-    for (int k = 0; k < 2 * L + 1; ++k) {
-      if (sa.identity) {
-        Ys[k] = Y[L * L + k];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) dYs[c][k] = dY[c][L * L + k];
-      } else {
-        double v = 0, g0 = 0, g1 = 0, g2 = 0;
-#pragma unroll
-        for (int m = 0; m < 2 * L + 1; ++m) {
-          const double cf = sa.c[L][k][m];
-          v += cf * Y[L * L + m];
-          g0 += cf * dY[0][L * L + m];
-          g1 += cf * dY[1][L * L + m];
-          g2 += cf * dY[2][L * L + m];
-        }
-        Ys[k] = v; dYs[0][k] = g0; dYs[1][k] = g1; dYs[2][k] = g2;
-      }
-      ymax = fmax(ymax, fabs(Ys[k]));
-    }
-    const int64_t row0 = (it.slot - io.s0) * 128 + threadIdx.x;
-    double vmax = 0.0;
+    const int64_t row0 = (it.slot - io.s0) * 128 + p0;
     // radial function k of the item: its 2 L + 1 functions
-    auto store = [&](int k, double Rv, double dRv) {
-      vmax = fmax(vmax, fabs(Rv));
+    auto store = [&](int k, const double (&R)[N], const double (&dR)[N]) {
 #pragma unroll
-      for (int m = 0; m < 2 * L + 1; ++m) {
+      for (int u = 0; u < N; ++u) vmax[u] = fmax(vmax[u], fabs(R[u]));
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
         const int64_t o = row0 + (m * nsel + k) * 128;
-        io.phi[o] = Ys[m] * Rv;
+        double v[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) v[u] = Ys[u][m] * R[u];
+        put_points(io.phi + o, v);
         if (GRAD) {
-          const double h = Ys[m] * dRv;
-          io.gx[o] = (GT)(x * h + dYs[0][m] * Rv);
-          io.gy[o] = (GT)(y * h + dYs[1][m] * Rv);
-          io.gz[o] = (GT)(z * h + dYs[2][m] * Rv);
+          double g[3][N];
+#pragma unroll
+          for (int u = 0; u < N; ++u) {
+            const double h = Ys[u][m] * dR[u];
+            g[0][u] = x[u] * h + dYs[u][0][m] * R[u];
+            g[1][u] = y[u] * h + dYs[u][1][m] * R[u];
+            g[2][u] = z[u] * h + dYs[u][2][m] * R[u];
+          }
+          put_points(io.gx + o, g[0]);
+          put_points(io.gy + o, g[1]);
+          put_points(io.gz + o, g[2]);
         }
       }
     };
@@ -425,13 +471,16 @@ __device__ __forceinline__ void basis_items(const BasisItem* __restrict__ items,
         const int rr = __ffsll((long long)rem) - 1;
         rem &= rem - 1;
         const int2 rg = __ldg(io.rng + it.rad_off + rr);
-        double Rr = 0.0, dR = 0.0;
+        double R[N] = {}, dR[N] = {};
         auto add = [&](int e) {
           const double2 p = __ldg(pr + e);
-          const double ar2 = p.x * r2;
-          const double v = ar2 < 50.0 ? p.y * exp(-ar2) : 0.0;
-          Rr += v;
-          dR += (-2.0 * p.x) * v;
+#pragma unroll
+          for (int u = 0; u < N; ++u) {
+            const double ar2 = p.x * r2[u];
+            const double v = ar2 < 50.0 ? p.y * exp(-ar2) : 0.0;
+            R[u] += v;
+            dR[u] += (-2.0 * p.x) * v;
+          }
         };
         if (nexp <= 32) {
           unsigned m = rg.y > rg.x ? live & (0xffffffffu >> (32 - (rg.y - rg.x))) << rg.x : 0u;
@@ -439,83 +488,80 @@ __device__ __forceinline__ void basis_items(const BasisItem* __restrict__ items,
         } else {
           for (int e = rg.x; e < rg.y; ++e) add(e);
         }
-        store(k, Rr, dR);
+        store(k, R, dR);
       }
     } else {
-      for (int k0 = 0; k0 < nsel; k0 += kRadGroup) {
-        int rr[kRadGroup];
+      // general contractions: each radial function over all primitives (bare ones: its own)
+      for (int k = 0; k < nsel; ++k) {
+        const int rr = __ffsll((long long)rem) - 1;
+        rem &= rem - 1;
+        const bool bare = rr < it.nunc;
+        const double* cc = io.contr + it.con_off + (int64_t)nexp * (rr - it.nunc);
+        double R[N] = {}, dR[N] = {};
+        for (int e = bare ? rr : 0; e < (bare ? rr + 1 : nexp); ++e) {
+          const double alpha = __ldg(io.exps + it.exp_off + e), nrm = __ldg(io.norms + it.exp_off + e);
+          const double cf = bare ? 1.0 : __ldg(cc + e);
 #pragma unroll
-        for (int r = 0; r < kRadGroup; ++r) {
-          if (k0 + r < nsel) {
-            rr[r] = __ffsll((long long)rem) - 1;
-            rem &= rem - 1;
-          } else {
-            rr[r] = -1;
+          for (int u = 0; u < N; ++u) {
+            const double v = prim_value(alpha, nrm, r2[u]);
+            R[u] += cf * v;
+            dR[u] += cf * ((-2.0 * alpha) * v);
           }
         }
-        double Rr[kRadGroup], dR[kRadGroup];
-#pragma unroll
-        for (int r = 0; r < kRadGroup; ++r) { Rr[r] = 0.0; dR[r] = 0.0; }
-        for (int e = 0; e < nexp; ++e) {
-          const double alpha = __ldg(io.exps + it.exp_off + e);
-          const double v = prim_value(alpha, __ldg(io.norms + it.exp_off + e), r2);
-          const double dv = (-2.0 * alpha) * v;
-#pragma unroll
-          for (int r = 0; r < kRadGroup; ++r) {
-            if (rr[r] >= 0) {
-              const double cf = rr[r] < it.nunc ? (e == rr[r] ? 1.0 : 0.0)
-                                                : __ldg(io.contr + it.con_off + e + (int64_t)nexp * (rr[r] - it.nunc));
-              Rr[r] += cf * v;
-              dR[r] += cf * dv;
-            }
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < kRadGroup; ++r)
-          if (rr[r] >= 0) store(k0 + r, Rr[r], dR[r]);
+        store(k, R, dR);
       }
     }
     // largest |phi| of each point over the tile's functions, max-reduced once per run of
     // items of one tile (non-negative doubles order like their bits)
-    tmax = fmax(tmax, ymax * vmax);
-    if (io.pmax && (nx.tile != it.tile || i + 1 == i1)) {
-      atomicMax(io.pmax + ((int64_t)it.tile - io.t0) * 128 + threadIdx.x,
-                (unsigned long long)__double_as_longlong(tmax));
-      tmax = 0.0;
+#pragma unroll
+    for (int u = 0; u < N; ++u) tmax[u] = fmax(tmax[u], ymax[u] * vmax[u]);
+    if (io.pmax && (ntile != it.tile || i + 1 == i1)) {
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        atomicMax(io.pmax + ((int64_t)it.tile - io.t0) * 128 + p0 + u,
+                  (unsigned long long)__double_as_longlong(tmax[u]));
+        tmax[u] = 0.0;
+      }
     }
-    if (nx.tile != it.tile) {
-      const int64_t qn = (int64_t)nx.tile * 128 + threadIdx.x;
-      px = __ldg(io.qx + qn); py = __ldg(io.qy + qn); pz = __ldg(io.qz + qn);
-    }
-    it = nx;
+    if (ntile != it.tile) points(ntile);
   }
+}
+
+// One block of 128 threads: kBasisPts<L> item ranges side by side (range `v` of
+// `ranges`, `per` items each).
+template <int L, bool GRAD, typename GT>
+__device__ __forceinline__ void basis_block(const BasisItem* __restrict__ items, int64_t nitems, int64_t per,
+                                            unsigned block, const BasisIO<GT>& io, const DevSA& sa) {
+  constexpr int N = kBasisPts<L>, T = 128 / N;  // threads of an item
+  const int64_t i0 = ((int64_t)block * N + threadIdx.x / T) * per;
+  basis_items<L, GRAD, GT>(items, i0, min(nitems, i0 + per), (int)(threadIdx.x % T) * N, io, sa);
 }
 
 template <int L, bool GRAD, typename GT>
 __global__ void __launch_bounds__(128, (basis_blocks<L, GRAD>()))
     k_basis_items(const BasisItem* __restrict__ items, int64_t nitems, BasisIO<GT> io, DevSA sa) {
-  const int64_t per = (nitems + gridDim.x - 1) / gridDim.x;
-  const int64_t i0 = (int64_t)blockIdx.x * per;
-  basis_items<L, GRAD, GT>(items, i0, min(nitems, i0 + per), io, sa);
+  constexpr int N = kBasisPts<L>;
+  const int64_t ranges = (int64_t)gridDim.x * N;
+  basis_block<L, GRAD, GT>(items, nitems, (nitems + ranges - 1) / ranges, blockIdx.x, io, sa);
 }
 
-// The same for every l in one launch, one item per block: grids of few tiles,
+// The same for every l in one launch, one item per range: grids of few tiles,
 // where each launch is one short wave and the launches one after another are
-// what takes the time.  n.v[l] items of each l.
+// what takes the time.  n.v[l] blocks for the n.n[l] items of each l.
 struct BasisCounts {
   const BasisItem* items[kMaxL + 1];
-  unsigned v[kMaxL + 1];
+  unsigned n[kMaxL + 1], v[kMaxL + 1];
 };
 template <bool GRAD, typename GT>
-__global__ void __launch_bounds__(128, 4) k_basis_small(BasisCounts n, BasisIO<GT> io, DevSA sa) {
+__global__ void __launch_bounds__(128, 3) k_basis_small(BasisCounts n, BasisIO<GT> io, DevSA sa) {
   unsigned b = blockIdx.x;
-  if (b < n.v[0]) return basis_items<0, GRAD, GT>(n.items[0], b, b + 1, io, sa);
+  if (b < n.v[0]) return basis_block<0, GRAD, GT>(n.items[0], n.n[0], 1, b, io, sa);
   b -= n.v[0];
-  if (b < n.v[1]) return basis_items<1, GRAD, GT>(n.items[1], b, b + 1, io, sa);
+  if (b < n.v[1]) return basis_block<1, GRAD, GT>(n.items[1], n.n[1], 1, b, io, sa);
   b -= n.v[1];
-  if (b < n.v[2]) return basis_items<2, GRAD, GT>(n.items[2], b, b + 1, io, sa);
+  if (b < n.v[2]) return basis_block<2, GRAD, GT>(n.items[2], n.n[2], 1, b, io, sa);
   b -= n.v[2];
-  basis_items<3, GRAD, GT>(n.items[3], b, b + 1, io, sa);
+  basis_block<3, GRAD, GT>(n.items[3], n.n[3], 1, b, io, sa);
 }
 
 // Basis values of a chunk: items[l][0 .. n[l]).  One launch per l, blocks that
@@ -528,18 +574,22 @@ int launch_basis_items(const BasisItem* const (&items)[kMaxL + 1], const int64_t
   if (all == 0) return 0;
   if (all <= most) {
     BasisCounts c;
+    constexpr int pts[kMaxL + 1] = {kBasisPts<0>, kBasisPts<1>, kBasisPts<2>, kBasisPts<3>};
+    unsigned blocks = 0;
     for (int l = 0; l <= kMaxL; ++l) {
       c.items[l] = items[l];
-      c.v[l] = (unsigned)n[l];
+      c.n[l] = (unsigned)n[l];
+      blocks += c.v[l] = (unsigned)((n[l] + pts[l] - 1) / pts[l]);
     }
-    k_basis_small<GRAD, GT><<<(unsigned)all, 128, 0, st>>>(c, io, sa);
+    k_basis_small<GRAD, GT><<<blocks, 128, 0, st>>>(c, io, sa);
     return 1;
   }
   int launches = 0;
   auto one = [&](auto Lc) {
     constexpr int L = decltype(Lc)::value;
     if (n[L] == 0) return;
-    k_basis_items<L, GRAD, GT><<<(unsigned)(n[L] < most ? n[L] : most), 128, 0, st>>>(items[L], n[L], io, sa);
+    const int64_t nb = (n[L] + kBasisPts<L> - 1) / kBasisPts<L>;
+    k_basis_items<L, GRAD, GT><<<(unsigned)(nb < most ? nb : most), 128, 0, st>>>(items[L], n[L], io, sa);
     ++launches;
   };
   one(std::integral_constant<int, 0>());

@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(128) k_grad_weights(const double* __restrict__
       const double sxy = __dmul_rn(0.5, __dsub_rn(1.0, q3)), syx = __dmul_rn(0.5, __dadd_rn(1.0, q3));
       // leave-one-out products of rows x (without y) and y (without x)
       const double Lxy = zx == -1 ? (sxy != 0.0 ? pnx / sxy : 0.0) : (zx == y ? pnx : 0.0);
-      const double pny = spnz[y * ld + p];
+      const double pny = ly ? spnz[y * ld + p] : 0.0;
       const double Lyx = zy == -1 ? (syx != 0.0 ? pny / syx : 0.0) : (zy == x ? pny : 0.0);
       const double cy = e * ((y == h ? 1.0 : 0.0) - Wh) * iZ;
       const double kxy = cx * Lxy * ds, kyx = cy * Lyx * ds;
