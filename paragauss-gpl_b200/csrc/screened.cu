@@ -316,8 +316,8 @@ __device__ __forceinline__ void load_sfn(int* sfn, const int* __restrict__ slot_
 // K3 (screened): CTA = (tile, half of its 128 points).  X = phi_t P[S_t, S_t]
 // in 64-wide column blocks, P gathered element-wise by 8-byte cp.async (thread
 // = one column, every second row of a stage); each finished block of X passes
-// through shared memory so that a thread then owns one point: the phi and grad phi it meets are read in whole rows and the sums take
-// 4 registers.
+// through shared memory so that a thread then owns one point: the phi and grad phi
+// it meets are read in whole rows and the sums take 4 registers.
 // tri (GGA = false: only rho, a quadratic form): P is symmetric, so column
 // block J takes the rows of the blocks before it doubled and its own block, half
 // the products.  Grid z selects the operand plane and its sum (the three tau
@@ -326,6 +326,8 @@ __device__ __forceinline__ void load_sfn(int* sfn, const int* __restrict__ slot_
 // Three CTAs per SM: 60 atoms, 304 of 690 functions per tile (226 GF, 6.4 ms at
 // the pipe's rate) 10.8 -> 8.9 ms against one 128-thread CTA form that kept two
 // CTAs at 254 registers; four CTAs at 128 registers 9.2, 32-deep stages 9.4.
+// The sums' loop has eight slots' loads in flight: 8.9 -> 8.7 ms against four
+// (20 atoms meta-GGA 1.04 -> 1.01).
 template <bool GGA, bool STORE = false>
 __global__ void __launch_bounds__(kSThreads, 3)
     k_sdensity(SPlanes pl, const double* __restrict__ gx, const double* __restrict__ gy,
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
     __syncthreads();
     const int cn = min(kSBlk, nl - n0);
     const int64_t o0 = (sb + n0) * 128 + m0 + col;
-#pragma unroll 4
+#pragma unroll 8
     for (int c = kq; c < cn; c += 2) {
       const double x = sX[c * kXLd + col];
       const int64_t o = o0 + c * 128;
