@@ -799,6 +799,26 @@ void screen_stats(const ScreenPlan* sp, int64_t* ntiles, int64_t* nslots, int64_
     }                                                                            \
   } while (0)
 
+// Even tile lists of every chunk [t0[c], t0[c + 1]) (screen_mixed_order) on the device.
+template <typename Alloc>
+static cudaError_t make_order(const int64_t* tso, const std::vector<int64_t>& t0, int nsm, std::vector<char>& used,
+                              Alloc alloc, int** order, int** start) {
+  const size_t nch = t0.size() - 1;
+  std::vector<int> ho((size_t)t0.back()), hs(nch * (size_t)(nsm + 1));
+  used.assign(nch, 0);
+  bool any = false;
+  for (size_t c = 0; c < nch; ++c) {
+    used[c] = screen_mixed_order(tso + t0[c], t0[c + 1] - t0[c], nsm, ho.data() + t0[c], hs.data() + c * (nsm + 1));
+    any = any || used[c];
+  }
+  if (!any) return cudaSuccess;
+  cudaError_t e = alloc(order, ho.size());
+  if (e == cudaSuccess) e = alloc(start, hs.size());
+  if (e == cudaSuccess) e = cudaMemcpy(*order, ho.data(), sizeof(int) * ho.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(*start, hs.data(), sizeof(int) * hs.size(), cudaMemcpyHostToDevice);
+  return e;
+}
+
 int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, cudaStream_t st, std::string& err) {
   *out = nullptr;
   ScreenPlan* sp = new ScreenPlan();
@@ -948,6 +968,9 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     SP_TRY(sp_alloc(sp, &sp->b_off, boff.size()), "cudaMalloc");
     SP_TRY(cudaMemcpy(sp->b_off, boff.data(), sizeof(int64_t) * boff.size(), cudaMemcpyHostToDevice), "copy");
     mi.b_off = sp->b_off;
+    SP_TRY(make_order(tso.data(), sp->chunk_t0, sp->nsm, sp->ordered, [&](int** p, size_t k) { return sp_alloc(sp, p, k); },
+                      &sp->order, &sp->order_start),
+           "tile order");
     const int st2 = screen_mixed_create(&sp->mixed, mi, err);
     if (st2) {
       screen_destroy(sp);
@@ -1087,6 +1110,11 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
     float* fxc = gga && gf ? sp->fx + so * 128 : nullptr;
     float* fyc = gga && gf ? sp->fy + so * 128 : nullptr;
     float* fzc = gga && gf ? sp->fz + so * 128 : nullptr;
+    if (sp->mixed) {
+      const bool use = sp->ordered[c];
+      screen_mixed_set_order(sp->mixed, use ? sp->order + t0 : nullptr,
+                             use ? sp->order_start + c * (size_t)(sp->nsm + 1) : nullptr);
+    }
     if (timed) SR_TRY(cudaEventRecord(ev[0], st));
     // K1
     {

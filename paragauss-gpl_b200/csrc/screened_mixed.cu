@@ -26,6 +26,9 @@
 // the device error flag and the kernel winds down.
 #include <algorithm>
 #include <cstdint>
+#include <functional>
+#include <queue>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -70,6 +73,7 @@ struct ScreenMixed {
   int* err = nullptr;                // device view of h_err
   volatile int* h_err = nullptr;     // mapped host word: written by a kernel only when a wait runs out
   int nsm = 148;
+  const int *order = nullptr, *start = nullptr;  // tile lists of the persistent CTAs (null: round robin)
   std::vector<void*> allocs;
 };
 
@@ -85,6 +89,30 @@ cudaError_t sm_alloc(ScreenMixed* m, T** p, size_t n) {
   }
   return e;
 }
+
+// The tiles of one persistent CTA: every gridDim.x-th of the chunk's, or
+// (order not null) its own list order[start[c]] .. order[start[c + 1] - 1], made
+// when the plan is so that the CTAs' work is even.  Every role of a kernel walks
+// the same sequence.
+struct TileWalk {
+  const int* order;
+  const int* start;
+  int64_t k, k1, step;
+  __device__ __forceinline__ TileWalk(const int* o, const int* s, int64_t nt) : order(o), start(s) {
+    if (o) {
+      k = s[blockIdx.x];
+      k1 = s[blockIdx.x + 1];
+      step = 1;
+    } else {
+      k = blockIdx.x;
+      k1 = nt;
+      step = gridDim.x;
+    }
+  }
+  __device__ __forceinline__ bool more() const { return k < k1; }
+  __device__ __forceinline__ void next() { k += step; }
+  __device__ __forceinline__ int64_t tile() const { return order ? (int64_t)__ldg(order + k) : k; }
+};
 
 // ---------------------------------------------------------------------------
 // operands
@@ -308,7 +336,8 @@ __global__ void __launch_bounds__(kDensThreads, 1)
                  const int8_t* __restrict__ tB, const int64_t* __restrict__ b_off, const double* __restrict__ ps,
                  const double* __restrict__ phi, const GT* __restrict__ gx, const GT* __restrict__ gy,
                  const GT* __restrict__ gz, double* __restrict__ rho, double* __restrict__ grx,
-                 double* __restrict__ gry, double* __restrict__ grz, int* err) {
+                 double* __restrict__ gry, double* __restrict__ grz, int* err, const int* __restrict__ order,
+                 const int* __restrict__ start) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DensSmem& S = *reinterpret_cast<DensSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -336,7 +365,8 @@ __global__ void __launch_bounds__(kDensThreads, 1)
   if (warp == 10) {
     if (lane == 0) {  // epilogue operands: per slot block j, group u, third h: kECols slots of phi (grad phi)
       int e = 0;
-      for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x) {
+      for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+        const int64_t ti = wk.tile();
         const int64_t sb = tso[t0 + ti] - s0;
         const int n = (int)(tso[t0 + ti + 1] - tso[t0 + ti]);
         const int nN = (n + kN - 1) / kN;
@@ -373,7 +403,8 @@ __global__ void __launch_bounds__(kDensThreads, 1)
   } else if (warp == 8) {
     if (lane == 0) {  // MMA issuer
       int it = 0, jj = 0;
-      for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x) {
+      for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+        const int64_t ti = wk.tile();
         const int n = (int)(tso[t0 + ti + 1] - tso[t0 + ti]);
         const int nK = n / 32, nN = (n + kN - 1) / kN;
         for (int j = 0; j < nN && ok; ++j, ++jj) {
@@ -401,7 +432,8 @@ __global__ void __launch_bounds__(kDensThreads, 1)
   } else if (warp == 9) {
     if (lane == 0) {  // operand producer: per K step the phi digits (A) and the gathered P digits (B)
       int it = 0;
-      for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x) {
+      for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+        const int64_t ti = wk.tile();
         const int64_t sb = tso[t0 + ti] - s0;
         const int n = (int)(tso[t0 + ti + 1] - tso[t0 + ti]);
         const int nK = n / 32, nN = (n + kN - 1) / kN;
@@ -427,7 +459,8 @@ __global__ void __launch_bounds__(kDensThreads, 1)
     const int row = (warp & 3) * 32 + lane, third = warp < 8 ? (warp >> 2) : 2;
     const uint32_t trow = tbase + ((uint32_t)((warp & 3) * 32) << 16);
     int jj = 0;
-    for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x) {
+    for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+      const int64_t ti = wk.tile();
       const int64_t sg = tso[t0 + ti];
       const int64_t sb = sg - s0;
       const int n = (int)(tso[t0 + ti + 1] - sg);
@@ -535,7 +568,9 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
                                                             const double* __restrict__ By,
                                                             const double* __restrict__ Bz, int8_t* __restrict__ tZ,
                                                             int8_t* __restrict__ tF, double* __restrict__ zs,
-                                                            double* __restrict__ fs, int* err) {
+                                                            double* __restrict__ fs, int* err,
+                                                            const int* __restrict__ order,
+                                                            const int* __restrict__ start) {
   using L = ZLayout<GGA, GT>;
   extern __shared__ __align__(128) uint8_t zsm[];
   uint64_t* full = reinterpret_cast<uint64_t*>(zsm + L::kBar);
@@ -559,7 +594,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
   if (warp == kZWarps) {
     if (lane == 0) {  // producer
       int it = 0, tt = 0;
-      for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x, ++tt) {
+      for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next(), ++tt) {
+        const int64_t ti = wk.tile();
         const int64_t sb = tso[t0 + ti] - s0;
         const int n = (int)(tso[t0 + ti + 1] - tso[t0 + ti]);
         const int b = tt & 1;
@@ -603,7 +639,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
     const int p0 = lane * 4;
     const int kstep = lane >> 3, kin = (lane & 7) * 4;
     int it = 0, tt = 0;
-    for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x, ++tt) {
+    for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next(), ++tt) {
+      const int64_t ti = wk.tile();
       const int64_t sb = tso[t0 + ti] - s0;
       const int n = (int)(tso[t0 + ti + 1] - tso[t0 + ti]);
       const int b = tt & 1;
@@ -723,7 +760,8 @@ __global__ void __launch_bounds__(kVThreads, 1)
     k_sm_vpot(const int64_t* __restrict__ tso, const int* __restrict__ slot_fn, int64_t t0, int64_t nt, int64_t s0,
               const int8_t* __restrict__ tF, const int8_t* __restrict__ tZ, const double* __restrict__ fs,
               const double* __restrict__ zs, double* __restrict__ V, int64_t ldv, int* err,
-              const int* __restrict__ tile_mol, const SetMolDev* __restrict__ mols) {
+              const int* __restrict__ tile_mol, const SetMolDev* __restrict__ mols, const int* __restrict__ order,
+              const int* __restrict__ start) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   VSmem& S = *reinterpret_cast<VSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -751,7 +789,8 @@ __global__ void __launch_bounds__(kVThreads, 1)
   if (warp == kVEpiWarps + 1) {
     if (lane == 0) {  // producer: the phi block of each J once, the Z block of each (J, I) pair per K step
       int it = 0, ia = 0;
-      for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x) {
+      for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+        const int64_t ti = wk.tile();
         const int64_t sb = tso[t0 + ti] - s0;
         const int n = (int)(tso[t0 + ti + 1] - tso[t0 + ti]);
         const int nJ = (n + kM - 1) / kM, nI = (n + kN - 1) / kN;
@@ -786,7 +825,8 @@ __global__ void __launch_bounds__(kVThreads, 1)
   } else if (warp == kVEpiWarps) {
     if (lane == 0) {  // MMA issuer
       int it = 0, pp = 0, ia = 0;
-      for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x) {
+      for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+        const int64_t ti = wk.tile();
         const int n = (int)(tso[t0 + ti + 1] - tso[t0 + ti]);
         const int nJ = (n + kM - 1) / kM, nI = (n + kN - 1) / kN;
         for (int J = 0; J < nJ && ok; ++J, ++ia) {
@@ -826,7 +866,8 @@ __global__ void __launch_bounds__(kVThreads, 1)
     const int part = warp >> 2;
     const uint32_t trow = tbase + ((uint32_t)((warp & 3) * 32) << 16);
     int pp = 0;
-    for (int64_t ti = blockIdx.x; ti < nt && ok; ti += gridDim.x) {
+    for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+      const int64_t ti = wk.tile();
       const int64_t sg = tso[t0 + ti];
       const int64_t sb = sg - s0;
       const int n = (int)(tso[t0 + ti + 1] - sg);
@@ -982,6 +1023,46 @@ int screen_mixed_basis(ScreenMixed* m, const int64_t* tso, const int* slot_fn, i
 
 void screen_mixed_set_gga(ScreenMixed* m, bool gga) { m->gga = gga; }
 
+void screen_mixed_set_order(ScreenMixed* m, const int* order, const int* start) {
+  m->order = order;
+  m->start = start;
+}
+
+// Longest first: the tiles by falling work, each to the CTA with the least so
+// far; a CTA's tiles then in their grid order.  The work of a tile: its digit
+// products and what is streamed per slot (the fit matters little).  Where the
+// lists pay: with more tiles than CTAs, and few enough that round robin leaves
+// the slowest CTA behind (60 atoms, 16 tiles per CTA, 20% behind the mean:
+// potential 2.93 -> 2.79 ms, density 1.41 -> 1.39; 31 atoms LDA, build 1.345 ->
+// 1.31).  With the 45 and more per CTA of a 200-atom build's chunks both took
+// the same time (47.6 and 47.5 ms), so from 32 on nothing is made.
+bool screen_mixed_order(const int64_t* tso, int64_t nt, int nsm, int* order, int* start) {
+  if (nt <= nsm || nt > 32 * (int64_t)nsm) return false;
+  std::vector<std::pair<double, int>> work((size_t)nt);
+  for (int64_t t = 0; t < nt; ++t) {
+    const double n = (double)(tso[t + 1] - tso[t]);
+    work[(size_t)t] = {-(n * n + 150.0 * n + 1000.0), (int)t};
+  }
+  std::sort(work.begin(), work.end());
+  std::vector<std::vector<int>> mine((size_t)nsm);
+  std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<std::pair<double, int>>> q;
+  for (int c = 0; c < nsm; ++c) q.push({0.0, c});
+  for (const auto& w : work) {
+    const auto top = q.top();
+    q.pop();
+    mine[(size_t)top.second].push_back(w.second);
+    q.push({top.first - w.first, top.second});
+  }
+  int o = 0;
+  for (int c = 0; c < nsm; ++c) {
+    start[c] = o;
+    std::sort(mine[(size_t)c].begin(), mine[(size_t)c].end());
+    for (int t : mine[(size_t)c]) order[o++] = t;
+  }
+  start[nsm] = o;
+  return true;
+}
+
 int screen_mixed_gather(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_t t0, int64_t nt, int64_t s0,
                         int spin, cudaStream_t st, const int* tile_mol, const SetMolDev* mols) {
   k_sm_gather_B<<<(unsigned)nt, kGatherThreads, 4 * m->max_n, st>>>(
@@ -1001,11 +1082,12 @@ int mixed_density(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_
   const int smem = tc::kWholeSmSmem;
   if (m->gga)
     k_sm_density<true, GT><<<grid, kDensThreads, smem, st>>>(tso, slot_fn, t0, nt, s0, tA, e_pt, m->tB, m->b_off,
-                                                             m->ps, phi, gx, gy, gz, rho, grx, gry, grz, m->err);
+                                                             m->ps, phi, gx, gy, gz, rho, grx, gry, grz, m->err,
+                                                             m->order, m->start);
   else
     k_sm_density<false, GT><<<grid, kDensThreads, smem, st>>>(tso, slot_fn, t0, nt, s0, tA, e_pt, m->tB, m->b_off,
                                                               m->ps, phi, nullptr, nullptr, nullptr, rho, nullptr,
-                                                              nullptr, nullptr, m->err);
+                                                              nullptr, nullptr, m->err, m->order, m->start);
   return 1;
 }
 
@@ -1017,16 +1099,16 @@ int mixed_potential(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int6
   const unsigned zgrid = (unsigned)std::min<int64_t>(nt, m->nsm);
   if (m->gga)
     k_sm_zquant<true, GT><<<zgrid, kZThreads, ZLayout<true, GT>::kBytes, st>>>(
-        tso, t0, nt, s0, phi, gx, gy, gz, A, Bx, By, Bz, m->tZ, m->tF, m->zs, m->fs, m->err);
+        tso, t0, nt, s0, phi, gx, gy, gz, A, Bx, By, Bz, m->tZ, m->tF, m->zs, m->fs, m->err, m->order, m->start);
   else
     k_sm_zquant<false, GT><<<zgrid, kZThreads, ZLayout<false, GT>::kBytes, st>>>(
         tso, t0, nt, s0, phi, nullptr, nullptr, nullptr, A, nullptr, nullptr, nullptr, m->tZ, m->tF, m->zs, m->fs,
-        m->err);
+        m->err, m->order, m->start);
   if (k0) cudaEventRecord(k0, st);
   const unsigned grid = (unsigned)std::min<int64_t>(nt, m->nsm);
   auto launch = [&](auto kern) {
     kern<<<grid, kVThreads, tc::kWholeSmSmem, st>>>(tso, slot_fn, t0, nt, s0, m->tF, m->tZ, m->fs, m->zs, V, ldv, m->err,
-                                                   tile_mol, mols);
+                                                   tile_mol, mols, m->order, m->start);
   };
   if (m->gga) {
     if (tile_mol) launch(k_sm_vpot<true, true>);

@@ -56,6 +56,11 @@ int screen_mixed_basis(ScreenMixed* m, const int64_t* tso, const int* slot_fn, i
                        const int* tile_mol = nullptr, const SetMolDev* mols = nullptr);
 // the functional kind of the following launches (a set's chunks alternate)
 void screen_mixed_set_gga(ScreenMixed* m, bool gga);
+// Even tile lists for the persistent CTAs of a chunk (tso: its nt + 1 slot
+// offsets): order[nt], start[nsm + 1] on the host; false where round robin does.
+bool screen_mixed_order(const int64_t* tso, int64_t nt, int nsm, int* order, int* start);
+// the device copies used by the following density and potential launches (null: round robin)
+void screen_mixed_set_order(ScreenMixed* m, const int* order, const int* start);
 // the gathered digits of P_spin[S_t, S_t] of every tile (replaces the previous spin's);
 // with tile_mol, tile t's digits come from mols[tile_mol[t]] instead
 int screen_mixed_gather(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_t t0, int64_t nt, int64_t s0,

@@ -53,6 +53,8 @@ struct ScreenPlan {
   double* V = nullptr;       // [ispin][nbas][nbas]
   unsigned long long* pmax = nullptr;  // [chunk_tiles*128] largest |phi| per point (INT8 path)
   ScreenMixed* mixed = nullptr;
+  int *order = nullptr, *order_start = nullptr;  // INT8: even tile lists ([ntiles] chunk by chunk, [chunk][nsm + 1])
+  std::vector<char> ordered;                     // chunks that use them
   std::vector<std::array<cudaEvent_t, 9>> cev;  // timing events of each chunk (made by the first timed build)
   int nsm = 148;
   std::vector<void*> allocs;

@@ -37,6 +37,19 @@ def test_fp64_block_remainders(natoms, lmax, functional, ispin):
     _check(_case(natoms, lmax, functional, ispin), "fp64", 0.0, 1e-10)
 
 
+# 148 tiles (one per SM), a few more (even tile lists) and several per SM: INT8 against FP64
+@pytest.mark.parametrize("functional", ["VWN", "PBE"])
+@pytest.mark.parametrize("nrad,nang", [(24, 110), (25, 110), (40, 194)])
+def test_int8_tile_lists(nrad, nang, functional):
+    c = _case(7, 2, functional, nang=nang, nrad=nrad)
+    r = []
+    for precision in ("mixed", "fp64"):
+        with lib.Context(c, precision=precision, screen_threshold=1e-10) as ctx:
+            r.append(ctx.build())
+    assert abs(r[0][1] - r[1][1]) < 1e-7 and abs(r[0][2] - r[1][2]) < 1e-7
+    assert float(np.max(np.abs(r[0][0] - r[1][0]))) < 1e-7
+
+
 # the symmetric half of the products: rho of an LDA and the tau sums and terms
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 1e-7)])
 @pytest.mark.parametrize("natoms,lmax", [(3, 1), (4, 2), (7, 2), (9, 3)])
