@@ -56,6 +56,10 @@ struct BuildArgs {
   double* P = nullptr;        // [ldc][ldc]
   bool cleared = false;       // acc and the plan's potential matrix are already 0
   double* exc_nel = nullptr;  // device {E_xc, N_el} written by the packing, when not null
+  // orbital form of the screened FP64 density (nop > 0), per spin: C [function][nop], occ C
+  // [nop][ldc] (zero past nocc), occupations [nocc]
+  int nop = 0, nocc = 0;
+  const double *orb[2] = {}, *orb_scaled[2] = {}, *orb_occ[2] = {};
   bool p_symmetric = true;    // P formed here from C; false: the caller's P, which nothing checks
   // potential tiles
   int nt = 0;                 // ldc / 64
@@ -79,6 +83,9 @@ void launch_pmat_scaled(const BuildArgs& a, int64_t kpad, cudaStream_t st);
 // P from unpadded device orbitals C (nbas x nocc) and occ; z0[n0] and z1[n1] are cleared in the same launch
 void launch_pmat_raw(const BuildArgs& a, const double* C, const double* occ, int64_t nbas, int nocc, int64_t kpad,
                      double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st);
+// C and occ C turned for the orbital form: Ct [nbas][nop], Co [nop][ldc]; the same two clears
+void launch_turn_orbitals(const double* C, const double* occ, int64_t nbas, int nocc, int64_t ldc, int nop, double* Ct,
+                          double* Co, double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st);
 void launch_density_f64(const BuildArgs& a, bool gga, cudaStream_t st);
 void launch_functional_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool gga, cudaStream_t st);
 // the functional on ntiles whole 128-point tiles, one partial pair per tile (no reduction)

@@ -127,6 +127,44 @@ void launch_pmat_raw(const BuildArgs& a, const double* C, const double* occ, int
   launch_pmat_scaled(a, kpad, st);
 }
 
+// The caller's orbitals for the orbital form: Ct[mu][j] (nop per function) and
+// Co[j][mu] = occ_j C (ldc per orbital), zero past nocc, with the two clears of
+// k_load_orbitals.  Block = 32 functions x 16 orbitals, turned in shared memory.
+__global__ void __launch_bounds__(256) k_turn_orbitals(const double* __restrict__ C, const double* __restrict__ occ,
+                                                       int64_t nbas, int nocc, int64_t ldc, int nop,
+                                                       double* __restrict__ Ct, double* __restrict__ Co,
+                                                       double* __restrict__ z0, int64_t n0, double* __restrict__ z1,
+                                                       int64_t n1) {
+  __shared__ double t[16][33];
+  const int64_t mu0 = (int64_t)blockIdx.x * 32;
+  const int j0 = blockIdx.y * 16, tid = threadIdx.x;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int jj = (tid >> 5) + 8 * u, j = j0 + jj;
+    const int64_t mu = mu0 + (tid & 31);
+    const bool in = j < nocc && mu < nbas;
+    const double c = in ? C[j * nbas + mu] : 0.0;
+    t[jj][tid & 31] = c;
+    Co[j * ldc + mu] = in ? c * occ[j] : 0.0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int m = (tid >> 4) + 16 * u;
+    if (mu0 + m < nbas) Ct[(mu0 + m) * nop + j0 + (tid & 15)] = t[tid & 15][m];
+  }
+  const int64_t step = (int64_t)gridDim.x * gridDim.y * 256;
+  const int64_t first = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 256 + tid;
+  for (int64_t i = first; i < n0; i += step) z0[i] = 0.0;
+  for (int64_t i = first; i < n1; i += step) z1[i] = 0.0;
+}
+
+void launch_turn_orbitals(const double* C, const double* occ, int64_t nbas, int nocc, int64_t ldc, int nop, double* Ct,
+                          double* Co, double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st) {
+  k_turn_orbitals<<<dim3((unsigned)(ldc / 32), (unsigned)(nop / 16)), 256, 0, st>>>(C, occ, nbas, nocc, ldc, nop, Ct, Co,
+                                                                                    z0, n0, z1, n1);
+}
+
 void launch_pmat_scaled(const BuildArgs& a, int64_t kpad, cudaStream_t st) {
   constexpr int smem = gemm_smem_bytes<false, false>();
   raise_smem_limit(k_pmat, smem);

@@ -714,7 +714,19 @@ static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given, cons
     int64_t nv = 0;
     double* V = screen_potential(c->screen, &nv);
     if (!as.cleared) CUDA_TRY(c, cudaMemsetAsync(a.acc, 0, 4 * sizeof(double), s));
-    for (int sp = 0; sp < c->opt.ispin && !p_given; ++sp) {
+    const bool orbitals = rawC && screen_orbital_form(c->screen, (int)kpad);
+    for (int sp = 0; sp < c->opt.ispin && orbitals; ++sp) {
+      // no P is formed: the second spin's scaled orbitals lie in its place (nop <= ldc)
+      double *Ct = sp ? c->C2 : a.C, *Co = sp ? c->P2 : a.Cocc;
+      as.orb_occ[sp] = rawocc + (size_t)sp * nocc;
+      launch_turn_orbitals(rawC + (size_t)sp * c->nbas * nocc, as.orb_occ[sp], c->nbas, nocc, a.ldc, (int)kpad, Ct, Co, V,
+                           sp ? 0 : nv, a.acc, sp ? 0 : 4, s);
+      as.orb[sp] = Ct;
+      as.orb_scaled[sp] = Co;
+      as.nop = (int)kpad;
+      as.nocc = nocc;
+    }
+    for (int sp = 0; sp < c->opt.ispin && !p_given && !orbitals; ++sp) {
       BuildArgs b = a;
       if (sp) {  // second spin: its orbitals and occupations into P2 (Cocc is scratch)
         b.C = c->C2;
@@ -732,7 +744,7 @@ static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given, cons
     std::string e;
     const int st = screen_run(c->screen, as, c->P2, s, ham, &T, e);
     if (st) return set_err(c, st, e);
-    tm->kernel_launches = T.launches + (p_given ? 0 : 2 * c->opt.ispin);
+    tm->kernel_launches = T.launches + (p_given ? 0 : (orbitals ? 1 : 2) * c->opt.ispin);
     return PGXC_OK;
   }
   float t_basis = 0, t_dens = 0, t_func = 0, t_pot = 0, t_x = 0, t_v = 0;

@@ -304,6 +304,8 @@ struct SPlanes {
   __device__ __forceinline__ const double* phi(int z) const { return z == 0 ? phi0 : (z == 1 ? phi1 : phi2); }
   __device__ __forceinline__ double* rho(int z) const { return z == 0 ? rho0 : (z == 1 ? rho1 : rho2); }
 };
+// psi's way through memory and the second launch (screen_orbital_form)
+constexpr double kOrbitalMargin = 1.15;
 // The tile's slot -> function list in shared memory, -1 from its slots to a
 // whole block past them: every index the kernels form is inside it, guarded or
 // not (a guarded shared-memory load may be executed all the same).
@@ -328,13 +330,19 @@ __device__ __forceinline__ void load_sfn(int* sfn, const int* __restrict__ slot_
 // CTAs at 254 registers; four CTAs at 128 registers 9.2, 32-deep stages 9.4.
 // The sums' loop has eight slots' loads in flight: 8.9 -> 8.7 ms against four
 // (20 atoms meta-GGA 1.04 -> 1.01).
-template <bool GGA, bool STORE = false>
+// The orbital form of the same sums (FORM): kPsi, psi_o = sum_k phi_k C[k][o] of
+// the tile's points (columns = the nop padded orbitals; P = C, ldc = nop), with
+// rho = sum occ psi^2, written to X where grad rho follows; kFromPsi, X = sum_o
+// psi_o occ_o C[.][o] (rows = psi; P = occ C by orbitals) with grad rho alone.
+// Taken while 2 nocc is below the tiles' mean length (screen_orbital_form).
+enum { kFromP, kPsi, kFromPsi };
+template <bool GGA, bool STORE = false, int FORM = kFromP>
 __global__ void __launch_bounds__(kSThreads, 3)
     k_sdensity(SPlanes pl, const double* __restrict__ gx, const double* __restrict__ gy,
                const double* __restrict__ gz, const int64_t* __restrict__ tso, const int* __restrict__ listed,
                int64_t t0, int64_t s0, const int* __restrict__ slot_fn, const double* __restrict__ P, int64_t ldc,
                bool tri, double* __restrict__ grx, double* __restrict__ gry, double* __restrict__ grz,
-               double* __restrict__ X = nullptr) {
+               double* __restrict__ X = nullptr, int nop = 0, int nocc = 0, const double* __restrict__ occ = nullptr) {
   extern __shared__ double smem[];
   constexpr int E = kDK * kDLd;  // one operand of a stage
   static_assert(kSBlk * kXLd <= 2 * kDStages * E, "the X block lies in the stages");
@@ -349,15 +357,16 @@ __global__ void __launch_bounds__(kSThreads, 3)
   const int nl = listed[t];
   const int m0 = blockIdx.y * kSBlk;
   load_sfn(sfn, slot_fn + sb + s0, (int)(tso[t + 1] - tso[t]));
-  const double* A = phi + sb * 128 + m0;
+  const double* A = phi + (FORM == kFromPsi ? (int64_t)blockIdx.x * nop : sb) * 128 + m0;
+  const int nk = FORM == kFromPsi ? nop : nl, nn = FORM == kPsi ? nop : nl;  // rows summed over, columns
   const int wm0 = (warp >> 1) * 32, wn0 = (warp & 1) * 32, fr = lane >> 2, fk = lane & 3;
-  const int nslab = (nl + kDK - 1) / kDK;
+  const int nslab = (nk + kDK - 1) / kDK;
   const int col = tid & 63, kq = tid >> 6;  // this thread's column of every gathered stage, rows kq + 2 i
   double r = 0.0, g[3] = {0.0, 0.0, 0.0};   // of point m0 + (tid & 63), columns tid >> 6 mod 2
-  for (int n0 = 0; n0 < nl; n0 += kSBlk) {
+  for (int n0 = 0; n0 < nn; n0 += kSBlk) {
     const int ns = tri ? min(nslab, n0 / kDK + kSBlk / kDK) : nslab;
     __syncthreads();  // sfn written; the X block before this one read
-    const int fcol = sfn[n0 + col];
+    const int fcol = FORM != kPsi ? sfn[n0 + col] : (n0 + col < nop ? n0 + col : -1);
     auto load = [&](int it) {
       double* a = sA + it % kDStages * E;
       double* b = sB + it % kDStages * E;
@@ -369,7 +378,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
       }
 #pragma unroll
       for (int i = 0; i < kDK / 2; ++i) {
-        const int k = kq + 2 * i, f = sfn[k0 + k];
+        const int k = kq + 2 * i, f = FORM == kFromPsi ? k0 + k : sfn[k0 + k];  // (nop: whole stages)
         const bool ok = f >= 0 && fcol >= 0;
         cp_async8(b + k * kDLd + col, ok ? P + (int64_t)f * ldc + fcol : P, ok);
       }
@@ -379,7 +388,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
       if (s < ns) load(s);
       cp_async_commit();
     }
-    const int nj = live_frags(n0 + wn0, nl, 4);
+    const int nj = live_frags(n0 + wn0, nn, 4);
     SAcc<4, 4> acc;
     acc.zero();
     for (int it = 0; it < ns; ++it) {
@@ -411,14 +420,18 @@ __global__ void __launch_bounds__(kSThreads, 3)
         for (int e = 0; e < 2; ++e)
           sX[(wn0 + j * 8 + 2 * fk + e) * kXLd + wm0 + i * 8 + fr] = acc.v[i][j][e];
     __syncthreads();
-    const int cn = min(kSBlk, nl - n0);
-    const int64_t o0 = (sb + n0) * 128 + m0 + col;
+    const int cn = min(kSBlk, nn - n0);
+    const int64_t o0 = ((FORM == kPsi ? (int64_t)blockIdx.x * nop : sb) + n0) * 128 + m0 + col;
 #pragma unroll 8
     for (int c = kq; c < cn; c += 2) {
       const double x = sX[c * kXLd + col];
       const int64_t o = o0 + c * 128;
       if (STORE) X[o] = x;
-      r += x * phi[o];
+      if (FORM == kPsi) {
+        if (n0 + c < nocc) r += occ[n0 + c] * (x * x);
+      } else if (FORM == kFromP) {
+        r += x * phi[o];
+      }
       if (GGA) {
         g[0] += x * gx[o];
         g[1] += x * gy[o];
@@ -435,6 +448,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
   }
   __syncthreads();
   for (int q = kq; q < (GGA ? 4 : 1); q += 2) {
+    if (FORM == kFromPsi && q == 0) continue;
     const double v = red[q * kSThreads + col] + red[q * kSThreads + 64 + col];
     double* out = q == 0 ? pl.rho(blockIdx.z) : (q == 1 ? grx : (q == 2 ? gry : grz));
     out[(int64_t)blockIdx.x * 128 + m0 + col] = q == 0 ? v : 2.0 * v;
@@ -774,6 +788,7 @@ void screen_destroy(ScreenPlan* sp) {
   if (!sp) return;
   if (sp->mixed) screen_mixed_destroy(sp->mixed);
   for (void* p : sp->allocs) cudaFree(p);
+  cudaFree(sp->psi);
   for (auto& c : sp->cev)
     for (auto& e : c)
       if (e) cudaEventDestroy(e);
@@ -1047,6 +1062,74 @@ void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, con
   }
 }
 
+// The orbital form costs n (nop + nop) products per point where P costs n^2 (an
+// LDA, and each tau plane: n nop against n^2 / 2), and forms no P.  60 atoms, 304
+// functions per tile, 105 orbitals (2 nop / n = 0.74): contraction 8.7 -> 6.7 ms;
+// 25 atoms open shell 0.955 -> 0.79, 20 atoms meta-GGA 1.007 -> 0.615, 12 atoms
+// 0.155 -> 0.138.  Time over products is 1.04 of what P takes, so that with a
+// margin of 1.15 the form chosen is the faster one; above it P stays (nocc near
+// nbas, where the orbital form is up to twice the products).  INT8 keeps P, whose
+// digits are what its products read.
+bool screen_orbital_form(ScreenPlan* sp, int nop) {
+  if (sp->mixed || kOrbitalMargin * 2.0 * nop * (double)sp->nlisted >= sp->sum_n2) return false;
+  if (!sp->gga) return true;
+  // psi of as many tiles as 256 MB hold (the rest follow in further launches)
+  const int64_t per = (int64_t)nop * 128;
+  const int64_t tiles = std::min(sp->chunk_tiles, std::max<int64_t>(1, (int64_t(1) << 25) / per));
+  if (tiles * per > sp->psi_cap) {
+    cudaFree(sp->psi);
+    sp->psi = nullptr;
+    sp->psi_cap = 0;
+    if (cudaMalloc(&sp->psi, sizeof(double) * (size_t)(tiles * per)) != cudaSuccess) {
+      cudaGetLastError();  // no room: the build takes P instead
+      sp->psi = nullptr;
+      return false;
+    }
+    sp->psi_cap = tiles * per;
+  }
+  return true;
+}
+
+// rho, grad rho and (tau not null) the tau sums of one spin by its orbitals
+static int orbital_density(const ScreenPlan* sp, const BuildArgs& a, int s, int64_t t0, int64_t nt, int64_t s0,
+                           const double* phi, const double* gx, const double* gy, const double* gz, const BuildArgs& b,
+                           double* tau, int64_t cp, cudaStream_t st) {
+  const int smem = sdensity_smem(sp->max_n), nop = a.nop, nocc = a.nocc;
+  raise_smem_limit(k_sdensity<false, true, kPsi>, smem);
+  raise_smem_limit(k_sdensity<false, false, kPsi>, smem);
+  raise_smem_limit(k_sdensity<true, false, kFromPsi>, smem);
+  const SPlanes pl{phi, phi, phi, b.rho, b.rho, b.rho};
+  int launches = 0;
+  if (!gx) {
+    k_sdensity<false, false, kPsi><<<dim3((unsigned)nt, 2), kSThreads, smem, st>>>(
+        pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, a.orb[s], nop, false, nullptr, nullptr,
+        nullptr, nullptr, nop, nocc, a.orb_occ[s]);
+    return 1;
+  }
+  const int64_t step = sp->psi_cap / ((int64_t)nop * 128);
+  for (int64_t u = 0; u < nt; u += step) {
+    const dim3 grid((unsigned)std::min(step, nt - u), 2);
+    const int64_t p = u * 128;
+    const SPlanes pu{phi, phi, phi, b.rho + p, nullptr, nullptr};
+    k_sdensity<false, true, kPsi><<<grid, kSThreads, smem, st>>>(
+        pu, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb[s], nop, false, nullptr,
+        nullptr, nullptr, sp->psi, nop, nocc, a.orb_occ[s]);
+    const SPlanes px{sp->psi, nullptr, nullptr, nullptr, nullptr, nullptr};
+    k_sdensity<true, false, kFromPsi><<<grid, kSThreads, smem, st>>>(
+        px, gx, gy, gz, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb_scaled[s], a.ldc, false, b.grx + p,
+        b.gry + p, b.grz + p, nullptr, nop, nocc, nullptr);
+    launches += 2;
+  }
+  if (tau) {
+    const SPlanes pt{gx, gy, gz, tau, tau + cp, tau + 2 * cp};
+    k_sdensity<false, false, kPsi><<<dim3((unsigned)nt, 2, 3), kSThreads, smem, st>>>(
+        pt, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, a.orb[s], nop, false, nullptr, nullptr,
+        nullptr, nullptr, nop, nocc, a.orb_occ[s]);
+    ++launches;
+  }
+  return launches;
+}
+
 int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_t st, double* ham, ScreenTimes* tm,
                std::string& err, const ScreenExtra* extra) {
   const bool potential = !extra || extra->potential;
@@ -1165,6 +1248,10 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         else
           T.launches += screen_mixed_density(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, phi, gxc, gyc, gzc,
                                              b[s].rho, b[s].grx, b[s].gry, b[s].grz, so, to, st);
+      } else if (a.nop) {
+        T.launches += orbital_density(sp, a, s, t0, nt, s0, phi, gxc, gyc, gzc, b[s], sp->mgga ? sp->tq + 4 * s * cp : nullptr,
+                                      cp, st);
+        continue;
       } else {
         const int smem = sdensity_smem(sp->max_n);
         const SPlanes pl{phi, phi, phi, b[s].rho, b[s].rho, b[s].rho};

@@ -10,9 +10,9 @@ from pgxc import cases, lib
 pytestmark = pytest.mark.gpu
 
 
-def _case(natoms, lmax, functional, ispin=1, nang=26, nrad=9):
-    c = cases.small_case(functional, seed=40 + natoms, natoms=natoms, nrad=nrad, nang=nang, nocc=max(2, natoms),
-                         ispin=ispin, lmax=lmax)
+def _case(natoms, lmax, functional, ispin=1, nang=26, nrad=9, nocc=None):
+    c = cases.small_case(functional, seed=40 + natoms, natoms=natoms, nrad=nrad, nang=nang,
+                         nocc=max(2, natoms) if nocc is None else nocc, ispin=ispin, lmax=lmax)
     O.weight_case(c)
     return c
 
@@ -48,6 +48,18 @@ def test_int8_tile_lists(nrad, nang, functional):
             r.append(ctx.build())
     assert abs(r[0][1] - r[1][1]) < 1e-7 and abs(r[0][2] - r[1][2]) < 1e-7
     assert float(np.max(np.abs(r[0][0] - r[1][0]))) < 1e-7
+
+
+# orbitals in the place of P, on either side of its 16-row stages and 64-column blocks and of the
+# length where P is taken instead; occupations of both signs and none
+@pytest.mark.parametrize("functional,ispin", [("VWN", 1), ("PBE", 1), ("PBE", 2), ("TPSS", 1), ("TPSS", 2)])
+@pytest.mark.parametrize("nocc", [1, 15, 16, 17, 33, 64, 65, 100])
+def test_fp64_orbital_remainders(nocc, functional, ispin):
+    c = _case(12, 2, functional, ispin, nocc=nocc)
+    c.occ[-1] *= -0.125
+    c.occ[nocc // 2] = 0.0
+    c.occ[0] = 2.0
+    _check(c, "fp64", 0.0, 1e-10)
 
 
 # the symmetric half of the products: rho of an LDA and the tau sums and terms
