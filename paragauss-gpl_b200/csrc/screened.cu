@@ -334,6 +334,8 @@ __device__ __forceinline__ void load_sfn(int* sfn, const int* __restrict__ slot_
 // the tile's points (columns = the nop padded orbitals; P = C, ldc = nop), with
 // rho = sum occ psi^2, written to X where grad rho follows; kFromPsi, X = sum_o
 // psi_o occ_o C[.][o] (rows = psi; P = occ C by orbitals) with grad rho alone.
+// kPsi with GGA: the planes are grad phi's (grid z), so that x = d_z psi: the tau
+// sum, and grad rho_z = 2 sum occ psi d_z psi with psi from X (no kFromPsi).
 // Taken while 2 nocc is below the tiles' mean length (screen_orbital_form).
 enum { kFromP, kPsi, kFromPsi };
 template <bool GGA, bool STORE = false, int FORM = kFromP>
@@ -428,11 +430,15 @@ __global__ void __launch_bounds__(kSThreads, 3)
       const int64_t o = o0 + c * 128;
       if (STORE) X[o] = x;
       if (FORM == kPsi) {
-        if (n0 + c < nocc) r += occ[n0 + c] * (x * x);
+        if (n0 + c < nocc) {
+          const double y = occ[n0 + c] * x;
+          r += y * x;
+          if (GGA) g[0] += y * X[o];
+        }
       } else if (FORM == kFromP) {
         r += x * phi[o];
       }
-      if (GGA) {
+      if (GGA && FORM != kPsi) {
         g[0] += x * gx[o];
         g[1] += x * gy[o];
         g[2] += x * gz[o];
@@ -442,15 +448,18 @@ __global__ void __launch_bounds__(kSThreads, 3)
   __syncthreads();
   double* red = smem;  // [4 quantities][2 column groups][64 points]
   red[tid] = r;
-  if (GGA) {
+  if (GGA && FORM == kPsi) {
+    red[kSThreads + tid] = g[0];
+  } else if (GGA) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) red[(q + 1) * kSThreads + tid] = g[q];
   }
   __syncthreads();
-  for (int q = kq; q < (GGA ? 4 : 1); q += 2) {
+  for (int q = kq; q < (GGA ? (FORM == kPsi ? 2 : 4) : 1); q += 2) {
     if (FORM == kFromPsi && q == 0) continue;
     const double v = red[q * kSThreads + col] + red[q * kSThreads + 64 + col];
-    double* out = q == 0 ? pl.rho(blockIdx.z) : (q == 1 ? grx : (q == 2 ? gry : grz));
+    const int d = FORM == kPsi ? (int)blockIdx.z : q - 1;  // direction of grad rho
+    double* out = q == 0 ? pl.rho(blockIdx.z) : (d == 0 ? grx : (d == 1 ? gry : grz));
     out[(int64_t)blockIdx.x * 128 + m0 + col] = q == 0 ? v : 2.0 * v;
   }
 }
@@ -1064,8 +1073,8 @@ void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, con
 
 // The orbital form costs n (nop + nop) products per point where P costs n^2 (an
 // LDA, and each tau plane: n nop against n^2 / 2), and forms no P.  60 atoms, 304
-// functions per tile, 105 orbitals (2 nop / n = 0.74): contraction 8.7 -> 6.7 ms;
-// 25 atoms open shell 0.955 -> 0.79, 20 atoms meta-GGA 1.007 -> 0.615, 12 atoms
+// functions per tile, 105 orbitals (2 nop / n = 0.74): contraction 8.7 -> 6.45 ms;
+// 25 atoms open shell 0.955 -> 0.79, 20 atoms meta-GGA 1.007 -> 0.485, 12 atoms
 // 0.155 -> 0.138.  Time over products is 1.04 of what P takes, so that with a
 // margin of 1.15 the form chosen is the faster one; above it P stays (nocc near
 // nbas, where the orbital form is up to twice the products).  INT8 keeps P, whose
@@ -1073,9 +1082,10 @@ void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, con
 bool screen_orbital_form(ScreenPlan* sp, int nop) {
   if (sp->mixed || kOrbitalMargin * 2.0 * nop * (double)sp->nlisted >= sp->sum_n2) return false;
   if (!sp->gga) return true;
-  // psi of as many tiles as 256 MB hold (the rest follow in further launches)
+  // psi of as many tiles as 1 GB holds, the rest in further launches (60 atoms: 256 MB 6.7 ms, 1 GB 6.45: fewer
+  // half-empty last waves)
   const int64_t per = (int64_t)nop * 128;
-  const int64_t tiles = std::min(sp->chunk_tiles, std::max<int64_t>(1, (int64_t(1) << 25) / per));
+  const int64_t tiles = std::min(sp->chunk_tiles, std::max<int64_t>(1, (int64_t(1) << 27) / per));
   if (tiles * per > sp->psi_cap) {
     cudaFree(sp->psi);
     sp->psi = nullptr;
@@ -1097,6 +1107,7 @@ static int orbital_density(const ScreenPlan* sp, const BuildArgs& a, int s, int6
   const int smem = sdensity_smem(sp->max_n), nop = a.nop, nocc = a.nocc;
   raise_smem_limit(k_sdensity<false, true, kPsi>, smem);
   raise_smem_limit(k_sdensity<false, false, kPsi>, smem);
+  raise_smem_limit(k_sdensity<true, false, kPsi>, smem);
   raise_smem_limit(k_sdensity<true, false, kFromPsi>, smem);
   const SPlanes pl{phi, phi, phi, b.rho, b.rho, b.rho};
   int launches = 0;
@@ -1106,7 +1117,8 @@ static int orbital_density(const ScreenPlan* sp, const BuildArgs& a, int s, int6
         nullptr, nullptr, nop, nocc, a.orb_occ[s]);
     return 1;
   }
-  const int64_t step = sp->psi_cap / ((int64_t)nop * 128);
+  const int64_t most = sp->psi_cap / ((int64_t)nop * 128), parts = (nt + most - 1) / most;
+  const int64_t step = (nt + parts - 1) / parts;
   for (int64_t u = 0; u < nt; u += step) {
     const dim3 grid((unsigned)std::min(step, nt - u), 2);
     const int64_t p = u * 128;
@@ -1114,18 +1126,18 @@ static int orbital_density(const ScreenPlan* sp, const BuildArgs& a, int s, int6
     k_sdensity<false, true, kPsi><<<grid, kSThreads, smem, st>>>(
         pu, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb[s], nop, false, nullptr,
         nullptr, nullptr, sp->psi, nop, nocc, a.orb_occ[s]);
+    launches += 2;
+    if (tau) {
+      const SPlanes pt{gx, gy, gz, tau + p, tau + cp + p, tau + 2 * cp + p};
+      k_sdensity<true, false, kPsi><<<dim3(grid.x, 2, 3), kSThreads, smem, st>>>(
+          pt, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb[s], nop, false, b.grx + p,
+          b.gry + p, b.grz + p, sp->psi, nop, nocc, a.orb_occ[s]);
+      continue;
+    }
     const SPlanes px{sp->psi, nullptr, nullptr, nullptr, nullptr, nullptr};
     k_sdensity<true, false, kFromPsi><<<grid, kSThreads, smem, st>>>(
         px, gx, gy, gz, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb_scaled[s], a.ldc, false, b.grx + p,
         b.gry + p, b.grz + p, nullptr, nop, nocc, nullptr);
-    launches += 2;
-  }
-  if (tau) {
-    const SPlanes pt{gx, gy, gz, tau, tau + cp, tau + 2 * cp};
-    k_sdensity<false, false, kPsi><<<dim3((unsigned)nt, 2, 3), kSThreads, smem, st>>>(
-        pt, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, a.orb[s], nop, false, nullptr, nullptr,
-        nullptr, nullptr, nop, nocc, a.orb_occ[s]);
-    ++launches;
   }
   return launches;
 }
