@@ -671,11 +671,11 @@ void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan*
     double* d = g.den + (int64_t)(7 * s) * ld;
     double* X = XY + (int64_t)(nxy * s) * plane;
     grad_contract(sp, t0, nt, s0, B, g.gga ? gx : nullptr, gy, gz, g.P[s], a.ldc, X, d, d + ld, d + 2 * ld, d + 3 * ld,
-                  st);
+                  g.orb[s], st);
     // the Y_j only for meta-GGAs (tau and its terms), GGAs take V = W P after the coefficients
     for (int j = 0; j < 3 && g.mgga; ++j)
       grad_contract(sp, t0, nt, s0, B + (1 + j) * plane, nullptr, nullptr, nullptr, g.P[s], a.ldc, X + (1 + j) * plane,
-                    d + (4 + j) * ld, nullptr, nullptr, nullptr, st);
+                    d + (4 + j) * ld, nullptr, nullptr, nullptr, g.orb[s], st);
   }
   k_grad_coef<<<(unsigned)nt, 128, 0, st>>>(a.xc, g.functional, g.gga, g.ispin, ld, sp->qw + t0 * 128,
                                             sp->qwraw + t0 * 128, g.den, g.coef, g.ef + t0 * 128, g.exc);
@@ -683,7 +683,7 @@ void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan*
     k_grad_w<<<(unsigned)nt, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, B, plane,
                                            g.coef + (int64_t)(kCoefPlanes * s + 1) * ld, ld, W);
     grad_contract(sp, t0, nt, s0, W, nullptr, nullptr, nullptr, g.P[s], a.ldc, XY + (int64_t)(nxy * s + 1) * plane,
-                  g.den, nullptr, nullptr, nullptr, st);  // (rho is done with: its sum goes to scratch)
+                  g.den, nullptr, nullptr, nullptr, g.orb[s], st);  // (rho is done with: its sum goes to scratch)
   }
   const int smem = (int)sizeof(double) * 3 * g.natm;
   if (smem > 48 * 1024) raise_smem_limit(k_grad_orb, smem);

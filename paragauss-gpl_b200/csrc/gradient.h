@@ -27,10 +27,12 @@ struct ScreenPlan;
 int64_t grad_planes(bool gga, bool mgga, int ispin);
 
 // One gradient's buffers and kind.
+struct GradOrbitals;
 struct GradChunk {
   bool gga, mgga;            // meta-GGAs set both
   int ispin, functional, natm;
   const double* P[2];        // density matrices, leading dimension BuildArgs::ldc
+  const GradOrbitals* orb[2]; // not null: the orbitals instead
   const int* fatom;          // atom of each function
   double* rows;              // grad_planes planes of `plane` doubles
   int64_t plane;

@@ -83,8 +83,8 @@ void launch_pmat_scaled(const BuildArgs& a, int64_t kpad, cudaStream_t st);
 // P from unpadded device orbitals C (nbas x nocc) and occ; z0[n0] and z1[n1] are cleared in the same launch
 void launch_pmat_raw(const BuildArgs& a, const double* C, const double* occ, int64_t nbas, int nocc, int64_t kpad,
                      double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st);
-// C and occ C turned for the orbital form: Ct [nbas][nop], Co [nop][ldc]; the same two clears
-void launch_turn_orbitals(const double* C, const double* occ, int64_t nbas, int nocc, int64_t ldc, int nop, double* Ct,
+// C (lds doubles per orbital) and occ C turned for the orbital form: Ct [nbas][nop], Co [nop][ldc]; the same two clears
+void launch_turn_orbitals(const double* C, int64_t lds, const double* occ, int64_t nbas, int nocc, int64_t ldc, int nop, double* Ct,
                           double* Co, double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st);
 void launch_density_f64(const BuildArgs& a, bool gga, cudaStream_t st);
 void launch_functional_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool gga, cudaStream_t st);

@@ -127,11 +127,11 @@ void launch_pmat_raw(const BuildArgs& a, const double* C, const double* occ, int
   launch_pmat_scaled(a, kpad, st);
 }
 
-// The caller's orbitals for the orbital form: Ct[mu][j] (nop per function) and
+// The orbitals (lds doubles each) for the orbital form: Ct[mu][j] (nop per function) and
 // Co[j][mu] = occ_j C (ldc per orbital), zero past nocc, with the two clears of
 // k_load_orbitals.  Block = 32 functions x 16 orbitals, turned in shared memory.
-__global__ void __launch_bounds__(256) k_turn_orbitals(const double* __restrict__ C, const double* __restrict__ occ,
-                                                       int64_t nbas, int nocc, int64_t ldc, int nop,
+__global__ void __launch_bounds__(256) k_turn_orbitals(const double* __restrict__ C, int64_t lds,
+                                                       const double* __restrict__ occ, int64_t nbas, int nocc, int64_t ldc, int nop,
                                                        double* __restrict__ Ct, double* __restrict__ Co,
                                                        double* __restrict__ z0, int64_t n0, double* __restrict__ z1,
                                                        int64_t n1) {
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) k_turn_orbitals(const double* __restrict_
     const int jj = (tid >> 5) + 8 * u, j = j0 + jj;
     const int64_t mu = mu0 + (tid & 31);
     const bool in = j < nocc && mu < nbas;
-    const double c = in ? C[j * nbas + mu] : 0.0;
+    const double c = in ? C[j * lds + mu] : 0.0;
     t[jj][tid & 31] = c;
     Co[j * ldc + mu] = in ? c * occ[j] : 0.0;
   }
@@ -159,9 +159,9 @@ __global__ void __launch_bounds__(256) k_turn_orbitals(const double* __restrict_
   for (int64_t i = first; i < n1; i += step) z1[i] = 0.0;
 }
 
-void launch_turn_orbitals(const double* C, const double* occ, int64_t nbas, int nocc, int64_t ldc, int nop, double* Ct,
+void launch_turn_orbitals(const double* C, int64_t lds, const double* occ, int64_t nbas, int nocc, int64_t ldc, int nop, double* Ct,
                           double* Co, double* z0, int64_t n0, double* z1, int64_t n1, cudaStream_t st) {
-  k_turn_orbitals<<<dim3((unsigned)(ldc / 32), (unsigned)(nop / 16)), 256, 0, st>>>(C, occ, nbas, nocc, ldc, nop, Ct, Co,
+  k_turn_orbitals<<<dim3((unsigned)(ldc / 32), (unsigned)(nop / 16)), 256, 0, st>>>(C, lds, occ, nbas, nocc, ldc, nop, Ct, Co,
                                                                                     z0, n0, z1, n1);
 }
 

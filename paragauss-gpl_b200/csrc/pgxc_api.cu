@@ -719,7 +719,7 @@ static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given, cons
       // no P is formed: the second spin's scaled orbitals lie in its place (nop <= ldc)
       double *Ct = sp ? c->C2 : a.C, *Co = sp ? c->P2 : a.Cocc;
       as.orb_occ[sp] = rawocc + (size_t)sp * nocc;
-      launch_turn_orbitals(rawC + (size_t)sp * c->nbas * nocc, as.orb_occ[sp], c->nbas, nocc, a.ldc, (int)kpad, Ct, Co, V,
+      launch_turn_orbitals(rawC + (size_t)sp * c->nbas * nocc, c->nbas, as.orb_occ[sp], c->nbas, nocc, a.ldc, (int)kpad, Ct, Co, V,
                            sp ? 0 : nv, a.acc, sp ? 0 : 4, s);
       as.orb[sp] = Ct;
       as.orb_scaled[sp] = Co;
@@ -995,14 +995,6 @@ int pgxc_build_device(pgxc_ctx* c, const double* d_C, const double* d_occ, int32
 static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad, double* grad, double* exc) {
   BuildArgs& a = c->a;
   cudaStream_t s = c->stream;
-  launch_pmat_f64(a, kpad, s);
-  if (ispin == 2) {
-    BuildArgs b = a;
-    b.C = c->C2;
-    b.occ = c->occ2;
-    b.P = c->P2;
-    launch_pmat_f64(b, kpad, s);
-  }
   // function -> atom
   std::vector<int> fatom((size_t)nbas);
   for (const DevShell& S : c->shells)
@@ -1029,12 +1021,15 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   // one scratch buffer, carved in 256-byte aligned pieces and kept in the
   // context for the next call (allocation and release of several GB per call
   // would cost more than the gradient's kernels)
-  const size_t sizes[8] = {sizeof(double) * (size_t)(planes * plane), sizeof(double) * 7 * ispin * (size_t)ld,
+  size_t sizes[9] = {sizeof(double) * (size_t)(planes * plane), sizeof(double) * 7 * ispin * (size_t)ld,
                            sizeof(double) * 5 * ispin * (size_t)ld,   sizeof(double) * (size_t)nq,
                            sizeof(double) * 3 * c->natm,              sizeof(double),
-                           sizeof(double) * ((size_t)7 * c->natm * ldw / 2 + 1), sizeof(int) * (size_t)nbas};
-  size_t offs[8], total = 0;
-  for (int i = 0; i < 8; ++i) {
+                           sizeof(double) * ((size_t)7 * c->natm * ldw / 2 + 1), sizeof(int) * (size_t)nbas, 0};
+  bool orbitals = orbital_form_pays(gp, kpad);
+  const int64_t psi_tiles = orbital_psi_tiles(gp, kpad);
+  if (orbitals) sizes[8] = sizeof(double) * (size_t)(psi_tiles * kpad * 128);
+  size_t offs[9], total = 0;
+  for (int i = 0; i < 9; ++i) {
     offs[i] = total;
     total += (sizes[i] + 255) / 256 * 256;
   }
@@ -1043,6 +1038,12 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     c->grad_scr = nullptr;
     c->grad_scr_bytes = 0;
     cudaError_t e = cudaMalloc(&c->grad_scr, total);
+    if (e != cudaSuccess && orbitals) {  // no room for psi: P instead
+      cudaGetLastError();
+      orbitals = false;
+      total = offs[8];
+      e = cudaMalloc(&c->grad_scr, total);
+    }
     if (e != cudaSuccess) {
       c->grad_scr = nullptr;
       return set_err(c, PGXC_ENOMEM, std::string("gradient scratch: ") + cudaGetErrorString(e));
@@ -1058,6 +1059,24 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   g.natm = c->natm;
   g.P[0] = a.P;
   g.P[1] = c->P2;
+  GradOrbitals orb[2];
+  for (int sp = 0; sp < ispin; ++sp) {
+    BuildArgs b = a;
+    if (sp) {
+      b.C = c->C2;
+      b.occ = c->occ2;
+      b.P = c->P2;
+    }
+    g.orb[sp] = nullptr;
+    if (orbitals) {  // both turned forms lie in P's place (2 nop <= ldc)
+      double *Ct = b.P, *Co = b.P + kpad * a.ldc;
+      launch_turn_orbitals(b.C, a.ldc, b.occ, nbas, (int)kpad, a.ldc, (int)kpad, Ct, Co, nullptr, 0, nullptr, 0, s);
+      orb[sp] = {(int)kpad, Ct, Co, b.occ, (double*)(base + offs[8]), psi_tiles};
+      g.orb[sp] = &orb[sp];
+    } else {
+      launch_pmat_f64(b, kpad, s);
+    }
+  }
   g.rows = (double*)(base + offs[0]);
   g.plane = plane;
   g.ld = ld;

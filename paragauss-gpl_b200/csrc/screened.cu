@@ -1056,8 +1056,31 @@ int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npt
 
 void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
                    const double* gy, const double* gz, const double* P, int64_t ldc, double* X, double* rho,
-                   double* grx, double* gry, double* grz, cudaStream_t st) {
+                   double* grx, double* gry, double* grz, const GradOrbitals* orb, cudaStream_t st) {
   const int smem = sdensity_smem(sp->max_n);
+  if (orb) {
+    raise_smem_limit(k_sdensity<false, true, kPsi>, smem);
+    raise_smem_limit(k_sdensity<true, true, kFromPsi>, smem);
+    raise_smem_limit(k_sdensity<false, true, kFromPsi>, smem);
+    const int64_t parts = (nt + orb->psi_tiles - 1) / orb->psi_tiles, step = (nt + parts - 1) / parts;
+    for (int64_t u = 0; u < nt; u += step) {
+      const dim3 grid((unsigned)std::min(step, nt - u), 2);
+      const int64_t p = u * 128;
+      const SPlanes pu{F, F, F, rho + p, nullptr, nullptr}, px{orb->psi, nullptr, nullptr, nullptr, nullptr, nullptr};
+      k_sdensity<false, true, kPsi><<<grid, kSThreads, smem, st>>>(
+          pu, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, orb->orb, orb->nop, false, nullptr,
+          nullptr, nullptr, orb->psi, orb->nop, orb->nop, orb->occ);
+      if (gx)
+        k_sdensity<true, true, kFromPsi><<<grid, kSThreads, smem, st>>>(
+            px, gx, gy, gz, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, orb->scaled, ldc, false, grx + p, gry + p,
+            grz + p, X, orb->nop, orb->nop, nullptr);
+      else
+        k_sdensity<false, true, kFromPsi><<<grid, kSThreads, smem, st>>>(
+            px, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, orb->scaled, ldc, false, nullptr,
+            nullptr, nullptr, X, orb->nop, orb->nop, nullptr);
+    }
+    return;
+  }
   const SPlanes pl{F, F, F, rho, rho, rho};
   const dim3 grid((unsigned)nt, 2);
   if (gx) {
@@ -1079,13 +1102,17 @@ void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, con
 // margin of 1.15 the form chosen is the faster one; above it P stays (nocc near
 // nbas, where the orbital form is up to twice the products).  INT8 keeps P, whose
 // digits are what its products read.
+bool orbital_form_pays(const ScreenPlan* sp, int64_t nop) {
+  return kOrbitalMargin * 2.0 * (double)nop * (double)sp->nlisted < sp->sum_n2;
+}
+// (60 atoms: 256 MB of psi 6.7 ms, 1 GB 6.45: fewer half-empty last waves)
+int64_t orbital_psi_tiles(const ScreenPlan* sp, int64_t nop) {
+  return std::min(sp->chunk_tiles, std::max<int64_t>(1, (int64_t(1) << 27) / (nop * 128)));
+}
 bool screen_orbital_form(ScreenPlan* sp, int nop) {
-  if (sp->mixed || kOrbitalMargin * 2.0 * nop * (double)sp->nlisted >= sp->sum_n2) return false;
+  if (sp->mixed || !orbital_form_pays(sp, nop)) return false;
   if (!sp->gga) return true;
-  // psi of as many tiles as 1 GB holds, the rest in further launches (60 atoms: 256 MB 6.7 ms, 1 GB 6.45: fewer
-  // half-empty last waves)
-  const int64_t per = (int64_t)nop * 128;
-  const int64_t tiles = std::min(sp->chunk_tiles, std::max<int64_t>(1, (int64_t(1) << 27) / per));
+  const int64_t per = (int64_t)nop * 128, tiles = orbital_psi_tiles(sp, nop);
   if (tiles * per > sp->psi_cap) {
     cudaFree(sp->psi);
     sp->psi = nullptr;

@@ -71,11 +71,22 @@ struct ScreenPlan {
 int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
                      const std::vector<double>& R2, const std::vector<int>& r2off, const double* wraw,
                      const int* owner, int64_t max_rows, cudaStream_t st, std::string& err);
-// X = F_t P[S_t, S_t] of the chunk's tiles ([slot][128] rows, padding rows of F
+// The orbitals in the place of P (orbital_form_pays): nop padded, C [function][nop], occ C
+// [nop][ldc], occupations [nop], and psi for psi_tiles tiles at a time.
+struct GradOrbitals {
+  int nop;
+  const double *orb, *scaled, *occ;
+  double* psi;
+  int64_t psi_tiles;
+};
+bool orbital_form_pays(const ScreenPlan* sp, int64_t nop);
+// tiles whose psi is held at once: those of a chunk, as many as 1 GB holds
+int64_t orbital_psi_tiles(const ScreenPlan* sp, int64_t nop);
+// X = F_t P[S_t, S_t] (by the orbitals when orb is not null) of the chunk's tiles ([slot][128] rows, padding rows of F
 // zero), with rho[p] = sum X F and (gx not null) gr[p] = 2 sum X grad phi.
 void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
                    const double* gy, const double* gz, const double* P, int64_t ldc, double* X, double* rho,
-                   double* grx, double* gry, double* grz, cudaStream_t st);
+                   double* grx, double* gry, double* grz, const GradOrbitals* orb, cudaStream_t st);
 
 
 }  // namespace pgxc
