@@ -3,14 +3,15 @@
 // Per geometry (screen_create):
 //   Morton order of the grid, tiles of 128 points (padded with weight-0 copies);
 //   k_tile_atom_d2    smallest squared distance of each tile to each atom;
-//   host plan         per tile the listed functions (slots, padded to 32), the
-//                     basis work items (tile, shell, radial mask) and chunks.
+//   k_plan_count, k_plan_fill  per tile the listed functions (slots, padded to
+//                     32) and the basis work items (tile, shell, radial mask);
+//                     the host sums the counts and makes the chunks.
 // Per build (screen_run), per chunk of tiles:
 //   k_basis_items     phi, grad phi of listed functions only     [K1]
 //   k_tile_init       (first) clears: the padding slots at the end of each tile's
 //                     list, and what the INT8 stages add or max into
 //   k_sdensity        X = phi_t P[S_t, S_t] on DMMA, P gathered by cp.async,
-//                     fused rho, grad rho                          [K3]
+//                     fused rho, grad rho (or by the orbitals)     [K3]
 //   k_functional      (kernels_fp64.cu)                            [K2]
 //   k_svpot           H[S_t, S_t] += Z_t^T phi_t on DMMA with Z = A phi
 //                     (+ B . grad phi) formed in shared memory, scatter-added
@@ -306,6 +307,8 @@ struct SPlanes {
 };
 // psi's way through memory and the second launch (screen_orbital_form)
 constexpr double kOrbitalMargin = 1.15;
+// elements of psi held at once, 1 GB (60 atoms: 256 MB 6.7 ms, 1 GB 6.45: fewer half-empty last waves)
+constexpr int64_t kPsiMost = int64_t(1) << 27;
 // The tile's slot -> function list in shared memory, -1 from its slots to a
 // whole block past them: every index the kernels form is inside it, guarded or
 // not (a guarded shared-memory load may be executed all the same).
@@ -527,7 +530,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
       b[1] = By[pt];
       b[2] = Bz[pt];
     }
-#pragma unroll 8
+#pragma unroll(GRAD ? 8 : 16)  // (16 with gradients: 8.35 -> 8.6 ms; without, 20 atoms meta-GGA 1.03 -> 1.00)
     for (int i = 0; i < kRows; ++i) {  // rows past the listed functions are the tile's zero padding
       const int64_t o = (sb + I0 + i) * 128 + tid;
       double z = a * phi[o];
@@ -797,7 +800,6 @@ void screen_destroy(ScreenPlan* sp) {
   if (!sp) return;
   if (sp->mixed) screen_mixed_destroy(sp->mixed);
   for (void* p : sp->allocs) cudaFree(p);
-  cudaFree(sp->psi);
   for (auto& c : sp->cev)
     for (auto& e : c)
       if (e) cudaEventDestroy(e);
@@ -953,7 +955,21 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     if (e == cudaSuccess) e = cudaMemsetAsync(*p + (brows - kSlack * 128), 0, sizeof(**p) * kSlack * 128, st);
     return e;
   };
-  SP_TRY(plane(&sp->phi), "cudaMalloc (phi)");
+  // psi of the orbital form lies behind phi: up to the longest that the form is taken for, so that no build
+  // allocates (a 12-atom context's first build 0.98 ms with an allocation of its own, 0.61 without)
+  if (in.gga && !mixed && sp->nlisted > 0) {
+    const int64_t most = (int64_t)(sp->sum_n2 / (2.0 * kOrbitalMargin * (double)sp->nlisted));
+    const int64_t cap = std::min(kPsiMost, sp->chunk_tiles * most * 128);
+    if (8.0 * (double)cap < 0.1 * (double)freeb && sp_alloc(sp, &sp->phi, brows + (size_t)cap) == cudaSuccess) {
+      sp->psi = sp->phi + brows;
+      sp->psi_cap = cap;
+    } else {
+      cudaGetLastError();  // no room: the builds take P
+      sp->phi = nullptr;
+    }
+  }
+  if (sp->phi) SP_TRY(cudaMemsetAsync(sp->phi + (brows - kSlack * 128), 0, sizeof(double) * kSlack * 128, st), "memset");
+  else SP_TRY(plane(&sp->phi), "cudaMalloc (phi)");
   if (in.gga && sp->gf32) {
     SP_TRY(plane(&sp->fx), "cudaMalloc (grad phi)");
     SP_TRY(plane(&sp->fy), "cudaMalloc (grad phi)");
@@ -1105,26 +1121,12 @@ void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, con
 bool orbital_form_pays(const ScreenPlan* sp, int64_t nop) {
   return kOrbitalMargin * 2.0 * (double)nop * (double)sp->nlisted < sp->sum_n2;
 }
-// (60 atoms: 256 MB of psi 6.7 ms, 1 GB 6.45: fewer half-empty last waves)
 int64_t orbital_psi_tiles(const ScreenPlan* sp, int64_t nop) {
-  return std::min(sp->chunk_tiles, std::max<int64_t>(1, (int64_t(1) << 27) / (nop * 128)));
+  return std::min(sp->chunk_tiles, std::max<int64_t>(1, kPsiMost / (nop * 128)));
 }
-bool screen_orbital_form(ScreenPlan* sp, int nop) {
+bool screen_orbital_form(const ScreenPlan* sp, int nop) {
   if (sp->mixed || !orbital_form_pays(sp, nop)) return false;
-  if (!sp->gga) return true;
-  const int64_t per = (int64_t)nop * 128, tiles = orbital_psi_tiles(sp, nop);
-  if (tiles * per > sp->psi_cap) {
-    cudaFree(sp->psi);
-    sp->psi = nullptr;
-    sp->psi_cap = 0;
-    if (cudaMalloc(&sp->psi, sizeof(double) * (size_t)(tiles * per)) != cudaSuccess) {
-      cudaGetLastError();  // no room: the build takes P instead
-      sp->psi = nullptr;
-      return false;
-    }
-    sp->psi_cap = tiles * per;
-  }
-  return true;
+  return !sp->gga || (int64_t)nop * 128 <= sp->psi_cap;
 }
 
 // rho, grad rho and (tau not null) the tau sums of one spin by its orbitals

@@ -324,7 +324,7 @@ __device__ __forceinline__ void acc_cols(uint32_t taddr, double* x) {
   }
 }
 // Persistent: CTA c takes the chunk's tiles c, c + G, c + 2G, ... (G = grid
-// size); the copy / MMA / epilogue pipeline runs on across tile boundaries.
+// size) or its list (TileWalk); the copy / MMA / epilogue pipeline runs on across tile boundaries.
 // rho and grad rho are accumulated with atomics (the two column halves of a
 // point and nothing else), so they must be zero on entry.
 // GT: element type of the grad phi planes (staged beside phi in the same
@@ -735,6 +735,9 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
 // blocks I (B, Z); K = the tile's 128 points in 4 steps; each A block is one
 // copy of whole 8-slot groups and stays resident for its 48-slot blocks.
 // Persistent like k_sm_density.
+// Bound by the L2's write path into V: 60 atoms 1.53 ms, 200 atoms 12.7; without
+// the additions 0.98 and 7.6, with plain stores in their place unchanged, without
+// the TMEM loads and the digit combination 1.48 and 11.9.
 // ---------------------------------------------------------------------------
 constexpr int kVStages = 8;
 struct VSmem {

@@ -49,7 +49,7 @@ struct ScreenPlan {
   bool mgga = false;
   int functional = 0;        // PGXC_XC_* (the meta-GGA step selects its functional by id)
   double* tq = nullptr;      // meta-GGA: 4 point arrays per spin (2 tau_x, 2 tau_y, 2 tau_z, C)
-  double* psi = nullptr;     // [tile][padded orbital][128] of the orbital form (GGA), made by the first build that takes it
+  double* psi = nullptr;     // [tile][padded orbital][128] of the orbital form (FP64 GGA), psi_cap elements behind phi
   int64_t psi_cap = 0;
   double* partial = nullptr;
   double* V = nullptr;       // [ispin][nbas][nbas]
