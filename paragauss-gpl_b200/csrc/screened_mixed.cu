@@ -293,8 +293,12 @@ struct DensSmem {
   uint64_t acc_empty[2];
   uint64_t e_full[kERing];
   uint64_t e_empty[kERing];
+  double part[2][4][128];  // rho, grad rho of the first two column thirds, for the last one to add
+  uint64_t p_full[4];      // per TMEM lane quarter
+  uint64_t p_empty[4];
   uint32_t tslot;
 };
+static_assert(sizeof(DensSmem) <= tc::kWholeSmSmem, "one CTA's shared memory");
 // warps 0-7 and 11-14 epilogue (three per TMEM lane quarter), 8 MMA, 9 operand
 // copies, 10 epilogue-operand copies, 15 idle
 constexpr int kDensThreads = tc::kWholeSmThreads;
@@ -325,8 +329,9 @@ __device__ __forceinline__ void acc_cols(uint32_t taddr, double* x) {
 }
 // Persistent: CTA c takes the chunk's tiles c, c + G, c + 2G, ... (G = grid
 // size) or its list (TileWalk); the copy / MMA / epilogue pipeline runs on across tile boundaries.
-// rho and grad rho are accumulated with atomics (the two column halves of a
-// point and nothing else), so they must be zero on entry.
+// The three column thirds of a point are added in a fixed order through shared
+// memory (as atomics their order, and with it the last bits of E_xc, could
+// differ from run to run).
 // GT: element type of the grad phi planes (staged beside phi in the same
 // ring entry: phi in doubles, then the three gradient blocks in GT).
 template <bool GGA, typename GT>
@@ -354,6 +359,10 @@ __global__ void __launch_bounds__(kDensThreads, 1)
     for (int r = 0; r < kERing; ++r) {
       tc::mbar_init(&S.e_full[r], 1);
       tc::mbar_init(&S.e_empty[r], 128);  // the four warps of one column third
+    }
+    for (int q = 0; q < 4; ++q) {
+      tc::mbar_init(&S.p_full[q], 64);  // the quarter's warps of the first two thirds
+      tc::mbar_init(&S.p_empty[q], 32);
     }
     tc::mbar_fence_init();
   }
@@ -458,8 +467,8 @@ __global__ void __launch_bounds__(kDensThreads, 1)
   } else {  // epilogue: point row = 32 (warp & 3) + lane, columns 16 third .. +15 of each slot block
     const int row = (warp & 3) * 32 + lane, third = warp < 8 ? (warp >> 2) : 2;
     const uint32_t trow = tbase + ((uint32_t)((warp & 3) * 32) << 16);
-    int jj = 0;
-    for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next()) {
+    int jj = 0, tt = 0;
+    for (TileWalk wk(order, start, nt); wk.more() && ok; wk.next(), ++tt) {
       const int64_t ti = wk.tile();
       const int64_t sg = tso[t0 + ti];
       const int64_t sb = sg - s0;
@@ -506,13 +515,35 @@ __global__ void __launch_bounds__(kDensThreads, 1)
           tc::mbar_arrive(&S.e_empty[r]);
         }
       }
-      if (!ok) break;
-      const int64_t p = ti * 128 + row;
-      atomicAdd(rho + p, r_acc);
-      if (GGA) {
-        atomicAdd(grx + p, 2.0 * g_acc[0]);
-        atomicAdd(gry + p, 2.0 * g_acc[1]);
-        atomicAdd(grz + p, 2.0 * g_acc[2]);
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        break;
+      }
+      const int q = warp & 3;
+      if (third < 2) {
+        if (!tc::mbar_wait_warp(&S.p_empty[q], (tt & 1) ^ 1)) {
+          ok = false;
+          break;
+        }
+        S.part[third][0][row] = r_acc;
+        if (GGA) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) S.part[third][1 + d][row] = g_acc[d];
+        }
+        tc::mbar_arrive(&S.p_full[q]);
+      } else {
+        if (!tc::mbar_wait_warp(&S.p_full[q], tt & 1)) {
+          ok = false;
+          break;
+        }
+        const int64_t p = ti * 128 + row;
+        rho[p] = S.part[0][0][row] + S.part[1][0][row] + r_acc;
+        if (GGA) {
+          grx[p] = 2.0 * (S.part[0][1][row] + S.part[1][1][row] + g_acc[0]);
+          gry[p] = 2.0 * (S.part[0][2][row] + S.part[1][2][row] + g_acc[1]);
+          grz[p] = 2.0 * (S.part[0][3][row] + S.part[1][3][row] + g_acc[2]);
+        }
+        tc::mbar_arrive(&S.p_empty[q]);
       }
     }
     if (!ok) atomicExch(err, 1);
