@@ -1007,7 +1007,7 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     // identically zero on a tile is listed), in chunks of under ~4 GB of slot rows
     std::string e;
     const int st = grad_plan_create(&c->gplan, a, c->natm, c->npts, c->shells, c->grad_r2, c->grad_r2off, c->d_wraw,
-                                    c->d_owner, (int64_t)(4.0e9 / (1024.0 * planes)), s, e);
+                                    c->d_owner, c->screen, (int64_t)(4.0e9 / (1024.0 * planes)), s, e);
     if (st) return set_err(c, st, "gradient plan: " + e);
   }
   const ScreenPlan* gp = c->gplan;

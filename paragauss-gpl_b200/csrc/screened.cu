@@ -687,8 +687,8 @@ void screen_listing_radii(const std::vector<DevShell>& shells, const double* exp
 // atom) and the basis items.  perm: the Morton order is kept in it (caller
 // frees) when not null.
 static int build_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
-                       const std::vector<double>& R2, const std::vector<int>& r2off, int64_t** perm, cudaStream_t st,
-                       std::string& err) {
+                       const std::vector<double>& R2, const std::vector<int>& r2off, const int64_t* order,
+                       cudaStream_t st, std::string& err) {
 #define BL_TRY(call, what)                                                       \
   do {                                                                           \
     cudaError_t e_ = (call);                                                     \
@@ -705,20 +705,21 @@ static int build_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npt
   {
     // Morton order of the points, on the device (ties by point index)
     const int64_t nq = ntiles * 128;
-    int64_t* dperm;
-    BL_TRY(cudaMalloc(&dperm, sizeof(int64_t) * nq), "cudaMalloc");
-    cudaError_t e = morton_perm_device(a.px, a.py, a.pz, n, nq, dperm, st);
+    cudaError_t e = cudaSuccess;
+    if (!order) {  // (kept with the plan: a gradient plan of the same grid takes it)
+      BL_TRY(sp_alloc(sp, &sp->perm, (size_t)nq), "cudaMalloc");
+      e = morton_perm_device(a.px, a.py, a.pz, n, nq, sp->perm, st);
+      order = sp->perm;
+    }
     if (e == cudaSuccess) e = sp_alloc(sp, &sp->qx, 4 * nq);
     if (e == cudaSuccess) {
       sp->qy = sp->qx + nq;
       sp->qz = sp->qx + 2 * nq;
       sp->qw = sp->qx + 3 * nq;
-      k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(dperm, nq, a.px, a.py, a.pz, a.w, sp->qx,
+      k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(order, nq, a.px, a.py, a.pz, a.w, sp->qx,
                                                                    sp->qy, sp->qz, sp->qw);
-      e = cudaStreamSynchronize(st);
+      e = cudaGetLastError();
     }
-    if (perm && e == cudaSuccess) *perm = dperm;
-    else cudaFree(dperm);
     BL_TRY(e, "grid reordering");
   }
   // --- per-tile lists, on the device: distances, counts, then (their places known) the lists.  On the
@@ -1035,14 +1036,13 @@ __global__ void k_gather_hosts(const int64_t* __restrict__ perm, int64_t nq, con
 
 int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
                      const std::vector<double>& R2, const std::vector<int>& r2off, const double* wraw,
-                     const int* owner, int64_t max_rows, cudaStream_t st, std::string& err) {
+                     const int* owner, const ScreenPlan* from, int64_t max_rows, cudaStream_t st, std::string& err) {
   *out = nullptr;
   ScreenPlan* sp = new ScreenPlan();
   SP_TRY(cudaGetDevice(&sp->nsm), "cudaGetDevice");
   SP_TRY(cudaDeviceGetAttribute(&sp->nsm, cudaDevAttrMultiProcessorCount, sp->nsm), "cudaDeviceGetAttribute");
-  int64_t* perm = nullptr;
-  if (const int st2 = build_lists(sp, a, natm, npts, shells, R2, r2off, &perm, st, err)) {
-    cudaFree(perm);
+  const int64_t* perm = from ? from->perm : nullptr;
+  if (const int st2 = build_lists(sp, a, natm, npts, shells, R2, r2off, perm, st, err)) {
     screen_destroy(sp);
     return st2;
   }
@@ -1050,10 +1050,10 @@ int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npt
   cudaError_t e = sp_alloc(sp, &sp->qwraw, nq);
   if (e == cudaSuccess) e = sp_alloc(sp, &sp->qowner, nq);
   if (e == cudaSuccess) {
-    k_gather_hosts<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(perm, nq, wraw, owner, sp->qwraw, sp->qowner);
-    e = cudaStreamSynchronize(st);
+    k_gather_hosts<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(perm ? perm : sp->perm, nq, wraw, owner, sp->qwraw,
+                                                                 sp->qowner);
+    e = cudaGetLastError();
   }
-  cudaFree(perm);
   SP_TRY(e, "gradient plan");
   max_rows = std::max<int64_t>(max_rows, sp->max_n);
   sp->chunk_t0.push_back(0);

@@ -29,6 +29,7 @@ struct ScreenPlan {
   bool basis_ready = false;  // ... and a completed build has filled them
   // device, whole grid
   double *qx = nullptr, *qy = nullptr, *qz = nullptr, *qw = nullptr;  // Morton-ordered points [ntiles*128]
+  int64_t* perm = nullptr;  // their indices in the caller's grid (null: another plan's order was taken)
   int64_t* tso = nullptr;   // [ntiles+1] first slot of each tile
   int* slot_fn = nullptr;   // [nslots] function of each slot, -1 for padding
   int* listed = nullptr;    // [ntiles] listed (not padding) slots of each tile
@@ -67,10 +68,11 @@ struct ScreenPlan {
 
 // A plan of tiles and lists alone (no build buffers), in chunks of at most
 // max_rows slot rows, for the nuclear gradient; R2 with threshold 0, so that
-// unlisted functions and their derivatives are exactly zero on the tile.
+// unlisted functions and their derivatives are exactly zero on the tile.  from: the
+// context's own plan of the same grid, whose point order is taken, or null.
 int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
                      const std::vector<double>& R2, const std::vector<int>& r2off, const double* wraw,
-                     const int* owner, int64_t max_rows, cudaStream_t st, std::string& err);
+                     const int* owner, const ScreenPlan* from, int64_t max_rows, cudaStream_t st, std::string& err);
 // The orbitals in the place of P (orbital_form_pays): nop padded, C [function][nop], occ C
 // [nop][ldc], occupations [nop], and psi for psi_tiles tiles at a time.
 struct GradOrbitals {
