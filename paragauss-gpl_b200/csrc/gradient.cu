@@ -306,7 +306,11 @@ __global__ void __launch_bounds__(128) k_grad_w(const int64_t* __restrict__ tso,
 // point.  Block = a tile, thread = point; a tile's slots come atom by atom, so
 // -q is summed over an atom's functions in registers and reduced over the warp
 // once per atom (a reduction per function took most of the instructions), +q
-// goes to the point's host through the thread's running sum.
+// goes to the point's host through the thread's running sum.  The functions of
+// the point's own host are left out of both: -q + q = 0 on the same atom, and
+// near a nucleus these terms are by far the largest, so that rounded once on
+// each side they were most of the error (40 atoms: two runs differed by 4e-12
+// of the gradient's norm and its sum over atoms was 2e-12, now 3e-15 and 1e-14).
 __global__ void __launch_bounds__(128) k_grad_orb(bool gga, bool mgga, int ispin, int natm,
                                                   const int64_t* __restrict__ tso, const int* __restrict__ listed,
                                                   const int* __restrict__ slot_fn, int64_t t0, int64_t s0,
@@ -330,10 +334,11 @@ __global__ void __launch_bounds__(128) k_grad_orb(bool gga, bool mgga, int ispin
   }
   double tot[3] = {0, 0, 0}, qa[3] = {0, 0, 0};
   int atom = nl > 0 ? fatom[fn[0]] : 0;
+  const int h = owner[t * 128 + threadIdx.x];
   auto flush = [&]() {
     for (int k = 0; k < 3; ++k) {
-      tot[k] += qa[k];
-      double v = qa[k];
+      double v = atom == h ? 0.0 : qa[k];
+      tot[k] += v;
       for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
       if (lane == 0) atomicAdd(&gs[3 * atom + k], -v);
       qa[k] = 0.0;
@@ -379,7 +384,6 @@ __global__ void __launch_bounds__(128) k_grad_orb(bool gga, bool mgga, int ispin
   }
   flush();
   // host sums: one shared atomic per warp when its points share a host
-  const int h = owner[t * 128 + threadIdx.x];
   const int h0 = __shfl_sync(0xffffffffu, h, 0);
   if (__all_sync(0xffffffffu, h == h0)) {
     for (int k = 0; k < 3; ++k) {

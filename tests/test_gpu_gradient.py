@@ -45,6 +45,23 @@ def test_mgga_gradient_matches_oracle(xc, ispin, layout):
     np.testing.assert_allclose(g.sum(0), 0.0, atol=1e-9 * scale)
 
 
+@pytest.mark.parametrize("xc,ispin", [("VWN", 1), ("PBE", 2), ("TPSS", 1)])
+def test_core_terms_do_not_round_the_gradient(xc, ispin):
+    """What a function contributes on its own atom's points leaves and enters the
+    same atom.  With core functions (exponents up to 1e4) those terms are the
+    largest by far; a gradient that does not carry them has a sum over atoms,
+    and a difference between two calls, of the rounding of the other terms
+    alone: tiles (300) x eps (1.1e-16) of the largest component, three times over."""
+    case = cases.build_case("core", ["C", "H", "O", "H"], np.array([[0, 0, 0], [2.1, 0, 0], [0, 2.3, 0], [0, 0, 2.0]]),
+                            seed=5, exp_range=(0.05, 1e4), nrad=50, nang=194, functional=xc, nocc=8, ispin=ispin,
+                            orthonormalise=False)
+    with lib.Context(case, weighted=False) as ctx:
+        a, b = ctx.xc_gradient()[0], ctx.xc_gradient()[0]
+    scale = float(np.max(np.abs(a)))
+    assert float(np.max(np.abs(a.sum(0)))) < 1e-13 * scale
+    assert float(np.max(np.abs(a - b))) < 1e-13 * scale
+
+
 def test_gradient_needs_the_raw_grid():
     case = cases.small_case(functional="PBE", seed=63)
     O.weight_case(case)
