@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(128) k_grad_orb(bool gga, bool mgga, int ispin
   __syncthreads();
   const int64_t t = t0 + blockIdx.x, p = (int64_t)blockIdx.x * 128 + threadIdx.x;
   const int lane = threadIdx.x & 31, nl = listed[t];
-  const int* fn = slot_fn + tso[t];
+  const int* fn = slot_fn + (tso[t] - s0);
   double a[2] = {0, 0}, b[2][3] = {{0, 0, 0}, {0, 0, 0}}, ct[2] = {0, 0};
   for (int sp = 0; sp < ispin; ++sp) {
     a[sp] = coef[(kCoefPlanes * sp) * ld + p];
@@ -648,9 +648,11 @@ int64_t grad_planes(bool gga, bool mgga, int ispin) {
   return mgga ? 10 + 4 * ispin : gga ? 11 + 2 * ispin : 4 + ispin;
 }
 
-void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan* sp, size_t c, cudaStream_t st) {
+void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, ScreenPlan* sp, size_t c, cudaStream_t st) {
   const int64_t t0 = sp->chunk_t0[c], nt = sp->chunk_t0[c + 1] - t0, s0 = sp->h_tso[(size_t)t0], ld = g.ld;
   const int64_t plane = g.plane;
+  const int* slot_fn = g.lists->slot_fn;
+  grad_plan_lists(sp, a, c, *g.lists, st);
   double* B = g.rows;                                  // phi, grad phi and (GGAs) the Hessian
   double* XY = B + (g.gga ? 10 : 4) * plane;           // per spin X; X, V (GGA); X, Y_j (meta-GGA)
   const int nxy = g.mgga ? 4 : g.gga ? 2 : 1;
@@ -659,7 +661,7 @@ void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan*
                            s0,     t0,      nullptr, nullptr, nullptr, nullptr, nullptr};
   auto hess = [&](auto Lc) {
     constexpr int L = decltype(Lc)::value;
-    const BasisItem* it = sp->items[L] + sp->tile_item[L][(size_t)t0];
+    const BasisItem* it = g.lists->items[L];
     const int64_t n = sp->tile_item[L][(size_t)(t0 + nt)] - sp->tile_item[L][(size_t)t0];
     if (n > 0)
       k_hess_items<L><<<(unsigned)std::min<int64_t>(n, (int64_t)sp->nsm * 32), 128, 0, st>>>(it, n, io, a.sa, g.gga,
@@ -674,11 +676,11 @@ void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan*
   for (int s = 0; s < g.ispin; ++s) {
     double* d = g.den + (int64_t)(7 * s) * ld;
     double* X = XY + (int64_t)(nxy * s) * plane;
-    grad_contract(sp, t0, nt, s0, B, g.gga ? gx : nullptr, gy, gz, g.P[s], a.ldc, X, d, d + ld, d + 2 * ld, d + 3 * ld,
+    grad_contract(sp, slot_fn, t0, nt, s0, B, g.gga ? gx : nullptr, gy, gz, g.P[s], a.ldc, X, d, d + ld, d + 2 * ld, d + 3 * ld,
                   g.orb[s], st);
     // the Y_j only for meta-GGAs (tau and its terms), GGAs take V = W P after the coefficients
     for (int j = 0; j < 3 && g.mgga; ++j)
-      grad_contract(sp, t0, nt, s0, B + (1 + j) * plane, nullptr, nullptr, nullptr, g.P[s], a.ldc, X + (1 + j) * plane,
+      grad_contract(sp, slot_fn, t0, nt, s0, B + (1 + j) * plane, nullptr, nullptr, nullptr, g.P[s], a.ldc, X + (1 + j) * plane,
                     d + (4 + j) * ld, nullptr, nullptr, nullptr, g.orb[s], st);
   }
   k_grad_coef<<<(unsigned)nt, 128, 0, st>>>(a.xc, g.functional, g.gga, g.ispin, ld, sp->qw + t0 * 128,
@@ -686,12 +688,12 @@ void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan*
   for (int s = 0; s < g.ispin && g.gga && !g.mgga; ++s) {
     k_grad_w<<<(unsigned)nt, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, B, plane,
                                            g.coef + (int64_t)(kCoefPlanes * s + 1) * ld, ld, W);
-    grad_contract(sp, t0, nt, s0, W, nullptr, nullptr, nullptr, g.P[s], a.ldc, XY + (int64_t)(nxy * s + 1) * plane,
+    grad_contract(sp, slot_fn, t0, nt, s0, W, nullptr, nullptr, nullptr, g.P[s], a.ldc, XY + (int64_t)(nxy * s + 1) * plane,
                   g.den, nullptr, nullptr, nullptr, g.orb[s], st);  // (rho is done with: its sum goes to scratch)
   }
   const int smem = (int)sizeof(double) * 3 * g.natm;
   if (smem > 48 * 1024) raise_smem_limit(k_grad_orb, smem);
-  k_grad_orb<<<(unsigned)nt, 128, smem, st>>>(g.gga, g.mgga, g.ispin, g.natm, sp->tso, sp->listed, sp->slot_fn, t0, s0,
+  k_grad_orb<<<(unsigned)nt, 128, smem, st>>>(g.gga, g.mgga, g.ispin, g.natm, sp->tso, sp->listed, slot_fn, t0, s0,
                                               g.fatom, sp->qowner, B, plane, XY, nxy, g.coef, ld, g.grad);
 }
 

@@ -28,12 +28,14 @@ int64_t grad_planes(bool gga, bool mgga, int ispin);
 
 // One gradient's buffers and kind.
 struct GradOrbitals;
+struct TileLists;
 struct GradChunk {
   bool gga, mgga;            // meta-GGAs set both
   int ispin, functional, natm;
   const double* P[2];        // density matrices, leading dimension BuildArgs::ldc
   const GradOrbitals* orb[2]; // not null: the orbitals instead
   const int* fatom;          // atom of each function
+  const TileLists* lists;    // room for the lists of any chunk
   double* rows;              // grad_planes planes of `plane` doubles
   int64_t plane;
   int64_t ld;                // points of the largest chunk
@@ -45,7 +47,7 @@ struct GradChunk {
 };
 // The orbital terms of chunk c of the plan (grad_plan_create): -sum_g q to atom(mu)
 // and +sum_mu q to host(g); also ef and E_xc.
-void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, const ScreenPlan* sp, size_t c, cudaStream_t st);
+void launch_grad_chunk(const GradChunk& g, const BuildArgs& a, ScreenPlan* sp, size_t c, cudaStream_t st);
 
 // The weight term sum_g ef_g dW_host(r_g)/dR over the chunk's points; dist is
 // the natm x natm atom distance matrix followed by its reciprocals (the

@@ -1010,7 +1010,7 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
                                     c->d_owner, c->screen, (int64_t)(4.0e9 / (1024.0 * planes)), s, e);
     if (st) return set_err(c, st, "gradient plan: " + e);
   }
-  const ScreenPlan* gp = c->gplan;
+  ScreenPlan* gp = c->gplan;
   const int64_t nq = gp->ntiles * 128, ld = gp->chunk_tiles * 128;
   const int64_t plane = (gp->chunk_slots + kSlack) * 128;
   // The weight term needs only each point's w_raw f and runs after the chunk loop in launches of ldw
@@ -1021,15 +1021,18 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   // one scratch buffer, carved in 256-byte aligned pieces and kept in the
   // context for the next call (allocation and release of several GB per call
   // would cost more than the gradient's kernels)
-  size_t sizes[9] = {sizeof(double) * (size_t)(planes * plane), sizeof(double) * 7 * ispin * (size_t)ld,
-                           sizeof(double) * 5 * ispin * (size_t)ld,   sizeof(double) * (size_t)nq,
-                           sizeof(double) * 3 * c->natm,              sizeof(double),
-                           sizeof(double) * ((size_t)7 * c->natm * ldw / 2 + 1), sizeof(int) * (size_t)nbas, 0};
+  constexpr int kLists = 8, kPsiAt = kLists + kMaxL + 2;  // the chunk's lists: slot_fn, items of each l; then psi
+  size_t sizes[kPsiAt + 1] = {sizeof(double) * (size_t)(planes * plane), sizeof(double) * 7 * ispin * (size_t)ld,
+                              sizeof(double) * 5 * ispin * (size_t)ld,   sizeof(double) * (size_t)nq,
+                              sizeof(double) * 3 * c->natm,              sizeof(double),
+                              sizeof(double) * ((size_t)7 * c->natm * ldw / 2 + 1), sizeof(int) * (size_t)nbas,
+                              sizeof(int) * (size_t)gp->chunk_slots};
+  for (int l = 0; l <= kMaxL; ++l) sizes[kLists + 1 + l] = sizeof(BasisItem) * (size_t)gp->chunk_items[l];
   bool orbitals = orbital_form_pays(gp, kpad);
   const int64_t psi_tiles = orbital_psi_tiles(gp, kpad);
-  if (orbitals) sizes[8] = sizeof(double) * (size_t)(psi_tiles * kpad * 128);
-  size_t offs[9], total = 0;
-  for (int i = 0; i < 9; ++i) {
+  if (orbitals) sizes[kPsiAt] = sizeof(double) * (size_t)(psi_tiles * kpad * 128);
+  size_t offs[kPsiAt + 1], total = 0;
+  for (int i = 0; i <= kPsiAt; ++i) {
     offs[i] = total;
     total += (sizes[i] + 255) / 256 * 256;
   }
@@ -1037,11 +1040,12 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     if (c->grad_scr) cudaFree(c->grad_scr);
     c->grad_scr = nullptr;
     c->grad_scr_bytes = 0;
+    gp->filled = -1;
     cudaError_t e = cudaMalloc(&c->grad_scr, total);
     if (e != cudaSuccess && orbitals) {  // no room for psi: P instead
       cudaGetLastError();
       orbitals = false;
-      total = offs[8];
+      total = offs[kPsiAt];
       e = cudaMalloc(&c->grad_scr, total);
     }
     if (e != cudaSuccess) {
@@ -1071,7 +1075,7 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     if (orbitals) {  // both turned forms lie in P's place (2 nop <= ldc)
       double *Ct = b.P, *Co = b.P + kpad * a.ldc;
       launch_turn_orbitals(b.C, a.ldc, b.occ, nbas, (int)kpad, a.ldc, (int)kpad, Ct, Co, nullptr, 0, nullptr, 0, s);
-      orb[sp] = {(int)kpad, Ct, Co, b.occ, (double*)(base + offs[8]), psi_tiles};
+      orb[sp] = {(int)kpad, Ct, Co, b.occ, (double*)(base + offs[kPsiAt]), psi_tiles};
       g.orb[sp] = &orb[sp];
     } else {
       launch_pmat_f64(b, kpad, s);
@@ -1088,6 +1092,10 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   double* wscr = (double*)(base + offs[6]);
   int* dfatom = (int*)(base + offs[7]);
   g.fatom = dfatom;
+  TileLists lists{};
+  lists.slot_fn = (int*)(base + offs[kLists]);
+  for (int l = 0; l <= kMaxL; ++l) lists.items[l] = (BasisItem*)(base + offs[kLists + 1 + l]);
+  g.lists = &lists;
   int rc = PGXC_OK;
   do {
     if (cudaMemcpyAsync(dfatom, fatom.data(), sizeof(int) * nbas, cudaMemcpyHostToDevice, s) != cudaSuccess ||
@@ -1120,6 +1128,7 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     if (exc) *exc += he;
   } while (false);
   cudaStreamSynchronize(s);
+  if (rc) gp->filled = -1;  // the lists may not have been made
   return rc;
 }
 

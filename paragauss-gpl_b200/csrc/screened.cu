@@ -120,24 +120,21 @@ __global__ void __launch_bounds__(128) k_plan_count(const float* __restrict__ d2
   if (threadIdx.x < 2 + kMaxL) cnt[t * (2 + kMaxL) + threadIdx.x] = sum[threadIdx.x];
 }
 
-struct PlanItems {
-  BasisItem* items[kMaxL + 1];
-};
 // The slot list (shell by shell: independent function -> radial function, then
-// padding) and the basis items of every tile, in shell order: 128 shells at a
+// padding) and the basis items of tiles t0 + block, in shell order: 128 shells at a
 // time, their places by a block scan.  start[t] = {first item of l = 0..3}.
 __global__ void __launch_bounds__(128) k_plan_fill(const float* __restrict__ d2, int natm,
                                                    const double* __restrict__ atoms,
                                                    const DevShell* __restrict__ shells, int nsh,
                                                    const double* __restrict__ r2, const int* __restrict__ r2off,
                                                    const int64_t* __restrict__ tso, const int64_t* __restrict__ start,
-                                                   int* __restrict__ slot_fn, PlanItems out) {
+                                                   int64_t t0, TileLists out) {
   __shared__ int scan_n[128];
   __shared__ unsigned scan_l[128];  // four 8-bit counts (at most 128 shells each)
-  const int64_t t = blockIdx.x;
+  const int64_t t = t0 + blockIdx.x;
   const int tid = threadIdx.x;
   int64_t slot0 = tso[t], item0[kMaxL + 1];
-  for (int l = 0; l <= kMaxL; ++l) item0[l] = start[t * (kMaxL + 1) + l];
+  for (int l = 0; l <= kMaxL; ++l) item0[l] = start[t * (kMaxL + 1) + l] - out.i0[l];
   for (int s0 = 0; s0 < nsh; s0 += 128) {
     const int s = s0 + tid;
     DevShell S{};
@@ -176,15 +173,15 @@ __global__ void __launch_bounds__(128) k_plan_fill(const float* __restrict__ d2,
       it.nunc = S.nunc;
       it.seg = S.seg;
       out.items[S.l][item0[S.l] + ((scan_l[tid] - one) >> (8 * S.l) & 255u)] = it;
-      int64_t o = slot;
+      int64_t o = slot - out.s0;
       for (int i = 0; i < 2 * S.l + 1; ++i)
-        for (unsigned long long m = mask; m; m &= m - 1) slot_fn[o++] = S.f0 + i * S.nrad + __ffsll((long long)m) - 1;
+        for (unsigned long long m = mask; m; m &= m - 1) out.slot_fn[o++] = S.f0 + i * S.nrad + __ffsll((long long)m) - 1;
     }
     slot0 += scan_n[127];
     for (int l = 0; l <= kMaxL; ++l) item0[l] += scan_l[127] >> (8 * l) & 255u;
     __syncthreads();
   }
-  for (int64_t o = slot0 + tid; o < tso[t + 1]; o += 128) slot_fn[o] = -1;
+  for (int64_t o = slot0 + tid; o < tso[t + 1]; o += 128) out.slot_fn[o - out.s0] = -1;
 }
 
 // ---------------------------------------------------------------------------
@@ -309,7 +306,8 @@ struct SPlanes {
 constexpr double kOrbitalMargin = 1.15;
 // elements of psi held at once, 1 GB (60 atoms: 256 MB 6.7 ms, 1 GB 6.45: fewer half-empty last waves)
 constexpr int64_t kPsiMost = int64_t(1) << 27;
-// The tile's slot -> function list in shared memory, -1 from its slots to a
+// The tile's slot -> function list (slot_fn of the kernels below begins at the
+// chunk's first slot s0) in shared memory, -1 from its slots to a
 // whole block past them: every index the kernels form is inside it, guarded or
 // not (a guarded shared-memory load may be executed all the same).
 __host__ __device__ constexpr int sfn_len(int n) { return (n + kSBlk - 1) / kSBlk * kSBlk + kSBlk; }
@@ -361,7 +359,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
   const int64_t sb = tso[t] - s0;
   const int nl = listed[t];
   const int m0 = blockIdx.y * kSBlk;
-  load_sfn(sfn, slot_fn + sb + s0, (int)(tso[t + 1] - tso[t]));
+  load_sfn(sfn, slot_fn + sb, (int)(tso[t + 1] - tso[t]));
   const double* A = phi + (FORM == kFromPsi ? (int64_t)blockIdx.x * nop : sb) * 128 + m0;
   const int nk = FORM == kFromPsi ? nop : nl, nn = FORM == kPsi ? nop : nl;  // rows summed over, columns
   const int wm0 = (warp >> 1) * 32, wn0 = (warp & 1) * 32, fr = lane >> 2, fk = lane & 3;
@@ -520,7 +518,7 @@ __global__ void __launch_bounds__(kSThreads, 3)
     }
   };
   load();
-  load_sfn(sfn, slot_fn + sb + s0, (int)(tso[t + 1] - tso[t]));
+  load_sfn(sfn, slot_fn + sb, (int)(tso[t + 1] - tso[t]));
   {
     const int64_t pt = (int64_t)tile * 128 + tid;  // thread = point
     const double a = A[pt];
@@ -682,11 +680,14 @@ void screen_listing_radii(const std::vector<DevShell>& shells, const double* exp
   }
 }
 
-// The tiles and their lists: Morton-ordered points, per tile the listed
-// functions (those whose listing radius exceeds the tile's distance to their
-// atom) and the basis items.  perm: the Morton order is kept in it (caller
-// frees) when not null.
-static int build_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
+// The tiles and the lengths of their lists: Morton-ordered points, per tile the
+// number of listed functions (those whose listing radius exceeds the tile's
+// distance to their atom) and of basis items, and so their places.  order: the
+// points' order, or null: it is made here and kept in sp->perm.  The tables that
+// fill_lists reads stay in sp->tab.  On the host the lists of a 41-atom grid
+// (2,710 tiles, 170,000 items of 80 bytes, copied from pageable memory) were most
+// of the 30 ms of a context's creation.
+static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
                        const std::vector<double>& R2, const std::vector<int>& r2off, const int64_t* order,
                        cudaStream_t st, std::string& err) {
 #define BL_TRY(call, what)                                                       \
@@ -697,110 +698,85 @@ static int build_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npt
       return e_ == cudaErrorMemoryAllocation ? PGXC_ENOMEM : PGXC_ECUDA;         \
     }                                                                            \
   } while (0)
-  const int nsh = (int)shells.size();
-  // --- Morton-ordered, 128-point tiles -----------------------------------
-  const int64_t n = npts;
-  const int64_t ntiles = (n + 127) / 128;
+  constexpr int kCnt = 2 + kMaxL;
+  const int64_t ntiles = (npts + 127) / 128, nq = ntiles * 128;
+  ListTables& T = sp->tab;
   sp->ntiles = ntiles;
-  {
-    // Morton order of the points, on the device (ties by point index)
-    const int64_t nq = ntiles * 128;
-    cudaError_t e = cudaSuccess;
-    if (!order) {  // (kept with the plan: a gradient plan of the same grid takes it)
-      BL_TRY(sp_alloc(sp, &sp->perm, (size_t)nq), "cudaMalloc");
-      e = morton_perm_device(a.px, a.py, a.pz, n, nq, sp->perm, st);
-      order = sp->perm;
-    }
-    if (e == cudaSuccess) e = sp_alloc(sp, &sp->qx, 4 * nq);
-    if (e == cudaSuccess) {
-      sp->qy = sp->qx + nq;
-      sp->qz = sp->qx + 2 * nq;
-      sp->qw = sp->qx + 3 * nq;
-      k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(order, nq, a.px, a.py, a.pz, a.w, sp->qx,
-                                                                   sp->qy, sp->qz, sp->qw);
-      e = cudaGetLastError();
-    }
-    BL_TRY(e, "grid reordering");
+  T.natm = natm;
+  T.nsh = (int)shells.size();
+  if (!order) {  // Morton order of the points, on the device (ties by point index)
+    BL_TRY(sp_alloc(sp, &sp->perm, (size_t)nq), "cudaMalloc");
+    BL_TRY(morton_perm_device(a.px, a.py, a.pz, npts, nq, sp->perm, st), "grid reordering");
+    order = sp->perm;
   }
-  // --- per-tile lists, on the device: distances, counts, then (their places known) the lists.  On the
-  // host the lists of a 41-atom grid (2,710 tiles, 170,000 items of 80 bytes, copied from pageable
-  // memory) were most of the 30 ms of a context's creation.
-  std::vector<int64_t> tso((size_t)ntiles + 1, 0);
-  std::vector<int> listed_t((size_t)ntiles, 0);
-  {
-    constexpr int kCnt = 2 + kMaxL;
-    float* dd2 = nullptr;
-    double* dR2 = nullptr;
-    int *dr2off = nullptr, *dcnt = nullptr;
-    int64_t* dstart = nullptr;
-    std::vector<int> cnt((size_t)ntiles * kCnt);
-    std::vector<int64_t> start((size_t)ntiles * (kMaxL + 1));
-    auto plan = [&]() -> cudaError_t {
-#define PL_TRY(call)                      \
-  do {                                    \
-    cudaError_t e_ = (call);              \
-    if (e_ != cudaSuccess) return e_;     \
-  } while (0)
-      // one scratch allocation for the five tables
-      const size_t n8 = (size_t)ntiles * (kMaxL + 1) + std::max<size_t>(R2.size(), 1);
-      const size_t n4 = (size_t)ntiles * natm + (size_t)ntiles * kCnt + (size_t)nsh;
-      PL_TRY(cudaMalloc(&dstart, 8 * n8 + 4 * n4));
-      dR2 = (double*)(dstart + (size_t)ntiles * (kMaxL + 1));
-      dd2 = (float*)(dstart + n8);
-      dcnt = (int*)(dd2 + (size_t)ntiles * natm);
-      dr2off = dcnt + (size_t)ntiles * kCnt;
-      PL_TRY(cudaMemcpyAsync(dR2, R2.data(), sizeof(double) * R2.size(), cudaMemcpyHostToDevice, st));
-      PL_TRY(cudaMemcpyAsync(dr2off, r2off.data(), sizeof(int) * r2off.size(), cudaMemcpyHostToDevice, st));
-      k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, natm, dd2);
-      k_plan_count<<<(unsigned)ntiles, 128, 0, st>>>(dd2, natm, a.shells, nsh, dR2, dr2off, dcnt);
-      PL_TRY(cudaGetLastError());
-      PL_TRY(cudaMemcpyAsync(cnt.data(), dcnt, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, st));
-      PL_TRY(cudaStreamSynchronize(st));
-      int64_t items[kMaxL + 1] = {};
-      for (int l = 0; l <= kMaxL; ++l) sp->tile_item[l].assign((size_t)ntiles + 1, 0);
-      for (int64_t t = 0; t < ntiles; ++t) {
-        const int* c = &cnt[(size_t)t * kCnt];
-        listed_t[(size_t)t] = c[0];
-        const int nt = (c[0] + kSlotAlign - 1) / kSlotAlign * kSlotAlign;
-        sp->nlisted += c[0];
-        sp->sum_n2 += (double)c[0] * (double)c[0];
-        sp->max_n = std::max(sp->max_n, nt);
-        tso[(size_t)t + 1] = tso[(size_t)t] + nt;
-        for (int l = 0; l <= kMaxL; ++l) {
-          start[(size_t)t * (kMaxL + 1) + l] = items[l];
-          items[l] += c[1 + l];
-          sp->tile_item[l][(size_t)t + 1] = items[l];
-        }
-      }
-      sp->nslots = tso[(size_t)ntiles];
-      PL_TRY(sp_alloc(sp, &sp->tso, tso.size()));
-      PL_TRY(sp_alloc(sp, &sp->listed, listed_t.size()));
-      PL_TRY(sp_alloc(sp, &sp->slot_fn, (size_t)sp->nslots));
-      for (int l = 0; l <= kMaxL; ++l) PL_TRY(sp_alloc(sp, &sp->items[l], (size_t)items[l]));
-      PL_TRY(cudaMemcpyAsync(sp->tso, tso.data(), sizeof(int64_t) * tso.size(), cudaMemcpyHostToDevice, st));
-      PL_TRY(cudaMemcpyAsync(sp->listed, listed_t.data(), sizeof(int) * listed_t.size(), cudaMemcpyHostToDevice, st));
-      PL_TRY(cudaMemcpyAsync(dstart, start.data(), sizeof(int64_t) * start.size(), cudaMemcpyHostToDevice, st));
-      PlanItems out{};
-      for (int l = 0; l <= kMaxL; ++l) out.items[l] = sp->items[l];
-      k_plan_fill<<<(unsigned)ntiles, 128, 0, st>>>(dd2, natm, a.atoms, a.shells, nsh, dR2, dr2off, sp->tso, dstart,
-                                                    sp->slot_fn, out);
-      PL_TRY(cudaGetLastError());
-      return cudaStreamSynchronize(st);
-#undef PL_TRY
-    };
-    const cudaError_t e = plan();
-    cudaFree(dstart);
-    BL_TRY(e, "tile lists");
+  BL_TRY(sp_alloc(sp, &sp->qx, 4 * (size_t)nq), "grid reordering");
+  sp->qy = sp->qx + nq;
+  sp->qz = sp->qx + 2 * nq;
+  sp->qw = sp->qx + 3 * nq;
+  k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(order, nq, a.px, a.py, a.pz, a.w, sp->qx, sp->qy, sp->qz,
+                                                               sp->qw);
+  BL_TRY(cudaGetLastError(), "grid reordering");
+  // one allocation for the five tables
+  const size_t n8 = (size_t)ntiles * (kMaxL + 1) + std::max<size_t>(R2.size(), 1);
+  const size_t n4 = (size_t)ntiles * natm + (size_t)ntiles * kCnt + shells.size();
+  BL_TRY(cudaMalloc(&T.base, 8 * n8 + 4 * n4), "tile lists");
+  T.start = (int64_t*)T.base;
+  T.r2 = (double*)(T.start + (size_t)ntiles * (kMaxL + 1));
+  T.d2 = (float*)(T.start + n8);
+  T.cnt = (int*)(T.d2 + (size_t)ntiles * natm);
+  T.r2off = T.cnt + (size_t)ntiles * kCnt;
+  BL_TRY(cudaMemcpyAsync(T.r2, R2.data(), sizeof(double) * R2.size(), cudaMemcpyHostToDevice, st), "tile lists");
+  BL_TRY(cudaMemcpyAsync(T.r2off, r2off.data(), sizeof(int) * r2off.size(), cudaMemcpyHostToDevice, st), "tile lists");
+  k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, natm, T.d2);
+  k_plan_count<<<(unsigned)ntiles, 128, 0, st>>>(T.d2, natm, a.shells, T.nsh, T.r2, T.r2off, T.cnt);
+  BL_TRY(cudaGetLastError(), "tile lists");
+  std::vector<int> cnt((size_t)ntiles * kCnt), listed((size_t)ntiles);
+  std::vector<int64_t> start((size_t)ntiles * (kMaxL + 1));
+  BL_TRY(cudaMemcpyAsync(cnt.data(), T.cnt, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, st), "tile lists");
+  BL_TRY(cudaStreamSynchronize(st), "tile lists");
+  std::vector<int64_t>& tso = sp->h_tso;
+  tso.assign((size_t)ntiles + 1, 0);
+  int64_t items[kMaxL + 1] = {};
+  for (int l = 0; l <= kMaxL; ++l) sp->tile_item[l].assign((size_t)ntiles + 1, 0);
+  for (int64_t t = 0; t < ntiles; ++t) {
+    const int* c = &cnt[(size_t)t * kCnt];
+    listed[(size_t)t] = c[0];
+    const int nt = (c[0] + kSlotAlign - 1) / kSlotAlign * kSlotAlign;
+    sp->nlisted += c[0];
+    sp->sum_n2 += (double)c[0] * (double)c[0];
+    sp->max_n = std::max(sp->max_n, nt);
+    tso[(size_t)t + 1] = tso[(size_t)t] + nt;
+    for (int l = 0; l <= kMaxL; ++l) {
+      start[(size_t)t * (kMaxL + 1) + l] = items[l];
+      items[l] += c[1 + l];
+      sp->tile_item[l][(size_t)t + 1] = items[l];
+    }
   }
-  sp->h_tso = std::move(tso);
+  sp->nslots = tso[(size_t)ntiles];
+  BL_TRY(sp_alloc(sp, &sp->tso, tso.size()), "tile lists");
+  BL_TRY(sp_alloc(sp, &sp->listed, listed.size()), "tile lists");
+  BL_TRY(cudaMemcpyAsync(sp->tso, tso.data(), sizeof(int64_t) * tso.size(), cudaMemcpyHostToDevice, st), "tile lists");
+  BL_TRY(cudaMemcpyAsync(sp->listed, listed.data(), sizeof(int) * listed.size(), cudaMemcpyHostToDevice, st),
+         "tile lists");
+  BL_TRY(cudaMemcpyAsync(T.start, start.data(), sizeof(int64_t) * start.size(), cudaMemcpyHostToDevice, st),
+         "tile lists");
   return PGXC_OK;
 #undef BL_TRY
+}
+
+// The lists of tiles [t0, t0 + nt) at the places counted for them.
+static void fill_lists(const ScreenPlan* sp, const BuildArgs& a, int64_t t0, int64_t nt, const TileLists& out,
+                       cudaStream_t st) {
+  const ListTables& T = sp->tab;
+  k_plan_fill<<<(unsigned)nt, 128, 0, st>>>(T.d2, T.natm, a.atoms, a.shells, T.nsh, T.r2, T.r2off, sp->tso, T.start, t0,
+                                            out);
 }
 
 void screen_destroy(ScreenPlan* sp) {
   if (!sp) return;
   if (sp->mixed) screen_mixed_destroy(sp->mixed);
   for (void* p : sp->allocs) cudaFree(p);
+  if (sp->tab.base) cudaFree(sp->tab.base);
   for (auto& c : sp->cev)
     for (auto& e : c)
       if (e) cudaEventDestroy(e);
@@ -883,10 +859,22 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     std::vector<double> R2;
     std::vector<int> r2off;
     screen_listing_radii(shells, in.exps, in.norms, in.contr, in.threshold, a.sa, R2, r2off);
-    if (const int st2 = build_lists(sp, a, in.natm, in.npts, shells, R2, r2off, nullptr, st, err)) {
+    if (const int st2 = count_lists(sp, a, in.natm, in.npts, shells, R2, r2off, nullptr, st, err)) {
       screen_destroy(sp);
       return st2;
     }
+    TileLists L{};
+    SP_TRY(sp_alloc(sp, &sp->slot_fn, (size_t)sp->nslots), "tile lists");
+    L.slot_fn = sp->slot_fn;
+    for (int l = 0; l <= kMaxL; ++l) {
+      SP_TRY(sp_alloc(sp, &sp->items[l], (size_t)sp->tile_item[l].back()), "tile lists");
+      L.items[l] = sp->items[l];
+    }
+    fill_lists(sp, a, 0, sp->ntiles, L, st);
+    SP_TRY(cudaGetLastError(), "tile lists");
+    SP_TRY(cudaStreamSynchronize(st), "tile lists");
+    cudaFree(sp->tab.base);  // (a build's lists are filled once)
+    sp->tab = ListTables{};
   }
   const std::vector<int64_t>& tso = sp->h_tso;
   const int64_t ntiles = sp->ntiles;
@@ -1042,7 +1030,7 @@ int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npt
   SP_TRY(cudaGetDevice(&sp->nsm), "cudaGetDevice");
   SP_TRY(cudaDeviceGetAttribute(&sp->nsm, cudaDevAttrMultiProcessorCount, sp->nsm), "cudaDeviceGetAttribute");
   const int64_t* perm = from ? from->perm : nullptr;
-  if (const int st2 = build_lists(sp, a, natm, npts, shells, R2, r2off, perm, st, err)) {
+  if (const int st2 = count_lists(sp, a, natm, npts, shells, R2, r2off, perm, st, err)) {
     screen_destroy(sp);
     return st2;
   }
@@ -1065,12 +1053,25 @@ int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npt
     const int64_t t0 = sp->chunk_t0[c], t1 = sp->chunk_t0[c + 1];
     sp->chunk_tiles = std::max(sp->chunk_tiles, t1 - t0);
     sp->chunk_slots = std::max(sp->chunk_slots, sp->h_tso[(size_t)t1] - sp->h_tso[(size_t)t0]);
+    for (int l = 0; l <= kMaxL; ++l)
+      sp->chunk_items[l] =
+          std::max(sp->chunk_items[l], sp->tile_item[l][(size_t)t1] - sp->tile_item[l][(size_t)t0]);
   }
   *out = sp;
   return PGXC_OK;
 }
 
-void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
+void grad_plan_lists(ScreenPlan* sp, const BuildArgs& a, size_t c, const TileLists& lists, cudaStream_t st) {
+  if (sp->filled == (int64_t)c) return;
+  const int64_t t0 = sp->chunk_t0[c];
+  TileLists L = lists;
+  L.s0 = sp->h_tso[(size_t)t0];
+  for (int l = 0; l <= kMaxL; ++l) L.i0[l] = sp->tile_item[l][(size_t)t0];
+  fill_lists(sp, a, t0, sp->chunk_t0[c + 1] - t0, L, st);
+  sp->filled = (int64_t)c;
+}
+
+void grad_contract(const ScreenPlan* sp, const int* slot_fn, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
                    const double* gy, const double* gz, const double* P, int64_t ldc, double* X, double* rho,
                    double* grx, double* gry, double* grz, const GradOrbitals* orb, cudaStream_t st) {
   const int smem = sdensity_smem(sp->max_n);
@@ -1084,15 +1085,15 @@ void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, con
       const int64_t p = u * 128;
       const SPlanes pu{F, F, F, rho + p, nullptr, nullptr}, px{orb->psi, nullptr, nullptr, nullptr, nullptr, nullptr};
       k_sdensity<false, true, kPsi><<<grid, kSThreads, smem, st>>>(
-          pu, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, orb->orb, orb->nop, false, nullptr,
+          pu, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, slot_fn, orb->orb, orb->nop, false, nullptr,
           nullptr, nullptr, orb->psi, orb->nop, orb->nop, orb->occ);
       if (gx)
         k_sdensity<true, true, kFromPsi><<<grid, kSThreads, smem, st>>>(
-            px, gx, gy, gz, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, orb->scaled, ldc, false, grx + p, gry + p,
+            px, gx, gy, gz, sp->tso, sp->listed, t0 + u, s0, slot_fn, orb->scaled, ldc, false, grx + p, gry + p,
             grz + p, X, orb->nop, orb->nop, nullptr);
       else
         k_sdensity<false, true, kFromPsi><<<grid, kSThreads, smem, st>>>(
-            px, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, orb->scaled, ldc, false, nullptr,
+            px, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, slot_fn, orb->scaled, ldc, false, nullptr,
             nullptr, nullptr, X, orb->nop, orb->nop, nullptr);
     }
     return;
@@ -1101,12 +1102,12 @@ void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, con
   const dim3 grid((unsigned)nt, 2);
   if (gx) {
     raise_smem_limit(k_sdensity<true, true>, smem);
-    k_sdensity<true, true><<<grid, kSThreads, smem, st>>>(pl, gx, gy, gz, sp->tso, sp->listed, t0, s0, sp->slot_fn, P,
+    k_sdensity<true, true><<<grid, kSThreads, smem, st>>>(pl, gx, gy, gz, sp->tso, sp->listed, t0, s0, slot_fn, P,
                                                           ldc, false, grx, gry, grz, X);
   } else {
     raise_smem_limit(k_sdensity<false, true>, smem);
     k_sdensity<false, true><<<grid, kSThreads, smem, st>>>(pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0,
-                                                           sp->slot_fn, P, ldc, false, nullptr, nullptr, nullptr, X);
+                                                           slot_fn, P, ldc, false, nullptr, nullptr, nullptr, X);
   }
 }
 
@@ -1142,7 +1143,7 @@ static int orbital_density(const ScreenPlan* sp, const BuildArgs& a, int s, int6
   int launches = 0;
   if (!gx) {
     k_sdensity<false, false, kPsi><<<dim3((unsigned)nt, 2), kSThreads, smem, st>>>(
-        pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, a.orb[s], nop, false, nullptr, nullptr,
+        pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn + s0, a.orb[s], nop, false, nullptr, nullptr,
         nullptr, nullptr, nop, nocc, a.orb_occ[s]);
     return 1;
   }
@@ -1153,19 +1154,19 @@ static int orbital_density(const ScreenPlan* sp, const BuildArgs& a, int s, int6
     const int64_t p = u * 128;
     const SPlanes pu{phi, phi, phi, b.rho + p, nullptr, nullptr};
     k_sdensity<false, true, kPsi><<<grid, kSThreads, smem, st>>>(
-        pu, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb[s], nop, false, nullptr,
+        pu, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn + s0, a.orb[s], nop, false, nullptr,
         nullptr, nullptr, sp->psi, nop, nocc, a.orb_occ[s]);
     launches += 2;
     if (tau) {
       const SPlanes pt{gx, gy, gz, tau + p, tau + cp + p, tau + 2 * cp + p};
       k_sdensity<true, false, kPsi><<<dim3(grid.x, 2, 3), kSThreads, smem, st>>>(
-          pt, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb[s], nop, false, b.grx + p,
+          pt, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn + s0, a.orb[s], nop, false, b.grx + p,
           b.gry + p, b.grz + p, sp->psi, nop, nocc, a.orb_occ[s]);
       continue;
     }
     const SPlanes px{sp->psi, nullptr, nullptr, nullptr, nullptr, nullptr};
     k_sdensity<true, false, kFromPsi><<<grid, kSThreads, smem, st>>>(
-        px, gx, gy, gz, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn, a.orb_scaled[s], a.ldc, false, b.grx + p,
+        px, gx, gy, gz, sp->tso, sp->listed, t0 + u, s0, sp->slot_fn + s0, a.orb_scaled[s], a.ldc, false, b.grx + p,
         b.gry + p, b.grz + p, nullptr, nop, nocc, nullptr);
   }
   return launches;
@@ -1299,12 +1300,12 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         if (gga) {
           raise_smem_limit(k_sdensity<true>, smem);
           k_sdensity<true><<<dim3((unsigned)nt, 2), kSThreads, smem, st>>>(
-              pl, gxc, gyc, gzc, sp->tso, sp->listed, t0, s0, sp->slot_fn, P[s], a.ldc, false, b[s].grx, b[s].gry,
+              pl, gxc, gyc, gzc, sp->tso, sp->listed, t0, s0, sp->slot_fn + s0, P[s], a.ldc, false, b[s].grx, b[s].gry,
               b[s].grz);
         } else {
           raise_smem_limit(k_sdensity<false>, smem);
           k_sdensity<false><<<dim3((unsigned)nt, 2), kSThreads, smem, st>>>(
-              pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, P[s], a.ldc, a.p_symmetric,
+              pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn + s0, P[s], a.ldc, a.p_symmetric,
               nullptr, nullptr, nullptr);
         }
         ++T.launches;
@@ -1317,7 +1318,7 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         double* tau = sp->tq + 4 * s * cp;
         const SPlanes pl{gxc, gyc, gzc, tau, tau + cp, tau + 2 * cp};
         k_sdensity<false><<<dim3((unsigned)nt, 2, 3), kSThreads, smem, st>>>(
-            pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, P[s], a.ldc, a.p_symmetric,
+            pl, nullptr, nullptr, nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn + s0, P[s], a.ldc, a.p_symmetric,
             nullptr, nullptr, nullptr);
         ++T.launches;
       }
@@ -1358,11 +1359,11 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         if (gga) {
           raise_smem_limit(k_svpot<kFull, true>, smem);
           k_svpot<kFull, true><<<grid, kSThreads, smem, st>>>(pl, gxc, gyc, gzc, b[s].A, b[s].Bx, b[s].By, b[s].Bz,
-                                                              sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas, nI);
+                                                              sp->tso, sp->listed, t0, s0, sp->slot_fn + s0, Vs, sp->nbas, nI);
         } else {
           raise_smem_limit(k_svpot<kUpper, false>, smem);
           k_svpot<kUpper, false><<<grid, kSThreads, smem, st>>>(pl, nullptr, nullptr, nullptr, b[s].A, nullptr, nullptr,
-                                                                nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs,
+                                                                nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn + s0, Vs,
                                                                 sp->nbas, nI);
         }
         if (timed) SR_TRY(cudaEventRecord(k1, st));
@@ -1377,7 +1378,7 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         const unsigned nI = (unsigned)((sp->max_n + kRows - 1) / kRows);
         k_svpot<kTwice, false><<<dim3((unsigned)nt * nI, 1, 3), kSThreads, smem,
                                  st>>>(pl, nullptr, nullptr, nullptr, sp->tq + (4 * s + 3) * cp, nullptr, nullptr,
-                                       nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn, Vs, sp->nbas, nI);
+                                       nullptr, sp->tso, sp->listed, t0, s0, sp->slot_fn + s0, Vs, sp->nbas, nI);
         ++T.launches;
       }
     }

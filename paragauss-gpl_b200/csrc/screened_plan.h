@@ -17,6 +17,25 @@ constexpr int kSlotAlign = 32;   // slots per tile are padded to this (INT8 K st
 constexpr int64_t kSlack = 128;  // zero rows after the last slot of a chunk
 constexpr int kBasisBlocksPerSM = 16;  // blocks of the basis kernels per SM (each walks a range of items)
 
+// What the listing of tiles reads (device; one allocation): each tile's first
+// item of each l, the listing radii, the tiles' smallest squared distances to the atoms.
+struct ListTables {
+  void* base = nullptr;
+  int64_t* start = nullptr;  // [ntiles][kMaxL + 1]
+  double* r2 = nullptr;
+  float* d2 = nullptr;       // [ntiles][natm]
+  int* cnt = nullptr;        // [ntiles] {listed functions, items of each l}
+  int* r2off = nullptr;
+  int natm = 0, nsh = 0;
+};
+// Where the lists of a run of tiles go: slot_fn from its first slot s0 on, items[l] from its first item i0[l] on.
+struct TileLists {
+  int* slot_fn;
+  int64_t s0;
+  BasisItem* items[kMaxL + 1];
+  int64_t i0[kMaxL + 1];
+};
+
 struct ScreenPlan {
   int64_t ntiles = 0, nslots = 0, nlisted = 0;
   double sum_n2 = 0.0;
@@ -61,18 +80,26 @@ struct ScreenPlan {
   std::vector<std::array<cudaEvent_t, 9>> cev;  // timing events of each chunk (made by the first timed build)
   int nsm = 148;
   std::vector<void*> allocs;
-  // gradient plans: raw weight and host atom of the Morton-ordered points
+  ListTables tab;  // gradient plans (a build's are released with its creation)
+  // gradient plans: raw weight and host atom of the Morton-ordered points; the lists lie in the gradient's scratch,
+  // one chunk's at a time (chunk_items: the most items of a chunk; filled: the chunk whose lists lie there, or -1)
   double* qwraw = nullptr;
   int* qowner = nullptr;
+  int64_t chunk_items[kMaxL + 1] = {};
+  int64_t filled = -1;
 };
 
-// A plan of tiles and lists alone (no build buffers), in chunks of at most
-// max_rows slot rows, for the nuclear gradient; R2 with threshold 0, so that
+// A plan of tiles and list lengths alone (no lists, no build buffers), in chunks of
+// at most max_rows slot rows, for the nuclear gradient; R2 with threshold 0, so that
 // unlisted functions and their derivatives are exactly zero on the tile.  from: the
-// context's own plan of the same grid, whose point order is taken, or null.
+// context's own plan of the same grid, whose point order is taken, or null.  The lists
+// themselves are made chunk by chunk (grad_plan_lists): of a whole grid they would grow
+// with tiles x shells (200 atoms, 13,300 tiles: 0.4 GB) and stay until the context goes.
 int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
                      const std::vector<double>& R2, const std::vector<int>& r2off, const double* wraw,
                      const int* owner, const ScreenPlan* from, int64_t max_rows, cudaStream_t st, std::string& err);
+// Chunk c's lists into `lists` (s0 and i0 are set here), unless they are what it holds.
+void grad_plan_lists(ScreenPlan* sp, const BuildArgs& a, size_t c, const TileLists& lists, cudaStream_t st);
 // The orbitals in the place of P (orbital_form_pays): nop padded, C [function][nop], occ C
 // [nop][ldc], occupations [nop], and psi for psi_tiles tiles at a time.
 struct GradOrbitals {
@@ -84,9 +111,9 @@ struct GradOrbitals {
 bool orbital_form_pays(const ScreenPlan* sp, int64_t nop);
 // tiles whose psi is held at once: those of a chunk, as many as 1 GB holds
 int64_t orbital_psi_tiles(const ScreenPlan* sp, int64_t nop);
-// X = F_t P[S_t, S_t] (by the orbitals when orb is not null) of the chunk's tiles ([slot][128] rows, padding rows of F
+// X = F_t P[S_t, S_t] (by the orbitals when orb is not null) of the chunk's tiles (slot_fn: the chunk's; [slot][128] rows, padding rows of F
 // zero), with rho[p] = sum X F and (gx not null) gr[p] = 2 sum X grad phi.
-void grad_contract(const ScreenPlan* sp, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
+void grad_contract(const ScreenPlan* sp, const int* slot_fn, int64_t t0, int64_t nt, int64_t s0, const double* F, const double* gx,
                    const double* gy, const double* gz, const double* P, int64_t ldc, double* X, double* rho,
                    double* grx, double* gry, double* grz, const GradOrbitals* orb, cudaStream_t st);
 

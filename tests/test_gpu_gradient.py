@@ -1,6 +1,8 @@
 """Post-SCF XC nuclear gradient on the device (pgxc_xc_gradient) against the
 oracle's independent restatement (itself checked against finite differences
 in tests/test_gradient.py); every layout, both spins, LDA, GGA and meta-GGA."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -60,6 +62,43 @@ def test_core_terms_do_not_round_the_gradient(xc, ispin):
     scale = float(np.max(np.abs(a)))
     assert float(np.max(np.abs(a.sum(0)))) < 1e-13 * scale
     assert float(np.max(np.abs(a - b))) < 1e-13 * scale
+
+
+def test_gradient_of_many_chunks():
+    """200 atoms with f shells, about 70 chunks of slot rows: the lists are made chunk by
+    chunk, so what the context holds after a gradient is one chunk's rows (at most
+    4 GB), the weight term's scratch (at most 2 GB) and arrays by point, not the
+    lists of the whole grid (0.4 GB here).  Two halves of the grid, chunked in
+    their own way, sum to the whole; a second call finds the chunks again."""
+    import torch
+    n = 200
+    rng = np.random.default_rng(21)
+    els, xyz = cases.random_cluster(rng, [("C", 80), ("H", 60), ("O", 40), ("N", 20)], 18.0, 1.0)
+    case = cases.build_case("many", els, xyz, seed=21, exp_range=(0.05, 1e4), nrad=50, nang=194, functional="VWN",
+                            nocc=16, shells=cases.SHELLS_F, orthonormalise=False)
+    torch.cuda.init()
+    with lib.Context(case, weighted=False, screen_threshold=1e-10) as ctx:
+        free = torch.cuda.mem_get_info()[0]
+        g, e = ctx.xc_gradient()
+        held = free - torch.cuda.mem_get_info()[0]
+        again, _ = ctx.xc_gradient()
+    points = (case.npts + 127) // 128 * 128
+    weights = points
+    while 28 * n * weights > 2e9:
+        weights = (weights // 2 + 127) // 128 * 128
+    assert held < 4.0e9 + 28 * n * weights + 0.35e9
+    scale = float(np.max(np.abs(g)))
+    assert float(np.max(np.abs(again - g))) < 1e-12 * scale
+    half = np.zeros_like(g)
+    for pick in (slice(0, case.npts // 2), slice(case.npts // 2, None)):
+        c = dataclasses.replace(case, grid_xyz=case.grid_xyz[pick], grid_wraw=case.grid_wraw[pick],
+                                point_atom=case.point_atom[pick])
+        with lib.Context(c, weighted=False, screen_threshold=1e-10) as ctx:
+            gh, eh = ctx.xc_gradient()
+        half += gh
+        e -= eh
+    assert abs(e) < 1e-10
+    assert float(np.max(np.abs(half - g))) < 1e-11 * scale
 
 
 def test_gradient_needs_the_raw_grid():
