@@ -1006,8 +1006,8 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     // tiles and lists, once per context (its threshold does not matter: every function that is not
     // identically zero on a tile is listed), in chunks of under ~4 GB of slot rows
     std::string e;
-    const int st = grad_plan_create(&c->gplan, a, c->natm, c->npts, c->shells, c->grad_r2, c->grad_r2off, c->d_wraw,
-                                    c->d_owner, c->screen, (int64_t)(4.0e9 / (1024.0 * planes)), s, e);
+    const int st = grad_plan_create(&c->gplan, a, c->natm, c->npts, c->shells, c->grad_r2, c->grad_r2off,
+                                    c->screen, (int64_t)(4.0e9 / (1024.0 * planes)), s, e);
     if (st) return set_err(c, st, "gradient plan: " + e);
   }
   ScreenPlan* gp = c->gplan;
@@ -1021,11 +1021,13 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   // one scratch buffer, carved in 256-byte aligned pieces and kept in the
   // context for the next call (allocation and release of several GB per call
   // would cost more than the gradient's kernels)
-  constexpr int kLists = 8, kPsiAt = kLists + kMaxL + 2;  // the chunk's lists: slot_fn, items of each l; then psi
+  // the points' raw weights and hosts; the chunk's lists: slot_fn, items of each l; psi
+  constexpr int kHosts = 8, kLists = 10, kPsiAt = kLists + kMaxL + 2;
   size_t sizes[kPsiAt + 1] = {sizeof(double) * (size_t)(planes * plane), sizeof(double) * 7 * ispin * (size_t)ld,
                               sizeof(double) * 5 * ispin * (size_t)ld,   sizeof(double) * (size_t)nq,
                               sizeof(double) * 3 * c->natm,              sizeof(double),
                               sizeof(double) * ((size_t)7 * c->natm * ldw / 2 + 1), sizeof(int) * (size_t)nbas,
+                              sizeof(double) * (size_t)nq,               sizeof(int) * (size_t)nq,
                               sizeof(int) * (size_t)gp->chunk_slots};
   for (int l = 0; l <= kMaxL; ++l) sizes[kLists + 1 + l] = sizeof(BasisItem) * (size_t)gp->chunk_items[l];
   bool orbitals = orbital_form_pays(gp, kpad);
@@ -1096,6 +1098,7 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   lists.slot_fn = (int*)(base + offs[kLists]);
   for (int l = 0; l <= kMaxL; ++l) lists.items[l] = (BasisItem*)(base + offs[kLists + 1 + l]);
   g.lists = &lists;
+  grad_plan_hosts(gp, c->d_wraw, c->d_owner, (double*)(base + offs[kHosts]), (int*)(base + offs[kHosts + 1]), s);
   int rc = PGXC_OK;
   do {
     if (cudaMemcpyAsync(dfatom, fatom.data(), sizeof(int) * nbas, cudaMemcpyHostToDevice, s) != cudaSuccess ||

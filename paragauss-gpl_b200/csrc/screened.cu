@@ -682,13 +682,16 @@ void screen_listing_radii(const std::vector<DevShell>& shells, const double* exp
 
 // The tiles and the lengths of their lists: Morton-ordered points, per tile the
 // number of listed functions (those whose listing radius exceeds the tile's
-// distance to their atom) and of basis items, and so their places.  order: the
-// points' order, or null: it is made here and kept in sp->perm.  The tables that
-// fill_lists reads stay in sp->tab.  On the host the lists of a 41-atom grid
+// distance to their atom) and of basis items, and so their places.  The tables that
+// fill_lists reads stay in sp->tab.  from: a plan of the same grid whose points are
+// taken as they lie there, or null: they are put in order here.  one: the plan's own
+// arrays lie behind the tables (an allocation of 2 MB or more takes 0.35 ms whatever its
+// size: the gradient of 6 atoms 1.03 ms before it had a plan, 1.6 with eight allocations
+// of the plan's, 0.92 now).  On the host the lists of a 41-atom grid
 // (2,710 tiles, 170,000 items of 80 bytes, copied from pageable memory) were most
 // of the 30 ms of a context's creation.
 static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
-                       const std::vector<double>& R2, const std::vector<int>& r2off, const int64_t* order,
+                       const std::vector<double>& R2, const std::vector<int>& r2off, const ScreenPlan* from, bool one,
                        cudaStream_t st, std::string& err) {
 #define BL_TRY(call, what)                                                       \
   do {                                                                           \
@@ -704,27 +707,34 @@ static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npt
   sp->ntiles = ntiles;
   T.natm = natm;
   T.nsh = (int)shells.size();
-  if (!order) {  // Morton order of the points, on the device (ties by point index)
-    BL_TRY(sp_alloc(sp, &sp->perm, (size_t)nq), "cudaMalloc");
-    BL_TRY(morton_perm_device(a.px, a.py, a.pz, npts, nq, sp->perm, st), "grid reordering");
-    order = sp->perm;
+  if (from) {
+    sp->order_of_points = from->order_of_points;
+    sp->qx = from->qx;
+    sp->qy = from->qy;
+    sp->qz = from->qz;
+    sp->qw = from->qw;
+  } else {  // Morton order of the points, on the device (ties by point index)
+    BL_TRY(sp_alloc(sp, &sp->order_of_points, (size_t)nq), "cudaMalloc");
+    BL_TRY(morton_perm_device(a.px, a.py, a.pz, npts, nq, sp->order_of_points, st), "grid reordering");
+    BL_TRY(sp_alloc(sp, &sp->qx, 4 * (size_t)nq), "grid reordering");
+    sp->qy = sp->qx + nq;
+    sp->qz = sp->qx + 2 * nq;
+    sp->qw = sp->qx + 3 * nq;
+    k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(sp->order_of_points, nq, a.px, a.py, a.pz, a.w, sp->qx,
+                                                                 sp->qy, sp->qz, sp->qw);
+    BL_TRY(cudaGetLastError(), "grid reordering");
   }
-  BL_TRY(sp_alloc(sp, &sp->qx, 4 * (size_t)nq), "grid reordering");
-  sp->qy = sp->qx + nq;
-  sp->qz = sp->qx + 2 * nq;
-  sp->qw = sp->qx + 3 * nq;
-  k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(order, nq, a.px, a.py, a.pz, a.w, sp->qx, sp->qy, sp->qz,
-                                                               sp->qw);
-  BL_TRY(cudaGetLastError(), "grid reordering");
-  // one allocation for the five tables
-  const size_t n8 = (size_t)ntiles * (kMaxL + 1) + std::max<size_t>(R2.size(), 1);
-  const size_t n4 = (size_t)ntiles * natm + (size_t)ntiles * kCnt + shells.size();
+  // one allocation for the tables (and, with `one`, tso and listed)
+  const size_t nstart = (size_t)ntiles * (kMaxL + 1), n8 = nstart + (size_t)ntiles + 1 + std::max<size_t>(R2.size(), 1);
+  const size_t n4 = (size_t)ntiles * natm + (size_t)ntiles * kCnt + shells.size() + (size_t)ntiles;
   BL_TRY(cudaMalloc(&T.base, 8 * n8 + 4 * n4), "tile lists");
   T.start = (int64_t*)T.base;
-  T.r2 = (double*)(T.start + (size_t)ntiles * (kMaxL + 1));
+  sp->tso = T.start + nstart;
+  T.r2 = (double*)(sp->tso + ntiles + 1);
   T.d2 = (float*)(T.start + n8);
   T.cnt = (int*)(T.d2 + (size_t)ntiles * natm);
   T.r2off = T.cnt + (size_t)ntiles * kCnt;
+  sp->listed = T.r2off + shells.size();
   BL_TRY(cudaMemcpyAsync(T.r2, R2.data(), sizeof(double) * R2.size(), cudaMemcpyHostToDevice, st), "tile lists");
   BL_TRY(cudaMemcpyAsync(T.r2off, r2off.data(), sizeof(int) * r2off.size(), cudaMemcpyHostToDevice, st), "tile lists");
   k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, natm, T.d2);
@@ -753,8 +763,10 @@ static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npt
     }
   }
   sp->nslots = tso[(size_t)ntiles];
-  BL_TRY(sp_alloc(sp, &sp->tso, tso.size()), "tile lists");
-  BL_TRY(sp_alloc(sp, &sp->listed, listed.size()), "tile lists");
+  if (!one) {
+    BL_TRY(sp_alloc(sp, &sp->tso, tso.size()), "tile lists");
+    BL_TRY(sp_alloc(sp, &sp->listed, listed.size()), "tile lists");
+  }
   BL_TRY(cudaMemcpyAsync(sp->tso, tso.data(), sizeof(int64_t) * tso.size(), cudaMemcpyHostToDevice, st), "tile lists");
   BL_TRY(cudaMemcpyAsync(sp->listed, listed.data(), sizeof(int) * listed.size(), cudaMemcpyHostToDevice, st),
          "tile lists");
@@ -859,7 +871,7 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
     std::vector<double> R2;
     std::vector<int> r2off;
     screen_listing_radii(shells, in.exps, in.norms, in.contr, in.threshold, a.sa, R2, r2off);
-    if (const int st2 = count_lists(sp, a, in.natm, in.npts, shells, R2, r2off, nullptr, st, err)) {
+    if (const int st2 = count_lists(sp, a, in.natm, in.npts, shells, R2, r2off, nullptr, false, st, err)) {
       screen_destroy(sp);
       return st2;
     }
@@ -1023,26 +1035,16 @@ __global__ void k_gather_hosts(const int64_t* __restrict__ perm, int64_t nq, con
 }  // namespace
 
 int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
-                     const std::vector<double>& R2, const std::vector<int>& r2off, const double* wraw,
-                     const int* owner, const ScreenPlan* from, int64_t max_rows, cudaStream_t st, std::string& err) {
+                     const std::vector<double>& R2, const std::vector<int>& r2off, const ScreenPlan* from,
+                     int64_t max_rows, cudaStream_t st, std::string& err) {
   *out = nullptr;
   ScreenPlan* sp = new ScreenPlan();
   SP_TRY(cudaGetDevice(&sp->nsm), "cudaGetDevice");
   SP_TRY(cudaDeviceGetAttribute(&sp->nsm, cudaDevAttrMultiProcessorCount, sp->nsm), "cudaDeviceGetAttribute");
-  const int64_t* perm = from ? from->perm : nullptr;
-  if (const int st2 = count_lists(sp, a, natm, npts, shells, R2, r2off, perm, st, err)) {
+  if (const int st2 = count_lists(sp, a, natm, npts, shells, R2, r2off, from, true, st, err)) {
     screen_destroy(sp);
     return st2;
   }
-  const int64_t nq = sp->ntiles * 128;
-  cudaError_t e = sp_alloc(sp, &sp->qwraw, nq);
-  if (e == cudaSuccess) e = sp_alloc(sp, &sp->qowner, nq);
-  if (e == cudaSuccess) {
-    k_gather_hosts<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(perm ? perm : sp->perm, nq, wraw, owner, sp->qwraw,
-                                                                 sp->qowner);
-    e = cudaGetLastError();
-  }
-  SP_TRY(e, "gradient plan");
   max_rows = std::max<int64_t>(max_rows, sp->max_n);
   sp->chunk_t0.push_back(0);
   for (int64_t t = 1; t <= sp->ntiles; ++t) {
@@ -1059,6 +1061,14 @@ int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npt
   }
   *out = sp;
   return PGXC_OK;
+}
+
+void grad_plan_hosts(ScreenPlan* sp, const double* wraw, const int* owner, double* qwraw, int* qowner, cudaStream_t st) {
+  sp->qwraw = qwraw;
+  sp->qowner = qowner;
+  if (sp->filled >= 0) return;
+  const int64_t nq = sp->ntiles * 128;
+  k_gather_hosts<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(sp->order_of_points, nq, wraw, owner, qwraw, qowner);
 }
 
 void grad_plan_lists(ScreenPlan* sp, const BuildArgs& a, size_t c, const TileLists& lists, cudaStream_t st) {

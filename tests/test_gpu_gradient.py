@@ -101,6 +101,26 @@ def test_gradient_of_many_chunks():
     assert float(np.max(np.abs(half - g))) < 1e-11 * scale
 
 
+@pytest.mark.parametrize("layout", [("fp64", 0.0), ("mixed", 1e-10)], ids=["screened", "int8-screened"])
+def test_first_gradient_allocates_twice(layout):
+    """A gradient is asked for once per geometry, so the first call counts: the
+    tables of its lists (by tile, small) and its scratch are all that it
+    allocates, and nothing is released (each large allocation takes 0.35 ms)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    precision, thr = layout
+    case = cases.small_case(functional="PBE", seed=65, natoms=6, nrad=50, nang=194)
+    with lib.Context(case, weighted=False, precision=precision, screen_threshold=thr) as ctx:
+        ctx.build()
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as prof:
+            ctx.xc_gradient()
+        names = [e.name for e in prof.events()]
+    if "cudaLaunchKernel" not in names:
+        pytest.skip("the profiler records no runtime calls here")
+    assert names.count("cudaMalloc") <= 2 and "cudaFree" not in names
+
+
 def test_gradient_needs_the_raw_grid():
     case = cases.small_case(functional="PBE", seed=63)
     O.weight_case(case)
