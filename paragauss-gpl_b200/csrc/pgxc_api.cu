@@ -198,6 +198,7 @@ void pgxc_destroy(pgxc_ctx* c) {
   for (void* p : c->allocs) cudaFree(p);
   if (c->gplan) screen_destroy(c->gplan);
   if (c->grad_scr) cudaFree(c->grad_scr);
+  if (c->d_raw) cudaFree(c->d_raw);
   if (c->h_ham) cudaFreeHost(c->h_ham);
   if (c->h_acc) cudaFreeHost(c->h_acc);
   for (auto& e : c->ev)
@@ -840,13 +841,24 @@ static int finish_build(pgxc_ctx* c, pgxc_timings* tm) {
 }
 
 // Device copy of host orbitals and occupations as the caller holds them (one
-// buffer: C of both spins, then occ of both), grown when nocc grows.
+// buffer: C of both spins, then occ of both).  It grows in steps of 16 orbitals as
+// ensure_occ does; the outgrown one is released (nothing but the build that
+// filled it has its address, and that build has ended).
 static int stage_orbitals(pgxc_ctx* c, const double* C, const double* occ, int32_t nbas, int32_t nocc, double** dC,
                           double** docc) {
   const int64_t nC = (int64_t)c->opt.ispin * nbas * nocc, no = (int64_t)c->opt.ispin * nocc;
   if (nC + no > c->raw_cap || !c->d_raw) {
-    if (int st = dalloc(c, &c->d_raw, (size_t)(nC + no))) return st;
-    c->raw_cap = nC + no;
+    if (c->d_raw) cudaFree(c->d_raw);
+    c->d_raw = nullptr;
+    c->raw_cap = 0;
+    const int64_t cap = (int64_t)c->opt.ispin * (nbas + 1) * round_up(std::max(nocc, 1), 16);
+    const cudaError_t e = cudaMalloc(&c->d_raw, sizeof(double) * (size_t)cap);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      c->d_raw = nullptr;
+      return set_err(c, PGXC_ENOMEM, std::string("orbitals: ") + cudaGetErrorString(e));
+    }
+    c->raw_cap = cap;
   }
   *dC = c->d_raw;
   *docc = c->d_raw + nC;

@@ -119,3 +119,25 @@ def test_gradient_block_remainders(natoms, lmax):
     scale = max(1.0, float(np.max(np.abs(ref))))
     assert abs(e - re) < 1e-10 * max(1.0, abs(re))
     np.testing.assert_allclose(g, ref, rtol=0, atol=1e-10 * scale)
+
+
+# a caller whose number of orbitals creeps upwards: one staging buffer (with the padded buffers of
+# every 16 orbitals, 2 ldc kpad doubles each, which a captured batch may hold: 13 MB), not one per step (72 MB)
+def test_outgrown_orbital_buffers_are_released():
+    import torch
+    c = _case(16, 2, "VWN", nrad=6)
+    rng = np.random.default_rng(8)
+    C = rng.normal(size=(c.nbas, c.nbas, 1)) / c.nbas
+    torch.cuda.init()
+    with lib.Context(c, screen_threshold=0.0) as ctx:
+        c.nocc = 1
+        ctx.build(C=C[:, :1].T, occ=np.full(1, 2.0))
+        free = torch.cuda.mem_get_info()[0]
+        for c.nocc in range(2, c.nbas + 1):
+            last = ctx.build(C=C[:, :c.nocc, 0].T, occ=np.full(c.nocc, 2.0))
+        held = free - torch.cuda.mem_get_info()[0]
+    steps = np.arange(16, c.nbas + 16, 16)
+    assert held < 8 * (2 * (c.nbas + 64) * steps.sum() + (c.nbas + 1) * (c.nbas + 16)) + (8 << 20)
+    with lib.Context(c, screen_threshold=0.0) as ctx:
+        ref = ctx.build(C=C[:, :, 0].T, occ=np.full(c.nbas, 2.0))
+    assert abs(last[1] - ref[1]) < 1e-10 and float(np.max(np.abs(last[0] - ref[0]))) < 1e-10
