@@ -1033,13 +1033,14 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   // one scratch buffer, carved in 256-byte aligned pieces and kept in the
   // context for the next call (allocation and release of several GB per call
   // would cost more than the gradient's kernels)
-  // the points' raw weights and hosts; the chunk's lists: slot_fn, items of each l; psi
-  constexpr int kHosts = 8, kLists = 10, kPsiAt = kLists + kMaxL + 2;
+  // the points' raw weights and hosts, and (dense layout) the points; the chunk's lists: slot_fn, items of each l; psi
+  constexpr int kHosts = 8, kLists = 11, kPsiAt = kLists + kMaxL + 2;
   size_t sizes[kPsiAt + 1] = {sizeof(double) * (size_t)(planes * plane), sizeof(double) * 7 * ispin * (size_t)ld,
                               sizeof(double) * 5 * ispin * (size_t)ld,   sizeof(double) * (size_t)nq,
                               sizeof(double) * 3 * c->natm,              sizeof(double),
                               sizeof(double) * ((size_t)7 * c->natm * ldw / 2 + 1), sizeof(int) * (size_t)nbas,
                               sizeof(double) * (size_t)nq,               sizeof(int) * (size_t)nq,
+                              c->screen ? 0 : sizeof(double) * 4 * (size_t)nq,
                               sizeof(int) * (size_t)gp->chunk_slots};
   for (int l = 0; l <= kMaxL; ++l) sizes[kLists + 1 + l] = sizeof(BasisItem) * (size_t)gp->chunk_items[l];
   bool orbitals = orbital_form_pays(gp, kpad);
@@ -1110,7 +1111,8 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   lists.slot_fn = (int*)(base + offs[kLists]);
   for (int l = 0; l <= kMaxL; ++l) lists.items[l] = (BasisItem*)(base + offs[kLists + 1 + l]);
   g.lists = &lists;
-  grad_plan_hosts(gp, c->d_wraw, c->d_owner, (double*)(base + offs[kHosts]), (int*)(base + offs[kHosts + 1]), s);
+  grad_plan_hosts(gp, a, c->npts, c->d_wraw, c->d_owner, c->screen ? nullptr : (double*)(base + offs[kHosts + 2]),
+                  (double*)(base + offs[kHosts]), (int*)(base + offs[kHosts + 1]), s);
   int rc = PGXC_OK;
   do {
     if (cudaMemcpyAsync(dfatom, fatom.data(), sizeof(int) * nbas, cudaMemcpyHostToDevice, s) != cudaSuccess ||

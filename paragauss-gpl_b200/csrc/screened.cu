@@ -54,16 +54,21 @@ cudaError_t sp_alloc(ScreenPlan* sp, T** p, size_t n) {
 // ---------------------------------------------------------------------------
 // planning kernels
 // ---------------------------------------------------------------------------
-__global__ void k_gather_points(const int64_t* __restrict__ perm, int64_t nq, const double* __restrict__ px,
-                                const double* __restrict__ py, const double* __restrict__ pz,
-                                const double* __restrict__ w, double* __restrict__ qx, double* __restrict__ qy,
-                                double* __restrict__ qz, double* __restrict__ qw) {
+// index of point q of the tiles among the n of the grid (order null: as they lie there), or -1: padding
+__device__ __forceinline__ int64_t point_index(const int64_t* __restrict__ order, int64_t n, int64_t q) {
+  return order ? order[q] : (q < n ? q : -1);
+}
+
+__global__ void k_gather_points(const int64_t* __restrict__ order, int64_t n, int64_t nq,
+                                const double* __restrict__ px, const double* __restrict__ py,
+                                const double* __restrict__ pz, const double* __restrict__ w, double* __restrict__ qx,
+                                double* __restrict__ qy, double* __restrict__ qz, double* __restrict__ qw) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nq) return;
-  int64_t i = perm[q];
+  int64_t i = point_index(order, n, q);
   double wt = 0.0;
   if (i >= 0) wt = w[i];
-  else i = perm[q & ~(int64_t)127];  // padding: a weight-0 copy of the tile's first point
+  else i = point_index(order, n, q & ~(int64_t)127);  // padding: a weight-0 copy of the tile's first point
   qx[q] = px[i];
   qy[q] = py[i];
   qz[q] = pz[i];
@@ -71,13 +76,15 @@ __global__ void k_gather_points(const int64_t* __restrict__ perm, int64_t nq, co
 }
 
 // d2[t][a] = min over the tile's points of |r - R_a|^2, rounded down to float
-__global__ void __launch_bounds__(128) k_tile_atom_d2(const double* __restrict__ qx, const double* __restrict__ qy,
-                                                      const double* __restrict__ qz, const double* __restrict__ atoms,
+__global__ void __launch_bounds__(128) k_tile_atom_d2(const int64_t* __restrict__ order, int64_t n,
+                                                      const double* __restrict__ px, const double* __restrict__ py,
+                                                      const double* __restrict__ pz, const double* __restrict__ atoms,
                                                       int natm, float* __restrict__ d2) {
   __shared__ float red[4];
   const int64_t t = blockIdx.x;
-  const int64_t q = t * 128 + threadIdx.x;
-  const double x = qx[q], y = qy[q], z = qz[q];
+  int64_t i = point_index(order, n, t * 128 + threadIdx.x);
+  if (i < 0) i = point_index(order, n, t * 128);
+  const double x = px[i], y = py[i], z = pz[i];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int a = 0; a < natm; ++a) {
     const double dx = x - atoms[3 * a], dy = y - atoms[3 * a + 1], dz = z - atoms[3 * a + 2];
@@ -680,18 +687,26 @@ void screen_listing_radii(const std::vector<DevShell>& shells, const double* exp
   }
 }
 
+constexpr int64_t kSortFrom = int64_t(1) << 17;  // points
+
 // The tiles and the lengths of their lists: Morton-ordered points, per tile the
 // number of listed functions (those whose listing radius exceeds the tile's
 // distance to their atom) and of basis items, and so their places.  The tables that
-// fill_lists reads stay in sp->tab.  from: a plan of the same grid whose points are
-// taken as they lie there, or null: they are put in order here.  one: the plan's own
-// arrays lie behind the tables (an allocation of 2 MB or more takes 0.35 ms whatever its
+// fill_lists reads stay in sp->tab.
+// A build's plan (gradient false) keeps its points in Morton order.  A gradient's
+// takes those of `from`, a plan of the same grid; without one its points go into
+// the gradient's scratch (grad_plan_hosts), in Morton order from kSortFrom on: a
+// grid of few points is that of few atoms, whose functions reach most of its
+// points in any order, and the sort would be most of a first call (dense layout,
+// 6 atoms: 1.0 ms before there was a plan, 2.1 with the sort, 0.95 without;
+// 12 atoms 2.5, 3.4 and 1.7, a repeated call 1.09 with it and 1.18 without).
+// A gradient's own arrays lie behind its tables (an allocation of 2 MB or more takes 0.35 ms whatever its
 // size: the gradient of 6 atoms 1.03 ms before it had a plan, 1.6 with eight allocations
 // of the plan's, 0.92 now).  On the host the lists of a 41-atom grid
 // (2,710 tiles, 170,000 items of 80 bytes, copied from pageable memory) were most
 // of the 30 ms of a context's creation.
 static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
-                       const std::vector<double>& R2, const std::vector<int>& r2off, const ScreenPlan* from, bool one,
+                       const std::vector<double>& R2, const std::vector<int>& r2off, const ScreenPlan* from, bool gradient,
                        cudaStream_t st, std::string& err) {
 #define BL_TRY(call, what)                                                       \
   do {                                                                           \
@@ -707,24 +722,31 @@ static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npt
   sp->ntiles = ntiles;
   T.natm = natm;
   T.nsh = (int)shells.size();
+  const double *px = a.px, *py = a.py, *pz = a.pz;
+  int64_t n = npts;
+  const int64_t* order = nullptr;
   if (from) {
     sp->order_of_points = from->order_of_points;
-    sp->qx = from->qx;
-    sp->qy = from->qy;
-    sp->qz = from->qz;
+    px = sp->qx = from->qx;
+    py = sp->qy = from->qy;
+    pz = sp->qz = from->qz;
     sp->qw = from->qw;
-  } else {  // Morton order of the points, on the device (ties by point index)
+    n = nq;
+  } else if (!gradient || npts >= kSortFrom) {  // Morton order of the points, on the device (ties by point index)
     BL_TRY(sp_alloc(sp, &sp->order_of_points, (size_t)nq), "cudaMalloc");
     BL_TRY(morton_perm_device(a.px, a.py, a.pz, npts, nq, sp->order_of_points, st), "grid reordering");
+    order = sp->order_of_points;
+  }
+  if (!gradient) {
     BL_TRY(sp_alloc(sp, &sp->qx, 4 * (size_t)nq), "grid reordering");
     sp->qy = sp->qx + nq;
     sp->qz = sp->qx + 2 * nq;
     sp->qw = sp->qx + 3 * nq;
-    k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(sp->order_of_points, nq, a.px, a.py, a.pz, a.w, sp->qx,
-                                                                 sp->qy, sp->qz, sp->qw);
+    k_gather_points<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(order, npts, nq, a.px, a.py, a.pz, a.w, sp->qx, sp->qy,
+                                                                 sp->qz, sp->qw);
     BL_TRY(cudaGetLastError(), "grid reordering");
   }
-  // one allocation for the tables (and, with `one`, tso and listed)
+  // one allocation for the tables (and a gradient's tso and listed)
   const size_t nstart = (size_t)ntiles * (kMaxL + 1), n8 = nstart + (size_t)ntiles + 1 + std::max<size_t>(R2.size(), 1);
   const size_t n4 = (size_t)ntiles * natm + (size_t)ntiles * kCnt + shells.size() + (size_t)ntiles;
   BL_TRY(cudaMalloc(&T.base, 8 * n8 + 4 * n4), "tile lists");
@@ -737,7 +759,7 @@ static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npt
   sp->listed = T.r2off + shells.size();
   BL_TRY(cudaMemcpyAsync(T.r2, R2.data(), sizeof(double) * R2.size(), cudaMemcpyHostToDevice, st), "tile lists");
   BL_TRY(cudaMemcpyAsync(T.r2off, r2off.data(), sizeof(int) * r2off.size(), cudaMemcpyHostToDevice, st), "tile lists");
-  k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(sp->qx, sp->qy, sp->qz, a.atoms, natm, T.d2);
+  k_tile_atom_d2<<<(unsigned)ntiles, 128, 0, st>>>(order, n, px, py, pz, a.atoms, natm, T.d2);
   k_plan_count<<<(unsigned)ntiles, 128, 0, st>>>(T.d2, natm, a.shells, T.nsh, T.r2, T.r2off, T.cnt);
   BL_TRY(cudaGetLastError(), "tile lists");
   std::vector<int> cnt((size_t)ntiles * kCnt), listed((size_t)ntiles);
@@ -763,7 +785,7 @@ static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npt
     }
   }
   sp->nslots = tso[(size_t)ntiles];
-  if (!one) {
+  if (!gradient) {
     BL_TRY(sp_alloc(sp, &sp->tso, tso.size()), "tile lists");
     BL_TRY(sp_alloc(sp, &sp->listed, listed.size()), "tile lists");
   }
@@ -1023,14 +1045,15 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
 }
 
 namespace {
-// raw weight (0 for padding) and host atom of the Morton-ordered points
-__global__ void k_gather_hosts(const int64_t* __restrict__ perm, int64_t nq, const double* __restrict__ wraw,
-                               const int* __restrict__ owner, double* __restrict__ qwraw, int* __restrict__ qowner) {
+// raw weight (0 for padding) and host atom of the plan's points
+__global__ void k_gather_hosts(const int64_t* __restrict__ order, int64_t n, int64_t nq,
+                               const double* __restrict__ wraw, const int* __restrict__ owner,
+                               double* __restrict__ qwraw, int* __restrict__ qowner) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nq) return;
-  const int64_t i = perm[q];
+  const int64_t i = point_index(order, n, q);
   qwraw[q] = i >= 0 ? wraw[i] : 0.0;
-  qowner[q] = owner[i >= 0 ? i : perm[q & ~(int64_t)127]];
+  qowner[q] = owner[i >= 0 ? i : point_index(order, n, q & ~(int64_t)127)];
 }
 }  // namespace
 
@@ -1063,12 +1086,23 @@ int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npt
   return PGXC_OK;
 }
 
-void grad_plan_hosts(ScreenPlan* sp, const double* wraw, const int* owner, double* qwraw, int* qowner, cudaStream_t st) {
+void grad_plan_hosts(ScreenPlan* sp, const BuildArgs& a, int64_t npts, const double* wraw, const int* owner,
+                     double* points, double* qwraw, int* qowner, cudaStream_t st) {
   sp->qwraw = qwraw;
   sp->qowner = qowner;
-  if (sp->filled >= 0) return;
   const int64_t nq = sp->ntiles * 128;
-  k_gather_hosts<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(sp->order_of_points, nq, wraw, owner, qwraw, qowner);
+  const unsigned nb = (unsigned)((nq + 255) / 256);
+  if (points) {
+    sp->qx = points;
+    sp->qy = points + nq;
+    sp->qz = points + 2 * nq;
+    sp->qw = points + 3 * nq;
+  }
+  if (sp->filled >= 0) return;
+  if (points)
+    k_gather_points<<<nb, 256, 0, st>>>(sp->order_of_points, npts, nq, a.px, a.py, a.pz, a.w, sp->qx, sp->qy, sp->qz,
+                                        sp->qw);
+  k_gather_hosts<<<nb, 256, 0, st>>>(sp->order_of_points, npts, nq, wraw, owner, qwraw, qowner);
 }
 
 void grad_plan_lists(ScreenPlan* sp, const BuildArgs& a, size_t c, const TileLists& lists, cudaStream_t st) {

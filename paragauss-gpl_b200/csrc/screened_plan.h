@@ -47,8 +47,8 @@ struct ScreenPlan {
   bool keep = false;         // basis values (and INT8 point digits) of all slots stay resident
   bool basis_ready = false;  // ... and a completed build has filled them
   // device, whole grid
-  double *qx = nullptr, *qy = nullptr, *qz = nullptr, *qw = nullptr;  // Morton-ordered points [ntiles*128]
-  int64_t* order_of_points = nullptr;  // their indices in the caller's grid
+  double *qx = nullptr, *qy = nullptr, *qz = nullptr, *qw = nullptr;  // points in the tiles' order [ntiles*128]
+  int64_t* order_of_points = nullptr;  // their indices in the caller's grid (null: as they lie there)
   int64_t* tso = nullptr;   // [ntiles+1] first slot of each tile
   int* slot_fn = nullptr;   // [nslots] function of each slot, -1 for padding
   int* listed = nullptr;    // [ntiles] listed (not padding) slots of each tile
@@ -93,14 +93,16 @@ struct ScreenPlan {
 // A plan of tiles and list lengths alone (no lists, no build buffers), in chunks of
 // at most max_rows slot rows, for the nuclear gradient; R2 with threshold 0, so that
 // unlisted functions and their derivatives are exactly zero on the tile.  from: the
-// context's own plan of the same grid, whose points are taken, or null.  The lists
+// context's own plan of the same grid, whose points are taken, or null (grad_plan_hosts).  The lists
 // themselves are made chunk by chunk (grad_plan_lists): of a whole grid they would grow
 // with tiles x shells (200 atoms, 13,300 tiles: 0.4 GB) and stay until the context goes.
 int grad_plan_create(ScreenPlan** out, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
                      const std::vector<double>& R2, const std::vector<int>& r2off, const ScreenPlan* from,
                      int64_t max_rows, cudaStream_t st, std::string& err);
-// Raw weights and host atoms in the plan's point order into qwraw, qowner ([ntiles * 128]), unless they lie there.
-void grad_plan_hosts(ScreenPlan* sp, const double* wraw, const int* owner, double* qwraw, int* qowner, cudaStream_t st);
+// Raw weights and host atoms in the plan's point order into qwraw, qowner ([ntiles * 128]), and (points not null:
+// the plan has none) the points and weights (4 [ntiles * 128]), unless they lie there.
+void grad_plan_hosts(ScreenPlan* sp, const BuildArgs& a, int64_t npts, const double* wraw, const int* owner,
+                     double* points, double* qwraw, int* qowner, cudaStream_t st);
 // Chunk c's lists into `lists` (s0 and i0 are set here), unless they are what it holds.
 void grad_plan_lists(ScreenPlan* sp, const BuildArgs& a, size_t c, const TileLists& lists, cudaStream_t st);
 // The orbitals in the place of P (orbital_form_pays): nop padded, C [function][nop], occ C

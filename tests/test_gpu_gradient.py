@@ -101,7 +101,8 @@ def test_gradient_of_many_chunks():
     assert float(np.max(np.abs(half - g))) < 1e-11 * scale
 
 
-@pytest.mark.parametrize("layout", [("fp64", 0.0), ("mixed", 1e-10)], ids=["screened", "int8-screened"])
+@pytest.mark.parametrize("layout", [("fp64", -1.0), ("fp64", 0.0), ("mixed", 1e-10)],
+                         ids=["dense", "screened", "int8-screened"])
 def test_first_gradient_allocates_twice(layout):
     """A gradient is asked for once per geometry, so the first call counts: the
     tables of its lists (by tile, small) and its scratch are all that it
@@ -119,6 +120,25 @@ def test_first_gradient_allocates_twice(layout):
     if "cudaLaunchKernel" not in names:
         pytest.skip("the profiler records no runtime calls here")
     assert names.count("cudaMalloc") <= 2 and "cudaFree" not in names
+
+
+@pytest.mark.parametrize("npts", [129, (1 << 17) - 1, 1 << 17])
+def test_dense_gradient_in_either_point_order(npts):
+    """The dense layout's gradient takes the points as they lie up to 2^17 of them
+    and in Morton order from there on; the last tile is ragged.  Against the
+    screened context, whose points are always in Morton order."""
+    case = cases.small_case(functional="PBE", seed=67, natoms=4, nrad=250, nang=194, nocc=5)
+    assert case.npts >= npts
+    pick = np.sort(np.random.default_rng(9).permutation(case.npts)[:npts])
+    case = dataclasses.replace(case, grid_xyz=case.grid_xyz[pick], grid_wraw=case.grid_wraw[pick],
+                               point_atom=case.point_atom[pick])
+    r = []
+    for thr in (-1.0, 0.0):
+        with lib.Context(case, weighted=False, screen_threshold=thr) as ctx:
+            r.append(ctx.xc_gradient())
+    scale = max(1.0, float(np.max(np.abs(r[1][0]))))
+    assert abs(r[0][1] - r[1][1]) < 1e-11 * max(1.0, abs(r[1][1]))
+    np.testing.assert_allclose(r[0][0], r[1][0], rtol=0, atol=1e-11 * scale)
 
 
 def test_gradient_needs_the_raw_grid():
