@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(128) k_basis_l(const DevShell* __restrict__ sh
 // 16-byte words, the same for every lane); consecutive items of a tile reuse the
 // point coordinates.
 // ---------------------------------------------------------------------------
-struct BasisItem {
+struct alignas(16) BasisItem {
   double ax, ay, az;        // words 0-5: atom position
   int64_t slot;             // 6-7: global slot of the shell's first significant function
   unsigned long long mask;  // 8-9: significant radial functions of the shell
@@ -309,13 +309,14 @@ struct BasisItem {
   int seg;                  // 17
   int pad_[2];
 };
-static_assert(sizeof(BasisItem) == 80, "BasisItem is read as five 16-byte words");
+static_assert(sizeof(BasisItem) == 80 && alignof(BasisItem) == 16, "BasisItem is read as five 16-byte words");
 
 __device__ __forceinline__ void load_item(BasisItem& it, const BasisItem* __restrict__ p) {
-  uint4* d = reinterpret_cast<uint4*>(&it);
+  uint4 w[5];
   const uint4* src = reinterpret_cast<const uint4*>(p);
 #pragma unroll
-  for (int i = 0; i < 5; ++i) d[i] = __ldg(src + i);
+  for (int i = 0; i < 5; ++i) w[i] = __ldg(src + i);
+  memcpy(&it, w, sizeof(it));
 }
 
 // GT: the element type of the gradient planes (double; float in the INT8
