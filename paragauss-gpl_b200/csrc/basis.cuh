@@ -309,15 +309,7 @@ struct alignas(16) BasisItem {
   int seg;                  // 17
   int pad_[2];
 };
-static_assert(sizeof(BasisItem) == 80 && alignof(BasisItem) == 16, "BasisItem is read as five 16-byte words");
-
-__device__ __forceinline__ void load_item(BasisItem& it, const BasisItem* __restrict__ p) {
-  uint4 w[5];
-  const uint4* src = reinterpret_cast<const uint4*>(p);
-#pragma unroll
-  for (int i = 0; i < 5; ++i) w[i] = __ldg(src + i);
-  memcpy(&it, w, sizeof(it));
-}
+static_assert(sizeof(BasisItem) == 80 && alignof(BasisItem) == 16, "a record is copied as five 16-byte words");
 
 // GT: the element type of the gradient planes (double; float in the INT8
 // build, whose potential and density gradient tolerate 24-bit gradients).
@@ -391,8 +383,7 @@ __device__ __forceinline__ void basis_items(const BasisItem* __restrict__ items,
   };
   points(__ldg(&items[i0].tile));
   for (int64_t i = i0; i < i1; ++i) {
-    BasisItem it;
-    load_item(it, items + i);
+    const BasisItem it = items[i];
     // the next item's tile: also what brings its record into L1 a whole item ahead
     const int ntile = __ldg(&items[min(i + 1, i1 - 1)].tile);
     const int nsel = it.nsig, nexp = it.nexp;

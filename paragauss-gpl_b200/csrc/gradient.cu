@@ -127,8 +127,7 @@ __global__ void __launch_bounds__(128) k_hess_items(const BasisItem* __restrict_
   const int64_t i0 = (int64_t)blockIdx.x * per, i1 = min(nitems, i0 + per);
   constexpr int ci[6] = {0, 0, 0, 1, 1, 2}, di[6] = {0, 1, 2, 1, 2, 2};
   for (int64_t i = i0; i < i1; ++i) {
-    BasisItem it;
-    load_item(it, items + i);
+    const BasisItem it = items[i];
     const int64_t q = (int64_t)it.tile * 128 + threadIdx.x;
     const double x = __ldg(io.qx + q) - it.ax, y = __ldg(io.qy + q) - it.ay, z = __ldg(io.qz + q) - it.az;
     double Y[16], dY[3][16], H[6][16];

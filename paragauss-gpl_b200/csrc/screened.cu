@@ -700,10 +700,10 @@ constexpr int64_t kSortFrom = int64_t(1) << 17;  // points
 // points in any order, and the sort would be most of a first call (dense layout,
 // 6 atoms: 1.0 ms before there was a plan, 2.1 with the sort, 0.95 without;
 // 12 atoms 2.5, 3.4 and 1.7, a repeated call 1.09 with it and 1.18 without).
-// A gradient's own arrays lie behind its tables (an allocation of 2 MB or more takes 0.35 ms whatever its
-// size: the gradient of 6 atoms 1.03 ms before it had a plan, 1.6 with eight allocations
-// of the plan's, 0.92 now).  On the host the lists of a 41-atom grid
-// (2,710 tiles, 170,000 items of 80 bytes, copied from pageable memory) were most
+// A gradient's own arrays lie behind its tables (an allocation of 2 MB or more takes
+// 0.35 ms whatever its size: the gradient of 6 atoms 1.03 ms before it had a plan, 1.6
+// with eight allocations of the plan's, 0.92 now).  On the host the lists of a 41-atom
+// grid (2,710 tiles, 170,000 items of 80 bytes, copied from pageable memory) were most
 // of the 30 ms of a context's creation.
 static int count_lists(ScreenPlan* sp, const BuildArgs& a, int natm, int64_t npts, const std::vector<DevShell>& shells,
                        const std::vector<double>& R2, const std::vector<int>& r2off, const ScreenPlan* from, bool gradient,
