@@ -359,7 +359,8 @@ int pgxc_build_density(pgxc_ctx* ctx, const double* P, int32_t nbas, int32_t isp
  * device (for callers that keep C on the GPU).  d_exc_nel receives
  * {E_xc, N_el} (overwritten, not accumulated); d_ham_xc_arr is overwritten
  * with the packed matrix of this build.  Runs on the context's stream and
- * synchronises before returning.
+ * synchronises before returning.  After PGXC_ETIMEOUT both outputs hold what
+ * they held before the call.
  */
 int pgxc_build_device(pgxc_ctx* ctx, const double* d_C, const double* d_occ,
                       int32_t nbas, int32_t nocc, int32_t ispin,

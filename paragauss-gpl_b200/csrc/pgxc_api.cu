@@ -1573,6 +1573,16 @@ int pgxc_build_sym(pgxc_ctx* c, const double* const* C, const double* const* occ
   return PGXC_OK;
 }
 
+// Not part of the ABI (no declaration in pgxc.h): leaves a screened INT8 context
+// as a build whose device wait ran out does, so that a test can see what the next
+// call reports and leaves alone without making a wait run out.
+int pgxc_test_raise_wait_error(pgxc_ctx* c) {
+  if (!c || !c->screen) return set_err(c, PGXC_ENOTSUP, "a screened INT8 context");
+  CUDA_TRY(c, cudaSetDevice(c->device));
+  if (int st = screen_raise_error(c->screen, c->stream)) return set_err(c, st, "no INT8 error word");
+  return PGXC_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Batched builds: the device builds of many screened contexts captured as the
 // parallel branches of one CUDA graph.

@@ -588,9 +588,12 @@ constexpr int svpot_smem(int max_n) {
 }  // namespace
 
 // ham[spin + ispin*(j(j+1)/2 + k)] = H(k, j), k <= j; GGA: H(k, j) + H(j, k)
-// (exc_nel not null: and {E_xc, N_el} from acc)
+// (exc_nel not null: and {E_xc, N_el} from acc).  failed not null and not 0: a
+// wait of the build ran out, and the caller's outputs keep what they hold.
 __global__ void k_spack(const double* __restrict__ V, int64_t nbas, bool sym2, int ispin, int spin,
-                        double* __restrict__ ham, const double* __restrict__ acc, double* __restrict__ exc_nel) {
+                        double* __restrict__ ham, const double* __restrict__ acc, double* __restrict__ exc_nel,
+                        const int* __restrict__ failed) {
+  if (failed && *failed) return;
   const int64_t len = nbas * (nbas + 1) / 2;
   if (exc_nel && blockIdx.x == 0 && threadIdx.x < 2) exc_nel[threadIdx.x] = acc[2 * threadIdx.x];
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < len;
@@ -1450,8 +1453,10 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
   if (potential) {
     const int64_t len = sp->nbas * (sp->nbas + 1) / 2;
     const unsigned nbk = (unsigned)std::min<int64_t>((len + 255) / 256, 148 * 8);
+    const int* failed = sp->mixed ? screen_mixed_error(sp->mixed) : nullptr;
     for (int s = 0; s < ispin; ++s) {
-      k_spack<<<nbk, 256, 0, st>>>(sp->V + s * nb2, sp->nbas, gga, ispin, s, ham, a.acc, s == 0 ? a.exc_nel : nullptr);
+      k_spack<<<nbk, 256, 0, st>>>(sp->V + s * nb2, sp->nbas, gga, ispin, s, ham, a.acc, s == 0 ? a.exc_nel : nullptr,
+                                   failed);
       ++T.launches;
     }
   }
@@ -1524,6 +1529,10 @@ int screen_enable_tau(ScreenPlan* sp, std::string& err) {
     return PGXC_ENOMEM;
   }
   return PGXC_OK;
+}
+
+int screen_raise_error(ScreenPlan* sp, cudaStream_t st) {
+  return sp->mixed ? screen_mixed_raise_error(sp->mixed, st) : PGXC_ENOTSUP;
 }
 
 int screen_error_flag(ScreenPlan* sp, cudaStream_t st, int* flag) {

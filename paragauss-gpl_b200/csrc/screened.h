@@ -82,6 +82,8 @@ struct ScreenExtra {
 int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_t st, double* ham, ScreenTimes* t,
                std::string& err, const ScreenExtra* extra = nullptr);
 int screen_error_flag(ScreenPlan* sp, cudaStream_t st, int* flag);
+// INT8 plans: the error state of a wait that ran out, set from the host (for tests)
+int screen_raise_error(ScreenPlan* sp, cudaStream_t st);
 // After a timed screen_run: waits for the stream, adds the phase times (the
 // time from `start` to the first chunk counts as density) to *t and reads the
 // error flag.

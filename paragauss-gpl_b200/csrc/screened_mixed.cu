@@ -53,6 +53,13 @@ constexpr int kDigBytesPerSlot = 640;      // 128 points x 5 slices
 
 }  // namespace
 
+// Set when a bounded wait ran out: a device word, which the packing reads before
+// it writes the caller's outputs, and a mapped host word, which the host reads.
+struct WaitError {
+  int flag;
+  int* host;
+};
+
 struct ScreenMixed {
   int64_t nbas = 0, ldc = 0;
   bool gga = false;
@@ -70,7 +77,7 @@ struct ScreenMixed {
   double* zs = nullptr;              // [chunk_slots] 2^e of each slot's Z digits
   double* fs = nullptr;              // [chunk_slots] 2^(e - 40) of each slot's phi digits (the combine shift folded in)
   double* ps = nullptr;              // [chunk_slots] 2^e_P of each slot's function (0 for padding)
-  int* err = nullptr;                // device view of h_err
+  WaitError* err = nullptr;
   volatile int* h_err = nullptr;     // mapped host word: written by a kernel only when a wait runs out
   int nsm = 148;
   const int *order = nullptr, *start = nullptr;  // tile lists of the persistent CTAs (null: round robin)
@@ -88,6 +95,11 @@ cudaError_t sm_alloc(ScreenMixed* m, T** p, size_t n) {
     *p = (T*)q;
   }
   return e;
+}
+
+__device__ __forceinline__ void wait_ran_out(WaitError* e) {
+  atomicExch(&e->flag, 1);
+  *(volatile int*)e->host = 1;
 }
 
 // The tiles of one persistent CTA: every gridDim.x-th of the chunk's, or
@@ -341,7 +353,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
                  const int8_t* __restrict__ tB, const int64_t* __restrict__ b_off, const double* __restrict__ ps,
                  const double* __restrict__ phi, const GT* __restrict__ gx, const GT* __restrict__ gy,
                  const GT* __restrict__ gz, double* __restrict__ rho, double* __restrict__ grx,
-                 double* __restrict__ gry, double* __restrict__ grz, int* err, const int* __restrict__ order,
+                 double* __restrict__ gry, double* __restrict__ grz, WaitError* err, const int* __restrict__ order,
                  const int* __restrict__ start) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   DensSmem& S = *reinterpret_cast<DensSmem*>(smem_raw);
@@ -407,7 +419,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
             }
         }
       }
-      if (!ok) atomicExch(err, 1);
+      if (!ok) wait_ran_out(err);
     }
   } else if (warp == 8) {
     if (lane == 0) {  // MMA issuer
@@ -436,7 +448,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
           tc::mma_commit(&S.acc_full[b]);
         }
       }
-      if (!ok) atomicExch(err, 1);
+      if (!ok) wait_ran_out(err);
     }
   } else if (warp == 9) {
     if (lane == 0) {  // operand producer: per K step the phi digits (A) and the gathered P digits (B)
@@ -460,7 +472,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
             tc::bulk_g2s(S.b[s], bsrc + (int64_t)(j * nK + k) * kOpB, kOpB, &S.full[s]);
           }
       }
-      if (!ok) atomicExch(err, 1);
+      if (!ok) wait_ran_out(err);
     }
   } else if (warp >= 15) {
     // idle: the CTA holds the whole SM
@@ -546,7 +558,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
         tc::mbar_arrive(&S.p_empty[q]);
       }
     }
-    if (!ok) atomicExch(err, 1);
+    if (!ok) wait_ran_out(err);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -599,7 +611,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
                                                             const double* __restrict__ By,
                                                             const double* __restrict__ Bz, int8_t* __restrict__ tZ,
                                                             int8_t* __restrict__ tF, double* __restrict__ zs,
-                                                            double* __restrict__ fs, int* err,
+                                                            double* __restrict__ fs, WaitError* err,
                                                             const int* __restrict__ order,
                                                             const int* __restrict__ start) {
   using L = ZLayout<GGA, GT>;
@@ -661,7 +673,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
           }
         }
       }
-      if (!ok) atomicExch(err, 1);
+      if (!ok) wait_ran_out(err);
       // the copies still in flight land before the CTA exits
       for (int j = max(0, it - L::kRing); j < it; ++j) tc::mbar_wait(&full[j % L::kRing], (j / L::kRing) & 1);
       for (int j = max(0, tt - 2); j < tt; ++j) tc::mbar_wait(&ab_full[j & 1], (j >> 1) & 1);
@@ -752,7 +764,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
         if (lane == 0) tc::mbar_arrive(&empty[r]);
       }
     }
-    if (!ok) atomicExch(err, 1);
+    if (!ok) wait_ran_out(err);
   }
 }
 
@@ -793,7 +805,7 @@ template <bool GGA, bool SET>
 __global__ void __launch_bounds__(kVThreads, 1)
     k_sm_vpot(const int64_t* __restrict__ tso, const int* __restrict__ slot_fn, int64_t t0, int64_t nt, int64_t s0,
               const int8_t* __restrict__ tF, const int8_t* __restrict__ tZ, const double* __restrict__ fs,
-              const double* __restrict__ zs, double* __restrict__ V, int64_t ldv, int* err,
+              const double* __restrict__ zs, double* __restrict__ V, int64_t ldv, WaitError* err,
               const int* __restrict__ tile_mol, const SetMolDev* __restrict__ mols, const int* __restrict__ order,
               const int* __restrict__ start) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -854,7 +866,7 @@ __global__ void __launch_bounds__(kVThreads, 1)
             }
         }
       }
-      if (!ok) atomicExch(err, 1);
+      if (!ok) wait_ran_out(err);
     }
   } else if (warp == kVEpiWarps) {
     if (lane == 0) {  // MMA issuer
@@ -892,7 +904,7 @@ __global__ void __launch_bounds__(kVThreads, 1)
           tc::mma_commit(&S.a_empty[qa]);
         }
       }
-      if (!ok) atomicExch(err, 1);
+      if (!ok) wait_ran_out(err);
     }
   } else if (warp > kVEpiWarps + 1) {
     // idle: the CTA holds the whole SM
@@ -943,7 +955,7 @@ __global__ void __launch_bounds__(kVThreads, 1)
         }
       }
     }
-    if (!ok) atomicExch(err, 1);
+    if (!ok) wait_ran_out(err);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -984,9 +996,12 @@ int screen_mixed_create(ScreenMixed** out, const ScreenMixedInput& in, std::stri
   if (e == cudaSuccess) e = sm_alloc(m, &m->fs, (size_t)in.chunk_slots);
   if (e == cudaSuccess) e = sm_alloc(m, &m->ps, (size_t)in.chunk_slots);
   if (e == cudaSuccess) e = cudaHostAlloc((void**)&m->h_err, sizeof(int), cudaHostAllocMapped);
+  if (e == cudaSuccess) e = sm_alloc(m, &m->err, 1);
   if (e == cudaSuccess) {
     *m->h_err = 0;
-    e = cudaHostGetDevicePointer((void**)&m->err, (void*)m->h_err, 0);
+    WaitError w{};
+    e = cudaHostGetDevicePointer((void**)&w.host, (void*)m->h_err, 0);
+    if (e == cudaSuccess) e = cudaMemcpy(m->err, &w, sizeof(w), cudaMemcpyHostToDevice);
   }
   // the slack rows after a chunk's last slot are read (never used) by whole-block copies
   const size_t slack = (size_t)std::min<int64_t>(in.chunk_slots, 128) * kDigBytesPerSlot;
@@ -1193,8 +1208,18 @@ void screen_mixed_p8(ScreenMixed* m, int spin, const unsigned long long** P8, co
 int screen_mixed_error_flag(ScreenMixed* m, cudaStream_t st, int* flag) {
   if (cudaStreamSynchronize(st) != cudaSuccess) return PGXC_ECUDA;
   *flag = *m->h_err;
-  *m->h_err = 0;
+  if (*flag) {
+    *m->h_err = 0;
+    if (cudaMemsetAsync(&m->err->flag, 0, sizeof(int), st) != cudaSuccess) return PGXC_ECUDA;
+  }
   return PGXC_OK;
+}
+
+const int* screen_mixed_error(const ScreenMixed* m) { return &m->err->flag; }
+
+int screen_mixed_raise_error(ScreenMixed* m, cudaStream_t st) {
+  *m->h_err = 1;
+  return cudaMemsetAsync(&m->err->flag, 1, sizeof(int), st) == cudaSuccess ? PGXC_OK : PGXC_ECUDA;
 }
 
 }  // namespace pgxc

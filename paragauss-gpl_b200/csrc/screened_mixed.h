@@ -91,5 +91,9 @@ int screen_mixed_potential(ScreenMixed* m, const int64_t* tso, const int* slot_f
 void screen_mixed_p8(ScreenMixed* m, int spin, const unsigned long long** P8, const int** e_P);
 // copies the device error flag (a bounded wait ran out) to *flag and clears it
 int screen_mixed_error_flag(ScreenMixed* m, cudaStream_t st, int* flag);
+// device word: not 0 from a wait that ran out until the host has read the flag
+const int* screen_mixed_error(const ScreenMixed* m);
+// leaves both words as a wait that ran out does (for tests of what follows it)
+int screen_mixed_raise_error(ScreenMixed* m, cudaStream_t st);
 
 }  // namespace pgxc

@@ -141,3 +141,26 @@ def test_outgrown_orbital_buffers_are_released():
     with lib.Context(c, screen_threshold=0.0) as ctx:
         ref = ctx.build(C=C[:, :, 0].T, occ=np.full(c.nbas, 2.0))
     assert abs(last[1] - ref[1]) < 1e-10 and float(np.max(np.abs(last[0] - ref[0]))) < 1e-10
+
+
+# a device wait that runs out (its error state set from the host, no wait is made to run out): the
+# call reports it, the caller's outputs stay as they were, and the next call is whole again
+def test_outputs_after_a_wait_that_ran_out():
+    import torch
+    from pgxc import abi
+    c = _case(4, 2, "PBE")
+    C, occ = torch.from_numpy(c.c_fortran()).cuda(), torch.from_numpy(c.occ_fortran()).cuda()
+    ham = torch.full((c.xc_length,), 7.0, dtype=torch.float64, device="cuda")
+    sums = torch.full((2,), 7.0, dtype=torch.float64, device="cuda")
+    with lib.Context(c, precision="mixed", screen_threshold=1e-10) as ctx:
+        ref = ctx.build()
+        for call in (lambda: ctx.build_device(C.data_ptr(), occ.data_ptr(), ham.data_ptr(), sums.data_ptr()), ctx.build):
+            assert lib.lib().pgxc_test_raise_wait_error(ctx.h) == 0
+            with pytest.raises(lib.PgxcError) as e:
+                call()
+            assert e.value.status == abi.PGXC_ETIMEOUT
+        torch.cuda.synchronize()
+        assert bool((ham == 7.0).all()) and bool((sums == 7.0).all())
+        ctx.build_device(C.data_ptr(), occ.data_ptr(), ham.data_ptr(), sums.data_ptr())
+        assert abs(float(sums[0]) - ref[1]) < 1e-12
+        assert float(np.max(np.abs(ham.cpu().numpy() - ref[0]))) < 1e-12
