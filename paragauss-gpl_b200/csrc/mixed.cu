@@ -233,6 +233,7 @@ struct OzSmem {
   uint64_t empty[kStages];
   uint64_t acc_full;
   uint64_t acc_empty;
+  uint64_t drain;       // the products in flight when a wait ran out
   uint32_t tslot;
 };
 static_assert(sizeof(OzSmem) + 1024 <= tc::kWholeSmSmem, "OzSmem");
@@ -297,6 +298,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
     }
     tc::mbar_init(&S.acc_full, 1);
     tc::mbar_init(&S.acc_empty, 256);
+    tc::mbar_init(&S.drain, 1);
     tc::mbar_fence_init();
   }
   tc::fence_before_sync();
@@ -308,7 +310,8 @@ __global__ void __launch_bounds__(kDensThreads, 1)
   double r_acc = 0.0, g_acc[3] = {0.0, 0.0, 0.0};
   if (warp == 8) {
     if (lane == 0) {  // producer
-      for (int it = 0; it < total && ok; ++it) {
+      int it = 0;
+      for (; it < total; ++it) {
         const int s = it % kStages, nb = it / nks, kb = it % nks;
         if (it >= kStages && !tc::mbar_wait(&S.empty[s], ((it / kStages) - 1) & 1)) ok = false;
         if (!ok) break;
@@ -317,6 +320,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
         tc::bulk_g2s(S.b[s], tB + ((int64_t)nb * nks + kb) * kOpB, kOpB, &S.full[s]);
       }
       if (!ok) atomicExch(err, 1);
+      tc::copies_land(S.full, kStages, it);
     }
   } else if (warp == 9) {
     if (lane == 0) {  // MMA issuer
@@ -335,6 +339,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
         atomicExch(err, 1);
         // release the epilogue warps of the remaining tiles (their data is discarded)
         for (int nb = it / nks; nb < nnb; ++nb) tc::mma_commit(&S.acc_full);
+        tc::products_end(&S.drain);
       }
     }
   } else if (warp >= 10) {
@@ -478,6 +483,7 @@ __global__ void __launch_bounds__(kVThreads, 1)
       tc::mbar_init(&S.empty[s], 1);
     }
     tc::mbar_init(&S.acc_full, 1);
+    tc::mbar_init(&S.drain, 1);
     tc::mbar_fence_init();
   }
   tc::fence_before_sync();
@@ -487,7 +493,8 @@ __global__ void __launch_bounds__(kVThreads, 1)
   bool ok = true;
   if (warp == 4) {
     if (lane == 0) {
-      for (int it = 0; it < total && ok; ++it) {
+      int it = 0;
+      for (; it < total; ++it) {
         const int s = it % kStages, kb = kb0 + it;
         if (it >= kStages && !tc::mbar_wait(&S.empty[s], ((it / kStages) - 1) & 1)) ok = false;
         if (!ok) break;
@@ -496,6 +503,7 @@ __global__ void __launch_bounds__(kVThreads, 1)
         tc::bulk_g2s(S.b[s], tP + ((int64_t)tj * nks + kb) * kOpB, kOpB, &S.full[s]);
       }
       if (!ok) atomicExch(err, 1);
+      tc::copies_land(S.full, kStages, it);
     }
   } else if (warp == 5) {
     if (lane == 0) {
@@ -510,7 +518,10 @@ __global__ void __launch_bounds__(kVThreads, 1)
         tc::mma_commit(&S.empty[s]);
       }
       tc::mma_commit(&S.acc_full);  // also on failure: lets the epilogue wind down
-      if (!ok) atomicExch(err, 1);
+      if (!ok) {
+        atomicExch(err, 1);
+        tc::products_end(&S.drain);
+      }
     }
   } else if (warp >= 6) {
     // idle: the CTA holds the whole SM

@@ -308,6 +308,7 @@ struct DensSmem {
   double part[2][4][128];  // rho, grad rho of the first two column thirds, for the last one to add
   uint64_t p_full[4];      // per TMEM lane quarter
   uint64_t p_empty[4];
+  uint64_t drain;          // the products in flight when a wait ran out
   uint32_t tslot;
 };
 static_assert(sizeof(DensSmem) <= tc::kWholeSmSmem, "one CTA's shared memory");
@@ -376,6 +377,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
       tc::mbar_init(&S.p_full[q], 64);  // the quarter's warps of the first two thirds
       tc::mbar_init(&S.p_empty[q], 32);
     }
+    tc::mbar_init(&S.drain, 1);
     tc::mbar_fence_init();
   }
   tc::fence_before_sync();
@@ -420,6 +422,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
         }
       }
       if (!ok) wait_ran_out(err);
+      tc::copies_land(S.e_full, kERing, e);
     }
   } else if (warp == 8) {
     if (lane == 0) {  // MMA issuer
@@ -448,7 +451,10 @@ __global__ void __launch_bounds__(kDensThreads, 1)
           tc::mma_commit(&S.acc_full[b]);
         }
       }
-      if (!ok) wait_ran_out(err);
+      if (!ok) {
+        wait_ran_out(err);
+        tc::products_end(&S.drain);
+      }
     }
   } else if (warp == 9) {
     if (lane == 0) {  // operand producer: per K step the phi digits (A) and the gathered P digits (B)
@@ -473,6 +479,7 @@ __global__ void __launch_bounds__(kDensThreads, 1)
           }
       }
       if (!ok) wait_ran_out(err);
+      tc::copies_land(S.full, kDStages, it);
     }
   } else if (warp >= 15) {
     // idle: the CTA holds the whole SM
@@ -674,9 +681,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_sm_zquant(const int64_t* __res
         }
       }
       if (!ok) wait_ran_out(err);
-      // the copies still in flight land before the CTA exits
-      for (int j = max(0, it - L::kRing); j < it; ++j) tc::mbar_wait(&full[j % L::kRing], (j / L::kRing) & 1);
-      for (int j = max(0, tt - 2); j < tt; ++j) tc::mbar_wait(&ab_full[j & 1], (j >> 1) & 1);
+      tc::copies_land(full, L::kRing, it);
+      tc::copies_land(ab_full, 2, tt);
     }
   } else if (warp < kZWarps) {
     const int p0 = lane * 4;
@@ -791,6 +797,7 @@ struct VSmem {
   uint64_t empty[kVStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+  uint64_t drain;
   uint32_t tslot;
 };
 // warps 0-15 epilogue (four per TMEM lane quarter, 12 columns of each 48-slot
@@ -825,6 +832,7 @@ __global__ void __launch_bounds__(kVThreads, 1)
       tc::mbar_init(&S.acc_full[b], 1);
       tc::mbar_init(&S.acc_empty[b], 32 * kVEpiWarps);
     }
+    tc::mbar_init(&S.drain, 1);
     tc::mbar_fence_init();
   }
   tc::fence_before_sync();
@@ -867,6 +875,8 @@ __global__ void __launch_bounds__(kVThreads, 1)
         }
       }
       if (!ok) wait_ran_out(err);
+      tc::copies_land(S.a_full, 2, ia);
+      tc::copies_land(S.full, kVStages, it);
     }
   } else if (warp == kVEpiWarps) {
     if (lane == 0) {  // MMA issuer
@@ -904,7 +914,10 @@ __global__ void __launch_bounds__(kVThreads, 1)
           tc::mma_commit(&S.a_empty[qa]);
         }
       }
-      if (!ok) wait_ran_out(err);
+      if (!ok) {
+        wait_ran_out(err);
+        tc::products_end(&S.drain);
+      }
     }
   } else if (warp > kVEpiWarps + 1) {
     // idle: the CTA holds the whole SM

@@ -186,5 +186,17 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* mbar, uint32_t parity) 
   return ok;
 }
 
+// Before a CTA ends, also one whose waits ran out, its asynchronous work has ended:
+// the copies into its shared memory (uses 0 .. n - 1 of a ring of barriers, the last
+// of each slot), and the products that read it and write TMEM (drain: a barrier of
+// one arrival, used by the issuer alone).  Bounded like every wait.
+__device__ __forceinline__ void copies_land(uint64_t* full, int ring, int n) {
+  for (int j = n > ring ? n - ring : 0; j < n; ++j) mbar_wait(&full[j % ring], (j / ring) & 1);
+}
+__device__ __forceinline__ void products_end(uint64_t* drain) {
+  mma_commit(drain);
+  mbar_wait(drain, 0);
+}
+
 }  // namespace tc
 }  // namespace pgxc
