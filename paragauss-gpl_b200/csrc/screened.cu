@@ -313,6 +313,8 @@ struct SPlanes {
 constexpr double kOrbitalMargin = 1.15;
 // elements of psi held at once, 1 GB (60 atoms: 256 MB 6.7 ms, 1 GB 6.45: fewer half-empty last waves)
 constexpr int64_t kPsiMost = int64_t(1) << 27;
+// elements up to which psi's place is made with the context, 128 MB
+constexpr int64_t kPsiReserved = int64_t(1) << 24;
 // The tile's slot -> function list (slot_fn of the kernels below begins at the
 // chunk's first slot s0) in shared memory, -1 from its slots to a
 // whole block past them: every index the kernels form is inside it, guarded or
@@ -814,6 +816,7 @@ void screen_destroy(ScreenPlan* sp) {
   if (sp->mixed) screen_mixed_destroy(sp->mixed);
   for (void* p : sp->allocs) cudaFree(p);
   if (sp->tab.base) cudaFree(sp->tab.base);
+  if (sp->psi_own) cudaFree(sp->psi_own);
   for (auto& c : sp->cev)
     for (auto& e : c)
       if (e) cudaEventDestroy(e);
@@ -975,35 +978,46 @@ int screen_create(ScreenPlan** out, const ScreenInput& in, const BuildArgs& a, c
   const size_t rows = (size_t)(sp->chunk_slots + kSlack) * 128;
   // basis arrays: one chunk's rows, or every slot of the grid when they stay resident
   const size_t brows = sp->keep ? (size_t)(sp->nslots + kSlack) * 128 : rows;
-  // (padding slots are zeroed by every evaluation; the rows after the last slot are read by whole-block copies)
-  auto plane = [&](auto** p) -> cudaError_t {
-    cudaError_t e = sp_alloc(sp, p, brows);
-    if (e == cudaSuccess) e = cudaMemsetAsync(*p + (brows - kSlack * 128), 0, sizeof(**p) * kSlack * 128, st);
-    return e;
-  };
-  // psi of the orbital form lies behind phi: up to the longest that the form is taken for, so that no build
-  // allocates (a 12-atom context's first build 0.98 ms with an allocation of its own, 0.61 without)
+  // psi of the orbital form lies behind phi where it is small, for the longest that the form is taken for, so that
+  // the first build does not allocate (12 atoms, first build 0.98 ms with an allocation of its own, 0.61 without).
+  // A large one is made by the first build that takes the form (screen_orbital_form): the caller's P, symmetric
+  // builds, energies and batches never do, and would hold up to 1 GB for nothing.
+  int64_t psi = 0;
   if (in.gga && !mixed && sp->nlisted > 0) {
     const int64_t most = (int64_t)(sp->sum_n2 / (2.0 * kOrbitalMargin * (double)sp->nlisted));
-    const int64_t cap = std::min(kPsiMost, sp->chunk_tiles * most * 128);
-    if (8.0 * (double)cap < 0.1 * (double)freeb && sp_alloc(sp, &sp->phi, brows + (size_t)cap) == cudaSuccess) {
-      sp->psi = sp->phi + brows;
-      sp->psi_cap = cap;
-    } else {
-      cudaGetLastError();  // no room: the builds take P
-      sp->phi = nullptr;
-    }
+    psi = sp->chunk_tiles * most * 128;
+    if (psi > kPsiReserved || 8.0 * (double)psi > 0.1 * (double)freeb) psi = 0;
   }
-  if (sp->phi) SP_TRY(cudaMemsetAsync(sp->phi + (brows - kSlack * 128), 0, sizeof(double) * kSlack * 128, st), "memset");
-  else SP_TRY(plane(&sp->phi), "cudaMalloc (phi)");
-  if (in.gga && sp->gf32) {
-    SP_TRY(plane(&sp->fx), "cudaMalloc (grad phi)");
-    SP_TRY(plane(&sp->fy), "cudaMalloc (grad phi)");
-    SP_TRY(plane(&sp->fz), "cudaMalloc (grad phi)");
-  } else if (in.gga) {
-    SP_TRY(plane(&sp->gx), "cudaMalloc (grad phi)");
-    SP_TRY(plane(&sp->gy), "cudaMalloc (grad phi)");
-    SP_TRY(plane(&sp->gz), "cudaMalloc (grad phi)");
+  // one allocation for phi, psi and grad phi (an allocation takes 0.35 ms, whatever its size; 41 atoms, create,
+  // weights, first build and destroy: 22.2 ms with four and psi behind phi, 22.0 with one and psi in the build)
+  {
+    const size_t gb = in.gga ? (sp->gf32 ? sizeof(float) : sizeof(double)) : 0;
+    auto planes = [&] { return sp_alloc(sp, (char**)&sp->phi, sizeof(double) * (brows + (size_t)psi) + 3 * gb * brows); };
+    cudaError_t e = planes();
+    if (e != cudaSuccess && psi) {
+      cudaGetLastError();
+      psi = 0;
+      e = planes();
+    }
+    SP_TRY(e, "cudaMalloc (phi, grad phi)");
+    if (psi) {
+      sp->psi = sp->phi + brows;
+      sp->psi_cap = psi;
+    }
+    // (padding slots are zeroed by every evaluation; the rows after the last slot are read by whole-block copies)
+    auto slack = [&](auto* p) { return cudaMemsetAsync(p + (brows - kSlack * 128), 0, sizeof(*p) * kSlack * 128, st); };
+    auto place = [&](auto* g, auto** gx, auto** gy, auto** gz) -> cudaError_t {
+      *gx = g;
+      *gy = g + brows;
+      *gz = g + 2 * brows;
+      cudaError_t r = slack(*gx);
+      if (r == cudaSuccess) r = slack(*gy);
+      return r == cudaSuccess ? slack(*gz) : r;
+    };
+    double* g = sp->phi + brows + psi;
+    SP_TRY(slack(sp->phi), "memset");
+    if (in.gga && sp->gf32) SP_TRY(place((float*)g, &sp->fx, &sp->fy, &sp->fz), "memset");
+    else if (in.gga) SP_TRY(place(g, &sp->gx, &sp->gy, &sp->gz), "memset");
   }
   const int64_t cp = sp->chunk_tiles * 128;
   SP_TRY(sp_alloc(sp, &sp->pt, 8 * (size_t)in.ispin * cp), "cudaMalloc");
@@ -1172,9 +1186,25 @@ bool orbital_form_pays(const ScreenPlan* sp, int64_t nop) {
 int64_t orbital_psi_tiles(const ScreenPlan* sp, int64_t nop) {
   return std::min(sp->chunk_tiles, std::max<int64_t>(1, kPsiMost / (nop * 128)));
 }
-bool screen_orbital_form(const ScreenPlan* sp, int nop) {
+bool screen_orbital_form(ScreenPlan* sp, int nop) {
   if (sp->mixed || !orbital_form_pays(sp, nop)) return false;
-  return !sp->gga || (int64_t)nop * 128 <= sp->psi_cap;
+  if (!sp->gga) return true;
+  const int64_t need = std::min(kPsiMost, sp->chunk_tiles * nop * 128);
+  if (need <= sp->psi_cap) return true;
+  // a buffer of its own (the builds before this one have ended); without room the builds take P from here on
+  if (sp->psi_refused) return false;
+  if (sp->psi_own) cudaFree(sp->psi_own);
+  sp->psi_own = sp->psi = nullptr;
+  sp->psi_cap = 0;
+  if (cudaMalloc(&sp->psi_own, sizeof(double) * (size_t)need) != cudaSuccess) {
+    cudaGetLastError();
+    sp->psi_own = nullptr;
+    sp->psi_refused = true;
+    return false;
+  }
+  sp->psi = sp->psi_own;
+  sp->psi_cap = need;
+  return true;
 }
 
 // rho, grad rho and (tau not null) the tau sums of one spin by its orbitals

@@ -90,8 +90,9 @@ int screen_raise_error(ScreenPlan* sp, cudaStream_t st);
 int screen_finish(ScreenPlan* sp, cudaStream_t st, cudaEvent_t start, ScreenTimes* t, std::string& err);
 // The plan's potential accumulator (both spins), which a caller may clear itself (BuildArgs::cleared).
 double* screen_potential(ScreenPlan* sp, int64_t* n);
-// whether the FP64 density takes the orbitals (nop of them, padded) instead of P
-bool screen_orbital_form(const ScreenPlan* sp, int nop);
+// whether the FP64 density of the next build takes the orbitals (nop of them, padded) instead of P; makes the room
+// for psi that it needs
+bool screen_orbital_form(ScreenPlan* sp, int nop);
 // The kinetic-energy density for meta-GGA energies on the density of a plan
 // that does not form it in its builds: its buffer, allocated once.  Needs FP64
 // gradient planes (a GGA plan of the FP64 build); PGXC_ENOTSUP otherwise.

@@ -69,8 +69,10 @@ struct ScreenPlan {
   bool mgga = false;
   int functional = 0;        // PGXC_XC_* (the meta-GGA step selects its functional by id)
   double* tq = nullptr;      // meta-GGA: 4 point arrays per spin (2 tau_x, 2 tau_y, 2 tau_z, C)
-  double* psi = nullptr;     // [tile][padded orbital][128] of the orbital form (FP64 GGA), psi_cap elements behind phi
+  double* psi = nullptr;     // [tile][padded orbital][128] of the orbital form (FP64 GGA), psi_cap elements
   int64_t psi_cap = 0;
+  double* psi_own = nullptr;  // psi's buffer where it does not lie behind phi
+  bool psi_refused = false;   // there was no room for it
   double* partial = nullptr;
   double* V = nullptr;       // [ispin][nbas][nbas]
   unsigned long long* pmax = nullptr;  // [chunk_tiles*128] largest |phi| per point (INT8 path)

@@ -164,3 +164,26 @@ def test_outputs_after_a_wait_that_ran_out():
         ctx.build_device(C.data_ptr(), occ.data_ptr(), ham.data_ptr(), sums.data_ptr())
         assert abs(float(sums[0]) - ref[1]) < 1e-12
         assert float(np.max(np.abs(ham.cpu().numpy() - ref[0]))) < 1e-12
+
+
+# psi of a larger grid (here 2,500 tiles x 48 orbitals, 120 MB) is held once a build by orbitals has been made, not
+# by a context that is given density matrices; a build with more orbitals than there is room for makes more
+def test_psi_is_made_by_the_builds_that_use_it():
+    import torch
+    c = _case(12, 2, "PBE", nrad=160, nang=194, nocc=40)
+    P = c.density_matrix()
+    torch.cuda.init()
+    with lib.Context(c, screen_threshold=0.0) as ctx:
+        ref = ctx.build_density(P)
+        free = torch.cuda.mem_get_info()[0]
+        c.nocc = 16
+        ctx.build(C=c.C[:, :16, 0].T, occ=c.occ[:16, 0])
+        few = free - torch.cuda.mem_get_info()[0]
+        c.nocc = 40
+        got = ctx.build()
+        held = free - torch.cuda.mem_get_info()[0]
+        tiles = ctx.screen_stats()["ntiles"]
+    for orbitals, bytes_held in ((16, few), (48, held)):
+        assert abs(bytes_held - orbitals * tiles * 1024) < 12 << 20  # (and the padded orbitals)
+    assert abs(got[1] - ref[1]) < 1e-10 and abs(got[2] - ref[2]) < 1e-10
+    assert float(np.max(np.abs(got[0] - ref[0]))) < 1e-10
