@@ -9,7 +9,7 @@
 // Per build (screen_run), per chunk of tiles:
 //   k_basis_items     phi, grad phi of listed functions only     [K1]
 //   k_tile_init       (first) clears: the padding slots at the end of each tile's
-//                     list, and what the INT8 stages add or max into
+//                     list, and what the INT8 stages max into
 //   k_sdensity        X = phi_t P[S_t, S_t] on DMMA, P gathered by cp.async,
 //                     fused rho, grad rho (or by the orbitals)     [K3]
 //   k_functional      (kernels_fp64.cu)                            [K2]
@@ -196,21 +196,13 @@ __global__ void __launch_bounds__(128) k_plan_fill(const float* __restrict__ d2,
 // ---------------------------------------------------------------------------
 // Clears of one chunk before its basis values (grid = chunk tiles): the padding
 // slots of each tile (after its listed functions: tso[t] + listed[t] ..
-// tso[t+1]; phi not null), the points' largest |phi| (pmax not null) and the
-// density columns the INT8 contraction adds into (rho not null: ncol columns of
-// ld per spin, spins 8 ld apart).
+// tso[t+1]) and the points' largest |phi| (pmax not null).
 template <bool GGA, typename GT = double>
 __global__ void __launch_bounds__(128) k_tile_init(const int64_t* __restrict__ tso, const int* __restrict__ listed,
                                                   int64_t t0, int64_t s0, double* __restrict__ phi,
                                                   GT* __restrict__ gx, GT* __restrict__ gy,
-                                                  GT* __restrict__ gz, unsigned long long* __restrict__ pmax,
-                                                  double* __restrict__ rho, int64_t ld, int nspin) {
-  const int64_t p = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (pmax) pmax[p] = 0;
-  if (rho)
-    for (int s = 0; s < nspin; ++s)
-      for (int c = 0; c < (GGA ? 4 : 1); ++c) rho[(8 * s + c) * ld + p] = 0.0;
-  if (!phi) return;
+                                                  GT* __restrict__ gz, unsigned long long* __restrict__ pmax) {
+  if (pmax) pmax[(int64_t)blockIdx.x * 128 + threadIdx.x] = 0;
   const int64_t t = t0 + blockIdx.x;
   const int64_t r0 = tso[t] - s0 + listed[t], r1 = tso[t + 1] - s0;
   for (int64_t e = r0 * 128 + threadIdx.x; e < r1 * 128; e += 128) {
@@ -1319,24 +1311,14 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
     }
     if (timed) SR_TRY(cudaEventRecord(ev[0], st));
     // K1
-    {
-      double* ip = eval_basis ? phi : nullptr;
-      double* ir = sp->mixed ? sp->pt : nullptr;
-      unsigned long long* im = eval_basis ? sp->pmax : nullptr;
-      const unsigned g = (unsigned)nt;
-      if (!ip && !ir) {
-      } else if (gga && gf) {
-        k_tile_init<true, float><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, ip, fxc, fyc, fzc, im, ir, cp, ispin);
-      } else if (gga) {
-        k_tile_init<true><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, ip, gxc, gyc, gzc, im, ir, cp, ispin);
-      } else {
-        k_tile_init<false><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, ip, gxc, gyc, gzc, im, ir, cp, ispin);
-      }
-      ++T.launches;
-    }
     if (!eval_basis) {
       if (sp->mixed) T.launches += screen_mixed_gather(sp->mixed, sp->tso, sp->slot_fn, t0, nt, s0, 0, st);
     } else {
+      const unsigned g = (unsigned)nt;
+      if (gga && gf) k_tile_init<true, float><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, phi, fxc, fyc, fzc, sp->pmax);
+      else if (gga) k_tile_init<true><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, phi, gxc, gyc, gzc, sp->pmax);
+      else k_tile_init<false><<<g, 128, 0, st>>>(sp->tso, sp->listed, t0, s0, phi, gxc, gyc, gzc, sp->pmax);
+      ++T.launches;
       const BasisItem* items[kMaxL + 1];
       int64_t ni[kMaxL + 1];
       for (int l = 0; l <= kMaxL; ++l) {
@@ -1958,11 +1940,9 @@ int screen_set_run(ScreenSet* S, cudaStream_t st, std::string& err) {
     float* gyc = gga ? S->gy : nullptr;
     float* gzc = gga ? S->gz : nullptr;
     if (gga)
-      k_tile_init<true, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc, S->pmax,
-                                                             S->pt, cp, 1);
+      k_tile_init<true, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc, S->pmax);
     else
-      k_tile_init<false, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc, S->pmax,
-                                                              S->pt, cp, 1);
+      k_tile_init<false, float><<<(unsigned)nt, 128, 0, st>>>(S->tso, S->listed, t0, s0, S->phi, gxc, gyc, gzc, S->pmax);
     ++launches;
     const BasisItem* items[kMaxL + 1];
     int64_t ni[kMaxL + 1];

@@ -65,7 +65,7 @@ void screen_mixed_set_order(ScreenMixed* m, const int* order, const int* start);
 // with tile_mol, tile t's digits come from mols[tile_mol[t]] instead
 int screen_mixed_gather(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_t t0, int64_t nt, int64_t s0,
                         int spin, cudaStream_t st, const int* tile_mol = nullptr, const SetMolDev* mols = nullptr);
-// (adds into rho, grx, gry, grz: cleared by the caller)
+// (rho, grx, gry, grz of every point of the tiles are written)
 int screen_mixed_density(ScreenMixed* m, const int64_t* tso, const int* slot_fn, int64_t t0, int64_t nt, int64_t s0,
                          const double* phi, const double* gx, const double* gy, const double* gz, double* rho,
                          double* grx, double* gry, double* grz, int64_t so, int64_t to, cudaStream_t st);

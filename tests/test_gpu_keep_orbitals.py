@@ -83,3 +83,20 @@ def test_kept_basis_in_a_batch():
     finally:
         for c in ctxs:
             c.close()
+
+
+@BUILDS
+def test_kept_basis_leaves_out_its_clears(precision, thr, tol):
+    """The clears before the basis values go with their evaluation: no kernel of
+    a later build has them left to do (the density stores every point)."""
+    from torch.profiler import ProfilerActivity, profile
+    c = cases.small_case(functional="PBE", seed=43, natoms=5)
+    O.weight_case(c)
+    with lib.Context(c, precision=precision, screen_threshold=thr, keep_orbitals=True) as ctx:
+        ctx.build()
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as prof:
+            ctx.build()
+        names = [e.name for e in prof.events()]
+    if not any("k_spack" in n for n in names):
+        pytest.skip("the profiler records no kernels here")
+    assert not any("k_tile_init" in n or "k_basis" in n for n in names)
