@@ -71,9 +71,10 @@ struct BuildArgs {
   double* vpart = nullptr;    // [nsplit][ntiles][64*64]
 };
 
-void launch_basis_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool grad, cudaStream_t st);
-// basis values (and gradients) of every shell at points [p0, p0+ld) of (px,py,pz), FP64, [f][ld] layout
-void launch_basis(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t p0,
+int launch_basis_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool grad, cudaStream_t st);
+// basis values (and gradients) of every shell at points [p0, p0+ld) of (px,py,pz), FP64, [f][ld] layout (both return
+// their launches, one for each l of the basis)
+int launch_basis(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t p0,
                   int64_t nvalid, int64_t ld, double* phi, double* gx, double* gy, double* gz, cudaStream_t st);
 void launch_basis_points_f64(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t n,
                              int64_t ld, double* phi, double* gx, double* gy, double* gz, cudaStream_t st);

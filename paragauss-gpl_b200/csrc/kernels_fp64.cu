@@ -31,10 +31,10 @@ namespace pgxc {
 // K1: basis functions, one launch per angular momentum (k_basis_l, basis.cuh)
 // ---------------------------------------------------------------------------
 template <int L>
-static void launch_basis_one_l(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t p0,
+static int launch_basis_one_l(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t p0,
                                int64_t nvalid, int64_t ld, double* phi, double* gx, double* gy, double* gz,
                                cudaStream_t st) {
-  if (a.nshl[L] == 0) return;
+  if (a.nshl[L] == 0) return 0;
   dim3 grid((unsigned)((ld + 127) / 128), (unsigned)a.nshl[L]);
   if (gx)
     k_basis_l<L, true><<<grid, 128, 0, st>>>(a.shells, a.shl[L], a.atoms, a.exps, a.norms, a.contr, a.rng, a.sa, px,
@@ -42,18 +42,19 @@ static void launch_basis_one_l(const BuildArgs& a, const double* px, const doubl
   else
     k_basis_l<L, false><<<grid, 128, 0, st>>>(a.shells, a.shl[L], a.atoms, a.exps, a.norms, a.contr, a.rng, a.sa,
                                                       px, py, pz, p0, nvalid, ld, phi, nullptr, nullptr, nullptr);
+  return 1;
 }
 
-void launch_basis(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t p0,
+int launch_basis(const BuildArgs& a, const double* px, const double* py, const double* pz, int64_t p0,
                   int64_t nvalid, int64_t ld, double* phi, double* gx, double* gy, double* gz, cudaStream_t st) {
-  launch_basis_one_l<0>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st);
-  launch_basis_one_l<1>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st);
-  launch_basis_one_l<2>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st);
-  launch_basis_one_l<3>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st);
+  return launch_basis_one_l<0>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st) +
+         launch_basis_one_l<1>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st) +
+         launch_basis_one_l<2>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st) +
+         launch_basis_one_l<3>(a, px, py, pz, p0, nvalid, ld, phi, gx, gy, gz, st);
 }
 
-void launch_basis_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool grad, cudaStream_t st) {
-  launch_basis(a, a.px, a.py, a.pz, p0, nvalid, a.ldp, a.phi, grad ? a.gx : nullptr, a.gy, a.gz, st);
+int launch_basis_f64(const BuildArgs& a, int64_t p0, int64_t nvalid, bool grad, cudaStream_t st) {
+  return launch_basis(a, a.px, a.py, a.pz, p0, nvalid, a.ldp, a.phi, grad ? a.gx : nullptr, a.gy, a.gz, st);
 }
 
 // basis on arbitrary points (pgxc_orbital_calculate): same kernels, caller arrays

@@ -686,10 +686,10 @@ int mixed_prepare_P(MixedState* m, const double* P, int64_t ldc, cudaStream_t st
 }
 
 int mixed_basis(MixedState* m, const BuildArgs& a, int64_t p0, int64_t nvalid, bool gga, cudaStream_t st) {
-  launch_basis(a, a.px, a.py, a.pz, p0, nvalid, m->ldp, m->phi, gga ? m->gx : nullptr, m->gy, m->gz, st);
+  const int n = launch_basis(a, a.px, a.py, a.pz, p0, nvalid, m->ldp, m->phi, gga ? m->gx : nullptr, m->gy, m->gz, st);
   const int nksf = (int)(m->ldk / kKStep);
   k_oz_quant_pts<<<(unsigned)(m->ldp / 128), 128, 0, st>>>(m->phi, m->ldp, m->nbas, nksf, m->e_pt, m->tA1);
-  return 5;
+  return n + 1;
 }
 
 int mixed_density(MixedState* m, const BuildArgs& a, bool gga, cudaStream_t st) {

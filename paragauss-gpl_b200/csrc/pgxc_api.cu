@@ -769,7 +769,7 @@ static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given, cons
     const int64_t nv = std::min<int64_t>(c->chunk, c->npts - p0);
     CUDA_TRY(c, cudaEventRecord(c->ev[3], s));
     if (c->mixed) launches += mixed_basis(c->mixed, a, p0, nv, gga, s);
-    else { launch_basis_f64(a, p0, nv, gga, s); launches += 4; }
+    else launches += launch_basis_f64(a, p0, nv, gga, s);
     CUDA_TRY(c, cudaEventRecord(c->ev[4], s));
     CUDA_TRY(c, cudaEventRecord(c->kev[0], s));
     if (c->mixed) launches += mixed_density(c->mixed, a, gga, s);
@@ -777,7 +777,7 @@ static int run_build(pgxc_ctx* c, int nocc, pgxc_timings* tm, bool p_given, cons
     CUDA_TRY(c, cudaEventRecord(c->kev[1], s));
     CUDA_TRY(c, cudaEventRecord(c->ev[5], s));
     launch_functional_f64(a, p0, nv, gga, s);
-    launches += 2;
+    launches += 1;
     CUDA_TRY(c, cudaEventRecord(c->ev[6], s));
     if (c->mixed) {
       launches += mixed_potential(c->mixed, a, gga, s, c->kev[2], c->kev[3]);
@@ -1568,7 +1568,7 @@ int pgxc_build_sym(pgxc_ctx* c, const double* const* C, const double* const* occ
     tm->h2d_ms = h2d;
     tm->d2h_ms = d2h;
     tm->total_ms = tot;
-    tm->kernel_launches += ispin + 1;
+    tm->kernel_launches += ispin + 1 + (P->p2_pairs > 0 && P->p2_quads > 0);
   }
   return PGXC_OK;
 }

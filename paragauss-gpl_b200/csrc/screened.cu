@@ -1456,7 +1456,7 @@ int screen_run(ScreenPlan* sp, const BuildArgs& a, const double* Pb, cudaStream_
         launch_functional2_f64(extra->xc[i], sp->qw, b[0].rho, b[1].rho, cp, t0 * 128, npt, extra->gga[i] != 0,
                                sp->partial, extra->acc + 4 * i, st);
       }
-      T.launches += 2;
+      T.launches += extra->fid && PGXC_XC_IS_MGGA(extra->fid[i]) ? 2 : 1;
     }
     SR_TRY(cudaGetLastError());
     // the packing counts with the last chunk's potential
