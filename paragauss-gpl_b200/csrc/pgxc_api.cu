@@ -79,6 +79,7 @@ struct pgxc_ctx {
   std::vector<double> grad_r2;     // listing radii of the exact (threshold 0) lists of the gradient
   std::vector<int> grad_r2off;
   ScreenPlan* gplan = nullptr;  // tiles and lists of pgxc_xc_gradient, made by the first call
+  int64_t psi_limit = 0;           // pgxc_test_limit_psi
   void* grad_scr = nullptr;     // scratch of pgxc_xc_gradient, kept across calls (grows only)
   size_t grad_scr_bytes = 0;
   int eacc_cap = 0;
@@ -1023,6 +1024,7 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     if (st) return set_err(c, st, "gradient plan: " + e);
   }
   ScreenPlan* gp = c->gplan;
+  gp->psi_tiles_most = c->psi_limit;
   const int64_t nq = gp->ntiles * 128, ld = gp->chunk_tiles * 128;
   const int64_t plane = (gp->chunk_slots + kSlack) * 128;
   // The weight term needs only each point's w_raw f and runs after the chunk loop in launches of ldw
@@ -1570,6 +1572,16 @@ int pgxc_build_sym(pgxc_ctx* c, const double* const* C, const double* const* occ
     tm->total_ms = tot;
     tm->kernel_launches += ispin + 1 + (P->p2_pairs > 0 && P->p2_quads > 0);
   }
+  return PGXC_OK;
+}
+
+// Not part of the ABI (no declaration in pgxc.h): psi of at most `tiles` tiles at
+// once in the builds and gradients of a screened context that follow (0: no
+// limit), so that a test sees on a small grid what a large one does in parts.
+int pgxc_test_limit_psi(pgxc_ctx* c, int64_t tiles) {
+  if (!c || !c->screen || tiles < 0) return set_err(c, PGXC_EINVAL, "a screened context and tiles >= 0");
+  c->psi_limit = tiles;
+  c->screen->psi_tiles_most = tiles;
   return PGXC_OK;
 }
 

@@ -1176,12 +1176,13 @@ bool orbital_form_pays(const ScreenPlan* sp, int64_t nop) {
   return kOrbitalMargin * 2.0 * (double)nop * (double)sp->nlisted < sp->sum_n2;
 }
 int64_t orbital_psi_tiles(const ScreenPlan* sp, int64_t nop) {
-  return std::min(sp->chunk_tiles, std::max<int64_t>(1, kPsiMost / (nop * 128)));
+  const int64_t most = sp->psi_tiles_most > 0 ? std::min(sp->chunk_tiles, sp->psi_tiles_most) : sp->chunk_tiles;
+  return std::min(most, std::max<int64_t>(1, kPsiMost / (nop * 128)));
 }
 bool screen_orbital_form(ScreenPlan* sp, int nop) {
   if (sp->mixed || !orbital_form_pays(sp, nop)) return false;
   if (!sp->gga) return true;
-  const int64_t need = std::min(kPsiMost, sp->chunk_tiles * nop * 128);
+  const int64_t need = orbital_psi_tiles(sp, nop) * nop * 128;
   if (need <= sp->psi_cap) return true;
   // a buffer of its own (the builds before this one have ended); without room the builds take P from here on
   if (sp->psi_refused) return false;
@@ -1216,7 +1217,7 @@ static int orbital_density(const ScreenPlan* sp, const BuildArgs& a, int s, int6
         nullptr, nullptr, nop, nocc, a.orb_occ[s]);
     return 1;
   }
-  const int64_t most = sp->psi_cap / ((int64_t)nop * 128), parts = (nt + most - 1) / most;
+  const int64_t most = orbital_psi_tiles(sp, nop), parts = (nt + most - 1) / most;
   const int64_t step = (nt + parts - 1) / parts;
   for (int64_t u = 0; u < nt; u += step) {
     const dim3 grid((unsigned)std::min(step, nt - u), 2);

@@ -73,6 +73,7 @@ struct ScreenPlan {
   int64_t psi_cap = 0;
   double* psi_own = nullptr;  // psi's buffer where it does not lie behind phi
   bool psi_refused = false;   // there was no room for it
+  int64_t psi_tiles_most = 0; // tiles whose psi is held at once, at most (0: as many as kPsiMost holds)
   double* partial = nullptr;
   double* V = nullptr;       // [ispin][nbas][nbas]
   unsigned long long* pmax = nullptr;  // [chunk_tiles*128] largest |phi| per point (INT8 path)

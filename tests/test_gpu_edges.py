@@ -1,6 +1,8 @@
 """Builds at the sizes where the tile kernels' remainders change: basis sizes
 off the 32-, 48-, 64- and 128-slot blocks, single and ragged tiles, both
 precisions, against the CPU oracle (FP64 1e-10, INT8 1e-7)."""
+import ctypes as ct
+
 import numpy as np
 import pytest
 
@@ -187,3 +189,50 @@ def test_psi_is_made_by_the_builds_that_use_it():
         assert abs(bytes_held - orbitals * tiles * 1024) < 12 << 20  # (and the padded orbitals)
     assert abs(got[1] - ref[1]) < 1e-10 and abs(got[2] - ref[2]) < 1e-10
     assert float(np.max(np.abs(got[0] - ref[0]))) < 1e-10
+
+
+# psi held for a few tiles at a time, as grids of more than 2^20 tiles x orbitals have it: parts of one and two
+# tiles, and a ragged last part, against the whole and against the same density by P
+@pytest.mark.parametrize("functional,ispin", [("PBE", 1), ("PBE", 2), ("TPSS", 1), ("TPSS", 2)])
+@pytest.mark.parametrize("nocc", [5, 20])
+def test_psi_in_parts(nocc, functional, ispin):
+    c = _case(9, 2, functional, ispin, nocc=nocc)
+    with lib.Context(c, screen_threshold=0.0) as ctx:
+        tiles = ctx.screen_stats()["ntiles"]
+        assert tiles > 5
+        whole, by_p = ctx.build(), ctx.build_density(c.density_matrix())
+        for most in (1, 2, tiles - 1):
+            assert lib.lib().pgxc_test_limit_psi(ctx.h, ct.c_int64(most)) == 0
+            got = ctx.build()
+            for ref, tol in ((whole, 1e-13), (by_p, 1e-11)):
+                assert abs(got[1] - ref[1]) < tol * max(1.0, abs(ref[1])) and abs(got[2] - ref[2]) < tol * abs(ref[2])
+                assert float(np.max(np.abs(got[0] - ref[0]))) < tol * max(1.0, float(np.max(np.abs(ref[0]))))
+
+
+@pytest.mark.parametrize("functional,ispin", [("VWN", 1), ("PBE", 1), ("PBE", 2), ("TPSS", 1), ("TPSS", 2)])
+def test_gradient_psi_in_parts(functional, ispin):
+    c = cases.small_case(functional, seed=49, natoms=9, nrad=9, nang=26, nocc=20, ispin=ispin)
+    with lib.Context(c, weighted=False, screen_threshold=0.0) as ctx:
+        tiles = ctx.screen_stats()["ntiles"]
+        whole = ctx.xc_gradient()
+        scale = max(1.0, float(np.max(np.abs(whole[0]))))
+        for most in (1, 2, tiles - 1):
+            assert lib.lib().pgxc_test_limit_psi(ctx.h, ct.c_int64(most)) == 0
+            got = ctx.xc_gradient()
+            assert abs(got[1] - whole[1]) < 1e-13 * max(1.0, abs(whole[1]))
+            assert float(np.max(np.abs(got[0] - whole[0]))) < 1e-12 * scale
+
+
+# the gradient on either side of the line between orbitals and P: 5 atoms, 60 functions, so that 16 padded orbitals
+# lie below it and 32 and 48 above
+@pytest.mark.parametrize("nocc", [4, 30, 40])
+@pytest.mark.parametrize("functional,ispin", [("VWN", 1), ("PBE", 1), ("PBE", 2), ("TPSS", 1), ("TPSS", 2)])
+def test_gradient_by_orbitals_and_by_p(functional, ispin, nocc):
+    c = cases.small_case(functional, seed=50, natoms=5, nrad=12, nang=50, nocc=nocc, ispin=ispin)
+    assert c.nbas < 2.3 * 32 and c.nbas > 2.3 * 16
+    ref, re = O.xc_gradient(c)
+    with lib.Context(c, weighted=False, screen_threshold=0.0) as ctx:
+        g, e = ctx.xc_gradient()
+    scale = max(1.0, float(np.max(np.abs(ref))))
+    assert abs(e - re) < 1e-10 * max(1.0, abs(re))
+    np.testing.assert_allclose(g, ref, rtol=0, atol=1e-10 * scale)
