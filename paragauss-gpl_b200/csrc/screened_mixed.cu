@@ -9,10 +9,9 @@
 //   k_sm_quant_P     word), one scale per row nu                       (B of X)
 //   k_sm_gather_B    per tile, the digits of P[S_t, S_t] in the MMA layout
 //   k_sm_density     X = phi_t P[S_t, S_t], 128 points x 48 slots per MMA;
-//                    A by bulk copy, B gathered from P8 by four producer
-//                    warps, two TMEM accumulator sets (MMA of slot block j+1
-//                    overlaps the epilogue of block j); fused FP64 epilogue
-//                    rho += X phi, grad rho += 2 X grad phi
+//                    A and B by bulk copy, two TMEM accumulator sets (MMA of
+//                    slot block j+1 overlaps the epilogue of block j); fused FP64
+//                    epilogue rho = sum X phi, grad rho = 2 sum X grad phi
 //   k_sm_zquant      Z = A phi (+ B . grad phi) in FP64 and the digits of phi
 //                    (slice-interleaved per 8 slots: one copy per A block) and
 //                    of Z (slices one after another), one scale per
@@ -23,7 +22,8 @@
 //                    into the full matrix with atomics that run along rows
 //
 // Every mbarrier wait is bounded (tc::kWaitLimit); a wait that runs out sets
-// the device error flag and the kernel winds down.
+// the error state (WaitError) and the kernel winds down, its copies and products
+// in flight first.
 #include <algorithm>
 #include <cstdint>
 #include <functional>
