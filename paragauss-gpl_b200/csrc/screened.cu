@@ -1184,15 +1184,16 @@ bool screen_orbital_form(ScreenPlan* sp, int nop) {
   if (!sp->gga) return true;
   const int64_t need = orbital_psi_tiles(sp, nop) * nop * 128;
   if (need <= sp->psi_cap) return true;
-  // a buffer of its own (the builds before this one have ended); without room the builds take P from here on
-  if (sp->psi_refused) return false;
+  // a buffer of its own (the builds before this one have ended); without room the builds take P, as long as they
+  // would need as much
+  if (need >= sp->psi_refused) return false;
   if (sp->psi_own) cudaFree(sp->psi_own);
   sp->psi_own = sp->psi = nullptr;
   sp->psi_cap = 0;
   if (cudaMalloc(&sp->psi_own, sizeof(double) * (size_t)need) != cudaSuccess) {
     cudaGetLastError();
     sp->psi_own = nullptr;
-    sp->psi_refused = true;
+    sp->psi_refused = need;
     return false;
   }
   sp->psi = sp->psi_own;

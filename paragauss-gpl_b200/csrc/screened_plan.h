@@ -72,7 +72,7 @@ struct ScreenPlan {
   double* psi = nullptr;     // [tile][padded orbital][128] of the orbital form (FP64 GGA), psi_cap elements
   int64_t psi_cap = 0;
   double* psi_own = nullptr;  // psi's buffer where it does not lie behind phi
-  bool psi_refused = false;   // there was no room for it
+  int64_t psi_refused = INT64_MAX;  // elements that there was no room for
   int64_t psi_tiles_most = 0; // tiles whose psi is held at once, at most (0: as many as kPsiMost holds)
   double* partial = nullptr;
   double* V = nullptr;       // [ispin][nbas][nbas]

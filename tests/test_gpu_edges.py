@@ -191,6 +191,31 @@ def test_psi_is_made_by_the_builds_that_use_it():
     assert float(np.max(np.abs(got[0] - ref[0]))) < 1e-10
 
 
+# no room for psi (the rest of the device memory is taken): the build takes P; one that needs less is made by
+# orbitals again once there is room
+def test_builds_without_room_for_psi():
+    import torch
+    c = _case(12, 2, "PBE", nrad=160, nang=194, nocc=40)
+    P = c.density_matrix()
+    torch.cuda.init()
+    with lib.Context(c, screen_threshold=0.0) as ctx:
+        ref = ctx.build_density(P)
+        tiles = ctx.screen_stats()["ntiles"]
+        assert 48 * tiles * 1024 > 112 << 20
+        torch.cuda.empty_cache()
+        taken = torch.empty(torch.cuda.mem_get_info()[0] - (72 << 20), dtype=torch.uint8, device="cuda")
+        got = ctx.build()
+        del taken
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        c.nocc = 16
+        ctx.build(C=c.C[:, :16, 0].T, occ=c.occ[:16, 0])
+        held = free - torch.cuda.mem_get_info()[0]
+    assert abs(got[1] - ref[1]) < 1e-10 and abs(got[2] - ref[2]) < 1e-10
+    assert float(np.max(np.abs(got[0] - ref[0]))) < 1e-10
+    assert abs(held - 16 * tiles * 1024) < 12 << 20
+
+
 # psi held for a few tiles at a time, as grids of more than 2^20 tiles x orbitals have it: parts of one and two
 # tiles, and a ragged last part, against the whole and against the same density by P
 @pytest.mark.parametrize("functional,ispin", [("PBE", 1), ("PBE", 2), ("TPSS", 1), ("TPSS", 2)])
