@@ -82,6 +82,7 @@ struct pgxc_ctx {
   int64_t psi_limit = 0;           // pgxc_test_limit_psi
   void* grad_scr = nullptr;     // scratch of pgxc_xc_gradient, kept across calls (grows only)
   size_t grad_scr_bytes = 0;
+  size_t grad_psi_refused = SIZE_MAX;  // bytes of psi that it had no room for
   int eacc_cap = 0;
   int* d_owner = nullptr;       // host atom of each point (raw-weight grids)
   double* d_wraw = nullptr;     // the raw weights of those grids
@@ -1047,7 +1048,9 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
   for (int l = 0; l <= kMaxL; ++l) sizes[kLists + 1 + l] = sizeof(BasisItem) * (size_t)gp->chunk_items[l];
   bool orbitals = orbital_form_pays(gp, kpad);
   const int64_t psi_tiles = orbital_psi_tiles(gp, kpad);
-  if (orbitals) sizes[kPsiAt] = sizeof(double) * (size_t)(psi_tiles * kpad * 128);
+  const size_t psi = sizeof(double) * (size_t)(psi_tiles * kpad * 128);
+  orbitals = orbitals && psi < c->grad_psi_refused;
+  if (orbitals) sizes[kPsiAt] = psi;
   size_t offs[kPsiAt + 1], total = 0;
   for (int i = 0; i <= kPsiAt; ++i) {
     offs[i] = total;
@@ -1062,6 +1065,7 @@ static int gradient_core(pgxc_ctx* c, int32_t nbas, int32_t ispin, int64_t kpad,
     if (e != cudaSuccess && orbitals) {  // no room for psi: P instead
       cudaGetLastError();
       orbitals = false;
+      c->grad_psi_refused = psi;
       total = offs[kPsiAt];
       e = cudaMalloc(&c->grad_scr, total);
     }

@@ -122,6 +122,35 @@ def test_first_gradient_allocates_twice(layout):
     assert names.count("cudaMalloc") <= 2 and "cudaFree" not in names
 
 
+def test_gradient_without_room_for_psi():
+    """No room for psi beside the rows: the gradient takes P, and a second one does not ask again."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    case = cases.small_case(functional="PBE", seed=68, natoms=12, nrad=160, nang=194, nocc=40)
+    torch.cuda.init()
+    with lib.Context(case, weighted=False, screen_threshold=0.0) as ctx:
+        tiles = ctx.screen_stats()["ntiles"]
+        assert 48 * tiles * 1024 > 112 << 20
+        many, case.nocc = case.nocc, 1
+        ctx.xc_gradient(C=case.C[:, :1, 0].T, occ=case.occ[:1, 0])  # the scratch, with psi of 16 orbitals
+        case.nocc = many
+        torch.cuda.empty_cache()
+        taken = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+        got = ctx.xc_gradient()
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as prof:
+            again = ctx.xc_gradient()
+        names = [e.name for e in prof.events()]
+        del taken
+        torch.cuda.empty_cache()
+    with lib.Context(case, weighted=False, screen_threshold=0.0) as ctx:
+        ref = ctx.xc_gradient()
+    scale = max(1.0, float(np.max(np.abs(ref[0]))))
+    for g, e in (got, again):
+        assert abs(e - ref[1]) < 1e-11 * max(1.0, abs(ref[1]))
+        np.testing.assert_allclose(g, ref[0], rtol=0, atol=1e-11 * scale)
+    assert "cudaMalloc" not in names and "cudaFree" not in names
+
+
 @pytest.mark.parametrize("npts", [129, (1 << 17) - 1, 1 << 17])
 def test_dense_gradient_in_either_point_order(npts):
     """The dense layout's gradient takes the points as they lie up to 2^17 of them
